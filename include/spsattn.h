@@ -280,6 +280,19 @@ int spsattn_decode_step(const void* q, int nq, void* out, int out_dtype,
                         void* workspace, size_t workspace_bytes,
                         int* device_status, void* stream);
 
+/* The same with the tickets in a buffer of their own: `workspace` holds records only
+ * (spsattn_decode_workspace_bytes) and may be anything, `tickets` at least (S*H + S) * 4 bytes that
+ * must be zero before the first call and are left zero.  One zeroed ticket buffer then serves
+ * calls of different sizes, whose tickets would otherwise sit at different places of a workspace. */
+int spsattn_decode_step_tickets(const void* q, int nq, void* out, int out_dtype,
+                                const spsattn_segment* segs, int n_segments,
+                                const spsattn_extra* extras, int n_extras,
+                                const spsattn_kv_append* append_or_null,
+                                int S, int H, int D, int dtype, float sm_scale,
+                                void* workspace, size_t workspace_bytes,
+                                int* tickets, size_t ticket_bytes,
+                                int* device_status, void* stream);
+
 /* Test hook: which kernel spsattn_decode_step uses.  0 = automatic (the tensor-core kernel when
  * head_dim is 64 or 128, no segment is packed through seq_offset and there are at least 444
  * (sequence, head, long segment) triples, else the CUDA-core kernel),

@@ -23,7 +23,8 @@ EXPORTS = (
     "spsattn_prefill_workspace_bytes", "spsattn_prefill_fwd", "spsattn_prefill_fwd_strided",
     "spsattn_decode_workspace_bytes", "spsattn_decode_fwd", "spsattn_decode_fwd_noalloc",
     "spsattn_kv_update", "spsattn_fill_decode_caches", "spsattn_rope_cast", "spsattn_debug_visibility",
-    "spsattn_decode_step_workspace_bytes", "spsattn_decode_step", "spsattn_qkv_rope_cast",
+    "spsattn_decode_step_workspace_bytes", "spsattn_decode_step", "spsattn_decode_step_tickets",
+    "spsattn_qkv_rope_cast",
     "spsattn_add_rmsnorm", "spsattn_swiglu", "spsattn_debug_decode_path", "spsattn_debug_prefill_path", "spsattn_debug_wait_expiry",
     "spsattn_prefill_bwd_workspace_bytes", "spsattn_prefill_bwd", "spsattn_prefill_bwd_strided",
 )
@@ -122,6 +123,9 @@ def load() -> C.CDLL:
     lib.spsattn_decode_step.restype = i32
     lib.spsattn_decode_step.argtypes = [vp, i32, vp, i32, C.POINTER(Segment), i32, C.POINTER(Extra), i32,
                                         C.POINTER(KvAppend), i32, i32, i32, i32, f32, vp, sz, vp, vp]
+    lib.spsattn_decode_step_tickets.restype = i32
+    lib.spsattn_decode_step_tickets.argtypes = [vp, i32, vp, i32, C.POINTER(Segment), i32, C.POINTER(Extra), i32,
+                                                C.POINTER(KvAppend), i32, i32, i32, i32, f32, vp, sz, vp, sz, vp, vp]
     lib.spsattn_qkv_rope_cast.restype = i32
     lib.spsattn_qkv_rope_cast.argtypes = [vp, i32, i64, i64, i64, vp, i64, C.POINTER(RopeGroup), i32, i32,
                                           i32, i32, i32, i32, vp]
@@ -139,6 +143,24 @@ def load() -> C.CDLL:
     lib.spsattn_debug_visibility.argtypes = [vp, vp, i32, i64, i64, i32, i32, i32, i32, i32, i32, vp, sz, vp]
     _lib = lib
     return lib
+
+
+_native = None
+
+
+def native():
+    """The extension module that holds the host path of the public functions (csrc/native.cpp)."""
+    global _native
+    if _native is None:
+        load()                                   # the library that it calls, with its own message when missing
+        try:
+            from . import _native as ext
+        except ImportError as e:
+            raise SpsAttnError(f"sps_b200/_native.so does not load: {e} (python -m sps_b200.build)") from e
+        from .decode import PackedKVSegment
+        ext.setup(SpsAttnError, PackedKVSegment)
+        _native = ext
+    return _native
 
 
 def check(code: int, what: str) -> None:

@@ -703,8 +703,8 @@ size_t spsattn_decode_step_workspace_bytes(int S, int H, int D, int nq, const sp
 static int decode_impl(const void* q, int nq, void* out, int out_dtype, const spsattn_segment* segs,
                        int n_segments, const spsattn_extra* extras, int n_extras,
                        const spsattn_kv_append* append, bool single_launch, int S, int H, int D, int dtype,
-                       float sm_scale, void* workspace, size_t workspace_bytes, int* device_status,
-                       void* stream) {
+                       float sm_scale, void* workspace, size_t workspace_bytes, int* tickets,
+                       size_t ticket_bytes, int* device_status, void* stream) {
   if (!q || !out) return SPSATTN_ERR_ARG;
   if (nq != 1 && nq != 2) return SPSATTN_ERR_ARG;
   if (S <= 0 || H <= 0) return SPSATTN_ERR_ARG;
@@ -773,8 +773,11 @@ static int decode_impl(const void* q, int nq, void* out, int out_dtype, const sp
   if (n_chunks > 65535) return SPSATTN_ERR_TOO_LARGE;
   prm.n_chunks = (int)n_chunks;
   const size_t raw = (size_t)S * H * n_chunks * nq * (D + 2) * sizeof(float);
-  const size_t records = single_launch ? decode_records_bytes(S, H, D, nq, segs, n_segments) : align_up(raw, 256);
-  const size_t need = single_launch ? records + decode_ticket_bytes(S, H) : raw;
+  // single launch: tickets behind the records unless the caller keeps them elsewhere
+  const bool own_tickets = single_launch && tickets == nullptr;
+  const size_t records = own_tickets ? decode_records_bytes(S, H, D, nq, segs, n_segments) : align_up(raw, 256);
+  const size_t need = own_tickets ? records + decode_ticket_bytes(S, H) : raw;
+  if (tickets && ticket_bytes < ((size_t)S * H + S) * sizeof(int)) return SPSATTN_ERR_WORKSPACE;
   if (!workspace || workspace_bytes < need) return SPSATTN_ERR_WORKSPACE;
   if (append && !single_launch) return SPSATTN_ERR_ARG;
   if (!aligned16(workspace)) return SPSATTN_ERR_ALIGN;
@@ -805,7 +808,8 @@ static int decode_impl(const void* q, int nq, void* out, int out_dtype, const sp
     d.retained_storage = a.retained_storage;
     d.window_tokens = a.window_tokens > 0 ? a.window_tokens : 0;
   }
-  if (single_launch) prm.tickets = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(workspace) + records);
+  if (single_launch)
+    prm.tickets = own_tickets ? reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(workspace) + records) : tickets;
   prm.q = q;
   prm.out = out;
   prm.out16 = out_dtype != SPSATTN_DTYPE_FP32;
@@ -846,7 +850,7 @@ int spsattn_decode_fwd(const void* q, int nq, float* out, const spsattn_segment*
                        float sm_scale, void* workspace, size_t workspace_bytes, int* device_status,
                        void* stream) {
   return decode_impl(q, nq, out, SPSATTN_DTYPE_FP32, segs, n_segments, extras, n_extras, nullptr, false, S, H,
-                     D, dtype, sm_scale, workspace, workspace_bytes, device_status, stream);
+                     D, dtype, sm_scale, workspace, workspace_bytes, nullptr, 0, device_status, stream);
 }
 
 int spsattn_decode_step(const void* q, int nq, void* out, int out_dtype, const spsattn_segment* segs,
@@ -854,7 +858,17 @@ int spsattn_decode_step(const void* q, int nq, void* out, int out_dtype, const s
                         const spsattn_kv_append* append, int S, int H, int D, int dtype, float sm_scale,
                         void* workspace, size_t workspace_bytes, int* device_status, void* stream) {
   return decode_impl(q, nq, out, out_dtype, segs, n_segments, extras, n_extras, append, true, S, H, D, dtype,
-                     sm_scale, workspace, workspace_bytes, device_status, stream);
+                     sm_scale, workspace, workspace_bytes, nullptr, 0, device_status, stream);
+}
+
+int spsattn_decode_step_tickets(const void* q, int nq, void* out, int out_dtype, const spsattn_segment* segs,
+                                int n_segments, const spsattn_extra* extras, int n_extras,
+                                const spsattn_kv_append* append, int S, int H, int D, int dtype, float sm_scale,
+                                void* workspace, size_t workspace_bytes, int* tickets, size_t ticket_bytes,
+                                int* device_status, void* stream) {
+  if (!tickets || (reinterpret_cast<uintptr_t>(tickets) & 3u)) return SPSATTN_ERR_ARG;
+  return decode_impl(q, nq, out, out_dtype, segs, n_segments, extras, n_extras, append, true, S, H, D, dtype,
+                     sm_scale, workspace, workspace_bytes, tickets, ticket_bytes, device_status, stream);
 }
 
 int spsattn_debug_wait_expiry(int* device_status, unsigned long long limit_ns, int* device_result,

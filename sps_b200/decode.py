@@ -5,8 +5,6 @@ decode_attention_fast.py).  All compute happens in libspsattn.so; there is no fa
 
 from __future__ import annotations
 
-import ctypes as C
-import math
 from dataclasses import dataclass
 from typing import Optional, Sequence
 
@@ -14,7 +12,6 @@ import torch
 from torch import Tensor
 
 from . import _lib
-from .attention import _dtype_code, _forward_only, _status
 
 
 @dataclass
@@ -46,45 +43,6 @@ class PackedKVSegment:
     max_rows: int
 
 
-def _segment_scan_len(seg: KVSegment) -> int:
-    # decode_attention.py:381-390
-    max_t = int(seg.k.size(2))
-    if max_t == 0:
-        return 0
-    if seg.max_len_cap is None:
-        return max_t
-    cap = int(seg.max_len_cap)
-    if cap < 0:
-        raise ValueError(f"KVSegment.max_len_cap must be non-negative, got {cap}")
-    return max(1, min(max_t, cap))
-
-
-_step_ws: dict = {}
-
-
-def _step_workspace(device, stream_handle: int, nbytes: int) -> Tensor:
-    """Zeroed workspace of the single-launch decode, one per (device, stream): the kernel leaves its
-    completion tickets at zero, and calls on one stream are ordered, so the buffer is cleared only
-    when it is (re)allocated.  A buffer of another size starts over: the tickets sit at its end."""
-    if torch.cuda.is_current_stream_capturing():
-        # memory of a graph's private pool must not outlive the capture in this cache
-        return torch.zeros(nbytes, dtype=torch.uint8, device=device)
-    key = (device.index, stream_handle)
-    ws = _step_ws.get(key)
-    if ws is None or ws.numel() != nbytes:
-        ws = torch.zeros(nbytes, dtype=torch.uint8, device=device)
-        _step_ws[key] = ws
-    return ws
-
-
-def _lengths_i64(lengths: Tensor, device) -> Tensor:
-    if lengths.device != device:
-        raise RuntimeError("Segment lengths must live on the same device as query")
-    if lengths.dtype != torch.int64:
-        lengths = lengths.to(torch.int64)
-    return lengths.contiguous()
-
-
 def decode_attention(
     q: Tensor,                                   # [S, nq, H, D]
     segments: Sequence,                          # KVSegment | PackedKVSegment, with query masks
@@ -96,74 +54,7 @@ def decode_attention(
     """nq (1 or 2) queries per (sequence, head) over the live rows of every segment plus the
     extra single-token entries; returns fp32 [S, nq, H, D].  Bit i of a query mask says whether
     query slot i sees that segment / entry."""
-    lib = _lib.load()
-    if not q.is_cuda:
-        raise RuntimeError("CUDA tensors are required for segmented decode attention")
-    # decode is the generation path: no backward kernels behind it
-    _forward_only(q, *[t for seg in segments for t in (seg.k, seg.v)], *[t for e in extras for t in e[:2]])
-    S, nq, H, D = q.shape
-    q = q.contiguous()
-    dt = _dtype_code(q)
-    dev = q.device
-    n_seg = len(segments)
-    keep = [q]
-    seg_arr = (_lib.Segment * max(1, n_seg))()
-    for i, seg in enumerate(segments):
-        qm = 0xFF if segment_query_masks is None else int(segment_query_masks[i])
-        lengths = _lengths_i64(seg.lengths, dev)
-        keep.append(lengths)
-        st = seg_arr[i]
-        if isinstance(seg, PackedKVSegment):
-            off = seg.seq_offset.to(torch.int64).contiguous()
-            keep.append(off)
-            st.k, st.v = seg.k.data_ptr(), seg.v.data_ptr()
-            st.seq_offset, st.seq_stride = off.data_ptr(), 0
-            st.head_stride, st.row_stride = int(seg.head_stride), int(seg.row_stride)
-            st.max_rows = int(seg.max_rows)
-            kd = seg.k.dtype
-        else:
-            if seg.k.dim() != 4 or seg.v.dim() != 4:
-                raise RuntimeError("Segment K/V tensors must be rank-4 [B,H,T,D]")
-            if seg.k.shape != seg.v.shape:
-                raise RuntimeError(f"Segment K/V shapes differ: {tuple(seg.k.shape)} vs {tuple(seg.v.shape)}")
-            if seg.k.size(0) != S or seg.k.size(1) != H or seg.k.size(3) != D:
-                raise RuntimeError("Segment K/V tensors must match query batch/head/head_dim, got "
-                                   f"{tuple(seg.k.shape)} for query {(S, H, D)}")
-            if (not seg.k.is_cuda) or (not seg.v.is_cuda):
-                raise RuntimeError("Segment K/V tensors must be CUDA tensors")
-            if (not seg.k.is_contiguous()) or (not seg.v.is_contiguous()):
-                raise RuntimeError("Segment K/V tensors must be contiguous")
-            max_t = int(seg.k.size(2))
-            st.k, st.v = seg.k.data_ptr(), seg.v.data_ptr()
-            st.seq_offset, st.seq_stride = None, H * max_t * D
-            st.head_stride, st.row_stride = max_t * D, D
-            st.max_rows = _segment_scan_len(seg)
-            kd = seg.k.dtype
-        if st.max_rows > 0 and kd != q.dtype:
-            raise RuntimeError(f"Segment dtype {kd} differs from the attention dtype {q.dtype}")
-        st.lengths = lengths.data_ptr()
-        st.lengths_per_head = int(lengths.dim() == 2)
-        st.query_mask = qm
-    ex_arr = (_lib.Extra * max(1, len(extras)))()
-    for i, (ek, ev, qm) in enumerate(extras):
-        if (not ek.is_cuda) or (not ev.is_cuda):
-            raise RuntimeError("Current-token K/V tensors must be CUDA tensors")
-        if tuple(ek.shape) != (S, H, D) or tuple(ev.shape) != (S, H, D):
-            raise RuntimeError(f"Current-token K/V tensors must have shape {(S, H, D)}, got {tuple(ek.shape)}")
-        ek, ev = ek.to(q.dtype).contiguous(), ev.to(q.dtype).contiguous()
-        keep += [ek, ev]
-        ex_arr[i].k, ex_arr[i].v, ex_arr[i].query_mask = ek.data_ptr(), ev.data_ptr(), int(qm)
-    out = torch.empty((S, nq, H, D), device=dev, dtype=torch.float32)
-    ws_bytes = lib.spsattn_decode_step_workspace_bytes(S, H, D, nq, seg_arr, n_seg)
-    scale = 1.0 / math.sqrt(D) if sm_scale is None else float(sm_scale)
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream()
-        ws = _step_workspace(dev, stream.cuda_stream, ws_bytes)
-        rc = lib.spsattn_decode_step(q.data_ptr(), nq, out.data_ptr(), _lib.DTYPE_FP32, seg_arr, n_seg, ex_arr,
-                                     len(extras), None, S, H, D, dt, scale, ws.data_ptr(), ws_bytes,
-                                     _status(dev).data_ptr(), stream.cuda_stream)
-    _lib.check(rc, "spsattn_decode_step")
-    return out
+    return _lib.native().decode(q, segments, extras, segment_query_masks, sm_scale)
 
 
 def segmented_q2_attention(
@@ -181,19 +72,8 @@ def segmented_q2_attention(
     Slot 0 attends over the segments plus the current normal key; slot 1 over the same
     segments plus current normal and current predict.  Fail-fast like the reference.
     """
-    if not q_Bx2xHxD.is_cuda:
-        raise RuntimeError("CUDA tensors are required for SPS-family cached generation attention")
-    if len(segments) > 2:
-        raise RuntimeError(f"SPS-family q2 attention supports at most 2 segments, got {len(segments)}")
-    if q_Bx2xHxD.dim() != 4 or q_Bx2xHxD.shape[1] != 2:
-        raise RuntimeError(f"Expected q_Bx2xHxD slot dimension to be 2, got {tuple(q_Bx2xHxD.shape)}")
-    head_dim = q_Bx2xHxD.shape[3]
-    if head_dim <= 0 or head_dim > 256:
-        raise RuntimeError(f"Unsupported SPS-family q2 attention head_dim={head_dim}")
-    q = q_Bx2xHxD.to(attn_dtype)
-    extras = [(current_normal_k_BxHxD, current_normal_v_BxHxD, 0b11),
-              (current_predict_k_BxHxD, current_predict_v_BxHxD, 0b10)]
-    return decode_attention(q, segments, extras)
+    return _lib.native().decode_q2(q_Bx2xHxD, segments, current_normal_k_BxHxD, current_normal_v_BxHxD,
+                                   current_predict_k_BxHxD, current_predict_v_BxHxD, attn_dtype)
 
 
 # the name the reference binds (src/modeling/models/reverse_sps/inference.py:354)
@@ -203,13 +83,7 @@ triton_segmented_q2_attention = segmented_q2_attention
 def segmented_q1_attention(q_BxHxD: Tensor, segments: list, *, extra_kv=None,
                            attn_dtype: torch.dtype) -> Tensor:
     """q=1 variant: up to 3 segments and 2 always-valid extra entries (decode_attention.py:393-480)."""
-    if len(segments) > 3:
-        raise RuntimeError(f"q1 attention supports at most 3 segments, got {len(segments)}")
-    extras = [(ek, ev, 1) for ek, ev in (extra_kv or [])]
-    if len(extras) > 2:
-        raise RuntimeError(f"q1 attention supports at most 2 extra entries, got {len(extras)}")
-    q = q_BxHxD.to(attn_dtype).unsqueeze(1)
-    return decode_attention(q, segments, extras)[:, 0]
+    return _lib.native().decode_q1(q_BxHxD, segments, extra_kv, attn_dtype)
 
 
 def masked_kv_attention(q_BxHxD: Tensor, segments: list, *, extra_kv=None, attn_dtype: torch.dtype,
@@ -218,8 +92,7 @@ def masked_kv_attention(q_BxHxD: Tensor, segments: list, *, extra_kv=None, attn_
     """Attention of one query per (batch, head) over variable-length KV segments
     (decode_attention.py:597-704).  Always runs the CUDA kernel; ``prefer_triton`` /
     ``require_triton`` are accepted for signature compatibility."""
-    del prefer_triton, require_triton
-    out = segmented_q1_attention(q_BxHxD, segments, extra_kv=extra_kv, attn_dtype=attn_dtype)
+    out = _lib.native().decode_q1(q_BxHxD, segments, extra_kv, attn_dtype)
     if check_finite and not torch.isfinite(out).all():
         raise RuntimeError(f"Non-finite attention output{error_context}")
     return out
@@ -231,34 +104,8 @@ def fused_sps_kv_update(*, nw_k: Tensor, nw_v: Tensor, nw_len: Tensor, nw_pos: T
                         k_retained_BxHxD: Tensor, v_retained_BxHxD: Tensor,
                         active_mask_B: Tensor, window_tokens: int) -> None:
     """Single-launch in-place KV update for SPS-family decode (decode_attention_fast.py:139-221)."""
-    lib = _lib.load()
-    B, H, D = k_retained_BxHxD.shape
-    assert br_k.shape == br_v.shape and br_k.is_cuda and br_k.is_contiguous() and br_v.is_contiguous()
-    assert br_len.shape == (B, H) and br_len.dtype == torch.int64 and br_len.is_contiguous()
-    active = active_mask_B if active_mask_B.dtype == torch.int8 else active_mask_B.to(torch.int8)
-    active = active.contiguous()
-    kr = k_retained_BxHxD.to(br_k.dtype).contiguous()
-    vr = v_retained_BxHxD.to(br_v.dtype).contiguous()
-    args_w = [None, None, None, None]
-    kw = vw = None
-    window_storage = 0
-    if window_tokens > 0:
-        assert nw_k.shape == nw_v.shape, "nw.k/v shape mismatch"
-        assert nw_k.size(0) == B and nw_k.size(1) == H and nw_k.is_contiguous() and nw_v.is_contiguous()
-        assert nw_len.shape == (B,) and nw_pos.shape == (B,)
-        assert nw_len.dtype == torch.int64 and nw_pos.dtype == torch.int64
-        window_storage = int(nw_k.size(2))
-        kw = k_window_BxHxD.to(nw_k.dtype).contiguous()
-        vw = v_window_BxHxD.to(nw_v.dtype).contiguous()
-        args_w = [nw_k.data_ptr(), nw_v.data_ptr(), nw_len.data_ptr(), nw_pos.data_ptr()]
-    with torch.cuda.device(br_k.device):
-        rc = lib.spsattn_kv_update(
-            args_w[0], args_w[1], args_w[2], args_w[3], br_k.data_ptr(), br_v.data_ptr(), br_len.data_ptr(),
-            None if kw is None else kw.data_ptr(), None if vw is None else vw.data_ptr(),
-            kr.data_ptr(), vr.data_ptr(), active.data_ptr(), B, H, D, window_storage,
-            int(br_k.size(2)), int(window_tokens), br_k.element_size(),
-            torch.cuda.current_stream().cuda_stream)
-    _lib.check(rc, "spsattn_kv_update")
+    _lib.native().kv_update(nw_k, nw_v, nw_len, nw_pos, br_k, br_v, br_len, k_window_BxHxD, v_window_BxHxD,
+                            k_retained_BxHxD, v_retained_BxHxD, active_mask_B, window_tokens)
 
 
 def fill_decode_caches(k_Bx2TxHxD: Tensor, v_Bx2TxHxD: Tensor, current_doc_mask_BxT: Tensor, *,

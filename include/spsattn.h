@@ -81,8 +81,8 @@ int spsattn_version(void);
  * With SPSATTN_PARITY_NONE only the causal and document terms apply.  Rows with no visible key
  * produce 0.  doc_ids: [B, N] int64 (doc_is_i64 = 1) or int32, element strides given; NULL = none.
  * lse (nullable, [B, H, N] fp32) receives log2(sum_j exp2(score_ij * sm_scale * log2 e)), the
- * reference's M tensor (:265-267).  N must be even unless parity is NONE.  D in {64, 128} run on
- * the tcgen05/TMA kernel; D in {16, 32, 256} run on a plain CUDA-core kernel.  sm_scale > 0.
+ * reference's M tensor (:265-267).  N must be even unless parity is NONE.  All of D in
+ * {16, 32, 64, 128, 256} run on the tcgen05 / TMA kernel.  sm_scale > 0.
  * workspace: at least spsattn_prefill_workspace_bytes(B, H, N, D) bytes of device memory,
  * 256-byte aligned, private to this call until it completes.
  * ------------------------------------------------------------------------------------------- */
@@ -102,8 +102,8 @@ int spsattn_prefill_fwd(const void* q, const void* k, const void* v, void* o, fl
  * of token-major [B, N, H, D] projections (src/modeling/models/sps/core.py:45-55) and transposes
  * the result back (:79); with strides the kernel reads and writes those layouts in place — q, k, v
  * even straight out of a fused [B, N, 3*H*D] projection buffer — so the .contiguous() copies of
- * triton_sps_flash_attention.py:504-506 disappear.  D in {64, 128}; the other head dims need dense
- * operands. */
+ * triton_sps_flash_attention.py:504-506 disappear.
+ */
 int spsattn_prefill_fwd_strided(const void* q, const void* k, const void* v, void* o, float* lse,
                                 const int64_t* q_strides, const int64_t* k_strides,
                                 const int64_t* v_strides, const int64_t* o_strides,

@@ -194,19 +194,12 @@ Forward prefill_forward(Tensor q, Tensor k, Tensor v, const MaskArgs& m, const o
   // the tensor-core kernels read any layout whose rows are contiguous (the transposed views of
   // token-major projections that the reference's modules pass); only what they cannot address is
   // copied, where the reference copies always (triton_sps_flash_attention.py:504-506)
-  const bool strided_ok = d == 64 || d == 128;
-  if (!(strided_ok && addressable(q))) q = q.contiguous();
-  if (!(strided_ok && addressable(k))) k = k.contiguous();
-  if (!(strided_ok && addressable(v))) v = v.contiguous();
+  for (Tensor* x : {&q, &k, &v})
+    if (!addressable(*x)) *x = x->contiguous();
   const DocArgs ids(docs, b, n, q);
   const c10::cuda::CUDAGuard guard(q.device());
   Forward r;
-  if (out.has_value())
-    r.o = *out;
-  else if (strided_ok)
-    r.o = empty_like_layout(q);
-  else
-    r.o = at::detail::empty_cuda({b, h, n, d}, q.scalar_type(), q.device(), c10::nullopt);
+  r.o = out.has_value() ? *out : empty_like_layout(q);
   if (return_lse) r.lse = at::detail::empty_cuda({b, h, n}, at::kFloat, q.device(), c10::nullopt);
   const size_t ws_bytes = ids.ptr ? spsattn_prefill_workspace_bytes(b, h, n, d) : 0;
   Tensor ws;

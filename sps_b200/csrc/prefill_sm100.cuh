@@ -70,38 +70,47 @@ constexpr int kPrefillThreads = 192;
 template <int D>
 struct PrefillCfg {
   static constexpr int kStagesK = 2;
-  static constexpr int kStagesV = (D == 64) ? 2 : 1;
-  static constexpr int kSBufs = (D == 64) ? 1 : 2;            // S accumulators in TMEM
-  static constexpr uint32_t kTmemCols = (D == 64) ? 128 : 256;
+  static constexpr int kStagesV = (D == 128) ? 1 : 2;
+  static constexpr int kSBufs = (D <= 64) ? 1 : 2;             // S accumulators in TMEM
+  static constexpr uint32_t kTmemCols = (D <= 64) ? 128 : (D == 128) ? 256 : 512;
+  // Heads narrower than 64 keep the 128-byte rows of shared memory: the tensor maps end at D and
+  // the copies fill the rest of a row with zeros without reading it; the products run over D only.
+  static constexpr int kDP = D < 64 ? 64 : D;
   static constexpr uint32_t kColO = kSBufs * kTileN;           // O accumulator column offset
-  static constexpr int kQBytes = kTileM * D * 2;               // the Q tile
+  static constexpr int kQBytes = kTileM * kDP * 2;               // the Q tile
   static constexpr int kQSubBytes = kTileM * 128;              // 128 rows x 64 elements
-  static constexpr int kKVBytes = kTileN * D * 2;              // one K or V tile
+  static constexpr int kKVBytes = kTileN * kDP * 2;              // one K or V tile
   static constexpr int kKVSubBytes = kTileN * 128;             // 64 rows x 64 elements
-  static constexpr int kPBytes = (D == 64 && SPSATTN_P_SPLIT_DEFAULT) ? 0 : kTileM * kTileN * 2;
+  static constexpr int kPBytes = (D <= 64 && SPSATTN_P_SPLIT_DEFAULT) ? 0 : kTileM * kTileN * 2;
   static constexpr int kOffQ = 0;
   static constexpr int kOffK = kOffQ + kQBytes;
   static constexpr int kOffV = kOffK + kStagesK * kKVBytes;
   static constexpr int kOffP = kOffV + kStagesV * kKVBytes;
   static constexpr int kOffBar = kOffP + kPBytes;
   static constexpr int kSmemBytes = kOffBar + 256 + 1024;      // barriers + alignment slack
-  static constexpr int kBlocksPerSM = (D == 64) ? 3 : 2;
-  // head_dim 128 (two S accumulators): P never touches shared memory.  The softmax thread writes
+  static constexpr int kBlocksPerSM = (D <= 64) ? 3 : (D == 128) ? 2 : 1;
+  // head_dim 128 and 256 (two S accumulators): P never touches shared memory.  The softmax thread writes
   // it, as packed 16-bit pairs, over the S columns it has just read, and the P V product takes it
   // from tensor memory as its A operand, which also halves what that product reads from shared
   // memory.  The next Q K^T into the same accumulator is issued after this tile's P V, and the
   // tensor pipe runs in issue order.  (With the single accumulator of head_dim 64 the next Q K^T
   // would have to wait for P V; measured slower there.)
-  static constexpr bool kPTmem = (D == 128);
-  // head_dim 64: P also lives in tensor memory, but in 32 columns of its own (a second, small
+  static constexpr bool kPTmem = (D >= 128);
+  // head_dim <= 64: P also lives in tensor memory, but in 32 columns of its own (a second, small
   // allocation: 128 + 32 columns per block, three blocks per SM = 480 of 512), so the next Q K^T
   // does not have to wait for this tile's P V.  No shared-memory stores, no swizzle arithmetic,
   // no proxy fence; the P tile's 16 KB of shared memory are not needed.
 #ifndef SPSATTN_P_SPLIT
 #define SPSATTN_P_SPLIT 1
 #endif
-  static constexpr bool kPSplit = (D == 64) && (SPSATTN_P_SPLIT != 0);
+  static constexpr bool kPSplit = (D <= 64) && (SPSATTN_P_SPLIT != 0);
   static constexpr uint32_t kPCols = kTileN / 2;
+  // head_dim 16, 32 and 256: the probabilities keep more than 16 bits.  P goes to tensor memory as
+  // two 16-bit terms, p = hi + lo, and the product runs over both: these widths leave the tensor
+  // pipe idle (narrow) or are rare (256), and their results carry fp32 probabilities this way.
+  // lo lies behind O where the heads are narrow (columns 96-127), behind hi in the S columns else.
+  static constexpr bool kPLo = (D != 64 && D != 128);
+  static constexpr uint32_t kColPLo = (D <= 32) ? 96 : kTileN / 2;
 };
 
 struct TileInfo {
@@ -175,6 +184,7 @@ __global__ void __launch_bounds__(kPrefillThreads, PrefillCfg<D>::kBlocksPerSM)
 prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const PrefillParams prm) {
   using Cfg = PrefillCfg<D>;
+  constexpr int kOChunk = D < 32 ? D : 32;      // columns of O a thread moves at a time
   extern __shared__ uint8_t smem_raw[];
   __shared__ BlockPlan s_plan;
   __shared__ int s_tiles[kTileTable];
@@ -270,7 +280,7 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       // the Q tile depends on nothing but the block index: start it before the plan is known
       tma_prefetch_desc(&tm_q);
       mbar_arrive_expect_tx(bar_q_full, Cfg::kQBytes);
-      for (int c = 0; c < D / 64; ++c)
+      for (int c = 0; c < Cfg::kDP / 64; ++c)
         tma_load_4d(sQ + c * Cfg::kQSubBytes, &tm_q, bar_q_full, c * 64, i0, h, b);
       tma_prefetch_desc(&tm_k);
       tma_prefetch_desc(&tm_v);
@@ -296,7 +306,7 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const TileInfo t = tile_info(s_plan, 0);
     if (elect_one()) {
       mbar_arrive_expect_tx(bar_k_full, Cfg::kKVBytes);
-      for (int c = 0; c < D / 64; ++c)
+      for (int c = 0; c < Cfg::kDP / 64; ++c)
         tma_load_5d(sK + c * Cfg::kKVSubBytes, &tm_k, bar_k_full, c * 64, t.stream, t.k0, h, b);
     }
     __syncwarp();
@@ -322,7 +332,7 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           }
           if (elect_one()) {
             mbar_arrive_expect_tx(bar_k_full + 8 * st, Cfg::kKVBytes);
-            for (int c = 0; c < D / 64; ++c)
+            for (int c = 0; c < Cfg::kDP / 64; ++c)
               tma_load_5d(sK + st * Cfg::kKVBytes + c * Cfg::kKVSubBytes, &tm_k, bar_k_full + 8 * st,
                           c * 64, t.stream, t.k0, h, b);
           }
@@ -339,7 +349,7 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           }
           if (elect_one()) {
             mbar_arrive_expect_tx(bar_v_full + 8 * st, Cfg::kKVBytes);
-            for (int c = 0; c < D / 64; ++c)
+            for (int c = 0; c < Cfg::kDP / 64; ++c)
               tma_load_5d(sV + st * Cfg::kKVBytes + c * Cfg::kKVSubBytes, &tm_v, bar_v_full + 8 * st,
                           c * 64, t.stream, t.k0, h, b);
           }
@@ -418,6 +428,12 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 #pragma unroll
               for (int kk = 0; kk < kTileN / 16; ++kk)
                 umma_ts(od, pa + 8 * kk, vb0 + ((kk * 2048) >> 4), dv_hi, idesc_pv, j > 0 || kk > 0);
+              if constexpr (Cfg::kPLo) {
+                const uint32_t pl = Cfg::kPSplit ? tmem + Cfg::kColPLo : pa + Cfg::kColPLo;
+#pragma unroll
+                for (int kk = 0; kk < kTileN / 16; ++kk)
+                  umma_ts(od, pl + 8 * kk, vb0 + ((kk * 2048) >> 4), dv_hi, idesc_pv, true);
+              }
             } else {
               if (j > 0) {
                 umma_ss<true>(od, dp_lo, dp_hi, vb0, dv_hi, idesc_pv);
@@ -558,6 +574,7 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         const float2 c2 = make_float2(c, c), nm2 = make_float2(neg_mc, neg_mc);
         float2 sum_a = make_float2(0.f, 0.f), sum_b = make_float2(0.f, 0.f);
         uint32_t pk[kTileN / 2];
+        uint32_t pl[Cfg::kPLo ? kTileN / 2 : 1];
 #ifdef SPSATTN_EXP_PAIRWISE
 #pragma unroll
         for (int e = 0; e < kTileN; e += 4) {
@@ -595,6 +612,14 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
               sum_b = __fadd2_rn(sum_b, make_float2(s[e + 2], s[e + 3]));
               pk[e / 2] = pack2<FP16>(s[e], s[e + 1]);
               pk[e / 2 + 1] = pack2<FP16>(s[e + 2], s[e + 3]);
+              if constexpr (Cfg::kPLo) {
+#pragma unroll
+                for (int x = 0; x < 4; x += 2) {
+                  float h0, h1;
+                  unpack2<FP16>(pk[(e + x) / 2], h0, h1);
+                  pl[(e + x) / 2] = pack2<FP16>(s[e + x] - h0, s[e + x + 1] - h1);
+                }
+              }
             }
           }
         }
@@ -624,6 +649,11 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           tmem_st16(tmem_p + lane_addr, pk);
           tmem_st16(tmem_p + lane_addr + 16, pk + 16);
         }
+        if constexpr (Cfg::kPLo) {
+          const uint32_t at = tmem + lane_addr + (Cfg::kPSplit ? 0 : sb * kTileN) + Cfg::kColPLo;
+          tmem_st16(at, pl);
+          tmem_st16(at + 16, pl + 16);
+        }
         // P -> shared memory, K-major 128B-swizzled: 16-byte chunk ch of row r sits at
         // r * 128 + ((ch ^ (r & 7)) << 4) of the [128 x 64] tile
 #pragma unroll
@@ -643,13 +673,13 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         }
         if (j > 0 && rescale) {
 #pragma unroll
-          for (int q4 = 0; q4 < D / 32; ++q4) {
-            uint32_t r[32];
-            tmem_ld32(tmem + lane_addr + Cfg::kColO + q4 * 32, r);
+          for (int q4 = 0; q4 < D / kOChunk; ++q4) {
+            uint32_t r[kOChunk];
+            tmem_ld_chunk(tmem + lane_addr + Cfg::kColO + q4 * kOChunk, r);
             tmem_wait_ld();
 #pragma unroll
-            for (int e = 0; e < 32; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * alpha);
-            tmem_st32(tmem + lane_addr + Cfg::kColO + q4 * 32, r);
+            for (int e = 0; e < kOChunk; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * alpha);
+            tmem_st_chunk(tmem + lane_addr + Cfg::kColO + q4 * kOChunk, r);
           }
           tmem_wait_st();
         }
@@ -669,19 +699,19 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         uint8_t* o_row = reinterpret_cast<uint8_t*>(prm.o) +
                          (b * prm.o_stride_b + h * prm.o_stride_h + i * prm.o_stride_n) * 2;
 #pragma unroll
-        for (int q4 = 0; q4 < D / 32; ++q4) {
-          uint32_t r[32];
-          tmem_ld32(tmem + lane_addr + Cfg::kColO + q4 * 32, r);
+        for (int q4 = 0; q4 < D / kOChunk; ++q4) {
+          uint32_t r[kOChunk];
+          tmem_ld_chunk(tmem + lane_addr + Cfg::kColO + q4 * kOChunk, r);
           tmem_wait_ld();
           if (i < prm.N) {
 #pragma unroll
-            for (int e = 0; e < 32; e += 8) {
+            for (int e = 0; e < kOChunk; e += 8) {
               uint4 u;
               u.x = pack2<FP16>(__uint_as_float(r[e]) * inv_l, __uint_as_float(r[e + 1]) * inv_l);
               u.y = pack2<FP16>(__uint_as_float(r[e + 2]) * inv_l, __uint_as_float(r[e + 3]) * inv_l);
               u.z = pack2<FP16>(__uint_as_float(r[e + 4]) * inv_l, __uint_as_float(r[e + 5]) * inv_l);
               u.w = pack2<FP16>(__uint_as_float(r[e + 6]) * inv_l, __uint_as_float(r[e + 7]) * inv_l);
-              *reinterpret_cast<uint4*>(o_row + q4 * 64 + e * 2) = u;
+              *reinterpret_cast<uint4*>(o_row + (q4 * kOChunk + e) * 2) = u;
             }
           }
         }

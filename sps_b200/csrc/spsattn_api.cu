@@ -421,75 +421,68 @@ int spsattn_prefill_fwd_strided(const void* q, const void* k, const void* v, voi
   const float scale_log2 = sm_scale * 1.4426950408889634f;
   const bool fp16 = dtype == SPSATTN_DTYPE_FP16;
 
-  if (D == 64 || D == 128) {
-    CUtensorMap tq, tk, tv;
-    if ((rc = encode_q_map(&tq, q, B, H, N, D, sq, dtype)) != 0) return rc;
-    const bool wide = D == 64 && g_prefill_path.load() == 2;
-    const int box_tokens = wide ? kWideN : kTileN;
-    if ((rc = encode_kv_map(&tk, k, B, H, N, D, mask.ks, sk, dtype, box_tokens)) != 0) return rc;
-    if ((rc = encode_kv_map(&tv, v, B, H, N, D, mask.ks, sv, dtype, box_tokens)) != 0) return rc;
-    PrefillParams prm;
-    memset(&prm, 0, sizeof(prm));
-    prm.o = o;
-    prm.o_stride_b = so.b;
-    prm.o_stride_h = so.h;
-    prm.o_stride_n = so.n;
-    prm.lse = lse;
-    prm.docs = doc_ids;
-    prm.doc_stride_b = doc_stride_b;
-    prm.doc_stride_t = doc_stride_t;
-    prm.doc_is_i64 = doc_is_i64;
-    prm.lo = lo;
-    prm.mono = mono;
-    prm.B = B;
-    prm.H = H;
-    prm.N = N;
-    prm.n_qtiles = (N + kTileM - 1) / kTileM;
-    prm.mask = mask;
-    prm.scale_log2 = scale_log2;
-    prm.status = device_status;
+  CUtensorMap tq, tk, tv;
+  if ((rc = encode_q_map(&tq, q, B, H, N, D, sq, dtype)) != 0) return rc;
+  const bool wide = D == 64 && g_prefill_path.load() == 2;
+  const int box_tokens = wide ? kWideN : kTileN;
+  if ((rc = encode_kv_map(&tk, k, B, H, N, D, mask.ks, sk, dtype, box_tokens)) != 0) return rc;
+  if ((rc = encode_kv_map(&tv, v, B, H, N, D, mask.ks, sv, dtype, box_tokens)) != 0) return rc;
+  PrefillParams prm;
+  memset(&prm, 0, sizeof(prm));
+  prm.o = o;
+  prm.o_stride_b = so.b;
+  prm.o_stride_h = so.h;
+  prm.o_stride_n = so.n;
+  prm.lse = lse;
+  prm.docs = doc_ids;
+  prm.doc_stride_b = doc_stride_b;
+  prm.doc_stride_t = doc_stride_t;
+  prm.doc_is_i64 = doc_is_i64;
+  prm.lo = lo;
+  prm.mono = mono;
+  prm.B = B;
+  prm.H = H;
+  prm.N = N;
+  prm.n_qtiles = (N + kTileM - 1) / kTileM;
+  prm.mask = mask;
+  prm.scale_log2 = scale_log2;
+  prm.status = device_status;
 #ifdef SPSATTN_TRACE
-    prm.trace = g_trace_buffer;
+  prm.trace = g_trace_buffer;
 #endif
-    // heads whose K and V (2 * N * D * 2 bytes each) share about 48 MB of L2 at a time
-    const long long kv_bytes = 4LL * N * D;
-    const long long gh = (48LL << 20) / (kv_bytes > 0 ? kv_bytes : 1);
-    prm.group_heads = (int)(gh < 1 ? 1 : (gh > 32 ? 32 : gh));
+  // heads whose K and V (2 * N * D * 2 bytes each) share about 48 MB of L2 at a time
+  const long long kv_bytes = 4LL * N * D;
+  const long long gh = (48LL << 20) / (kv_bytes > 0 ? kv_bytes : 1);
+  prm.group_heads = (int)(gh < 1 ? 1 : (gh > 32 ? 32 : gh));
 #ifdef SPSATTN_NO_GROUP
-    prm.group_heads = 1;      // tuning builds: one head after the other
+  prm.group_heads = 1;      // tuning builds: one head after the other
 #endif
-    if (wide) {
-      // the item counter lives behind the pre-pass flags: the pre-pass has zeroed it when ids were
-      // given, else it is cleared here; without a workspace the blocks take items with a stride
-      if (mono != nullptr) {
-        prm.work_counter = mono + B;
-      } else if (workspace != nullptr && workspace_bytes >= prefill_ws_mono_bytes(B) &&
-                 (reinterpret_cast<uintptr_t>(workspace) & 3u) == 0) {
-        prm.work_counter = reinterpret_cast<int*>(workspace) + B;
-        cudaError_t me = cudaMemsetAsync(prm.work_counter, 0, sizeof(int), st);
-        if (me != cudaSuccess) return (int)me;
-      }
-      return fp16 ? launch_prefill_wide<true>(tq, tk, tv, prm, st)
-                  : launch_prefill_wide<false>(tq, tk, tv, prm, st);
+  if (wide) {
+    // the item counter lives behind the pre-pass flags: the pre-pass has zeroed it when ids were
+    // given, else it is cleared here; without a workspace the blocks take items with a stride
+    if (mono != nullptr) {
+      prm.work_counter = mono + B;
+    } else if (workspace != nullptr && workspace_bytes >= prefill_ws_mono_bytes(B) &&
+               (reinterpret_cast<uintptr_t>(workspace) & 3u) == 0) {
+      prm.work_counter = reinterpret_cast<int*>(workspace) + B;
+      cudaError_t me = cudaMemsetAsync(prm.work_counter, 0, sizeof(int), st);
+      if (me != cudaSuccess) return (int)me;
     }
-    if (D == 64) return fp16 ? launch_prefill_sm100<64, true>(tq, tk, tv, prm, st)
-                             : launch_prefill_sm100<64, false>(tq, tk, tv, prm, st);
-    return fp16 ? launch_prefill_sm100<128, true>(tq, tk, tv, prm, st)
-                : launch_prefill_sm100<128, false>(tq, tk, tv, prm, st);
+    return fp16 ? launch_prefill_wide<true>(tq, tk, tv, prm, st)
+                : launch_prefill_wide<false>(tq, tk, tv, prm, st);
   }
-  // the CUDA-core kernel for the other head dims reads dense [B, H, N, D] operands only
-  const Strides dense = {(int64_t)H * N * D, (int64_t)N * D, (int64_t)D};
-  auto is_dense = [&](Strides x) { return x.b == dense.b && x.h == dense.h && x.n == dense.n; };
-  if (!is_dense(sq) || !is_dense(sk) || !is_dense(sv) || !is_dense(so)) return SPSATTN_ERR_ALIGN;
-  dim3 grid((N + 3) / 4, B * H);
-  const size_t smem = 4 * (size_t)D * sizeof(float);
-  if (fp16)
-    prefill_generic_kernel<true><<<grid, 128, smem, st>>>(q, k, v, o, lse, doc_ids, doc_is_i64, doc_stride_b,
-                                                          doc_stride_t, lo, mono, H, N, D, mask, scale_log2);
-  else
-    prefill_generic_kernel<false><<<grid, 128, smem, st>>>(q, k, v, o, lse, doc_ids, doc_is_i64, doc_stride_b,
-                                                           doc_stride_t, lo, mono, H, N, D, mask, scale_log2);
-  return (int)cudaGetLastError();
+  switch (D) {
+    case 16: return fp16 ? launch_prefill_sm100<16, true>(tq, tk, tv, prm, st)
+                         : launch_prefill_sm100<16, false>(tq, tk, tv, prm, st);
+    case 32: return fp16 ? launch_prefill_sm100<32, true>(tq, tk, tv, prm, st)
+                         : launch_prefill_sm100<32, false>(tq, tk, tv, prm, st);
+    case 64: return fp16 ? launch_prefill_sm100<64, true>(tq, tk, tv, prm, st)
+                         : launch_prefill_sm100<64, false>(tq, tk, tv, prm, st);
+    case 128: return fp16 ? launch_prefill_sm100<128, true>(tq, tk, tv, prm, st)
+                          : launch_prefill_sm100<128, false>(tq, tk, tv, prm, st);
+    default: return fp16 ? launch_prefill_sm100<256, true>(tq, tk, tv, prm, st)
+                         : launch_prefill_sm100<256, false>(tq, tk, tv, prm, st);
+  }
 }
 
 size_t spsattn_prefill_bwd_workspace_bytes(int B, int H, int N, int D) {

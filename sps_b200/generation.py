@@ -261,12 +261,9 @@ class SPSGenerator:
             _lib.check(rc, "spsattn_qkv_rope_cast")
             if state is not None:
                 self._fill_caches(state, layer, ops[1], ops[2], doc_mask)
-            in_place = hd in (64, 128)     # the tensor-core kernel reads and writes token-major rows
-            o = prefill_attention(ops[0].transpose(1, 2), ops[1].transpose(1, 2), ops[2].transpose(1, 2),
-                                  scale, persistent_parity=self.parity, temporary_window=self.window_tokens,
-                                  documents_idx=docs2, out=y.transpose(1, 2) if in_place else None)
-            if not in_place:
-                y.copy_(o.transpose(1, 2))
+            prefill_attention(ops[0].transpose(1, 2), ops[1].transpose(1, 2), ops[2].transpose(1, 2),
+                              scale, persistent_parity=self.parity, temporary_window=self.window_tokens,
+                              documents_idx=docs2, out=y.transpose(1, 2))
             y2 = y.view(rows, c)
             if pdt != self.attn_dtype:
                 y2 = y2.to(pdt)                                             # sps/core.py:80

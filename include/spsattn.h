@@ -66,6 +66,7 @@ extern "C" {
 
 /* device_status codes written by kernels (0 = ok) */
 #define SPSATTN_STATUS_WAIT_EXPIRED 1
+#define SPSATTN_STATUS_BAD_TOKEN 2      /* a decode step was given a token id outside the vocabulary */
 
 const char* spsattn_strerror(int code);
 int spsattn_version(void);
@@ -383,6 +384,74 @@ int spsattn_add_rmsnorm(void* x, const void* delta_or_null, const void* weight, 
                         int dtype, long long rows, int C, float eps, void* stream);
 
 int spsattn_swiglu(const void* gate_up, void* y, int dtype, long long rows, int I, void* stream);
+
+/* ---------------------------------------------------------------------------------------------
+ * A decode step of the decoder (reverse_sps/inference.py:364-503 without its host checks).  Nothing
+ * synchronises with the host, so the calls can be captured in a CUDA graph.
+ *
+ * spsattn_decoder_start: the tokens of the step (greedy choice over the logits of the step before,
+ *   or the caller's), counters, embedding; parameters and activations in `param_dtype`.
+ * spsattn_decoder_choose: the greedy choice alone (the last token of a generation).
+ * spsattn_decoder_step: start, every layer's projections around spsattn_decode_step, and the head on
+ *   the prediction slot, each launch a programmatic dependent of the one before it.  For sizes that
+ *   spsattn_decoder_step_supported takes (1 = yes): bf16, batch * slots <= 16 rows, hidden and
+ *   intermediate multiples of 16, hidden <= 2048.
+ * ------------------------------------------------------------------------------------------- */
+typedef struct spsattn_decoder_layer {
+  const void* attn_norm;      /* [C] */
+  const void* c_attn;         /* [3C, C] */
+  const void* c_proj;         /* [C, C] */
+  const void* mlp_norm;       /* [C] */
+  const void* gate_up;        /* [2I, C] */
+  const void* down;           /* [C, I] */
+  spsattn_segment segments[2];
+  spsattn_kv_append append;   /* k/v_window and k/v_retained point into k2 / v2 below */
+} spsattn_decoder_layer;
+
+typedef struct spsattn_decoder {
+  int32_t n_layer, batch, slots, n_head, head_dim, hidden, intermediate, vocab, pred_slot, n_segments;
+  int32_t param_dtype;        /* SPSATTN_DTYPE_BF16 or SPSATTN_DTYPE_FP32 */
+  float norm_eps;
+  int64_t eos, pad, predict;
+  const spsattn_decoder_layer* layers;   /* host array; only spsattn_decoder_step reads it */
+  const void* wte;            /* [vocab, C] */
+  const void* lm_head;        /* [vocab, C] */
+  const void* out_norm;       /* [C] */
+  const float* freqs;         /* [positions, head_dim / 2, 2] (cos, sin) */
+  int64_t* processed;         /* [batch] tokens per sequence, advanced */
+  uint8_t* next_doc_start;    /* [batch] */
+  int64_t *nw_len, *nw_pos;   /* [n_layer, batch] */
+  int64_t* br_len;            /* [n_layer, batch, n_head] */
+  /* step buffers */
+  int8_t* active;             /* [batch] */
+  int64_t* pos;               /* [batch] */
+  float* freqs_out;           /* [batch, head_dim / 2, 2] rows of this step's positions, or NULL */
+  void *x, *q, *k2, *v2, *y, *mlp_hidden;   /* [rows, C] x, q; [slots, batch, C] k2, v2; [rows, C] y; [rows, I] */
+  float* ssq;                 /* [rows, C / 8], or NULL for spsattn_decoder_start alone */
+  void* workspace;            /* spsattn_decode_step_workspace_bytes, zeroed once */
+  size_t workspace_bytes;
+} spsattn_decoder;
+
+/* Where the tokens of a step come from: logits (greedy choice among ids whose bit in `suppressed`
+ * is clear, first maximum) or token_in / active_in. */
+typedef struct spsattn_token_source {
+  const void* logits;         /* [batch, vocab] of param_dtype, or NULL */
+  const uint32_t* suppressed; /* [(vocab + 31) / 32] or NULL */
+  int64_t* generated;         /* [batch, max_new] */
+  int64_t* step;              /* [batch], advanced */
+  uint8_t* finished;          /* [batch] */
+  int32_t max_new, stop_on_eos;
+  const int64_t* token_in;    /* [batch] */
+  const uint8_t* active_in;   /* [batch] */
+} spsattn_token_source;
+
+int spsattn_decoder_start(const spsattn_decoder* d, const spsattn_token_source* source, int* device_status,
+                          void* stream);
+int spsattn_decoder_choose(const spsattn_decoder* d, const spsattn_token_source* source, void* stream);
+int spsattn_decoder_step_supported(const spsattn_decoder* d);
+/* logits_out: [batch, vocab] bf16, zeros for inactive sequences. */
+int spsattn_decoder_step(const spsattn_decoder* d, const spsattn_token_source* source, void* logits_out,
+                         int* device_status, void* stream);
 
 /* ---------------------------------------------------------------------------------------------
  * Prefill -> decode hand-over for one layer (src/modeling/models/reverse_sps/inference.py:568-613,

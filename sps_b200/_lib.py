@@ -17,6 +17,7 @@ PARITY_EVEN, PARITY_ODD, PARITY_NONE = 0, 1, -1
 NO_WINDOW = -2147483648
 NOALLOC_SCRATCH_BYTES = 16 << 20
 FLAG_PERSISTENT_Q_SKIPS_TEMPORARY = 1
+STATUS_BAD_TOKEN = 2
 
 EXPORTS = (
     "spsattn_version", "spsattn_strerror",
@@ -26,6 +27,7 @@ EXPORTS = (
     "spsattn_decode_step_workspace_bytes", "spsattn_decode_step", "spsattn_decode_step_tickets",
     "spsattn_qkv_rope_cast",
     "spsattn_add_rmsnorm", "spsattn_swiglu", "spsattn_debug_decode_path", "spsattn_debug_prefill_path", "spsattn_debug_wait_expiry",
+    "spsattn_decoder_start", "spsattn_decoder_choose", "spsattn_decoder_step_supported", "spsattn_decoder_step",
     "spsattn_prefill_bwd_workspace_bytes", "spsattn_prefill_bwd", "spsattn_prefill_bwd_strided",
 )
 
@@ -62,6 +64,36 @@ class RopeGroup(C.Structure):
     """struct spsattn_rope_group"""
     _fields_ = [("out", C.c_void_p), ("stride_b", C.c_int64), ("stride_n", C.c_int64),
                 ("stride_h", C.c_int64), ("rotate", C.c_int32), ("reserved", C.c_int32)]
+
+
+class DecoderLayer(C.Structure):
+    """struct spsattn_decoder_layer"""
+    _fields_ = [("attn_norm", C.c_void_p), ("c_attn", C.c_void_p), ("c_proj", C.c_void_p), ("mlp_norm", C.c_void_p),
+                ("gate_up", C.c_void_p), ("down", C.c_void_p), ("segments", Segment * 2), ("append", KvAppend)]
+
+
+class Decoder(C.Structure):
+    """struct spsattn_decoder"""
+    _fields_ = [
+        ("n_layer", C.c_int32), ("batch", C.c_int32), ("slots", C.c_int32), ("n_head", C.c_int32),
+        ("head_dim", C.c_int32), ("hidden", C.c_int32), ("intermediate", C.c_int32), ("vocab", C.c_int32),
+        ("pred_slot", C.c_int32), ("n_segments", C.c_int32), ("param_dtype", C.c_int32), ("norm_eps", C.c_float),
+        ("eos", C.c_int64), ("pad", C.c_int64), ("predict", C.c_int64), ("layers", C.POINTER(DecoderLayer)),
+        ("wte", C.c_void_p), ("lm_head", C.c_void_p), ("out_norm", C.c_void_p), ("freqs", C.c_void_p),
+        ("processed", C.c_void_p), ("next_doc_start", C.c_void_p), ("nw_len", C.c_void_p), ("nw_pos", C.c_void_p),
+        ("br_len", C.c_void_p), ("active", C.c_void_p), ("pos", C.c_void_p), ("freqs_out", C.c_void_p),
+        ("x", C.c_void_p), ("q", C.c_void_p), ("k2", C.c_void_p), ("v2", C.c_void_p), ("y", C.c_void_p),
+        ("mlp_hidden", C.c_void_p), ("ssq", C.c_void_p), ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t),
+    ]
+
+
+class TokenSource(C.Structure):
+    """struct spsattn_token_source"""
+    _fields_ = [
+        ("logits", C.c_void_p), ("suppressed", C.c_void_p), ("generated", C.c_void_p), ("step", C.c_void_p),
+        ("finished", C.c_void_p), ("max_new", C.c_int32), ("stop_on_eos", C.c_int32),
+        ("token_in", C.c_void_p), ("active_in", C.c_void_p),
+    ]
 
 
 class SpsAttnError(RuntimeError):
@@ -133,6 +165,14 @@ def load() -> C.CDLL:
     lib.spsattn_add_rmsnorm.argtypes = [vp, vp, vp, vp, i32, C.c_longlong, i32, f32, vp]
     lib.spsattn_swiglu.restype = i32
     lib.spsattn_swiglu.argtypes = [vp, vp, i32, C.c_longlong, i32, vp]
+    lib.spsattn_decoder_start.restype = i32
+    lib.spsattn_decoder_start.argtypes = [C.POINTER(Decoder), C.POINTER(TokenSource), vp, vp]
+    lib.spsattn_decoder_choose.restype = i32
+    lib.spsattn_decoder_choose.argtypes = [C.POINTER(Decoder), C.POINTER(TokenSource), vp]
+    lib.spsattn_decoder_step_supported.restype = i32
+    lib.spsattn_decoder_step_supported.argtypes = [C.POINTER(Decoder)]
+    lib.spsattn_decoder_step.restype = i32
+    lib.spsattn_decoder_step.argtypes = [C.POINTER(Decoder), C.POINTER(TokenSource), vp, vp, vp]
     lib.spsattn_debug_decode_path.restype = i32
     lib.spsattn_debug_decode_path.argtypes = [i32]
     lib.spsattn_debug_wait_expiry.restype = i32

@@ -31,7 +31,8 @@ def check_device_status(device=None) -> None:
     code = int(word.item())
     if code != 0:
         word.zero_()
-        raise _lib.SpsAttnError(f"device reported status {code} (a bounded wait expired)")
+        what = "a token id outside the vocabulary" if code == _lib.STATUS_BAD_TOKEN else "a bounded wait expired"
+        raise _lib.SpsAttnError(f"device reported status {code} ({what})")
 
 
 def _dtype_code(t: torch.Tensor) -> int:

@@ -481,6 +481,8 @@ decode_split_kernel(const DecodeParams prm) {
   // highest chunk first: blocks past the live length retire at once, at the start of the launch
   const int chunk = (int)gridDim.y - 1 - (int)blockIdx.y;
   const int tid = threadIdx.x;
+  grid_launch_dependents();
+  grid_dependency_wait();      // in a decode step: the queries and counters come from the launch before
 
   int seg_start[kMaxSegments + 1];
   seg_start[0] = 0;

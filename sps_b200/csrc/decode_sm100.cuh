@@ -86,6 +86,8 @@ decode_tc_kernel(const __grid_constant__ DecodeMaps maps, const DecodeParams prm
   // highest slot first: blocks past the live length retire at once, at the start of the launch
   const int slot = (int)gridDim.y - 1 - (int)blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  grid_launch_dependents();
+  grid_dependency_wait();      // in a decode step: the queries and counters come from the launch before
 
   int seg_live[kMaxSegments];
   int n_total = 0;

@@ -8,11 +8,13 @@
 
 #include <atomic>
 #include <mutex>
+#include <utility>
 
 #include "../../include/spsattn.h"
 #include "cache_fill.cuh"
 #include "decode.cuh"
 #include "decode_sm100.cuh"
+#include "decoder_step.cuh"
 #include "kv_update.cuh"
 #include "model_glue.cuh"
 #include "prefill_aux.cuh"
@@ -114,6 +116,34 @@ int encode_kv_map(CUtensorMap* tm, const void* ptr, int B, int H, int N, int D, 
 
 bool strides_ok(Strides st, int D) {
   return st.n >= D && st.h >= D && st.b >= D && (st.n % 8) == 0 && (st.h % 8) == 0 && (st.b % 8) == 0;
+}
+
+// A launch that may start while the kernel before it in the stream is still running; the kernel waits
+// (grid_dependency_wait) before it touches anything that one writes.
+template <typename... P, typename... A>
+int launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
+int multiprocessors() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+  static std::atomic<int> cached[64];
+  if (dev < 64 && cached[dev].load() > 0) return cached[dev].load();
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+  if (dev < 64) cached[dev].store(sms);
+  return sms;
 }
 
 template <int D, bool FP16>
@@ -236,9 +266,8 @@ static long long decode_max_rows(const spsattn_segment* segs, int n_segments) {
 template <int D, int NQ, bool FP16>
 static int launch_decode(const DecodeParams& prm, cudaStream_t st) {
   dim3 grid((unsigned)(prm.S * prm.H), (unsigned)prm.n_chunks);
-  decode_split_kernel<D, NQ, FP16><<<grid, kDecodeThreads, 0, st>>>(prm);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess || prm.tickets != nullptr) return (int)e;   // with tickets the last block merges
+  const int rc = launch_dependent(decode_split_kernel<D, NQ, FP16>, grid, dim3(kDecodeThreads), 0, st, prm);
+  if (rc != 0 || prm.tickets != nullptr) return rc;                // with tickets the last block merges
   decode_merge_kernel<D, NQ, FP16><<<(unsigned)(prm.S * prm.H), D, 0, st>>>(prm);
   return (int)cudaGetLastError();
 }
@@ -334,8 +363,7 @@ int launch_decode_tc(const DecodeMaps& maps, const DecodeParams& prm, cudaStream
   for (int x = 0; x < kMaxSegments; ++x) blocks_y += prm.seg_chunks[x];
   if (blocks_y < 1) blocks_y = 1;
   dim3 grid((unsigned)(prm.S * prm.H), (unsigned)blocks_y);
-  decode_tc_kernel<D, NQ, FP16><<<grid, kTcThreads, Cfg::kSmemBytes, st>>>(maps, prm);
-  return (int)cudaGetLastError();
+  return launch_dependent(decode_tc_kernel<D, NQ, FP16>, grid, dim3(kTcThreads), Cfg::kSmemBytes, st, maps, prm);
 }
 
 template <int D>
@@ -1122,6 +1150,213 @@ int spsattn_swiglu(const void* gate_up, void* y, int dtype, long long rows, int 
   else
     swiglu_kernel<false><<<(unsigned)blocks, 256, 0, st>>>(p);
   return (int)cudaGetLastError();
+}
+
+}  // extern "C"
+
+// ------------------------------------------------------------------------- decode step of a decoder
+
+namespace {
+
+template <int EPI>
+int launch_skinny(SkinnyParams p, cudaStream_t st) {
+  constexpr bool kNorm = EPI != kSkinnyResidual;
+  const int sms = multiprocessors(), tiles = (p.F + 7) / 8;
+  // Multiplying warps per block: one round for everybody if 12 warps suffice, else the number that
+  // leaves least of the last round empty.
+  p.warps = (tiles + sms - 1) / sms;
+  if (p.warps > kSkinnyMaxWarps) {
+    int best = 0;
+    for (int w = 4; w <= kSkinnyMaxWarps; ++w) {
+      const int work = w * ((tiles + sms * w - 1) / (sms * w));
+      if (best == 0 || work <= best) best = work, p.warps = w;
+    }
+  }
+  const int per_block = (tiles + p.warps - 1) / p.warps, blocks = per_block < sms ? per_block : sms;
+  const int rounds = (per_block + blocks - 1) / blocks;
+  // Ring: the widest pieces of rows that still give three stages, or all of a block's weights at once
+  // (a stage costs about 270 clocks of waiting beside its products: 2048 x 768 took 7.2 us in pieces
+  // of 256 columns, 4.8 in pieces of 1024).  Small rings leave room for a block of the next launch.
+  const int fixed = kNorm ? p.rows * skinny_pitch(p.K) : 0;
+  int ring = 190 * 1024 - fixed;
+  for (p.kc = 1024;; p.kc /= 2) {
+    const int stage = (p.warps * skinny_tile_rows(EPI) + (kNorm ? 0 : p.rows)) * skinny_pitch(p.kc);
+    const int loads = rounds * ((p.K + p.kc - 1) / p.kc);
+    p.stages = ring / stage;
+    if (p.stages > kSkinnyMaxStages) p.stages = kSkinnyMaxStages;
+    if (p.stages > loads) p.stages = loads;
+    if (p.stages >= 3 || p.stages == loads || p.kc == 64) {
+      if (p.stages < 1) return SPSATTN_ERR_TOO_LARGE;
+      ring = p.stages * stage;
+      break;
+    }
+  }
+  const int busy = 32 * p.warps + kSkinnyLoaders, threads = busy < kSkinnyMinThreads ? kSkinnyMinThreads : busy;
+  auto* kernel = p.rows <= 8 ? skinny_gemm_kernel<EPI, 1> : skinny_gemm_kernel<EPI, 2>;
+  static std::once_flag once;
+  static cudaError_t attr_err = cudaSuccess;
+  std::call_once(once, [] {
+    attr_err = cudaFuncSetAttribute(skinny_gemm_kernel<EPI, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (attr_err == cudaSuccess)
+      attr_err = cudaFuncSetAttribute(skinny_gemm_kernel<EPI, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  });
+  if (attr_err != cudaSuccess) return (int)attr_err;
+  return launch_dependent(kernel, dim3((unsigned)blocks), dim3((unsigned)threads), (size_t)(ring + fixed), st, p);
+}
+
+int launch_token_start(const spsattn_decoder* d, const spsattn_token_source* src, bool choose_only, int* status,
+                       cudaStream_t st) {
+  if (!d || !src || d->batch <= 0 || d->vocab <= 0) return SPSATTN_ERR_ARG;
+  if (!src->logits && (choose_only || !src->token_in || !src->active_in)) return SPSATTN_ERR_ARG;
+  if (src->logits && (!src->generated || !src->step || !src->finished)) return SPSATTN_ERR_ARG;
+  if (d->param_dtype != SPSATTN_DTYPE_BF16 && d->param_dtype != SPSATTN_DTYPE_FP32) return SPSATTN_ERR_ARG;
+  const bool f32 = d->param_dtype == SPSATTN_DTYPE_FP32;
+  if (src->logits && !aligned16(src->logits)) return SPSATTN_ERR_ALIGN;
+  TokenStartParams p;
+  memset(&p, 0, sizeof(p));
+  p.logits = src->logits;
+  p.suppressed = src->suppressed;
+  p.generated = src->generated;
+  p.step = src->step;
+  p.finished = src->finished;
+  p.max_new = src->max_new;
+  p.stop_on_eos = src->stop_on_eos;
+  p.choose_only = choose_only;
+  p.token_in = src->token_in;
+  p.active_in = src->active_in;
+  p.batch = d->batch;
+  p.vocab = d->vocab;
+  p.eos = d->eos;
+  p.pad = d->pad;
+  if (!choose_only) {
+    if (!d->processed || !d->next_doc_start || !d->nw_len || !d->nw_pos || !d->br_len || !d->active || !d->pos ||
+        !d->wte || !d->x || d->n_layer <= 0 || d->n_head <= 0 || d->hidden <= 0 || d->slots < 1 || d->slots > 2)
+      return SPSATTN_ERR_ARG;
+    if (d->hidden % (f32 ? 4 : 8) || !aligned16(d->wte) || !aligned16(d->x)) return SPSATTN_ERR_ALIGN;
+    p.processed = d->processed;
+    p.next_doc_start = d->next_doc_start;
+    p.nw_len = d->nw_len;
+    p.nw_pos = d->nw_pos;
+    p.br_len = d->br_len;
+    p.layers = d->n_layer;
+    p.heads = d->n_head;
+    p.predict = d->predict;
+    p.active = d->active;
+    p.pos = d->pos;
+    p.freqs = reinterpret_cast<const float2*>(d->freqs);
+    p.freqs_out = reinterpret_cast<float2*>(d->freqs_out);
+    p.half_dim = d->head_dim / 2;
+    p.wte = d->wte;
+    p.x = d->x;
+    p.ssq = d->ssq;
+    p.slots = d->slots;
+    p.C = d->hidden;
+    p.status = status;
+  }
+  return f32 ? launch_dependent(token_start_kernel<true>, dim3((unsigned)d->batch), dim3(kStartThreads), 0, st, p)
+             : launch_dependent(token_start_kernel<false>, dim3((unsigned)d->batch), dim3(kStartThreads), 0, st, p);
+}
+
+}  // namespace
+
+extern "C" {
+
+int spsattn_decoder_start(const spsattn_decoder* d, const spsattn_token_source* source, int* device_status,
+                          void* stream) {
+  return launch_token_start(d, source, false, device_status, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int spsattn_decoder_choose(const spsattn_decoder* d, const spsattn_token_source* source, void* stream) {
+  return launch_token_start(d, source, true, nullptr, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int spsattn_decoder_step_supported(const spsattn_decoder* d) {
+  if (!d || d->param_dtype != SPSATTN_DTYPE_BF16 || d->batch <= 0 || d->n_layer <= 0) return 0;
+  if ((d->slots != 1 && d->slots != 2) || d->n_head <= 0 || d->vocab <= 0) return 0;
+  if (d->hidden != d->n_head * d->head_dim || d->batch * d->slots > kSkinnyMaxRows) return 0;
+  // the norm's sums are those of a row of at most 256 vectors
+  return d->hidden % 16 == 0 && d->hidden <= kSkinnyMaxCols && d->intermediate > 0 && d->intermediate % 16 == 0 ? 1 : 0;
+}
+
+int spsattn_decoder_step(const spsattn_decoder* d, const spsattn_token_source* source, void* logits_out,
+                         int* device_status, void* stream) {
+  if (!spsattn_decoder_step_supported(d) || !logits_out || !d->layers || !d->ssq) return SPSATTN_ERR_ARG;
+  if (d->n_segments < 1 || d->n_segments > 2) return SPSATTN_ERR_ARG;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  int rc = launch_token_start(d, source, false, device_status, st);
+  if (rc != 0) return rc;
+  const int C = d->hidden, I = d->intermediate, rows = d->batch * d->slots;
+  // every slot sees the step's input row, only the <predict> slot its own (decode_attention.py:354-361)
+  spsattn_extra extras[2];
+  memset(extras, 0, sizeof(extras));
+  for (int s = 0; s < d->slots; ++s) {
+    extras[s].k = reinterpret_cast<const uint16_t*>(d->k2) + (size_t)s * d->batch * C;
+    extras[s].v = reinterpret_cast<const uint16_t*>(d->v2) + (size_t)s * d->batch * C;
+    extras[s].query_mask = s == 0 ? (1u << d->slots) - 1 : 2u;
+  }
+  SkinnyParams base;
+  memset(&base, 0, sizeof(base));
+  base.rows = rows;
+  base.eps = d->norm_eps;
+  base.status = device_status;
+  base.ssq = d->ssq;
+  base.ssq_out = d->ssq;
+  base.ssq_stride = C / 8;
+  base.x = reinterpret_cast<const uint16_t*>(d->x);
+  base.x_stride = C;
+  base.K = C;
+  for (int layer = 0; layer < d->n_layer; ++layer) {
+    const spsattn_decoder_layer& w = d->layers[layer];
+    SkinnyParams p = base;
+    p.w = reinterpret_cast<const uint16_t*>(w.c_attn);
+    p.F = 3 * C;
+    p.norm_w = reinterpret_cast<const uint16_t*>(w.attn_norm);
+    p.q = reinterpret_cast<uint16_t*>(d->q);
+    p.k = reinterpret_cast<uint16_t*>(d->k2);
+    p.v = reinterpret_cast<uint16_t*>(d->v2);
+    p.freqs = reinterpret_cast<const float2*>(d->freqs);
+    p.pos = d->pos;
+    p.slots = d->slots;
+    p.batch = d->batch;
+    p.head_dim = d->head_dim;
+    if ((rc = launch_skinny<kSkinnyQkv>(p, st)) != 0) return rc;
+    rc = spsattn_decode_step(d->q, d->slots, d->y, SPSATTN_DTYPE_BF16, w.segments, d->n_segments, extras, d->slots,
+                             &w.append, d->batch, d->n_head, d->head_dim, SPSATTN_DTYPE_BF16,
+                             1.0f / sqrtf((float)d->head_dim), d->workspace, d->workspace_bytes, device_status, stream);
+    if (rc != 0) return rc;
+    p = base;
+    p.w = reinterpret_cast<const uint16_t*>(w.c_proj);
+    p.x = reinterpret_cast<const uint16_t*>(d->y);
+    p.F = C;
+    p.out = reinterpret_cast<uint16_t*>(d->x);
+    if ((rc = launch_skinny<kSkinnyResidual>(p, st)) != 0) return rc;
+    p = base;
+    p.w = reinterpret_cast<const uint16_t*>(w.gate_up);
+    p.F = I;
+    p.norm_w = reinterpret_cast<const uint16_t*>(w.mlp_norm);
+    p.out = reinterpret_cast<uint16_t*>(d->mlp_hidden);
+    if ((rc = launch_skinny<kSkinnySwiglu>(p, st)) != 0) return rc;
+    p = base;
+    p.w = reinterpret_cast<const uint16_t*>(w.down);
+    p.x = reinterpret_cast<const uint16_t*>(d->mlp_hidden);
+    p.x_stride = I;
+    p.K = I;
+    p.F = C;
+    p.out = reinterpret_cast<uint16_t*>(d->x);
+    if ((rc = launch_skinny<kSkinnyResidual>(p, st)) != 0) return rc;
+  }
+  SkinnyParams p = base;
+  p.rows = d->batch;
+  p.w = reinterpret_cast<const uint16_t*>(d->lm_head);
+  p.x = base.x + (size_t)d->pred_slot * C;
+  p.x_stride = (int64_t)d->slots * C;
+  p.F = d->vocab;
+  p.norm_w = reinterpret_cast<const uint16_t*>(d->out_norm);
+  p.ssq = base.ssq + (size_t)d->pred_slot * (C / 8);
+  p.ssq_stride = (int64_t)d->slots * (C / 8);
+  p.out = reinterpret_cast<uint16_t*>(logits_out);
+  p.active = d->active;
+  return launch_skinny<kSkinnyLogits>(p, st);
 }
 
 }  // extern "C"

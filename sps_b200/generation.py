@@ -373,11 +373,8 @@ class SPSGenerator:
         s = type("StepBuffers", (), {})()
         s.state = state
         s.b = b
-        s.token = torch.zeros(b, device=dev, dtype=torch.long)
-        s.active = torch.zeros(b, device=dev, dtype=torch.bool)
         s.active_i8 = torch.zeros(b, device=dev, dtype=torch.int8)
         ns, wt = self.n_slot, self.window_tokens
-        s.idx_pair = torch.full((b, ns), max(d.predict_token_id, 0), device=dev, dtype=torch.long)
         s.pos = torch.zeros(b, device=dev, dtype=torch.long)
         s.fc = torch.zeros((b, hd // 2, 2), device=dev, dtype=torch.float32)
         s.x = torch.zeros((ns * b, c), device=dev, dtype=pdt)
@@ -391,8 +388,6 @@ class SPSGenerator:
         s.y_param = s.y if pdt == self.attn_dtype else torch.zeros((ns * b, c), device=dev, dtype=pdt)
         s.gate_up = torch.zeros((ns * b, 2 * inter), device=dev, dtype=pdt)
         s.hidden = torch.zeros((ns * b, inter), device=dev, dtype=pdt)
-        s.logits = torch.zeros((b, d.vocab_size), device=dev, dtype=pdt)
-        s.zero_tok = torch.zeros(b, device=dev, dtype=torch.long)
         # the [B, ns, 3C] projection seen as one row per sequence with 3 * ns head groups:
         # slot 0 q, k, v (, slot 1 q, k, v)
         groups = (_lib.RopeGroup * (3 * ns))()
@@ -449,24 +444,52 @@ class SPSGenerator:
             ws_bytes = max(ws_bytes, self.lib.spsattn_decode_step_workspace_bytes(b, h, hd, ns, segs, n_seg))
         s.ws = torch.zeros(ws_bytes, device=dev, dtype=torch.uint8)
         s.ws_bytes = ws_bytes
+        s.decoder = self._bind_decoder(s)
+        s.fused = bool(self.lib.spsattn_decoder_step_supported(C.byref(s.decoder)))
         self._step = s
 
-    def _step_body(self) -> None:
-        """One token for every row: reads ``token`` / ``active`` of the bound buffers, leaves the
-        prediction logits in ``logits`` and the caches and counters advanced.  No host sync."""
-        s, d, st = self._step, self.dims, self._step.state
+    def _bind_decoder(self, s) -> _lib.Decoder:
+        """The argument block of ``spsattn_decoder_start`` / ``_choose`` / ``_step`` for the bound buffers."""
+        d, st, w = self.dims, s.state, self.w
+        s.ssq = torch.zeros((s.x.shape[0], max(1, d.hidden_size // 8)), device=self.device, dtype=torch.float32)
+        s.layers = (_lib.DecoderLayer * d.n_layer)()
+        for layer, (segs, n_seg, _extras, ap) in enumerate(s.layer_args):
+            la = s.layers[layer]
+            la.attn_norm, la.c_attn, la.c_proj = (x[layer].data_ptr() for x in (w.attn_norm, w.c_attn, w.c_proj))
+            la.mlp_norm, la.gate_up, la.down = (x[layer].data_ptr() for x in (w.mlp_norm, w.gate_up, w.down))
+            for i in range(n_seg):
+                la.segments[i] = segs[i]
+            la.append = ap
+        dec = _lib.Decoder()
+        dec.n_layer, dec.batch, dec.slots, dec.n_head = d.n_layer, s.b, self.n_slot, d.n_head
+        dec.head_dim, dec.hidden, dec.intermediate = d.head_dim, d.hidden_size, d.intermediate_size
+        dec.vocab, dec.pred_slot, dec.n_segments = d.vocab_size, self.pred_slot, s.layer_args[0][1]
+        dec.param_dtype, dec.norm_eps = self.glue_dtype, float(d.norm_eps)
+        dec.eos, dec.pad, dec.predict = d.eos_token_id, d.pad_token_id, max(d.predict_token_id, 0)
+        dec.layers = s.layers
+        for name, x in (("wte", w.wte), ("lm_head", w.lm_head), ("out_norm", w.out_norm), ("freqs", self.freqs),
+                        ("processed", st.processed_tokens), ("next_doc_start", st.next_doc_start),
+                        ("nw_len", st.nw_len), ("nw_pos", st.nw_pos), ("br_len", st.br_len), ("active", s.active_i8),
+                        ("pos", s.pos), ("freqs_out", s.fc), ("x", s.x), ("q", s.q), ("k2", s.k2), ("v2", s.v2),
+                        ("y", s.y), ("mlp_hidden", s.hidden), ("ssq", s.ssq), ("workspace", s.ws)):
+            setattr(dec, name, x.data_ptr())
+        dec.workspace_bytes = s.ws_bytes
+        return dec
+
+    def _step_body(self, source, logits: Tensor) -> None:
+        """One token for every row, from ``source``: leaves the prediction logits in ``logits`` (zeros
+        for inactive rows when the projections are the library's own) and the caches and counters
+        advanced (reverse_sps/inference.py:391-503).  No host sync."""
+        s, d = self._step, self.dims
         b, c, h, hd, ns = s.b, d.hidden_size, d.n_head, d.head_dim, self.n_slot
         stream = self._stream()
-        torch.where(s.active, s.token, s.zero_tok, out=s.idx_pair[:, 0])     # inference.py:391-398
-        torch.where(s.active, st.processed_tokens, s.zero_tok, out=s.pos)    # :399-403
-        s.active_i8.copy_(s.active)
-        torch.index_select(self.freqs, 0, s.pos, out=s.fc)
-        # a row that starts a document forgets its caches, in every layer (:113-122, :408-409)
-        reset = st.next_doc_start & s.active
-        st.nw_len.masked_fill_(reset.unsqueeze(0), 0)
-        st.nw_pos.masked_fill_(reset.unsqueeze(0), 0)
-        st.br_len.masked_fill_(reset.view(1, b, 1), 0)
-        torch.index_select(self.w.wte, 0, s.idx_pair.view(-1), out=s.x)
+        if s.fused:
+            rc = self.lib.spsattn_decoder_step(C.byref(s.decoder), C.byref(source), logits.data_ptr(),
+                                               _status(self.device).data_ptr(), stream)
+            _lib.check(rc, "spsattn_decoder_step")
+            return
+        rc = self.lib.spsattn_decoder_start(C.byref(s.decoder), C.byref(source), _status(self.device).data_ptr(), stream)
+        _lib.check(rc, "spsattn_decoder_start")
         self._add_rmsnorm(s.x, None, self.w.attn_norm[0], s.xn)
         scale = 1.0 / math.sqrt(hd)
         for layer in range(d.n_layer):
@@ -489,10 +512,7 @@ class SPSGenerator:
             nxt = self.w.attn_norm[layer + 1] if layer + 1 < d.n_layer else self.w.out_norm
             self._add_rmsnorm(s.x, s.delta, nxt, s.xn)
         pred = s.xn.view(b, ns, c)[:, self.pred_slot]
-        torch.mm(pred, self.w.lm_head.t(), out=s.logits)
-        # _advance_decode_state (:487-503)
-        st.processed_tokens.add_(s.active.to(torch.long))
-        torch.where(s.active, s.token == d.eos_token_id, st.next_doc_start, out=st.next_doc_start)
+        torch.mm(pred, self.w.lm_head.t(), out=logits)
 
     @torch.no_grad()
     def decode_one_token(self, state: DecodeState, token_B: Tensor, active_B: Tensor) -> Tensor:
@@ -509,10 +529,18 @@ class SPSGenerator:
         if self._step is None or self._step.state is not state:
             self._bind_step(state)
         s = self._step
-        s.token.copy_(token_B.to(self.device))
-        s.active.copy_(active_B.to(self.device, torch.bool))
-        self._step_body()
-        return torch.where(s.active.unsqueeze(1), s.logits, torch.zeros_like(s.logits))
+        token = token_B.to(self.device, torch.long).contiguous()
+        active = active_B.to(self.device, torch.bool).contiguous()
+        if token.shape != (s.b,) or active.shape != (s.b,):
+            raise ValueError(f"token and active must have shape {(s.b,)}")
+        source = _lib.TokenSource()
+        source.token_in, source.active_in = token.data_ptr(), active.data_ptr()
+        logits = torch.empty((s.b, self.dims.vocab_size), device=self.device, dtype=self.param_dtype)
+        with torch.cuda.device(self.device):
+            self._step_body(source, logits)
+        if not s.fused:
+            logits.masked_fill_(~active.unsqueeze(1), 0)
+        return logits
 
     # ------------------------------------------------------------------ generation
     @torch.no_grad()
@@ -552,10 +580,6 @@ class SPSGenerator:
         # them, and they are bound again if a decode_one_token on another state replaced them
         self._step = g.step
         s = self._step
-        g.next_logits.copy_(next_logits)
-        g.generated.fill_(d.pad_token_id)
-        g.finished.fill_(False)
-        g.step_idx.zero_()
         n_steps = max_new_tokens - 1          # the last token is sampled without a further decode
         if n_steps > 0 and use_graph and g.graph is None:
             # warm-up with every row marked finished: the chain runs, nothing is sampled or stored
@@ -566,11 +590,13 @@ class SPSGenerator:
                 for _ in range(2):
                     self._token_body(g)
             torch.cuda.current_stream(self.device).wait_stream(side)
-            g.finished.fill_(False)
-            g.step_idx.zero_()
             g.graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g.graph):          # capture records, it does not execute
                 self._token_body(g)
+        g.next_logits.copy_(next_logits)
+        g.generated.fill_(d.pad_token_id)
+        g.finished.fill_(False)
+        g.step_idx.zero_()
         ev[2].record()
         for _ in range(n_steps):
             if use_graph:
@@ -578,7 +604,9 @@ class SPSGenerator:
             else:
                 self._token_body(g)
         ev[3].record()
-        self._sample(g)
+        with torch.cuda.device(self.device):
+            _lib.check(self.lib.spsattn_decoder_choose(C.byref(s.decoder), C.byref(g.source), self._stream()),
+                       "spsattn_decoder_choose")
         ev[4].record()
         state.host_tokens += n_steps
         if timings is not None:
@@ -598,37 +626,28 @@ class SPSGenerator:
         g = type("GenerationSession", (), {})()
         g.state, g.key, g.graph = state, key, None
         g.step = self._step
-        g.stop_on_eos = key[3]
-        g.suppressed = torch.tensor(list(key[4]), device=dev, dtype=torch.long)
         g.generated = torch.full((b, max_new), d.pad_token_id, device=dev, dtype=torch.long)
         g.finished = torch.zeros(b, device=dev, dtype=torch.bool)
-        g.step_idx = torch.zeros((1, 1), device=dev, dtype=torch.long)
-        g.pad_tok = torch.full((b,), d.pad_token_id, device=dev, dtype=torch.long)
+        g.step_idx = torch.zeros(b, device=dev, dtype=torch.long)
         g.next_logits = torch.zeros((b, d.vocab_size), device=dev, dtype=self.param_dtype)
+        words = torch.zeros((d.vocab_size + 31) // 32, dtype=torch.long)      # suppressed ids, a bit each
+        ids = torch.tensor(key[4], dtype=torch.long)
+        words.index_add_(0, ids >> 5, torch.ones_like(ids) << (ids & 31))
+        g.suppressed = torch.where(words >= 1 << 31, words - (1 << 32), words).to(torch.int32).to(dev)
+        src = g.source = _lib.TokenSource()
+        src.logits, src.suppressed = g.next_logits.data_ptr(), g.suppressed.data_ptr()
+        src.generated, src.step, src.finished = g.generated.data_ptr(), g.step_idx.data_ptr(), g.finished.data_ptr()
+        src.max_new, src.stop_on_eos = max_new, int(key[3])
         self._session = g
         return g
 
-    def _sample(self, g):
-        """utils/generation.py:171-181 with greedy sampling (utils/sampling.py:55-83)."""
-        live = ~g.finished
-        z = g.next_logits.float()
-        z.index_fill_(1, g.suppressed, float("-inf"))
-        tok = torch.where(live, z.argmax(dim=-1), g.pad_tok)
-        g.generated.scatter_(1, g.step_idx.expand(tok.shape[0], 1), tok.view(-1, 1))
-        newly = live & (tok == self.dims.eos_token_id) if g.stop_on_eos else torch.zeros_like(live)
-        return tok, live & ~newly, newly
-
     def _token_body(self, g) -> None:
-        """Sample one token per row, run the decode step on it, keep its logits for the next
-        (utils/generation.py:171-195); reads and writes only buffers of the session."""
-        s = self._step
-        tok, decode_active, newly = self._sample(g)
-        s.token.copy_(tok)
-        s.active.copy_(decode_active)
-        self._step_body()
-        torch.where(decode_active.unsqueeze(1), s.logits, g.next_logits, out=g.next_logits)
-        g.finished.logical_or_(newly)
-        g.step_idx.add_(1)
+        """Choose one token per row from the logits of the step before (utils/generation.py:171-181 with
+        greedy sampling, utils/sampling.py:55-83: first maximum, pad once a row has finished), run the
+        decode step on it and keep its logits for the next (:182-195); reads and writes only buffers
+        of the session."""
+        with torch.cuda.device(self.device):
+            self._step_body(g.source, g.next_logits)
 
 
 def generator_for(model, *, param_dtype: Optional[torch.dtype] = None) -> SPSGenerator:

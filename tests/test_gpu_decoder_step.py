@@ -1,0 +1,86 @@
+"""The fused decode step (spsattn_decoder_step) against the step made of library GEMMs and single
+kernels, at the edges of its tiles, stages and row counts; the greedy choice on the device."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _engine(variant, layers, heads, hidden, inter, vocab, seed=3):
+    import sps_b200
+    from sps_b200.generation import random_state_dict
+    dims = sps_b200.SPSDims(block_size=64, vocab_size=vocab, n_layer=layers, n_head=heads, hidden_size=hidden,
+                            intermediate_size=inter, eos_token_id=vocab - 3, pad_token_id=vocab - 1,
+                            predict_token_id=vocab - 2, window_size=5)
+    return sps_b200.SPSGenerator(random_state_dict(dims, seed=seed), dims, variant=variant), dims
+
+
+@pytest.mark.parametrize("variant,batch,heads,hidden,inter,vocab", [
+    ("standard", 1, 1, 64, 16, 33),           # one row, odd vocabulary, less than one stage
+    ("sps", 4, 2, 128, 80, 200),              # remainder of four steps of 16 columns
+    ("reverse_sps", 5, 3, 192, 1040, 1001),   # ten rows: two row tiles; a second stage of 16 columns
+    ("delayed_state", 8, 16, 1024, 2816, 2048),
+    ("standard", 16, 16, 2048, 8192, 50304),  # the widest rows, several rounds of the head
+    ("sps", 8, 16, 2048, 8192, 9473),
+])
+def test_fused_step_matches_the_separate_kernels(variant, batch, heads, hidden, inter, vocab):
+    import sps_b200
+    engine, dims = _engine(variant, 2, heads, hidden, inter, vocab)
+    g = torch.Generator().manual_seed(7)
+    prompt = torch.randint(0, vocab - 3, (batch, 9), generator=g)
+    tokens = torch.randint(0, vocab - 3, (3, batch), generator=g)
+    tokens[1, 0] = dims.eos_token_id                       # row 0 starts a new document in the third step
+    active = torch.ones(batch, dtype=torch.bool)
+    active[batch // 2] = batch == 1
+    outs, states = [], []
+    for fused in (True, False):
+        state, _ = engine.prefill(prompt, 8)
+        engine._bind_step(state)
+        assert engine._step.fused
+        engine._step.fused = fused
+        outs.append([engine.decode_one_token(state, t, active).float() for t in tokens])
+        states.append(state)
+    sps_b200.check_device_status()
+    for a, b in zip(*outs):
+        # both round every projection to bf16; where their fp32 sums round differently at all, a value
+        # moves by one unit of the last place (2^-8), and the logits by a fraction of their norm
+        assert float((a - b).norm()) <= 2.0 ** -6 * float(b.norm())
+        assert bool((a[~active] == 0).all())
+    for name in ("br_len", "nw_len", "nw_pos", "processed_tokens", "next_doc_start"):
+        assert torch.equal(getattr(states[0], name), getattr(states[1], name)), name
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("vocab", [7, 64, 1003, 50304])
+def test_greedy_choice_is_the_first_unsuppressed_maximum(dtype, vocab):
+    import ctypes as C
+    from sps_b200 import _lib
+    lib, dev, batch, new = _lib.load(), torch.device("cuda"), 6, 2
+    g = torch.Generator().manual_seed(vocab)
+    z = torch.randint(-3, 4, (batch, vocab), generator=g).to(dtype)              # many ties
+    z[1] = float("-inf")
+    z[2, vocab // 2] = float("nan")
+    z[3] = 0.0
+    z[3, 0] = -0.0
+    hidden = torch.randperm(vocab, generator=g)[: vocab // 3]
+    ref = z.float().clone()
+    ref[:, hidden] = float("-inf")
+    want = torch.stack([torch.argmax(r) for r in ref])
+    want[5] = vocab - 1                                                           # finished: pad
+    words = torch.zeros((vocab + 31) // 32, dtype=torch.long)
+    words.index_add_(0, hidden >> 5, torch.ones_like(hidden) << (hidden & 31))
+    words = torch.where(words >= 1 << 31, words - (1 << 32), words).to(torch.int32).to(dev)
+    zd = z.to(dev)
+    out = torch.full((batch, new), -1, dtype=torch.long, device=dev)
+    step = torch.ones(batch, dtype=torch.long, device=dev)
+    finished = torch.tensor([0, 0, 0, 0, 0, 1], dtype=torch.uint8, device=dev)
+    d, s = _lib.Decoder(), _lib.TokenSource()
+    d.batch, d.vocab, d.pad, d.eos = batch, vocab, vocab - 1, vocab - 2
+    d.param_dtype = _lib.DTYPE_BF16 if dtype == torch.bfloat16 else _lib.DTYPE_FP32
+    s.logits, s.suppressed, s.generated = zd.data_ptr(), words.data_ptr(), out.data_ptr()
+    s.step, s.finished, s.max_new, s.stop_on_eos = step.data_ptr(), finished.data_ptr(), new, 1
+    _lib.check(lib.spsattn_decoder_choose(C.byref(d), C.byref(s), torch.cuda.current_stream().cuda_stream), "choose")
+    keep = [i for i in range(batch) if not (i == 2 and vocab // 2 in hidden)]     # a hidden NaN counts as hidden
+    assert torch.equal(out[keep, 1].cpu(), want[keep])
+    assert bool((out[:, 0] == -1).all())

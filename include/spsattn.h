@@ -298,7 +298,8 @@ int spsattn_decode_step_tickets(const void* q, int nq, void* out, int out_dtype,
  * head_dim is 64 or 128, no segment is packed through seq_offset and there are at least 444
  * (sequence, head, long segment) triples, else the CUDA-core kernel),
  * 1 = always the CUDA-core kernel, 2 = the tensor-core kernel (head_dim 64 or 128, no packed
- * segment) or SPSATTN_ERR_ARG.  Process-wide. */
+ * segment) or SPSATTN_ERR_ARG, 3 = the CUDA-core kernel with one block per (sequence, head)
+ * (head_dim up to 128, at most 8 chunks) or SPSATTN_ERR_ARG.  Process-wide. */
 int spsattn_debug_decode_path(int path);
 
 /* Test hook: which tensor-core prefill kernel serves head_dim 64.  0 = automatic (today the

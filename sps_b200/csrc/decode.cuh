@@ -67,6 +67,7 @@ struct DecodeParams {
   // segment after segment, then one slot for the current-token entries.
   int seg_chunks[kMaxSegments];   // 0 for the short segments of small_segs
   int extras_slot;     // slot of the current-token entries and the short segments, -1 when none
+  int pair;            // one block per (sequence, head): decode_pair_kernel
   uint32_t small_segs; // bit x: segment x is short and handled with the entries, on the CUDA cores
   int* status;         // bounded-wait failures are reported here (may be null)
   DecodeAppend app;
@@ -515,6 +516,345 @@ decode_split_kernel(const DecodeParams prm) {
   for (int x = 0; x < kMaxSegments; ++x) seg_live[x] = seg_start[x + 1] - seg_start[x];
   decode_finish<D, NQ, FP16, false>(prm, sh, s, h, n_total, seg_live, ring_len, ring_pos, ret_len, !dead,
                                     tid, kDecodeThreads);
+}
+
+// ---------------------------------------------------------------------------------------------
+// The same attention with one block per (sequence, head), for few pairs with short caches, where a
+// launch is bound by latency: a pair's chunks are taken by groups of 128 threads of one block and
+// merged in its shared memory, so no record goes through global memory and no ticket is waited for
+// (about 3 us), the queries and current-token entries are asked for first, every batch of rows is
+// asked for while the one before it is worked on, and the rows are on their way to L2 before the
+// launch that produces the queries has ended.  Chunks, batches and sums are those of
+// decode_split_kernel, so the results are the same bits.
+constexpr int kPairMaxChunks = 8;
+constexpr int kPairMaxGroups = 4;
+
+template <int D, int NQ>
+struct PairScratch {
+  float m[4][NQ], l[4][NQ], acc[4][NQ][D];
+};
+
+__device__ __forceinline__ int live_rows_now(const DecodeSeg& sg, int s, int h, int H) {
+  long long len = __ldcg(sg.lengths + (sg.lengths_per_head ? (size_t)s * H + h : (size_t)s));
+  if (len < 0) len = 0;
+  return len < sg.max_rows ? (int)len : sg.max_rows;
+}
+
+template <int D, int NQ, bool FP16>
+__device__ __forceinline__ void pair_chunk(const DecodeParams& prm, int s, int h, int sh,
+                                           const int (&seg_start)[kMaxSegments + 1], int c_lo, int c_hi,
+                                           bool with_extras, float* rec, int tid, PairScratch<D, NQ>& scratch, int bar_id) {
+  constexpr int LPR = D / 8;          // lanes per row
+  constexpr int RPI = 32 / LPR;       // rows per warp load instruction
+  constexpr int U = kDecodeUnroll;
+  constexpr int STEP = 4 * RPI * U;   // rows per step of the group
+  const int warp = tid >> 5, lane = tid & 31;
+  const int g = lane / LPR;           // row inside a load instruction
+  const int dl = (lane % LPR) * 8;    // first of this lane's 8 dims
+  uint4 q_raw[NQ], ek[kMaxExtras], ev[kMaxExtras];
+#pragma unroll
+  for (int qi = 0; qi < NQ; ++qi)
+    q_raw[qi] = __ldcg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(prm.q) +
+                                                      (((size_t)s * NQ + qi) * prm.H + h) * D + dl));
+  const bool extras = with_extras && warp == 0;
+#pragma unroll
+  for (int e = 0; e < kMaxExtras; ++e) {
+    ek[e] = ev[e] = make_uint4(0, 0, 0, 0);
+    if (extras && e < prm.n_extras) {
+      ek[e] = __ldcg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(prm.extra_k[e]) + (size_t)sh * D + dl));
+      ev[e] = __ldcg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(prm.extra_v[e]) + (size_t)sh * D + dl));
+    }
+  }
+  // this lane's batches: rows r, r + 4 RPI, ... of segment x, then STEP further on
+  struct Batch {
+    int x, r, hi;
+    int64_t row_stride;
+    uint32_t mask;
+    const uint16_t *kb, *vb;
+  };
+  const int off = warp * RPI + g;
+  auto enter = [&](Batch& b) {        // first batch of segment b.x or a later one
+    const int from = b.x;
+    b.x = kMaxSegments;
+#pragma unroll
+    for (int x = kMaxSegments - 1; x >= 0; --x) {
+      const int lo = max(c_lo, seg_start[x]) - seg_start[x], hi = min(c_hi, seg_start[x + 1]) - seg_start[x];
+      if (x < from || x >= prm.n_segments || lo >= hi) continue;
+      const DecodeSeg& sg = prm.seg[x];
+      const int64_t base = (sg.seq_offset ? sg.seq_offset[s] : (int64_t)s * sg.seq_stride) + (int64_t)h * sg.head_stride + dl;
+      b.x = x;
+      b.hi = hi;
+      b.r = lo + off;
+      b.row_stride = sg.row_stride;
+      b.mask = sg.query_mask;
+      b.kb = reinterpret_cast<const uint16_t*>(sg.k) + base;
+      b.vb = reinterpret_cast<const uint16_t*>(sg.v) + base;
+    }
+  };
+  auto load = [&](const uint16_t* base, const Batch& b, uint4 (&rows)[U]) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int r = b.r + u * (4 * RPI);
+      rows[u] = make_uint4(0, 0, 0, 0);
+      if (r < b.hi) rows[u] = __ldg(reinterpret_cast<const uint4*>(base + (size_t)r * b.row_stride));
+    }
+  };
+  float q[NQ][8], m_run[NQ], l_run[NQ], acc[NQ][8];
+#pragma unroll
+  for (int qi = 0; qi < NQ; ++qi) {
+    m_run[qi] = -1.0e30f;
+    l_run[qi] = 0.f;
+#pragma unroll
+    for (int x = 0; x < 8; ++x) acc[qi][x] = 0.f;
+  }
+  auto unpack8 = [](const uint4& u, float (&f)[8]) {
+    unpack2<FP16>(u.x, f[0], f[1]);
+    unpack2<FP16>(u.y, f[2], f[3]);
+    unpack2<FP16>(u.z, f[4], f[5]);
+    unpack2<FP16>(u.w, f[6], f[7]);
+  };
+  // `ahead` runs between the scores and the sums: the keys are done with there
+  auto compute = [&](const uint4 (&kr)[U], const uint4 (&vr)[U], int r0, int r_hi, uint32_t qmask, auto ahead) {
+    float sc[NQ][U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      float kf[8];
+      unpack8(kr[u], kf);
+#pragma unroll
+      for (int qi = 0; qi < NQ; ++qi) {
+        float d = 0.f;
+#pragma unroll
+        for (int x = 0; x < 8; ++x) d = fmaf(q[qi][x], kf[x], d);
+#pragma unroll
+        for (int o = LPR / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+        sc[qi][u] = (r0 + u * (4 * RPI) < r_hi && ((qmask >> qi) & 1u)) ? d : -INFINITY;
+      }
+    }
+    ahead();
+    float pr[NQ][U];
+#pragma unroll
+    for (int qi = 0; qi < NQ; ++qi) {
+      float mx = m_run[qi];
+#pragma unroll
+      for (int u = 0; u < U; ++u) mx = fmaxf(mx, sc[qi][u]);
+      const float alpha = fast_exp2(m_run[qi] - mx);
+      float sum = 0.f;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        pr[qi][u] = fast_exp2(sc[qi][u] - mx);
+        sum += pr[qi][u];
+      }
+      l_run[qi] = l_run[qi] * alpha + sum;
+      m_run[qi] = mx;
+#pragma unroll
+      for (int x = 0; x < 8; ++x) acc[qi][x] *= alpha;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      float vf[8];
+      unpack8(vr[u], vf);
+#pragma unroll
+      for (int qi = 0; qi < NQ; ++qi)
+#pragma unroll
+        for (int x = 0; x < 8; ++x) acc[qi][x] = fmaf(pr[qi][u], vf[x], acc[qi][x]);
+    }
+  };
+
+  uint4 kr[U], vr[U];
+  Batch cur;
+  cur.x = 0;
+  enter(cur);
+  if (cur.x < kMaxSegments) {
+    load(cur.kb, cur, kr);
+    load(cur.vb, cur, vr);
+  }
+#pragma unroll
+  for (int qi = 0; qi < NQ; ++qi) {
+    // pre-scaled so that scores are in the log2 domain
+    unpack8(q_raw[qi], q[qi]);
+#pragma unroll
+    for (int x = 0; x < 8; ++x) q[qi][x] *= prm.scale_log2;
+  }
+  while (cur.x < kMaxSegments) {
+    Batch next = cur;
+    next.r += STEP;
+    if (next.r - off >= next.hi) {
+      ++next.x;
+      enter(next);
+    }
+    const bool more = next.x < kMaxSegments;
+    compute(kr, vr, cur.r, cur.hi, cur.mask, [&]() {
+      if (more) load(next.kb, next, kr);
+    });
+    if (more) load(next.vb, next, vr);
+    cur = next;
+  }
+  if (extras) {
+    // one row each, in lane group 0, as batches whose other rows are masked
+#pragma unroll
+    for (int e = 0; e < kMaxExtras; ++e) {
+      if (e >= prm.n_extras) break;
+      const uint4 zero = make_uint4(0, 0, 0, 0);
+      const uint4 k4[U] = {g == 0 ? ek[e] : zero, zero, zero, zero}, v4[U] = {g == 0 ? ev[e] : zero, zero, zero, zero};
+      compute(k4, v4, g, 1, prm.extra_mask[e], []() {});
+    }
+  }
+
+  // merge the lane groups of a warp, then the four warps, then write the record
+#pragma unroll
+  for (int qi = 0; qi < NQ; ++qi) {
+#pragma unroll
+    for (int o = LPR; o < 32; o <<= 1) {
+      const float m_o = __shfl_xor_sync(0xffffffffu, m_run[qi], o);
+      const float l_o = __shfl_xor_sync(0xffffffffu, l_run[qi], o);
+      const float mx = fmaxf(m_run[qi], m_o);
+      const float a = fast_exp2(m_run[qi] - mx), bsc = fast_exp2(m_o - mx);
+      l_run[qi] = l_run[qi] * a + l_o * bsc;
+#pragma unroll
+      for (int x = 0; x < 8; ++x) {
+        const float acc_o = __shfl_xor_sync(0xffffffffu, acc[qi][x], o);
+        acc[qi][x] = acc[qi][x] * a + acc_o * bsc;
+      }
+      m_run[qi] = mx;
+    }
+    if (g == 0) {
+      if (lane == 0) {
+        scratch.m[warp][qi] = m_run[qi];
+        scratch.l[warp][qi] = l_run[qi];
+      }
+#pragma unroll
+      for (int x = 0; x < 8; ++x) scratch.acc[warp][qi][dl + x] = acc[qi][x];
+    }
+  }
+  asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "n"(kDecodeThreads) : "memory");
+  for (int idx = tid; idx < NQ * D; idx += kDecodeThreads) {
+    const int qi = idx / D, d = idx % D;
+    float mx = scratch.m[0][qi];
+#pragma unroll
+    for (int v = 1; v < 4; ++v) mx = fmaxf(mx, scratch.m[v][qi]);
+    float a = 0.f, l = 0.f;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const float f = fast_exp2(scratch.m[v][qi] - mx);
+      a += scratch.acc[v][qi][d] * f;
+      l += scratch.l[v][qi] * f;
+    }
+    rec[qi * (D + 2) + 2 + d] = a;
+    if (d == 0) {
+      rec[qi * (D + 2)] = mx;
+      rec[qi * (D + 2) + 1] = l;
+    }
+  }
+}
+
+template <int D, int NQ, bool FP16>
+__global__ void __launch_bounds__(kPairMaxGroups * kDecodeThreads, 1) decode_pair_kernel(const DecodeParams prm) {
+  __shared__ PairScratch<D, NQ> s_scratch[kPairMaxGroups];
+  __shared__ float s_record[kPairMaxChunks][NQ * (D + 2)];
+  const int sh = blockIdx.x;
+  const int s = sh / prm.H, h = sh % prm.H;
+  const int tid = threadIdx.x, group = tid / kDecodeThreads, gt = tid % kDecodeThreads;
+  const int groups = blockDim.x / kDecodeThreads;
+  grid_launch_dependents();
+  // In a decode step nothing before this launch writes these rows (they are those of earlier steps);
+  // the lengths may still be about to be reset, which only makes this ask for rows in vain.
+#pragma unroll
+  for (int x = 0; x < kMaxSegments; ++x) {
+    if (x >= prm.n_segments) break;
+    const DecodeSeg& sg = prm.seg[x];
+    if (sg.seq_offset != nullptr) continue;
+    const int live = live_rows_now(sg, s, h, prm.H);
+    const int64_t base = (int64_t)s * sg.seq_stride + (int64_t)h * sg.head_stride;
+    for (int r = tid; r < live; r += blockDim.x) {
+#pragma unroll
+      for (int e = 0; e < D; e += 64) {        // lines of 128 bytes
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint16_t*>(sg.k) + base + r * sg.row_stride + e));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint16_t*>(sg.v) + base + r * sg.row_stride + e));
+      }
+    }
+  }
+  grid_dependency_wait();
+
+  int seg_start[kMaxSegments + 1];
+  seg_start[0] = 0;
+#pragma unroll
+  for (int x = 0; x < kMaxSegments; ++x)
+    seg_start[x + 1] = seg_start[x] + (x < prm.n_segments ? live_rows_now(prm.seg[x], s, h, prm.H) : 0);
+  const int n_total = seg_start[kMaxSegments];
+  // the counters as they are before this step's update
+  const DecodeAppend& ap = prm.app;
+  long long ring_len = 0, ring_pos = 0, ret_len = 0;
+  bool append = false;
+  if (ap.br_len != nullptr) {
+    append = ap.active[s] != 0;
+    ret_len = __ldcg(ap.br_len + sh);
+    if (ap.window_tokens > 0) {
+      ring_len = __ldcg(ap.nw_len + s);
+      ring_pos = __ldcg(ap.nw_pos + s);
+    }
+  }
+  const int chunks = max(1, (n_total + prm.chunk_rows - 1) / prm.chunk_rows);
+  for (int c = group; c < chunks; c += groups) {
+    // (the record of the group's chunk before is complete: its scratch may be written again)
+    if (c >= groups) asm volatile("bar.sync %0, %1;" ::"r"(2 + group), "n"(kDecodeThreads) : "memory");
+    pair_chunk<D, NQ, FP16>(prm, s, h, sh, seg_start, c * prm.chunk_rows, min((c + 1) * prm.chunk_rows, n_total), c == 0,
+                            s_record[c], gt, s_scratch[group], 2 + group);
+  }
+  __syncthreads();
+  // merge_records on shared memory: one group of eight
+  for (int idx = tid; idx < NQ * D; idx += blockDim.x) {
+    const int qi = idx / D, d = idx % D;
+    float mx = -1.0e30f;
+    for (int j = 0; j < chunks; ++j) mx = fmaxf(mx, s_record[j][qi * (D + 2)]);
+    float l_run = 0.f, a_run = 0.f;
+    for (int j = 0; j < chunks; ++j) {
+      const float* rec = s_record[j] + qi * (D + 2);
+      const float f = fast_exp2(rec[0] - mx);
+      l_run = fmaf(rec[1], f, l_run);
+      a_run = fmaf(rec[2 + d], f, a_run);
+    }
+    const float o = l_run > 0.f ? a_run / l_run : 0.f;
+    const size_t at = (((size_t)s * NQ + qi) * prm.H + h) * D + d;
+    if (prm.out16)
+      reinterpret_cast<uint16_t*>(prm.out)[at] = (uint16_t)(pack2<FP16>(o, 0.f) & 0xffffu);
+    else
+      reinterpret_cast<float*>(prm.out)[at] = o;
+  }
+  if (ap.br_k == nullptr) return;
+  const bool full = ring_len >= ap.window_tokens;
+  if (append) {
+    const long long ins = full ? ring_pos : ring_len;
+    for (int d = tid; d < D; d += blockDim.x) {
+      const size_t src = (size_t)sh * D + d;
+      if (ap.window_tokens > 0 && ins >= 0 && ins < ap.window_storage) {
+        const size_t dst = ((size_t)sh * ap.window_storage + (size_t)ins) * D + d;
+        ap.nw_k[dst] = __ldcg(ap.k_window + src);
+        ap.nw_v[dst] = __ldcg(ap.v_window + src);
+      }
+      if (ret_len >= 0 && ret_len < ap.retained_storage) {
+        const size_t dst = ((size_t)sh * ap.retained_storage + (size_t)ret_len) * D + d;
+        ap.br_k[dst] = __ldcg(ap.k_retained + src);
+        ap.br_v[dst] = __ldcg(ap.v_retained + src);
+      }
+    }
+  }
+  if (tid == 0) {
+    if (append && ret_len < ap.retained_storage) ap.br_len[sh] = ret_len + 1;
+    if (ap.window_tokens > 0) {
+      // the ring counters belong to the sequence: the last of its heads to get here advances them
+      __threadfence();
+      int* seq_ticket = prm.tickets + (size_t)prm.S * prm.H + s;
+      if (atomicAdd(seq_ticket, 1) == prm.H - 1) {
+        *seq_ticket = 0;
+        if (append) {
+          if (full)
+            ap.nw_pos[s] = (ring_pos + 1) % ap.window_tokens;
+          else
+            ap.nw_len[s] = ring_len + 1;
+        }
+      }
+    }
+  }
 }
 
 // Separate merge launch for callers whose workspace carries no tickets: one block of D threads

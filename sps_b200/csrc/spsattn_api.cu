@@ -257,6 +257,15 @@ static int decode_chunk_rows(int S, int H, long long max_rows_total) {
   return chunk;
 }
 
+// One block per (sequence, head) (decode_pair_kernel) where its rows and those of its neighbours on the
+// SM are read in less than the tickets and records of the split form cost.  Measured: 64 rows 5.6 ->
+// 4.3 us and 200 rows 6.2 -> 5.2 us at 2 x 12 x 64; even at 400 rows; slower where an SM has several
+// pairs of 200 rows of 128.
+static bool pair_fits(int S, int H, int D, long long rows) {
+  const long long pairs = (long long)S * H, per_sm = (pairs + 147) / 148;
+  return rows <= 384 && per_sm * rows * D * 4 <= 224 * 1024;
+}
+
 static long long decode_max_rows(const spsattn_segment* segs, int n_segments) {
   long long t = 0;
   for (int x = 0; x < n_segments; ++x) t += segs[x].max_rows > 0 ? segs[x].max_rows : 0;
@@ -266,6 +275,13 @@ static long long decode_max_rows(const spsattn_segment* segs, int n_segments) {
 template <int D, int NQ, bool FP16>
 static int launch_decode(const DecodeParams& prm, cudaStream_t st) {
   dim3 grid((unsigned)(prm.S * prm.H), (unsigned)prm.n_chunks);
+  if constexpr (D <= 128) {
+    if (prm.pair) {
+      const int groups = prm.n_chunks < kPairMaxGroups ? prm.n_chunks : kPairMaxGroups;
+      return launch_dependent(decode_pair_kernel<D, NQ, FP16>, dim3((unsigned)(prm.S * prm.H)),
+                              dim3((unsigned)(groups * kDecodeThreads)), 0, st, prm);
+    }
+  }
   const int rc = launch_dependent(decode_split_kernel<D, NQ, FP16>, grid, dim3(kDecodeThreads), 0, st, prm);
   if (rc != 0 || prm.tickets != nullptr) return rc;                // with tickets the last block merges
   decode_merge_kernel<D, NQ, FP16><<<(unsigned)(prm.S * prm.H), D, 0, st>>>(prm);
@@ -769,7 +785,7 @@ static int decode_impl(const void* q, int nq, void* out, int out_dtype, const sp
   const long long rows = decode_max_rows(segs, n_segments);
   const int path = g_decode_path.load();
   const bool tc_ok = single_launch && tc_supported(segs, n_segments, D);
-  if (path == 2 && !tc_ok) return SPSATTN_ERR_ARG;
+  if ((path == 2 && !tc_ok) || (path == 3 && D > 128)) return SPSATTN_ERR_ARG;
   // automatic choice: the tensor-core kernel when whole segments, one block each, already fill
   // the machine (two blocks per SM): then every block streams a long run of tiles, merges in
   // shared memory and its start-up is amortised (90 % of the copy bandwidth at 128 sequences x 16
@@ -790,6 +806,9 @@ static int decode_impl(const void* q, int nq, void* out, int out_dtype, const sp
     n_chunks = (rows + prm.chunk_rows - 1) / prm.chunk_rows;
     if (n_chunks < 1) n_chunks = 1;
     prm.extras_slot = -1;
+    const bool pair_ok = single_launch && D <= 128 && n_chunks <= kPairMaxChunks;
+    if (path == 3 && !pair_ok) return SPSATTN_ERR_ARG;
+    prm.pair = pair_ok && (path == 3 || (path == 0 && pair_fits(S, H, D, rows)));
   }
   if (n_chunks > 65535) return SPSATTN_ERR_TOO_LARGE;
   prm.n_chunks = (int)n_chunks;
@@ -908,7 +927,7 @@ int spsattn_debug_prefill_path(int path) {
 }
 
 int spsattn_debug_decode_path(int path) {
-  if (path < 0 || path > 2) return SPSATTN_ERR_ARG;
+  if (path < 0 || path > 3) return SPSATTN_ERR_ARG;
   g_decode_path.store(path);
   return 0;
 }

@@ -116,6 +116,27 @@ int spsattn_prefill_fwd_strided(const void* q, const void* k, const void* v, voi
                                 void* workspace, size_t workspace_bytes,
                                 int* device_status, void* stream);
 
+/* The same with the first row of every row's document given (run_start [B, N] int32 on the device;
+ * documents are runs of rows) instead of document ids: no pre-pass, for callers that attend over
+ * the same documents many times (the layers of a model). */
+int spsattn_prefill_fwd_runs(const void* q, const void* k, const void* v, void* o, float* lse,
+                             const int64_t* q_strides, const int64_t* k_strides,
+                             const int64_t* v_strides, const int64_t* o_strides,
+                             const int* run_start,
+                             int B, int H, int N, int D, int dtype, float sm_scale,
+                             int persistent_parity, int temporary_window, int persistent_window,
+                             int mask_flags, int* device_status, void* stream);
+
+/* What a batched prefill needs to know about left-padded prompts (model.py:39-99): ids [B, T] ->
+ * doubled ids and positions [B, T * slots] (slot 1 holds `predict`), run_start as above, doc_mask
+ * [B, T] (tokens of the last document; none when `empty_after_eos` and the row ends on EOS),
+ * real_len [B], ends_on_eos [B], flags [4] = {a pad stands after a real token, a row holds no real
+ * token, longest row, the device status word}. */
+int spsattn_prompt_scan(const int64_t* ids, int B, int T, int slots, int64_t eos, int64_t pad,
+                        int64_t predict, int empty_after_eos, int64_t* ids2, int64_t* pos2,
+                        int* run_start, uint8_t* doc_mask, int64_t* real_len, uint8_t* ends_on_eos,
+                        int64_t* flags, const int* device_status, void* stream);
+
 /* Backward of spsattn_prefill_fwd (the training path): dq, dk, dv from d_o, with the
  * probabilities recomputed from `lse` as written by the forward call on the same q, k, v, mask and
  * sm_scale (the reference's backward, triton_sps_flash_attention.py:623-720, does the same with

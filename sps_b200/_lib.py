@@ -21,7 +21,7 @@ STATUS_BAD_TOKEN = 2
 
 EXPORTS = (
     "spsattn_version", "spsattn_strerror",
-    "spsattn_prefill_workspace_bytes", "spsattn_prefill_fwd", "spsattn_prefill_fwd_strided",
+    "spsattn_prefill_workspace_bytes", "spsattn_prefill_fwd", "spsattn_prefill_fwd_strided", "spsattn_prefill_fwd_runs", "spsattn_prompt_scan",
     "spsattn_decode_workspace_bytes", "spsattn_decode_fwd", "spsattn_decode_fwd_noalloc",
     "spsattn_kv_update", "spsattn_fill_decode_caches", "spsattn_rope_cast", "spsattn_debug_visibility",
     "spsattn_decode_step_workspace_bytes", "spsattn_decode_step", "spsattn_decode_step_tickets",

@@ -21,8 +21,9 @@ NATIVE_PATH = os.path.join(PKG_DIR, "_native.so")
 ABI_HEADER = os.path.join("..", "..", "include", "spsattn.h")
 SOURCES = ["spsattn_api.cu"]
 HEADERS = ["common.cuh", "mask.cuh", "prefill_sm100.cuh", "prefill_wide_sm100.cuh", "prefill_bwd_sm100.cuh", "prefill_aux.cuh", "decode.cuh", "decode_sm100.cuh",
-           "kv_update.cuh", "model_glue.cuh", "rope.cuh", "cache_fill.cuh", "decoder_step.cuh", ABI_HEADER]
+           "kv_update.cuh", "model_glue.cuh", "rope.cuh", "cache_fill.cuh", "decoder_step.cuh", "prompt.cuh", ABI_HEADER]
 NATIVE_SOURCES = ["native.cpp"]
+NATIVE_HEADERS = ["native_engine.h"]
 
 
 def _nvcc() -> str:
@@ -39,7 +40,7 @@ def _stale(target: str, sources) -> bool:
 
 
 def is_stale() -> bool:
-    return _stale(LIB_PATH, SOURCES + HEADERS) or _stale(NATIVE_PATH, NATIVE_SOURCES + [ABI_HEADER])
+    return _stale(LIB_PATH, SOURCES + HEADERS) or _stale(NATIVE_PATH, NATIVE_SOURCES + NATIVE_HEADERS + [ABI_HEADER])
 
 
 def _run(cmd, verbose: bool) -> None:
@@ -81,7 +82,7 @@ def _build_native(verbose: bool) -> None:
 def build(force: bool = False, verbose: bool = False) -> str:
     if force or _stale(LIB_PATH, SOURCES + HEADERS):
         _build_library(verbose)
-    if force or _stale(NATIVE_PATH, NATIVE_SOURCES + [ABI_HEADER]):
+    if force or _stale(NATIVE_PATH, NATIVE_SOURCES + NATIVE_HEADERS + [ABI_HEADER]):
         _build_native(verbose)
     return LIB_PATH
 

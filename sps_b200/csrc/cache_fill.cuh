@@ -28,7 +28,10 @@ struct CacheFillParams {
   int retained_slot, window_slot;   // parity (0/1) of the row that feeds each cache
 };
 
+// Bound: HBM (each selected row is read and written once).  A block takes 64 tokens of a few heads
+// (grid z): with all heads in one block a batch of two short prompts had four blocks, 43 us a layer.
 constexpr int kFillChunk = 64;     // tokens per block
+constexpr int kFillHeads = 2;      // heads per block
 
 __global__ void __launch_bounds__(256) cache_fill_kernel(const CacheFillParams p) {
   __shared__ int s_warp[8];
@@ -83,14 +86,15 @@ __global__ void __launch_bounds__(256) cache_fill_kernel(const CacheFillParams p
   const int window_len = p.window_tokens > 0 ? min(p.window_tokens, doc_len) : 0;
   const int win_first = doc_len - window_len;   // rank of the first token that enters the ring
   const int vec_per_row = p.D / 8;              // 16-byte vectors per [D] row
-  const int vec_per_tok = p.H * vec_per_row;
+  const int h0 = blockIdx.z * kFillHeads, heads = min(kFillHeads, p.H - h0);
+  const int vec_per_tok = heads * vec_per_row;
   for (int idx = tid; idx < kFillChunk * vec_per_tok; idx += blockDim.x) {
     const int lt = idx / vec_per_tok;
     const int r = s_rank[lt];
     if (r < 0) continue;
     const int rank = s_before + r;
     const int rem = idx - lt * vec_per_tok;
-    const int h = rem / vec_per_row, x = rem - h * vec_per_row;
+    const int hl = rem / vec_per_row, x = rem - hl * vec_per_row, h = h0 + hl;
     const int t = t0 + lt;
     const size_t src_ret = (size_t)b * p.stride_b + (size_t)(2 * t + p.retained_slot) * p.stride_n +
                            (size_t)h * p.stride_h + x * 8;
@@ -107,7 +111,7 @@ __global__ void __launch_bounds__(256) cache_fill_kernel(const CacheFillParams p
       *reinterpret_cast<uint4*>(p.nw_v + dst) = *reinterpret_cast<const uint4*>(p.v + src_win);
     }
   }
-  if (blockIdx.x == 0) {
+  if (blockIdx.x == 0 && blockIdx.z == 0) {
     for (int h = tid; h < p.H; h += blockDim.x) p.br_len[(size_t)b * p.H + h] = doc_len;
     if (tid == 0 && p.window_tokens > 0) {
       p.nw_len[b] = window_len;

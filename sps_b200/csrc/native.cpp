@@ -18,9 +18,11 @@
 
 #include <algorithm>
 #include <cmath>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <unordered_map>
+#include <vector>
 
 #include "../../include/spsattn.h"
 
@@ -637,6 +639,8 @@ PyObject* kv_update_impl(PyObject* const* a, Py_ssize_t n) {
   Py_RETURN_NONE;
 }
 
+#include "native_engine.h"
+
 // ------------------------------------------------------------------------------------- module
 
 PyObject* status_word_impl(PyObject* const* a, Py_ssize_t n) {
@@ -678,6 +682,10 @@ PyMethodDef g_methods[] = {
     SPS_ENTRY("decode_q2", decode_q2_impl),
     SPS_ENTRY("decode_q1", decode_q1_impl),
     SPS_ENTRY("kv_update", kv_update_impl),
+    SPS_ENTRY("engine_model", engine_model_impl),
+    SPS_ENTRY("engine_scan", engine_scan_impl),
+    SPS_ENTRY("engine_prefill", engine_prefill_impl),
+    SPS_ENTRY("engine_step", engine_step_impl),
     SPS_ENTRY("status_word", status_word_impl),
     SPS_ENTRY("setup", setup_impl),
     {nullptr, nullptr, 0, nullptr}};

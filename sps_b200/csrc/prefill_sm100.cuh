@@ -32,7 +32,7 @@ struct PrefillParams {
   const void* docs;      // [B,N] ids or null
   int64_t doc_stride_b, doc_stride_t;
   int doc_is_i64;
-  const int* lo;         // [B,N] run starts (pre-pass) or null
+  const int* lo;         // [B,N] run starts (pre-pass, or the caller's) or null
   const int* mono;       // [B] 1 when ids of the row are non-decreasing, or null
   int B, H, N;
   int n_qtiles;
@@ -227,7 +227,7 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   const uint32_t bar_p_full = bar0 + 104;
   const uint32_t bar_pv_done = bar0 + 112;
 
-  const bool has_docs = prm.docs != nullptr;
+  const bool has_docs = prm.lo != nullptr;      // from document ids or given by the caller
 
   if (tid == 0 || tid == 32) {
     // Two planner threads, one per key stream (thread 0: the persistent stream, which holds the
@@ -242,7 +242,7 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     if (slot == 0 && prm.status != nullptr) st_word = *reinterpret_cast<volatile int*>(prm.status);
     const int mono_b = (has_docs && prm.mono != nullptr) ? prm.mono[b] : 1;
     int lo0 = 0, lo1 = 0;
-    if (has_docs && prm.lo != nullptr) {
+    if (has_docs) {
       const int i1 = min(i0 + kTileM - 1, prm.N - 1);
       lo0 = prm.lo[(size_t)b * prm.N + i0];
       lo1 = prm.lo[(size_t)b * prm.N + i1];

@@ -18,6 +18,7 @@
 #include "kv_update.cuh"
 #include "model_glue.cuh"
 #include "prefill_aux.cuh"
+#include "prompt.cuh"
 #include "prefill_sm100.cuh"
 #include "prefill_wide_sm100.cuh"
 #include "prefill_bwd_sm100.cuh"
@@ -176,7 +177,7 @@ int launch_prefill_sm100(const CUtensorMap& tq, const CUtensorMap& tk, const CUt
 #ifdef SPSATTN_NO_PDL
   cfg.numAttrs = 0;         // tuning builds: ordinary launch
 #else
-  cfg.numAttrs = prm.lo != nullptr ? 1 : 0;
+  cfg.numAttrs = prm.mono != nullptr ? 1 : 0;
 #endif
   const cudaError_t le = cudaLaunchKernelEx(&cfg, prefill_sm100_kernel<D, FP16>, tq, tk, tv, prm);
   return le != cudaSuccess ? (int)le : (int)cudaGetLastError();
@@ -429,14 +430,12 @@ size_t spsattn_prefill_workspace_bytes(int B, int H, int N, int D) {
   return prefill_ws_mono_bytes(B) + align_up((size_t)B * N * sizeof(int), 256);
 }
 
-int spsattn_prefill_fwd_strided(const void* q, const void* k, const void* v, void* o, float* lse,
-                                const int64_t* q_strides, const int64_t* k_strides,
-                                const int64_t* v_strides, const int64_t* o_strides, const void* doc_ids,
-                                int doc_is_i64, int64_t doc_stride_b, int64_t doc_stride_t, int B, int H,
-                                int N, int D, int dtype, float sm_scale, int persistent_parity,
-                                int temporary_window, int persistent_window, int mask_flags,
-                                void* workspace, size_t workspace_bytes, int* device_status,
-                                void* stream) {
+static int prefill_impl(const void* q, const void* k, const void* v, void* o, float* lse,
+                        const int64_t* q_strides, const int64_t* k_strides, const int64_t* v_strides,
+                        const int64_t* o_strides, const void* doc_ids, int doc_is_i64, int64_t doc_stride_b,
+                        int64_t doc_stride_t, const int* run_start, int B, int H, int N, int D, int dtype,
+                        float sm_scale, int persistent_parity, int temporary_window, int persistent_window,
+                        int mask_flags, void* workspace, size_t workspace_bytes, int* device_status, void* stream) {
   if (!q || !k || !v || !o || !q_strides || !k_strides || !v_strides || !o_strides) return SPSATTN_ERR_ARG;
   if (B <= 0 || H <= 0 || N <= 0) return SPSATTN_ERR_ARG;
   if (dtype != SPSATTN_DTYPE_BF16 && dtype != SPSATTN_DTYPE_FP16) return SPSATTN_ERR_ARG;
@@ -460,6 +459,7 @@ int spsattn_prefill_fwd_strided(const void* q, const void* k, const void* v, voi
   int rc = run_doc_prepass(doc_ids, doc_is_i64, doc_stride_b, doc_stride_t, B, N, workspace,
                            workspace_bytes, &lo, &mono, st);
   if (rc != 0) return rc;
+  if (run_start != nullptr) lo = const_cast<int*>(run_start);
 
   const MaskParams mask = make_mask(N, persistent_parity, temporary_window, persistent_window, mask_flags);
   const float scale_log2 = sm_scale * 1.4426950408889634f;
@@ -467,7 +467,7 @@ int spsattn_prefill_fwd_strided(const void* q, const void* k, const void* v, voi
 
   CUtensorMap tq, tk, tv;
   if ((rc = encode_q_map(&tq, q, B, H, N, D, sq, dtype)) != 0) return rc;
-  const bool wide = D == 64 && g_prefill_path.load() == 2;
+  const bool wide = D == 64 && g_prefill_path.load() == 2 && run_start == nullptr;
   const int box_tokens = wide ? kWideN : kTileN;
   if ((rc = encode_kv_map(&tk, k, B, H, N, D, mask.ks, sk, dtype, box_tokens)) != 0) return rc;
   if ((rc = encode_kv_map(&tv, v, B, H, N, D, mask.ks, sv, dtype, box_tokens)) != 0) return rc;
@@ -527,6 +527,59 @@ int spsattn_prefill_fwd_strided(const void* q, const void* k, const void* v, voi
     default: return fp16 ? launch_prefill_sm100<256, true>(tq, tk, tv, prm, st)
                          : launch_prefill_sm100<256, false>(tq, tk, tv, prm, st);
   }
+}
+
+int spsattn_prefill_fwd_strided(const void* q, const void* k, const void* v, void* o, float* lse,
+                                const int64_t* q_strides, const int64_t* k_strides,
+                                const int64_t* v_strides, const int64_t* o_strides, const void* doc_ids,
+                                int doc_is_i64, int64_t doc_stride_b, int64_t doc_stride_t, int B, int H,
+                                int N, int D, int dtype, float sm_scale, int persistent_parity,
+                                int temporary_window, int persistent_window, int mask_flags,
+                                void* workspace, size_t workspace_bytes, int* device_status,
+                                void* stream) {
+  return prefill_impl(q, k, v, o, lse, q_strides, k_strides, v_strides, o_strides, doc_ids, doc_is_i64, doc_stride_b,
+                      doc_stride_t, nullptr, B, H, N, D, dtype, sm_scale, persistent_parity, temporary_window,
+                      persistent_window, mask_flags, workspace, workspace_bytes, device_status, stream);
+}
+
+int spsattn_prefill_fwd_runs(const void* q, const void* k, const void* v, void* o, float* lse,
+                             const int64_t* q_strides, const int64_t* k_strides, const int64_t* v_strides,
+                             const int64_t* o_strides, const int* run_start, int B, int H, int N, int D, int dtype,
+                             float sm_scale, int persistent_parity, int temporary_window, int persistent_window,
+                             int mask_flags, int* device_status, void* stream) {
+  return prefill_impl(q, k, v, o, lse, q_strides, k_strides, v_strides, o_strides, nullptr, 0, 0, 0, run_start, B, H, N, D,
+                      dtype, sm_scale, persistent_parity, temporary_window, persistent_window, mask_flags, nullptr, 0,
+                      device_status, stream);
+}
+
+int spsattn_prompt_scan(const int64_t* ids, int B, int T, int slots, int64_t eos, int64_t pad, int64_t predict,
+                        int empty_after_eos, int64_t* ids2, int64_t* pos2, int* run_start, uint8_t* doc_mask,
+                        int64_t* real_len, uint8_t* ends_on_eos, int64_t* flags, const int* device_status,
+                        void* stream) {
+  if (!ids || !ids2 || !pos2 || !run_start || !doc_mask || !real_len || !ends_on_eos || !flags) return SPSATTN_ERR_ARG;
+  if (B <= 0 || T <= 0 || (slots != 1 && slots != 2) || (long long)T * slots > 0x7fffffffLL) return SPSATTN_ERR_ARG;
+  PromptParams p;
+  p.ids = ids;
+  p.B = B;
+  p.T = T;
+  p.slots = slots;
+  p.eos = eos;
+  p.pad = pad;
+  p.predict = predict;
+  p.empty_after_eos = empty_after_eos;
+  p.ids2 = ids2;
+  p.pos2 = pos2;
+  p.run_start = run_start;
+  p.doc_mask = doc_mask;
+  p.real_len = real_len;
+  p.ends_on_eos = ends_on_eos;
+  p.flags = flags;
+  p.status = device_status;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const cudaError_t e = cudaMemsetAsync(flags, 0, 4 * sizeof(int64_t), st);
+  if (e != cudaSuccess) return (int)e;
+  prompt_scan_kernel<<<(unsigned)B, kPromptThreads, 0, st>>>(p);
+  return (int)cudaGetLastError();
 }
 
 size_t spsattn_prefill_bwd_workspace_bytes(int B, int H, int N, int D) {
@@ -1044,7 +1097,7 @@ int spsattn_fill_decode_caches(const void* k, const void* v, int64_t stride_b, i
   p.window_tokens = window_tokens > 0 ? window_tokens : 0;
   p.retained_slot = retained_slot;
   p.window_slot = window_slot;
-  dim3 grid((T + kFillChunk - 1) / kFillChunk, B);
+  dim3 grid((T + kFillChunk - 1) / kFillChunk, B, (H + kFillHeads - 1) / kFillHeads);
   cache_fill_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(p);
   return (int)cudaGetLastError();
 }

@@ -36,7 +36,7 @@ import torch
 from torch import Tensor
 
 from . import _lib
-from .attention import _status, check_device_status, prefill_attention
+from .attention import _status, check_device_status
 
 _VARIANTS = {
     # name: (prediction slot, ring ("window") slot, retained slot, persistent-key parity)
@@ -192,104 +192,31 @@ class SPSGenerator:
         self.param_dtype = param_dtype
         self.attn_dtype = torch.bfloat16                       # reverse_sps/inference.py:637
         self.glue_dtype = _lib.DTYPE_BF16 if param_dtype == torch.bfloat16 else _lib.DTYPE_FP32
-        self.x_dtype_code = 0 if param_dtype == torch.bfloat16 else 2
         self.w = _Weights(state_dict, dims, self.device, param_dtype)
         hd = dims.head_dim
         # model.py:134-160, kept as (cos, sin) pairs: [block_size, hd/2, 2] fp32
         freqs = 1.0 / (10000.0 ** (torch.arange(0, hd, 2)[: hd // 2].float() / hd))
         ang = torch.outer(torch.arange(dims.block_size).float(), freqs)
         self.freqs = torch.stack([torch.cos(ang), torch.sin(ang)], dim=-1).to(self.device).contiguous()
+        self._model = None
         self._step = None
         self._session = None
 
-    # ------------------------------------------------------------------ library calls
     def _stream(self):
         return torch.cuda.current_stream(self.device).cuda_stream
 
-    def _add_rmsnorm(self, x: Tensor, delta: Optional[Tensor], weight: Tensor, y: Optional[Tensor]) -> None:
-        rows, c = x.shape
-        rc = self.lib.spsattn_add_rmsnorm(x.data_ptr(), None if delta is None else delta.data_ptr(),
-                                          weight.data_ptr(), None if y is None else y.data_ptr(),
-                                          self.glue_dtype, rows, c, float(self.dims.norm_eps), self._stream())
-        _lib.check(rc, "spsattn_add_rmsnorm")
-
-    def _swiglu(self, gate_up: Tensor, y: Tensor) -> None:
-        rows = gate_up.shape[0]
-        rc = self.lib.spsattn_swiglu(gate_up.data_ptr(), y.data_ptr(), self.glue_dtype, rows,
-                                     self.dims.intermediate_size, self._stream())
-        _lib.check(rc, "spsattn_swiglu")
-
-    def _mlp(self, layer: int, xn: Tensor, gate_up: Tensor, hidden: Tensor, delta: Tensor) -> None:
-        torch.mm(xn, self.w.gate_up[layer].t(), out=gate_up)
-        self._swiglu(gate_up, hidden)
-        torch.mm(hidden, self.w.down[layer].t(), out=delta)
+    def _native(self):
+        """(extension module, this model's parameters in it)."""
+        ext = _lib.native()
+        if self._model is None:
+            w, d = self.w, self.dims
+            self._model = ext.engine_model(
+                w.attn_norm, w.c_attn, w.c_proj, w.mlp_norm, w.gate_up, w.down, w.wte, w.out_norm, w.lm_head, self.freqs,
+                d.n_head, d.head_dim, self.n_slot, float(d.norm_eps), self.parity, self.window_tokens,
+                self.retained_slot, self.window_slot or 0)
+        return ext, self._model
 
     # ------------------------------------------------------------------ prefill
-    def _prefill_chain(self, idx: Tensor, positions: Tensor, docs2: Tensor,
-                       state: Optional[DecodeState], doc_mask: Optional[Tensor]) -> Tensor:
-        """Final-norm hidden states [B, 2T, C] of the doubled prompt; fills ``state`` on the way."""
-        d = self.dims
-        b, t = idx.shape
-        ns = self.n_slot
-        n, c, h, hd, inter = ns * t, d.hidden_size, d.n_head, d.head_dim, d.intermediate_size
-        rows = b * n
-        dev, pdt = self.device, self.param_dtype
-        idx2 = idx.repeat_interleave(ns, dim=1)
-        if ns == 2:
-            idx2[:, 1::2] = d.predict_token_id                              # reverse_sps/core.py:261-264
-        x = self.w.wte.index_select(0, idx2.reshape(-1))                    # [rows, C] residual stream
-        fc = self.freqs[positions.repeat_interleave(ns, dim=1)].contiguous()  # [B, N, hd/2, 2]
-        xn = torch.empty_like(x)
-        delta = torch.empty_like(x)
-        qkv = torch.empty((rows, 3 * c), device=dev, dtype=pdt)
-        ops = torch.empty((3, b, n, h, hd), device=dev, dtype=self.attn_dtype)   # q, k, v token-major
-        y = torch.empty((b, n, h, hd), device=dev, dtype=self.attn_dtype)
-        gate_up = torch.empty((rows, 2 * inter), device=dev, dtype=pdt)
-        hidden = torch.empty((rows, inter), device=dev, dtype=pdt)
-        groups = (_lib.RopeGroup * 3)()
-        for gi in range(3):
-            groups[gi].out = ops[gi].data_ptr()
-            groups[gi].stride_b, groups[gi].stride_n, groups[gi].stride_h = n * c, c, hd
-            groups[gi].rotate = int(gi < 2)
-        scale = 1.0 / math.sqrt(hd)
-        self._add_rmsnorm(x, None, self.w.attn_norm[0], xn)
-        for layer in range(d.n_layer):
-            torch.mm(xn, self.w.c_attn[layer].t(), out=qkv)
-            rc = self.lib.spsattn_qkv_rope_cast(qkv.data_ptr(), self.x_dtype_code, n * 3 * c, 3 * c, hd,
-                                                fc.data_ptr(), n * (hd // 2), groups, 3, _lib.DTYPE_BF16,
-                                                b, n, h, hd, self._stream())
-            _lib.check(rc, "spsattn_qkv_rope_cast")
-            if state is not None:
-                self._fill_caches(state, layer, ops[1], ops[2], doc_mask)
-            prefill_attention(ops[0].transpose(1, 2), ops[1].transpose(1, 2), ops[2].transpose(1, 2),
-                              scale, persistent_parity=self.parity, temporary_window=self.window_tokens,
-                              documents_idx=docs2, out=y.transpose(1, 2))
-            y2 = y.view(rows, c)
-            if pdt != self.attn_dtype:
-                y2 = y2.to(pdt)                                             # sps/core.py:80
-            torch.mm(y2, self.w.c_proj[layer].t(), out=delta)
-            self._add_rmsnorm(x, delta, self.w.mlp_norm[layer], xn)
-            self._mlp(layer, xn, gate_up, hidden, delta)
-            nxt = self.w.attn_norm[layer + 1] if layer + 1 < d.n_layer else self.w.out_norm
-            self._add_rmsnorm(x, delta, nxt, xn)
-        return xn.view(b, n, c)
-
-    def _fill_caches(self, st: DecodeState, layer: int, k: Tensor, v: Tensor, doc_mask: Tensor) -> None:
-        b, n, h, hd = k.shape
-        ring = [None] * 4
-        if self.window_tokens > 0:
-            ring = [st.nw_k[layer].data_ptr(), st.nw_v[layer].data_ptr(), st.nw_len[layer].data_ptr(),
-                    st.nw_pos[layer].data_ptr()]
-        # the entry point addresses row 2 * token + slot of a doubled sequence; with one row per
-        # token (Standard) half the row stride and slot 0 address row `token`
-        row_stride = k.stride(1) if self.n_slot == 2 else k.stride(1) // 2
-        rc = self.lib.spsattn_fill_decode_caches(
-            k.data_ptr(), v.data_ptr(), k.stride(0), row_stride, k.stride(2), doc_mask.data_ptr(),
-            st.br_k[layer].data_ptr(), st.br_v[layer].data_ptr(), st.br_len[layer].data_ptr(),
-            ring[0], ring[1], ring[2], ring[3], b, n // self.n_slot, h, hd, st.max_tokens, int(st.nw_k.shape[3]),
-            self.window_tokens, self.retained_slot, self.window_slot or 0, self._stream())
-        _lib.check(rc, "spsattn_fill_decode_caches")
-
     def build_decode_state(self, batch_size: int, max_tokens: int) -> DecodeState:
         """reverse_sps/inference.py:64-111, one allocation per kind instead of one per layer."""
         d = self.dims
@@ -317,8 +244,12 @@ class SPSGenerator:
             raise ValueError(f"Cannot forward sequence of length {self.n_slot * t}, block size is only {self.dims.block_size}")
         docs2 = left_padded_document_idx(idx, self.dims.eos_token_id, self.dims.pad_token_id)
         docs2 = docs2.repeat_interleave(self.n_slot, dim=1).contiguous()
-        pos = torch.arange(t, device=self.device).unsqueeze(0).expand(b, -1)
-        xn = self._prefill_chain(idx, pos, docs2, None, None)
+        pos2 = torch.arange(t, device=self.device).repeat_interleave(self.n_slot).expand(b, -1)
+        ids2 = idx.repeat_interleave(self.n_slot, dim=1)
+        if self.n_slot == 2:
+            ids2[:, 1::2] = self.dims.predict_token_id                      # reverse_sps/core.py:261-264
+        ext, model = self._native()
+        xn = ext.engine_prefill(model, ids2, pos2, docs2, None, None)
         pred = xn[:, self.pred_slot::self.n_slot].reshape(b * t, -1)
         return torch.mm(pred, self.w.lm_head.t()).view(b, t, -1)
 
@@ -328,15 +259,25 @@ class SPSGenerator:
         the logits [B, V] that predict the first new token.  ``state``: caches of an earlier call
         to fill again, used when their batch size and capacity fit."""
         d = self.dims
-        idx = idx_BxT.to(self.device)
+        idx = idx_BxT.to(self.device, torch.long).contiguous()
         b, t = idx.shape
-        _validate_left_padded(idx, d.pad_token_id, f"{self.variant} generation prefill prompts")
-        real = idx != d.pad_token_id
-        real_lengths = real.sum(dim=1).to(torch.long)
-        longest = int(real_lengths.max().item())
-        # the .item() above has synchronised: a bounded wait that expired in an earlier kernel
-        # shows in the status word now, before its empty outputs are used
-        check_device_status(self.device)
+        context = f"{self.variant} generation prefill prompts"
+        if t == 0:
+            raise ValueError(f"{context} must contain at least one real token per row")
+        ext, model = self._native()
+        # a Standard prompt that ends on EOS starts decoding with an empty cache
+        # (full_attention_model.py:703-705)
+        ids2, pos2, run_start, doc_mask, real_lengths, ends_on_eos, flags = ext.engine_scan(
+            model, idx, d.eos_token_id, d.pad_token_id, d.predict_token_id, self.variant == "standard")
+        pad_inside, empty_row, longest, status = flags.tolist()
+        # that has synchronised: a bounded wait that expired in an earlier kernel shows in the status
+        # word now, before its empty outputs are used
+        if status:
+            check_device_status(self.device)
+        if pad_inside:
+            raise ValueError(f"{context} must be left padded only")
+        if empty_row:
+            raise ValueError(f"{context} must contain at least one real token per row")
         total = longest + int(max_new_tokens)
         if total > d.block_size:
             raise ValueError(f"Cannot generate {max_new_tokens} new tokens from a prompt with "
@@ -346,20 +287,12 @@ class SPSGenerator:
                 t_.zero_()
         else:
             state = self.build_decode_state(b, total)
-        docs = left_padded_document_idx(idx, d.eos_token_id, d.pad_token_id)
-        docs2 = docs.repeat_interleave(self.n_slot, dim=1).contiguous()
-        doc_mask = real & (docs == docs[:, -1:])
-        if self.variant == "standard":
-            # a prompt that ends on EOS starts decoding with an empty cache
-            # (full_attention_model.py:703-705)
-            doc_mask = doc_mask & (idx[:, -1:] != d.eos_token_id)
-        doc_mask = doc_mask.to(torch.uint8).contiguous()
-        pos = left_padded_position_ids(idx, d.pad_token_id)
-        xn = self._prefill_chain(idx, pos, docs2, state, doc_mask)
+        caches = (state.nw_k, state.nw_v, state.nw_len, state.nw_pos, state.br_k, state.br_v, state.br_len)
+        xn = ext.engine_prefill(model, ids2, pos2, run_start, caches, doc_mask)
         last = xn[:, self.n_slot * (t - 1) + self.pred_slot]                # [B, C]
         next_logits = torch.mm(last, self.w.lm_head.t())
         state.processed_tokens.copy_(real_lengths)
-        state.next_doc_start.copy_(idx[:, -1] == d.eos_token_id)
+        state.next_doc_start.copy_(ends_on_eos)
         state.host_tokens = longest
         return state, next_logits
 
@@ -385,9 +318,9 @@ class SPSGenerator:
         s.k2 = torch.zeros((ns, b, h, hd), device=dev, dtype=self.attn_dtype)
         s.v2 = torch.zeros((ns, b, h, hd), device=dev, dtype=self.attn_dtype)
         s.y = torch.zeros((ns * b, c), device=dev, dtype=self.attn_dtype)
-        s.y_param = s.y if pdt == self.attn_dtype else torch.zeros((ns * b, c), device=dev, dtype=pdt)
         s.gate_up = torch.zeros((ns * b, 2 * inter), device=dev, dtype=pdt)
         s.hidden = torch.zeros((ns * b, inter), device=dev, dtype=pdt)
+        s.buffers = (s.x, s.xn, s.delta, s.qkv, s.y, s.gate_up, s.hidden, s.fc)
         # the [B, ns, 3C] projection seen as one row per sequence with 3 * ns head groups:
         # slot 0 q, k, v (, slot 1 q, k, v)
         groups = (_lib.RopeGroup * (3 * ns))()
@@ -480,39 +413,14 @@ class SPSGenerator:
         """One token for every row, from ``source``: leaves the prediction logits in ``logits`` (zeros
         for inactive rows when the projections are the library's own) and the caches and counters
         advanced (reverse_sps/inference.py:391-503).  No host sync."""
-        s, d = self._step, self.dims
-        b, c, h, hd, ns = s.b, d.hidden_size, d.n_head, d.head_dim, self.n_slot
-        stream = self._stream()
+        s = self._step
         if s.fused:
             rc = self.lib.spsattn_decoder_step(C.byref(s.decoder), C.byref(source), logits.data_ptr(),
-                                               _status(self.device).data_ptr(), stream)
+                                               _status(self.device).data_ptr(), self._stream())
             _lib.check(rc, "spsattn_decoder_step")
             return
-        rc = self.lib.spsattn_decoder_start(C.byref(s.decoder), C.byref(source), _status(self.device).data_ptr(), stream)
-        _lib.check(rc, "spsattn_decoder_start")
-        self._add_rmsnorm(s.x, None, self.w.attn_norm[0], s.xn)
-        scale = 1.0 / math.sqrt(hd)
-        for layer in range(d.n_layer):
-            segs, n_seg, extras, ap = s.layer_args[layer]
-            torch.mm(s.xn, self.w.c_attn[layer].t(), out=s.qkv)
-            rc = self.lib.spsattn_qkv_rope_cast(s.qkv.data_ptr(), self.x_dtype_code, 3 * ns * c, 0, hd,
-                                                s.fc.data_ptr(), hd // 2, s.groups, 3 * ns, _lib.DTYPE_BF16,
-                                                b, 1, h, hd, stream)
-            _lib.check(rc, "spsattn_qkv_rope_cast")
-            rc = self.lib.spsattn_decode_step(s.q.data_ptr(), ns, s.y.data_ptr(), _lib.DTYPE_BF16, segs, n_seg,
-                                              extras, ns, C.byref(ap), b, h, hd, _lib.DTYPE_BF16, scale,
-                                              s.ws.data_ptr(), s.ws_bytes, _status(self.device).data_ptr(),
-                                              stream)
-            _lib.check(rc, "spsattn_decode_step")
-            if s.y_param is not s.y:
-                s.y_param.copy_(s.y)                                        # inference.py:479-483
-            torch.mm(s.y_param, self.w.c_proj[layer].t(), out=s.delta)
-            self._add_rmsnorm(s.x, s.delta, self.w.mlp_norm[layer], s.xn)
-            self._mlp(layer, s.xn, s.gate_up, s.hidden, s.delta)
-            nxt = self.w.attn_norm[layer + 1] if layer + 1 < d.n_layer else self.w.out_norm
-            self._add_rmsnorm(s.x, s.delta, nxt, s.xn)
-        pred = s.xn.view(b, ns, c)[:, self.pred_slot]
-        torch.mm(pred, self.w.lm_head.t(), out=logits)
+        ext, model = self._native()
+        ext.engine_step(model, C.addressof(s.decoder), C.addressof(source), C.addressof(s.groups), s.buffers, logits)
 
     @torch.no_grad()
     def decode_one_token(self, state: DecodeState, token_B: Tensor, active_B: Tensor) -> Tensor:

@@ -171,6 +171,19 @@ int spsattn_prefill_bwd_strided(const void* q, const void* k, const void* v, con
                                 void* workspace, size_t workspace_bytes,
                                 int* device_status, void* stream);
 
+/* The same with the workspace that the forward call on the same document ids was given, untouched
+ * since: what that call found out about the documents is read from there instead of being worked out
+ * again (NULL: worked out). */
+int spsattn_prefill_bwd_after(const void* q, const void* k, const void* v, const void* o, const void* d_o,
+                                const float* lse, void* dq, void* dk, void* dv, const int64_t* strides,
+                                const void* doc_ids, int doc_is_i64, int64_t doc_stride_b,
+                                int64_t doc_stride_t,
+                                int B, int H, int N, int D, int dtype, float sm_scale,
+                                int persistent_parity, int temporary_window, int persistent_window,
+                                int mask_flags, void* forward_workspace,
+                                void* workspace, size_t workspace_bytes,
+                                int* device_status, void* stream);
+
 /* ---------------------------------------------------------------------------------------------
  * Decode: nq (1 or 2) queries per (sequence, head) over up to 3 length-masked KV segments plus up
  * to 2 single-token "current" K/V entries; fp32 output [S, nq, H, D].

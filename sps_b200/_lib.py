@@ -28,7 +28,7 @@ EXPORTS = (
     "spsattn_qkv_rope_cast",
     "spsattn_add_rmsnorm", "spsattn_swiglu", "spsattn_debug_decode_path", "spsattn_debug_prefill_path", "spsattn_debug_wait_expiry",
     "spsattn_decoder_start", "spsattn_decoder_choose", "spsattn_decoder_step_supported", "spsattn_decoder_step",
-    "spsattn_prefill_bwd_workspace_bytes", "spsattn_prefill_bwd", "spsattn_prefill_bwd_strided",
+    "spsattn_prefill_bwd_workspace_bytes", "spsattn_prefill_bwd", "spsattn_prefill_bwd_strided", "spsattn_prefill_bwd_after",
 )
 
 

@@ -180,7 +180,7 @@ struct DocArgs {
 };
 
 struct Forward {
-  Tensor o, lse;
+  Tensor o, lse, ws;       // ws: what the call found out about the documents (undefined without ids)
 };
 
 Forward prefill_forward(Tensor q, Tensor k, Tensor v, const MaskArgs& m, const optional<Tensor>& docs, bool return_lse,
@@ -204,13 +204,12 @@ Forward prefill_forward(Tensor q, Tensor k, Tensor v, const MaskArgs& m, const o
   r.o = out.has_value() ? *out : empty_like_layout(q);
   if (return_lse) r.lse = at::detail::empty_cuda({b, h, n}, at::kFloat, q.device(), c10::nullopt);
   const size_t ws_bytes = ids.ptr ? spsattn_prefill_workspace_bytes(b, h, n, d) : 0;
-  Tensor ws;
-  if (ws_bytes) ws = empty_bytes(ws_bytes, q);
+  if (ws_bytes) r.ws = empty_bytes(ws_bytes, q);
   const int rc = spsattn_prefill_fwd_strided(
       q.data_ptr(), k.data_ptr(), v.data_ptr(), r.o.data_ptr(), return_lse ? r.lse.data_ptr<float>() : nullptr,
       q.strides().data(), k.strides().data(), v.strides().data(), r.o.strides().data(), ids.ptr, ids.is_i64, ids.stride_b,
       ids.stride_t, b, h, n, d, dt, (float)m.sm_scale, (int)m.parity, m.temporary(n), m.persistent(n), (int)m.flags,
-      ws_bytes ? ws.data_ptr() : nullptr, ws_bytes, status_ptr(q), stream_of(q));
+      ws_bytes ? r.ws.data_ptr() : nullptr, ws_bytes, status_ptr(q), stream_of(q));
   check_rc(rc, "spsattn_prefill_fwd");
   return r;
 }
@@ -220,7 +219,7 @@ struct Gradients {
 };
 
 Gradients prefill_backward(Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, Tensor d_o, const MaskArgs& m,
-                           const optional<Tensor>& docs) {
+                           const optional<Tensor>& docs, const Tensor& forward_ws = Tensor()) {
   const int64_t b = q.size(0), h = q.size(1), n = q.size(2), d = q.size(3);
   if (!backward_head_dim(d))
     fail(PyExc_RuntimeError, "the backward kernels cover head_dim (64, 128), got " + std::to_string(d));
@@ -242,10 +241,11 @@ Gradients prefill_backward(Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, T
     for (int i = 0; i < 3; ++i) strides[at_++] = x->stride(i);
   const size_t ws_bytes = spsattn_prefill_bwd_workspace_bytes(b, h, n, d);
   const Tensor ws = empty_bytes(ws_bytes, q);
-  const int rc = spsattn_prefill_bwd_strided(
+  const int rc = spsattn_prefill_bwd_after(
       q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), d_o.data_ptr(), lse.data_ptr<float>(), g.dq.data_ptr(),
       g.dk.data_ptr(), g.dv.data_ptr(), strides, ids.ptr, ids.is_i64, ids.stride_b, ids.stride_t, b, h, n, d, dt,
-      (float)m.sm_scale, (int)m.parity, m.temporary(n), m.persistent(n), (int)m.flags, ws.data_ptr(), ws_bytes,
+      (float)m.sm_scale, (int)m.parity, m.temporary(n), m.persistent(n), (int)m.flags,
+      forward_ws.defined() ? forward_ws.data_ptr() : nullptr, ws.data_ptr(), ws_bytes,
       status_ptr(q), stream_of(q));
   check_rc(rc, "spsattn_prefill_bwd");
   return g;
@@ -256,7 +256,7 @@ struct PrefillAttention : public torch::autograd::Function<PrefillAttention> {
   static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v,
                         const MaskArgs& m, const optional<Tensor>& docs) {
     Forward r = prefill_forward(q, k, v, m, docs, true, c10::nullopt);
-    ctx->save_for_backward({q, k, v, r.o, r.lse});
+    ctx->save_for_backward({q, k, v, r.o, r.lse, r.ws});
     if (docs.has_value()) ctx->saved_data["docs"] = *docs;
     ctx->saved_data["scale"] = m.sm_scale;
     ctx->saved_data["mask"] = std::vector<int64_t>{m.parity, m.temporary_window, m.persistent_window, m.flags,
@@ -275,7 +275,7 @@ struct PrefillAttention : public torch::autograd::Function<PrefillAttention> {
     torch::autograd::variable_list out(5);
     try {
       const at::AutoGradMode no_grad(false);
-      Gradients g = prefill_backward(saved[0], saved[1], saved[2], saved[3], saved[4], grads[0].detach(), m, docs);
+      Gradients g = prefill_backward(saved[0], saved[1], saved[2], saved[3], saved[4], grads[0].detach(), m, docs, saved[5]);
       out[0] = g.dq;
       out[1] = g.dk;
       out[2] = g.dv;

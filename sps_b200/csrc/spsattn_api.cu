@@ -228,8 +228,8 @@ int launch_prefill_bwd(const CUtensorMap& x0, const CUtensorMap& x1, const CUten
   if (attr_err != cudaSuccess) return (int)attr_err;
   const long long blocks = (long long)prm.n_xtiles * prm.B * prm.H;
   if (blocks <= 0 || blocks > 0x7fffffffLL) return SPSATTN_ERR_TOO_LARGE;
-  prefill_bwd_sm100_kernel<D, FP16, MODE><<<(unsigned)blocks, Cfg::kThreads, Cfg::kSmemBytes, st>>>(x0, x1, y0, y1, prm);
-  return (int)cudaGetLastError();
+  return launch_dependent(prefill_bwd_sm100_kernel<D, FP16, MODE>, dim3((unsigned)blocks), dim3(Cfg::kThreads),
+                          Cfg::kSmemBytes, st, x0, x1, y0, y1, prm);
 }
 
 int run_doc_prepass(const void* doc_ids, int doc_is_i64, int64_t sb, int64_t stt, int B, int N,
@@ -588,12 +588,12 @@ size_t spsattn_prefill_bwd_workspace_bytes(int B, int H, int N, int D) {
          align_up((size_t)B * N * sizeof(int), 256);
 }
 
-int spsattn_prefill_bwd_strided(const void* q, const void* k, const void* v, const void* o, const void* d_o,
+static int prefill_bwd_impl(const void* q, const void* k, const void* v, const void* o, const void* d_o,
                                 const float* lse, void* dq, void* dk, void* dv, const int64_t* strides,
                                 const void* doc_ids, int doc_is_i64, int64_t doc_stride_b,
                                 int64_t doc_stride_t, int B, int H, int N, int D, int dtype, float sm_scale,
                                 int persistent_parity, int temporary_window, int persistent_window,
-                                int mask_flags, void* workspace, size_t workspace_bytes,
+                                int mask_flags, void* forward_workspace, void* workspace, size_t workspace_bytes,
                                 int* device_status, void* stream) {
   if (!q || !k || !v || !o || !d_o || !lse || !dq || !dk || !dv || !strides) return SPSATTN_ERR_ARG;
   if (B <= 0 || H <= 0 || N <= 0) return SPSATTN_ERR_ARG;
@@ -624,25 +624,35 @@ int spsattn_prefill_bwd_strided(const void* q, const void* k, const void* v, con
 
   int *lo = nullptr, *mono = nullptr;
   const size_t pre_bytes = spsattn_prefill_workspace_bytes(B, H, N, D);
-  int rc = run_doc_prepass(doc_ids, doc_is_i64, doc_stride_b, doc_stride_t, B, N, workspace, pre_bytes,
-                           &lo, &mono, st);
+  int rc = 0;
+  if (doc_ids != nullptr && forward_workspace != nullptr) {
+    mono = reinterpret_cast<int*>(forward_workspace);
+    lo = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(forward_workspace) + prefill_ws_mono_bytes(B));
+  } else {
+    rc = run_doc_prepass(doc_ids, doc_is_i64, doc_stride_b, doc_stride_t, B, N, workspace, pre_bytes, &lo, &mono, st);
+  }
   if (rc != 0) return rc;
   float* delta = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + pre_bytes);
   int* hi = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(delta) + align_up((size_t)B * H * N * sizeof(float), 256));
-  if (lo != nullptr) {
-    const long long total = (long long)B * N;
-    bwd_run_end_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(lo, hi, N, total);
-    if ((rc = (int)cudaGetLastError()) != 0) return rc;
-  }
-  const long long rows = (long long)B * H * N;
-  const unsigned dgrid = (unsigned)((rows * (D / 8) + 255) / 256);
-  const DeltaStrides ds = {{so.b, so.h, so.n}, {sg.b, sg.h, sg.n}};
+  BwdPrepareParams pp;
+  pp.o = o;
+  pp.d_o = d_o;
+  pp.delta = delta;
+  pp.rows = (long long)B * H * N;
+  pp.H = H;
+  pp.N = N;
+  pp.st = {{so.b, so.h, so.n}, {sg.b, sg.h, sg.n}};
+  pp.lo = lo;
+  pp.hi = hi;
+  pp.ids = lo != nullptr ? (long long)B * N : 0;
+  pp.delta_blocks = (unsigned)((pp.rows * (D / 8) + 255) / 256);
+  const unsigned pgrid = pp.delta_blocks + (unsigned)((pp.ids + 255) / 256);
   if (D == 64) {
-    if (fp16) bwd_delta_kernel<true, 64><<<dgrid, 256, 0, st>>>(o, d_o, delta, rows, H, N, ds);
-    else bwd_delta_kernel<false, 64><<<dgrid, 256, 0, st>>>(o, d_o, delta, rows, H, N, ds);
+    if (fp16) bwd_prepare_kernel<true, 64><<<pgrid, 256, 0, st>>>(pp);
+    else bwd_prepare_kernel<false, 64><<<pgrid, 256, 0, st>>>(pp);
   } else {
-    if (fp16) bwd_delta_kernel<true, 128><<<dgrid, 256, 0, st>>>(o, d_o, delta, rows, H, N, ds);
-    else bwd_delta_kernel<false, 128><<<dgrid, 256, 0, st>>>(o, d_o, delta, rows, H, N, ds);
+    if (fp16) bwd_prepare_kernel<true, 128><<<pgrid, 256, 0, st>>>(pp);
+    else bwd_prepare_kernel<false, 128><<<pgrid, 256, 0, st>>>(pp);
   }
   if ((rc = (int)cudaGetLastError()) != 0) return rc;
 
@@ -708,6 +718,30 @@ int spsattn_prefill_bwd_strided(const void* q, const void* k, const void* v, con
                 : launch_prefill_bwd<64, false, kBwdDQ>(q128, do128, ks_map, vs_map, prm, st);
   return fp16 ? launch_prefill_bwd<128, true, kBwdDQ>(q128, do128, ks_map, vs_map, prm, st)
               : launch_prefill_bwd<128, false, kBwdDQ>(q128, do128, ks_map, vs_map, prm, st);
+}
+
+int spsattn_prefill_bwd_strided(const void* q, const void* k, const void* v, const void* o, const void* d_o,
+                                const float* lse, void* dq, void* dk, void* dv, const int64_t* strides,
+                                const void* doc_ids, int doc_is_i64, int64_t doc_stride_b,
+                                int64_t doc_stride_t, int B, int H, int N, int D, int dtype, float sm_scale,
+                                int persistent_parity, int temporary_window, int persistent_window,
+                                int mask_flags, void* workspace, size_t workspace_bytes,
+                                int* device_status, void* stream) {
+  return prefill_bwd_impl(q, k, v, o, d_o, lse, dq, dk, dv, strides, doc_ids, doc_is_i64, doc_stride_b, doc_stride_t, B, H, N, D,
+                          dtype, sm_scale, persistent_parity, temporary_window, persistent_window, mask_flags, nullptr,
+                          workspace, workspace_bytes, device_status, stream);
+}
+
+int spsattn_prefill_bwd_after(const void* q, const void* k, const void* v, const void* o, const void* d_o,
+                                const float* lse, void* dq, void* dk, void* dv, const int64_t* strides,
+                                const void* doc_ids, int doc_is_i64, int64_t doc_stride_b,
+                                int64_t doc_stride_t, int B, int H, int N, int D, int dtype, float sm_scale,
+                                int persistent_parity, int temporary_window, int persistent_window,
+                                int mask_flags, void* forward_workspace, void* workspace, size_t workspace_bytes,
+                                int* device_status, void* stream) {
+  return prefill_bwd_impl(q, k, v, o, d_o, lse, dq, dk, dv, strides, doc_ids, doc_is_i64, doc_stride_b, doc_stride_t, B, H, N, D,
+                          dtype, sm_scale, persistent_parity, temporary_window, persistent_window, mask_flags, forward_workspace,
+                          workspace, workspace_bytes, device_status, stream);
 }
 
 int spsattn_prefill_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o,

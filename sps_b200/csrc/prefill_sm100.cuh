@@ -32,6 +32,7 @@ struct PrefillParams {
   const void* docs;      // [B,N] ids or null
   int64_t doc_stride_b, doc_stride_t;
   int doc_is_i64;
+  int scan_docs;         // no pre-pass: every block works its document starts out from the ids
   const int* lo;         // [B,N] run starts (pre-pass, or the caller's) or null
   const int* mono;       // [B] 1 when ids of the row are non-decreasing, or null
   int B, H, N;
@@ -60,6 +61,8 @@ constexpr int kTraceTiles = 40;
 constexpr int kTileM = 128;      // query rows per block
 constexpr int kTileN = 64;       // key tokens per tile
 constexpr int kPrefillThreads = 192;
+constexpr int kScanItems = 6;    // ids per thread where a block works out its document starts itself
+constexpr int kScanRows = kScanItems * kPrefillThreads;
 
 #ifndef SPSATTN_P_SPLIT
 #define SPSATTN_P_SPLIT_DEFAULT 1
@@ -191,6 +194,8 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   __shared__ uint32_t s_tmem_base;
   __shared__ uint32_t s_tmem_p;
   __shared__ int s_abort;
+  __shared__ int s_lo[kTileM];         // scan_docs: run starts of the block's rows
+  __shared__ int s_scan[kPrefillThreads / 32 + 1];
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
@@ -229,40 +234,6 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 
   const bool has_docs = prm.lo != nullptr;      // from document ids or given by the caller
 
-  if (tid == 0 || tid == 32) {
-    // Two planner threads, one per key stream (thread 0: the persistent stream, which holds the
-    // diagonal; thread 32: the other parity).  Launched as a programmatic dependent of the document
-    // pre-pass, the block has run up to here (and its producer warp sets up barriers, the Q load
-    // and tensor memory) beside that kernel; its outputs are read from here on.
-    grid_dependency_wait();
-    const int slot = tid >> 5;
-    // the global words the plan needs are asked for together (the document starts are read
-    // whether or not the ids turn out monotone: the table exists whenever ids were given)
-    int st_word = 0;
-    if (slot == 0 && prm.status != nullptr) st_word = *reinterpret_cast<volatile int*>(prm.status);
-    const int mono_b = (has_docs && prm.mono != nullptr) ? prm.mono[b] : 1;
-    int lo0 = 0, lo1 = 0;
-    if (has_docs) {
-      const int i1 = min(i0 + kTileM - 1, prm.N - 1);
-      lo0 = prm.lo[(size_t)b * prm.N + i0];
-      lo1 = prm.lo[(size_t)b * prm.N + i1];
-    }
-    SPS_TRACE(3 + 8 * slot, 15);
-    if (mono_b == 0) lo0 = lo1 = 0;
-    const bool two = prm.mask.ks != 1;
-    const int stream = two ? (slot == 0 ? prm.mask.pp : 1 - prm.mask.pp) : 0;
-    StreamPlan sp = plan_stream(prm.mask, i0, lo0, lo1, stream, kTileN);
-    if (!two && slot == 1) sp.ntiles = 0;
-    s_plan.sp[slot] = sp;
-    s_plan.stream_id[slot] = stream;
-    if (slot == 0) {
-      // a failure reported by an earlier block turns every later block into a no-op
-      s_abort = st_word != 0 ? 1 : 0;
-      s_plan.general_docs = mono_b == 0 ? 1 : 0;
-      s_plan.n_streams = two ? 2 : 1;
-    }
-    SPS_TRACE(4 + 8 * slot, 15);
-  }
   if (warp == 4) {
     if (lane == 0) {
       mbar_init(bar_q_full, 1);
@@ -291,6 +262,88 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     if constexpr (Cfg::kPSplit) tmem_alloc<Cfg::kPCols>(smem_u32(&s_tmem_p));
     tmem_relinquish();
     if (lane == 0) SPS_TRACE(6, 15);
+  }
+  if (prm.scan_docs) {
+    // Short rows (up to kScanRows) without a pre-pass launch, which costs more than it does: the ids
+    // before and inside this block's rows, kScanItems per thread.  Rows see no later key, so whether
+    // the ids decrease matters only up to here.
+    const uint8_t* ids = reinterpret_cast<const uint8_t*>(prm.docs) + (size_t)b * prm.doc_stride_b * (prm.doc_is_i64 ? 8 : 4);
+    auto id_at = [&](int i) {
+      const size_t off = (size_t)i * prm.doc_stride_t;
+      return prm.doc_is_i64 ? reinterpret_cast<const long long*>(ids)[off]
+                            : (long long)reinterpret_cast<const int*>(ids)[off];
+    };
+    const int n = min(i0 + kTileM, prm.N);
+    const int first = tid * kScanItems;
+    long long id[kScanItems + 1];
+#pragma unroll
+    for (int x = 0; x <= kScanItems; ++x) id[x] = (first + x - 1 >= 0 && first + x - 1 < n) ? id_at(first + x - 1) : 0;
+    int run[kScanItems], from = 0;
+    bool decreases = false;
+#pragma unroll
+    for (int x = 0; x < kScanItems; ++x) {
+      const int i = first + x;
+      if (i > 0 && i < n) {
+        if (id[x + 1] != id[x]) from = i;
+        decreases |= id[x + 1] < id[x];
+      }
+      run[x] = from;
+    }
+    int upto = from;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto = max(upto, u);
+    }
+    if (lane == 31) s_scan[warp] = upto;
+    const int any = __syncthreads_or(decreases);
+    int before = __shfl_up_sync(0xffffffffu, upto, 1);
+    if (lane == 0) before = 0;
+    for (int x = 0; x < warp; ++x) before = max(before, s_scan[x]);
+#pragma unroll
+    for (int x = 0; x < kScanItems; ++x) {
+      const int i = first + x;
+      if (i >= i0 && i < n) s_lo[i - i0] = max(run[x], before);
+    }
+    if (tid == 0) s_scan[kPrefillThreads / 32] = any;
+    __syncthreads();
+  }
+  if (tid == 0 || tid == 32) {
+    // Two planner threads, one per key stream (thread 0: the persistent stream, which holds the
+    // diagonal; thread 32: the other parity).  Launched as a programmatic dependent of the document
+    // pre-pass, the block has run up to here (and its producer warp sets up barriers, the Q load
+    // and tensor memory) beside that kernel; its outputs are read from here on.
+    grid_dependency_wait();
+    const int slot = tid >> 5;
+    // the global words the plan needs are asked for together (the document starts are read
+    // whether or not the ids turn out monotone: the table exists whenever ids were given)
+    int st_word = 0;
+    if (slot == 0 && prm.status != nullptr) st_word = *reinterpret_cast<volatile int*>(prm.status);
+    const int mono_b = prm.scan_docs ? !s_scan[kPrefillThreads / 32] : (has_docs && prm.mono != nullptr) ? prm.mono[b] : 1;
+    int lo0 = 0, lo1 = 0;
+    if (prm.scan_docs) {
+      lo0 = s_lo[0];
+      lo1 = s_lo[min(kTileM - 1, prm.N - 1 - i0)];
+    } else if (has_docs) {
+      const int i1 = min(i0 + kTileM - 1, prm.N - 1);
+      lo0 = prm.lo[(size_t)b * prm.N + i0];
+      lo1 = prm.lo[(size_t)b * prm.N + i1];
+    }
+    SPS_TRACE(3 + 8 * slot, 15);
+    if (mono_b == 0) lo0 = lo1 = 0;
+    const bool two = prm.mask.ks != 1;
+    const int stream = two ? (slot == 0 ? prm.mask.pp : 1 - prm.mask.pp) : 0;
+    StreamPlan sp = plan_stream(prm.mask, i0, lo0, lo1, stream, kTileN);
+    if (!two && slot == 1) sp.ntiles = 0;
+    s_plan.sp[slot] = sp;
+    s_plan.stream_id[slot] = stream;
+    if (slot == 0) {
+      // a failure reported by an earlier block turns every later block into a no-op
+      s_abort = st_word != 0 ? 1 : 0;
+      s_plan.general_docs = mono_b == 0 ? 1 : 0;
+      s_plan.n_streams = two ? 2 : 1;
+    }
+    SPS_TRACE(4 + 8 * slot, 15);
   }
   tc_fence_before();
   __syncthreads();
@@ -458,7 +511,10 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       const uint32_t lane_addr = static_cast<uint32_t>(warp * 32) << 16;
       const bool general = s_plan.general_docs != 0;
       int lo_i = 0;
-      if (has_docs && !general && i < prm.N) lo_i = prm.lo[(size_t)b * prm.N + i];
+      if (!general && i < prm.N) {
+        if (prm.scan_docs) lo_i = s_lo[row];
+        else if (has_docs) lo_i = prm.lo[(size_t)b * prm.N + i];
+      }
       int kmin_s[2], kmax_s[2];
       row_interval(prm.mask, i, lo_i, 0, kmin_s[0], kmax_s[0]);
       row_interval(prm.mask, i, lo_i, 1, kmin_s[1], kmax_s[1]);

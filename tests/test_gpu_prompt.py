@@ -42,3 +42,24 @@ def test_prompt_scan_matches_the_host_rules(t, variant):
     bad[1] = 39
     flags = ext.engine_scan(model, bad.cuda(), 37, 39, 38, False)[6].tolist()
     assert flags[:2] == [int(t > 1), 1]
+
+
+@pytest.mark.parametrize("n,parity", [(2, 0), (128, 1), (130, -1), (1152, 0), (1154, 1)])
+@pytest.mark.parametrize("mode", ["packed", "every_token", "arbitrary", "decreases_late"])
+def test_document_scan_inside_the_attention_equals_the_pre_pass(n, parity, mode):
+    import sps_b200
+    g = torch.Generator().manual_seed(n)
+    q, k, v = (torch.randn(2, 2, n, 64, generator=g).bfloat16().cuda() for _ in range(3))
+    ids = torch.arange(n).expand(2, n) // (50 if mode == "packed" else 2)
+    ids = ids.clone()
+    if mode == "arbitrary":
+        ids = torch.randint(0, 3, (2, n), generator=g)
+    if mode == "decreases_late":
+        ids[:, -1] = 0
+        ids[0, n // 2:] -= 1
+    wide = torch.zeros(2, n, 3, dtype=torch.int32)
+    wide[:, :, 1] = ids
+    for docs in (ids.cuda(), wide.cuda()[:, :, 1]):          # int64 dense, int32 strided
+        call = lambda lse: sps_b200.prefill_attention(q, k, v, 0.125, persistent_parity=parity, temporary_window=7,
+                                                      documents_idx=docs, return_lse=lse)
+        assert torch.equal(call(False), call(True)[0])       # with lse the pre-pass runs

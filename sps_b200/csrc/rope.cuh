@@ -24,7 +24,6 @@ struct RopeGroup {
 
 struct RopeParams {
   const void* x;
-  int x_dtype;                 // 0 bf16, 1 fp16, 2 fp32
   int64_t xs_b, xs_n, xs_h;    // elements
   const float2* freqs;         // [N, D/2] or [B, N, D/2] (cos, sin)
   int64_t fs_b;                // elements of float2 per batch row, 0 when shared
@@ -34,65 +33,87 @@ struct RopeParams {
   int B, N, H, D;
 };
 
-__global__ void __launch_bounds__(256) rope_cast_kernel(const RopeParams p) {
-  const int vec_per_row = p.D / 8;
-  const long long total = (long long)p.B * p.N * p.H * vec_per_row;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const int x8 = (int)(idx % vec_per_row);
-    long long r = idx / vec_per_row;
-    const int h = (int)(r % p.H);
-    r /= p.H;
-    const int n = (int)(r % p.N);
-    const int b = (int)(r / p.N);
-    const size_t src = (size_t)b * p.xs_b + (size_t)n * p.xs_n + (size_t)h * p.xs_h + x8 * 8;
-    float f[8];
-    if (p.x_dtype == 2) {
-      const float4 a = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.x) + src);
-      const float4 c = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.x) + src + 4);
-      f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
-      f[4] = c.x; f[5] = c.y; f[6] = c.z; f[7] = c.w;
-    } else {
-      const uint4 u = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.x) + src);
-      if (p.x_dtype == 1) {
-        unpack2<true>(u.x, f[0], f[1]); unpack2<true>(u.y, f[2], f[3]);
-        unpack2<true>(u.z, f[4], f[5]); unpack2<true>(u.w, f[6], f[7]);
-      } else {
-        unpack2<false>(u.x, f[0], f[1]); unpack2<false>(u.y, f[2], f[3]);
-        unpack2<false>(u.z, f[4], f[5]); unpack2<false>(u.w, f[6], f[7]);
-      }
-    }
-    const int gi = h / p.heads_per_group;
+// Bound: HBM.  A thread keeps its place in the row (head, group, eight elements) and walks down
+// `rows_per_block` rows, two loads in flight, so that nothing is divided per element: one flat index
+// per vector reached half of the bandwidth (65536 rows of 6144: 440 -> 283 us, 5.7 TB/s).
+// X_DTYPE: 0 bf16, 1 fp16, 2 fp32
+template <int X_DTYPE>
+__global__ void __launch_bounds__(256, 4) rope_cast_kernel(const RopeParams p, int rows_per_block) {
+  grid_dependency_wait();
+  const int vec_per_head = p.D / 8, vecs = p.H * vec_per_head;
+  const long long row0 = (long long)blockIdx.x * rows_per_block;
+  const int count = (int)min((long long)rows_per_block, (long long)p.B * p.N - row0);
+  const int b0 = (int)(row0 / p.N), n0 = (int)(row0 - (long long)b0 * p.N);
+  constexpr int kBytes = X_DTYPE == 2 ? 4 : 2, kLoads = kBytes / 2;      // 16-byte loads per vector
+  for (int v = blockIdx.y * 256 + threadIdx.x; v < vecs; v += gridDim.y * 256) {
+    const int h = v / vec_per_head, x8 = v - h * vec_per_head;
+    const int gi = h / p.heads_per_group, hg = h - gi * p.heads_per_group;
     RopeGroup grp = p.group[0];   // selected without indexing the parameter block dynamically
     if (gi == 1) grp = p.group[1];
     if (gi == 2) grp = p.group[2];
     if (gi == 3) grp = p.group[3];
     if (gi == 4) grp = p.group[4];
     if (gi == 5) grp = p.group[5];
-    if (grp.rotate) {
-      const float2* fr = p.freqs + (size_t)b * p.fs_b + (size_t)n * (p.D / 2) + x8 * 4;
-      const float4 c01 = *reinterpret_cast<const float4*>(fr);
-      const float4 c23 = *reinterpret_cast<const float4*>(fr + 2);
-      const float cs[8] = {c01.x, c01.y, c01.z, c01.w, c23.x, c23.y, c23.z, c23.w};
+    const uint8_t* src0 = reinterpret_cast<const uint8_t*>(p.x) + ((int64_t)h * p.xs_h + x8 * 8) * kBytes;
+    uint16_t* dst0 = grp.out + (int64_t)hg * grp.os_h + x8 * 8;
+    const float2* fr0 = p.freqs + x8 * 4;
+    int b = b0, n = n0;
+    constexpr int U = 2;
+    for (int r0 = 0; r0 < count; r0 += U) {
+      uint4 raw[U][kLoads];
+      float4 cs[U][2];
+      uint16_t* dst[U];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float a = f[2 * i], bb = f[2 * i + 1], c = cs[2 * i], s = cs[2 * i + 1];
-        // (a + bi)(c + si), products and sums rounded separately like the complex multiply
-        f[2 * i] = __fsub_rn(__fmul_rn(a, c), __fmul_rn(bb, s));
-        f[2 * i + 1] = __fadd_rn(__fmul_rn(a, s), __fmul_rn(bb, c));
+      for (int u = 0; u < U; ++u) {
+        if (r0 + u >= count) break;
+        const uint4* src = reinterpret_cast<const uint4*>(src0 + (b * p.xs_b + n * p.xs_n) * kBytes);
+#pragma unroll
+        for (int x = 0; x < kLoads; ++x) raw[u][x] = src[x];
+        dst[u] = dst0 + b * grp.os_b + n * grp.os_n;
+        if (grp.rotate) {
+          const float4* fr = reinterpret_cast<const float4*>(fr0 + b * p.fs_b + (int64_t)n * (p.D / 2));
+          cs[u][0] = __ldg(fr);
+          cs[u][1] = __ldg(fr + 1);
+        }
+        if (++n == p.N) n = 0, ++b;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (r0 + u >= count) break;
+        float f[8];
+        if constexpr (X_DTYPE == 2) {
+          const uint32_t w[8] = {raw[u][0].x, raw[u][0].y, raw[u][0].z, raw[u][0].w, raw[u][kLoads - 1].x,
+                                 raw[u][kLoads - 1].y, raw[u][kLoads - 1].z, raw[u][kLoads - 1].w};
+#pragma unroll
+          for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(w[e]);
+        } else {
+          constexpr bool kFp16 = X_DTYPE == 1;
+          unpack2<kFp16>(raw[u][0].x, f[0], f[1]);
+          unpack2<kFp16>(raw[u][0].y, f[2], f[3]);
+          unpack2<kFp16>(raw[u][0].z, f[4], f[5]);
+          unpack2<kFp16>(raw[u][0].w, f[6], f[7]);
+        }
+        if (grp.rotate) {
+          const float c[8] = {cs[u][0].x, cs[u][0].y, cs[u][0].z, cs[u][0].w, cs[u][1].x, cs[u][1].y, cs[u][1].z, cs[u][1].w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float a = f[2 * i], bb = f[2 * i + 1];
+            // (a + bi)(c + si), products and sums rounded separately like the complex multiply
+            f[2 * i] = __fsub_rn(__fmul_rn(a, c[2 * i]), __fmul_rn(bb, c[2 * i + 1]));
+            f[2 * i + 1] = __fadd_rn(__fmul_rn(a, c[2 * i + 1]), __fmul_rn(bb, c[2 * i]));
+          }
+        }
+        uint4 o;
+        if (p.out_fp16) {
+          o.x = pack2<true>(f[0], f[1]); o.y = pack2<true>(f[2], f[3]);
+          o.z = pack2<true>(f[4], f[5]); o.w = pack2<true>(f[6], f[7]);
+        } else {
+          o.x = pack2<false>(f[0], f[1]); o.y = pack2<false>(f[2], f[3]);
+          o.z = pack2<false>(f[4], f[5]); o.w = pack2<false>(f[6], f[7]);
+        }
+        *reinterpret_cast<uint4*>(dst[u]) = o;
       }
     }
-    uint4 o;
-    if (p.out_fp16) {
-      o.x = pack2<true>(f[0], f[1]); o.y = pack2<true>(f[2], f[3]);
-      o.z = pack2<true>(f[4], f[5]); o.w = pack2<true>(f[6], f[7]);
-    } else {
-      o.x = pack2<false>(f[0], f[1]); o.y = pack2<false>(f[2], f[3]);
-      o.z = pack2<false>(f[4], f[5]); o.w = pack2<false>(f[6], f[7]);
-    }
-    const int hg = h - gi * p.heads_per_group;
-    *reinterpret_cast<uint4*>(grp.out + (size_t)b * grp.os_b + (size_t)n * grp.os_n +
-                              (size_t)hg * grp.os_h + x8 * 8) = o;
   }
 }
 

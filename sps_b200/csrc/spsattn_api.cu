@@ -1054,7 +1054,6 @@ static int rope_impl(const void* x, int x_dtype, int64_t xs_b, int64_t xs_n, int
   }
   if (any_rotate && (!freqs_cis || !aligned16(freqs_cis))) return freqs_cis ? SPSATTN_ERR_ALIGN : SPSATTN_ERR_ARG;
   p.x = x;
-  p.x_dtype = x_dtype;
   p.xs_b = xs_b;
   p.xs_n = xs_n;
   p.xs_h = xs_h;
@@ -1066,11 +1065,16 @@ static int rope_impl(const void* x, int x_dtype, int64_t xs_b, int64_t xs_n, int
   p.N = N;
   p.H = heads_per_group * n_groups;
   p.D = D;
-  const long long total = (long long)B * N * p.H * (D / 8);
-  long long blocks = (total + 255) / 256;
-  if (blocks > 148LL * 32) blocks = 148LL * 32;
-  rope_cast_kernel<<<(unsigned)blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(p);
-  return (int)cudaGetLastError();
+  // eight rows per block once that still leaves several blocks per SM, and one block per 256 vectors of a row
+  const long long rows = (long long)B * N;
+  const int rows_per_block = rows >= 148LL * 32 ? 8 : rows >= 148LL * 8 ? 4 : 1;
+  const long long blocks = (rows + rows_per_block - 1) / rows_per_block;
+  if (blocks > 0x7fffffffLL) return SPSATTN_ERR_TOO_LARGE;
+  const unsigned across = (unsigned)((p.H * (D / 8) + 255) / 256);
+  const dim3 grid((unsigned)blocks, across < 65535u ? across : 65535u);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  auto* kernel = x_dtype == 2 ? rope_cast_kernel<2> : x_dtype == 1 ? rope_cast_kernel<1> : rope_cast_kernel<0>;
+  return launch_dependent(kernel, grid, dim3(256), 0, st, p, rows_per_block);
 }
 
 int spsattn_rope_cast(const void* x, int x_dtype, int64_t x_stride_b, int64_t x_stride_n,
@@ -1189,26 +1193,30 @@ int spsattn_kv_update(void* nw_k, void* nw_v, int64_t* nw_len, int64_t* nw_pos, 
     if (!nw_k || !nw_v || !nw_len || !nw_pos || !k_window || !v_window) return SPSATTN_ERR_ARG;
     if (window_storage <= 0) return SPSATTN_ERR_ARG;
   }
+  bool wide = (D * elem_bytes) % 16 == 0;
+  for (const void* ptr : {(const void*)br_k, (const void*)br_v, k_retained, v_retained}) wide = wide && aligned16(ptr);
+  if (window_tokens > 0)
+    for (const void* ptr : {(const void*)nw_k, (const void*)nw_v, k_window, v_window}) wide = wide && aligned16(ptr);
   KvUpdateParams p;
-  p.nw_k = reinterpret_cast<uint32_t*>(nw_k);
-  p.nw_v = reinterpret_cast<uint32_t*>(nw_v);
+  p.nw_k = nw_k;
+  p.nw_v = nw_v;
   p.nw_len = nw_len;
   p.nw_pos = nw_pos;
-  p.br_k = reinterpret_cast<uint32_t*>(br_k);
-  p.br_v = reinterpret_cast<uint32_t*>(br_v);
+  p.br_k = br_k;
+  p.br_v = br_v;
   p.br_len = br_len;
-  p.k_window = reinterpret_cast<const uint32_t*>(k_window);
-  p.v_window = reinterpret_cast<const uint32_t*>(v_window);
-  p.k_retained = reinterpret_cast<const uint32_t*>(k_retained);
-  p.v_retained = reinterpret_cast<const uint32_t*>(v_retained);
+  p.k_window = k_window;
+  p.v_window = v_window;
+  p.k_retained = k_retained;
+  p.v_retained = v_retained;
   p.active = active;
   p.H = H;
-  p.row_words = D * elem_bytes / 4;
+  p.row_vecs = D * elem_bytes / (wide ? 16 : 4);
   p.window_storage = window_storage;
   p.retained_storage = retained_storage;
   p.window_tokens = window_tokens > 0 ? window_tokens : 0;
-  kv_update_kernel<<<S, 256, (size_t)H * sizeof(long long), reinterpret_cast<cudaStream_t>(stream)>>>(p);
-  return (int)cudaGetLastError();
+  return launch_dependent(wide ? kv_update_kernel<uint4> : kv_update_kernel<uint32_t>, dim3((unsigned)S), dim3(256), 0,
+                          reinterpret_cast<cudaStream_t>(stream), p);
 }
 
 // ------------------------------------------------------------------------ block glue (norm, gate)
@@ -1232,11 +1240,10 @@ int spsattn_add_rmsnorm(void* x, const void* delta, const void* weight, void* y,
   p.eps = eps;
   const unsigned blocks = (unsigned)(rows < 148LL * 16 ? rows : 148LL * 16);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (dtype == SPSATTN_DTYPE_BF16)
-    add_rmsnorm_kernel<true><<<blocks, 256, 0, st>>>(p);
-  else
-    add_rmsnorm_kernel<false><<<blocks, 256, 0, st>>>(p);
-  return (int)cudaGetLastError();
+  const bool one = C / vec <= 256;
+  auto* kernel = dtype == SPSATTN_DTYPE_BF16 ? (one ? add_rmsnorm_kernel<true, 1> : add_rmsnorm_kernel<true, 4>)
+                                             : (one ? add_rmsnorm_kernel<false, 1> : add_rmsnorm_kernel<false, 4>);
+  return launch_dependent(kernel, dim3(blocks), dim3(256), 0, st, p);
 }
 
 int spsattn_swiglu(const void* gate_up, void* y, int dtype, long long rows, int I, void* stream) {
@@ -1255,11 +1262,8 @@ int spsattn_swiglu(const void* gate_up, void* y, int dtype, long long rows, int 
   long long blocks = (total + 255) / 256;
   if (blocks > 148LL * 32) blocks = 148LL * 32;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (dtype == SPSATTN_DTYPE_BF16)
-    swiglu_kernel<true><<<(unsigned)blocks, 256, 0, st>>>(p);
-  else
-    swiglu_kernel<false><<<(unsigned)blocks, 256, 0, st>>>(p);
-  return (int)cudaGetLastError();
+  return launch_dependent(dtype == SPSATTN_DTYPE_BF16 ? swiglu_kernel<true> : swiglu_kernel<false>, dim3((unsigned)blocks),
+                          dim3(256), 0, st, p);
 }
 
 }  // extern "C"

@@ -55,6 +55,7 @@ struct DecodeAppend {
   const uint16_t* v_retained;
   const int8_t* active;      // [S]
   int window_storage, retained_storage, window_tokens;
+  int ring_later;            // decode_pair_kernel: a later launch advances the ring counters
 };
 
 struct DecodeParams {
@@ -68,6 +69,7 @@ struct DecodeParams {
   int seg_chunks[kMaxSegments];   // 0 for the short segments of small_segs
   int extras_slot;     // slot of the current-token entries and the short segments, -1 when none
   int pair;            // one block per (sequence, head): decode_pair_kernel
+  int early_rows;      // decode_pair_kernel: nothing launched just before writes the segments' rows
   uint32_t small_segs; // bit x: segment x is short and handled with the entries, on the CUDA cores
   int* status;         // bounded-wait failures are reported here (may be null)
   DecodeAppend app;
@@ -522,10 +524,9 @@ decode_split_kernel(const DecodeParams prm) {
 // The same attention with one block per (sequence, head), for few pairs with short caches, where a
 // launch is bound by latency: a pair's chunks are taken by groups of 128 threads of one block and
 // merged in its shared memory, so no record goes through global memory and no ticket is waited for
-// (about 3 us), the queries and current-token entries are asked for first, every batch of rows is
-// asked for while the one before it is worked on, and the rows are on their way to L2 before the
-// launch that produces the queries has ended.  Chunks, batches and sums are those of
-// decode_split_kernel, so the results are the same bits.
+// (about 3 us), every batch of rows is asked for while the one before it is worked on, and the first
+// batch is in registers before the launch that produces the queries has ended.  Chunks, batches and
+// sums are those of decode_split_kernel, so the results are the same bits.
 constexpr int kPairMaxChunks = 8;
 constexpr int kPairMaxGroups = 4;
 
@@ -540,10 +541,52 @@ __device__ __forceinline__ int live_rows_now(const DecodeSeg& sg, int s, int h, 
   return len < sg.max_rows ? (int)len : sg.max_rows;
 }
 
+// A lane's batch of rows r, r + 4 RPI, ... (kDecodeUnroll of them) of segment x; the next one is
+// 4 RPI kDecodeUnroll rows further on, or the first of a later segment.
+struct PairBatch {
+  int x, r, hi;
+  int64_t row_stride;
+  uint32_t mask;
+  const uint16_t *kb, *vb;
+};
+
+// First batch of the chunk [c_lo, c_hi) in segment b.x or a later one; `off`: this lane's row in it.
+__device__ __forceinline__ void pair_enter(const DecodeParams& prm, int s, int h, const int (&seg_start)[kMaxSegments + 1],
+                                           int c_lo, int c_hi, int off, int dl, PairBatch& b) {
+  const int from = b.x;
+  b.x = kMaxSegments;
+#pragma unroll
+  for (int x = kMaxSegments - 1; x >= 0; --x) {
+    const int lo = max(c_lo, seg_start[x]) - seg_start[x], hi = min(c_hi, seg_start[x + 1]) - seg_start[x];
+    if (x < from || x >= prm.n_segments || lo >= hi) continue;
+    const DecodeSeg& sg = prm.seg[x];
+    const int64_t base = (sg.seq_offset ? sg.seq_offset[s] : (int64_t)s * sg.seq_stride) + (int64_t)h * sg.head_stride + dl;
+    b.x = x;
+    b.hi = hi;
+    b.r = lo + off;
+    b.row_stride = sg.row_stride;
+    b.mask = sg.query_mask;
+    b.kb = reinterpret_cast<const uint16_t*>(sg.k) + base;
+    b.vb = reinterpret_cast<const uint16_t*>(sg.v) + base;
+  }
+}
+
+template <int RPI>
+__device__ __forceinline__ void pair_load(const uint16_t* base, const PairBatch& b, uint4 (&rows)[kDecodeUnroll]) {
+#pragma unroll
+  for (int u = 0; u < kDecodeUnroll; ++u) {
+    const int r = b.r + u * (4 * RPI);
+    rows[u] = make_uint4(0, 0, 0, 0);
+    if (r < b.hi) rows[u] = __ldg(reinterpret_cast<const uint4*>(base + (size_t)r * b.row_stride));
+  }
+}
+
+// `cur`, kr, vr: the chunk's first batch and its rows
 template <int D, int NQ, bool FP16>
 __device__ __forceinline__ void pair_chunk(const DecodeParams& prm, int s, int h, int sh,
                                            const int (&seg_start)[kMaxSegments + 1], int c_lo, int c_hi,
-                                           bool with_extras, float* rec, int tid, PairScratch<D, NQ>& scratch, int bar_id) {
+                                           bool with_extras, float* rec, int tid, PairScratch<D, NQ>& scratch, int bar_id,
+                                           PairBatch cur, uint4 (&kr)[kDecodeUnroll], uint4 (&vr)[kDecodeUnroll]) {
   constexpr int LPR = D / 8;          // lanes per row
   constexpr int RPI = 32 / LPR;       // rows per warp load instruction
   constexpr int U = kDecodeUnroll;
@@ -551,6 +594,7 @@ __device__ __forceinline__ void pair_chunk(const DecodeParams& prm, int s, int h
   const int warp = tid >> 5, lane = tid & 31;
   const int g = lane / LPR;           // row inside a load instruction
   const int dl = (lane % LPR) * 8;    // first of this lane's 8 dims
+  const int off = warp * RPI + g;
   uint4 q_raw[NQ], ek[kMaxExtras], ev[kMaxExtras];
 #pragma unroll
   for (int qi = 0; qi < NQ; ++qi)
@@ -565,40 +609,6 @@ __device__ __forceinline__ void pair_chunk(const DecodeParams& prm, int s, int h
       ev[e] = __ldcg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(prm.extra_v[e]) + (size_t)sh * D + dl));
     }
   }
-  // this lane's batches: rows r, r + 4 RPI, ... of segment x, then STEP further on
-  struct Batch {
-    int x, r, hi;
-    int64_t row_stride;
-    uint32_t mask;
-    const uint16_t *kb, *vb;
-  };
-  const int off = warp * RPI + g;
-  auto enter = [&](Batch& b) {        // first batch of segment b.x or a later one
-    const int from = b.x;
-    b.x = kMaxSegments;
-#pragma unroll
-    for (int x = kMaxSegments - 1; x >= 0; --x) {
-      const int lo = max(c_lo, seg_start[x]) - seg_start[x], hi = min(c_hi, seg_start[x + 1]) - seg_start[x];
-      if (x < from || x >= prm.n_segments || lo >= hi) continue;
-      const DecodeSeg& sg = prm.seg[x];
-      const int64_t base = (sg.seq_offset ? sg.seq_offset[s] : (int64_t)s * sg.seq_stride) + (int64_t)h * sg.head_stride + dl;
-      b.x = x;
-      b.hi = hi;
-      b.r = lo + off;
-      b.row_stride = sg.row_stride;
-      b.mask = sg.query_mask;
-      b.kb = reinterpret_cast<const uint16_t*>(sg.k) + base;
-      b.vb = reinterpret_cast<const uint16_t*>(sg.v) + base;
-    }
-  };
-  auto load = [&](const uint16_t* base, const Batch& b, uint4 (&rows)[U]) {
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int r = b.r + u * (4 * RPI);
-      rows[u] = make_uint4(0, 0, 0, 0);
-      if (r < b.hi) rows[u] = __ldg(reinterpret_cast<const uint4*>(base + (size_t)r * b.row_stride));
-    }
-  };
   float q[NQ][8], m_run[NQ], l_run[NQ], acc[NQ][8];
 #pragma unroll
   for (int qi = 0; qi < NQ; ++qi) {
@@ -660,14 +670,6 @@ __device__ __forceinline__ void pair_chunk(const DecodeParams& prm, int s, int h
     }
   };
 
-  uint4 kr[U], vr[U];
-  Batch cur;
-  cur.x = 0;
-  enter(cur);
-  if (cur.x < kMaxSegments) {
-    load(cur.kb, cur, kr);
-    load(cur.vb, cur, vr);
-  }
 #pragma unroll
   for (int qi = 0; qi < NQ; ++qi) {
     // pre-scaled so that scores are in the log2 domain
@@ -676,17 +678,17 @@ __device__ __forceinline__ void pair_chunk(const DecodeParams& prm, int s, int h
     for (int x = 0; x < 8; ++x) q[qi][x] *= prm.scale_log2;
   }
   while (cur.x < kMaxSegments) {
-    Batch next = cur;
+    PairBatch next = cur;
     next.r += STEP;
     if (next.r - off >= next.hi) {
       ++next.x;
-      enter(next);
+      pair_enter(prm, s, h, seg_start, c_lo, c_hi, off, dl, next);
     }
     const bool more = next.x < kMaxSegments;
     compute(kr, vr, cur.r, cur.hi, cur.mask, [&]() {
-      if (more) load(next.kb, next, kr);
+      if (more) pair_load<RPI>(next.kb, next, kr);
     });
-    if (more) load(next.vb, next, vr);
+    if (more) pair_load<RPI>(next.vb, next, vr);
     cur = next;
   }
   if (extras) {
@@ -756,14 +758,42 @@ __global__ void __launch_bounds__(kPairMaxGroups * kDecodeThreads, 1) decode_pai
   const int tid = threadIdx.x, group = tid / kDecodeThreads, gt = tid % kDecodeThreads;
   const int groups = blockDim.x / kDecodeThreads;
   grid_launch_dependents();
-  // In a decode step nothing before this launch writes these rows (they are those of earlier steps);
-  // the lengths may still be about to be reset, which only makes this ask for rows in vain.
+  const DecodeAppend& ap = prm.app;
+  constexpr int RPI = 32 / (D / 8);
+  const int lane = gt & 31, off = (gt >> 5) * RPI + lane / (D / 8), dl = (lane % (D / 8)) * 8;
+  auto starts = [&](int (&seg_start)[kMaxSegments + 1]) {
+    seg_start[0] = 0;
+#pragma unroll
+    for (int x = 0; x < kMaxSegments; ++x)
+      seg_start[x + 1] = seg_start[x] + (x < prm.n_segments ? live_rows_now(prm.seg[x], s, h, prm.H) : 0);
+  };
+  auto first_batch = [&](const int (&seg_start)[kMaxSegments + 1], int c, PairBatch& cur, uint4 (&kr)[kDecodeUnroll],
+                         uint4 (&vr)[kDecodeUnroll]) {
+    cur.x = 0;
+    pair_enter(prm, s, h, seg_start, c * prm.chunk_rows, min((c + 1) * prm.chunk_rows, seg_start[kMaxSegments]), off, dl, cur);
+    if (cur.x < kMaxSegments) {
+      pair_load<RPI>(cur.kb, cur, kr);
+      pair_load<RPI>(cur.vb, cur, vr);
+    }
+  };
+  // Inside a decode step of a decoder nothing from its start on writes these rows (the launch that
+  // starts the step lets its dependents go only when everything before it is complete), so the first
+  // batch may be read and the other rows sent for before the wait.  Only the lengths may still be about
+  // to be reset: they are looked at again.
+  int seg_start[kMaxSegments + 1] = {};
+  PairBatch cur;
+  uint4 kr[kDecodeUnroll], vr[kDecodeUnroll];
+  bool same = prm.early_rows != 0;
+  if (same) {
+    starts(seg_start);
+    first_batch(seg_start, group, cur, kr, vr);
+  }
 #pragma unroll
   for (int x = 0; x < kMaxSegments; ++x) {
-    if (x >= prm.n_segments) break;
+    if (x >= prm.n_segments || !same) break;
     const DecodeSeg& sg = prm.seg[x];
     if (sg.seq_offset != nullptr) continue;
-    const int live = live_rows_now(sg, s, h, prm.H);
+    const int live = seg_start[x + 1] - seg_start[x];
     const int64_t base = (int64_t)s * sg.seq_stride + (int64_t)h * sg.head_stride;
     for (int r = tid; r < live; r += blockDim.x) {
 #pragma unroll
@@ -775,16 +805,13 @@ __global__ void __launch_bounds__(kPairMaxGroups * kDecodeThreads, 1) decode_pai
   }
   grid_dependency_wait();
 
-  int seg_start[kMaxSegments + 1];
-  seg_start[0] = 0;
-#pragma unroll
-  for (int x = 0; x < kMaxSegments; ++x)
-    seg_start[x + 1] = seg_start[x] + (x < prm.n_segments ? live_rows_now(prm.seg[x], s, h, prm.H) : 0);
-  const int n_total = seg_start[kMaxSegments];
-  // the counters as they are before this step's update
-  const DecodeAppend& ap = prm.app;
+  // the counters as they are before this step's update, and (a thread each) the vectors of the new rows:
+  // K and V for the retained cache, K and V for the ring
   long long ring_len = 0, ring_pos = 0, ret_len = 0;
   bool append = false;
+  constexpr int kRowVecs = D / 8;
+  uint4 fresh = make_uint4(0, 0, 0, 0);
+  const int kind = tid / kRowVecs;
   if (ap.br_len != nullptr) {
     append = ap.active[s] != 0;
     ret_len = __ldcg(ap.br_len + sh);
@@ -792,13 +819,31 @@ __global__ void __launch_bounds__(kPairMaxGroups * kDecodeThreads, 1) decode_pai
       ring_len = __ldcg(ap.nw_len + s);
       ring_pos = __ldcg(ap.nw_pos + s);
     }
+    if (kind < (ap.window_tokens > 0 ? 4 : 2)) {
+      const uint16_t* src = kind == 0 ? ap.k_retained : kind == 1 ? ap.v_retained : kind == 2 ? ap.k_window : ap.v_window;
+      fresh = __ldcg(reinterpret_cast<const uint4*>(src + (size_t)sh * D) + tid % kRowVecs);
+    }
   }
+  {
+    int now[kMaxSegments + 1];
+    starts(now);
+#pragma unroll
+    for (int x = 1; x <= kMaxSegments; ++x) {
+      same = same && now[x] == seg_start[x];
+      seg_start[x] = now[x];
+    }
+    if (!same) first_batch(seg_start, group, cur, kr, vr);
+  }
+  const int n_total = seg_start[kMaxSegments];
   const int chunks = max(1, (n_total + prm.chunk_rows - 1) / prm.chunk_rows);
   for (int c = group; c < chunks; c += groups) {
     // (the record of the group's chunk before is complete: its scratch may be written again)
-    if (c >= groups) asm volatile("bar.sync %0, %1;" ::"r"(2 + group), "n"(kDecodeThreads) : "memory");
+    if (c >= groups) {
+      first_batch(seg_start, c, cur, kr, vr);
+      asm volatile("bar.sync %0, %1;" ::"r"(2 + group), "n"(kDecodeThreads) : "memory");
+    }
     pair_chunk<D, NQ, FP16>(prm, s, h, sh, seg_start, c * prm.chunk_rows, min((c + 1) * prm.chunk_rows, n_total), c == 0,
-                            s_record[c], gt, s_scratch[group], 2 + group);
+                            s_record[c], gt, s_scratch[group], 2 + group, cur, kr, vr);
   }
   __syncthreads();
   // merge_records on shared memory: one group of eight
@@ -821,26 +866,19 @@ __global__ void __launch_bounds__(kPairMaxGroups * kDecodeThreads, 1) decode_pai
       reinterpret_cast<float*>(prm.out)[at] = o;
   }
   if (ap.br_k == nullptr) return;
+  // the pair's rows have all been read: its new rows may be stored
   const bool full = ring_len >= ap.window_tokens;
-  if (append) {
-    const long long ins = full ? ring_pos : ring_len;
-    for (int d = tid; d < D; d += blockDim.x) {
-      const size_t src = (size_t)sh * D + d;
-      if (ap.window_tokens > 0 && ins >= 0 && ins < ap.window_storage) {
-        const size_t dst = ((size_t)sh * ap.window_storage + (size_t)ins) * D + d;
-        ap.nw_k[dst] = __ldcg(ap.k_window + src);
-        ap.nw_v[dst] = __ldcg(ap.v_window + src);
-      }
-      if (ret_len >= 0 && ret_len < ap.retained_storage) {
-        const size_t dst = ((size_t)sh * ap.retained_storage + (size_t)ret_len) * D + d;
-        ap.br_k[dst] = __ldcg(ap.k_retained + src);
-        ap.br_v[dst] = __ldcg(ap.v_retained + src);
-      }
-    }
+  if (append && kind < 4) {
+    const bool ring = kind >= 2;
+    const long long at = ring ? (full ? ring_pos : ring_len) : ret_len;
+    const int storage = ring ? ap.window_storage : ap.retained_storage;
+    uint16_t* dst = kind == 0 ? ap.br_k : kind == 1 ? ap.br_v : kind == 2 ? ap.nw_k : ap.nw_v;
+    if ((!ring || ap.window_tokens > 0) && at >= 0 && at < storage)
+      reinterpret_cast<uint4*>(dst + ((size_t)sh * storage + (size_t)at) * D)[tid % kRowVecs] = fresh;
   }
   if (tid == 0) {
     if (append && ret_len < ap.retained_storage) ap.br_len[sh] = ret_len + 1;
-    if (ap.window_tokens > 0) {
+    if (ap.window_tokens > 0 && !ap.ring_later) {
       // the ring counters belong to the sequence: the last of its heads to get here advances them
       __threadfence();
       int* seq_ticket = prm.tickets + (size_t)prm.S * prm.H + s;

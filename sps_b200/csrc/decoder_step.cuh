@@ -52,12 +52,16 @@ struct SkinnyParams {
   float eps;
   uint16_t* out;             // SwiGLU, logits: [rows, F]; residual: x in place
   float* ssq_out;            // residual: [rows, F / 8]
-  const int8_t* active;      // logits: rows with 0 are written as zeros
+  const int8_t* active;      // [batch]; logits: rows with 0 are written as zeros
   // q, k, v: rows are (sequence, slot); q [rows, C], k and v [slots, batch, C]
   uint16_t *q, *k, *v;
   const float2* freqs;       // [positions, head_dim / 2] (cos, sin)
   const int64_t* pos;        // [batch]
   int slots, batch, head_dim;
+  // residual behind an attention that left it to this launch: the ring counters [batch] of the layer
+  // move on (all heads of that launch have read them), for sequences of `active`
+  int64_t *ring_len, *ring_pos;
+  int ring_tokens;
   int* status;
 };
 
@@ -171,6 +175,7 @@ __global__ void __launch_bounds__(32 * kSkinnyMaxWarps + kSkinnyLoaders) skinny_
   }
 
   // ------------------------------------------------------------------ input rows
+  int64_t pos[MT] = {};                // of the lane's rows (q, k, v)
   if constexpr (kNorm) {
     // a thread takes one vector of 8 columns (at most 256 of them) of every `at_once`-th row
     constexpr int kOwn = 4;            // rows a thread has in flight
@@ -180,6 +185,11 @@ __global__ void __launch_bounds__(32 * kSkinnyMaxWarps + kSkinnyLoaders) skinny_
     uint4 own[kOwn], wgt = make_uint4(0, 0, 0, 0);
     if (mine) wgt = __ldg(reinterpret_cast<const uint4*>(p.norm_w + i * 8));
     grid_dependency_wait();
+    // (asked for here so that the rotary factors can be asked for as soon as the products start)
+    if (EPI == kSkinnyQkv && warp < p.warps) {
+#pragma unroll
+      for (int m = 0; m < MT; ++m) pos[m] = g + 8 * m < p.rows ? __ldcg(p.pos + (g + 8 * m) / p.slots) : 0;
+    }
     const uint16_t* xp = p.x + (size_t)sub * p.x_stride + i * 8;
     const int64_t x_step = (int64_t)at_once * p.x_stride;
 #pragma unroll
@@ -216,6 +226,13 @@ __global__ void __launch_bounds__(32 * kSkinnyMaxWarps + kSkinnyLoaders) skinny_
     }
   } else {
     grid_dependency_wait();
+    if (p.ring_len != nullptr && blockIdx.x == gridDim.x - 1 && tid < p.batch && p.active[tid] != 0) {
+      const int64_t len = p.ring_len[tid], at = p.ring_pos[tid];
+      if (len >= p.ring_tokens)
+        p.ring_pos[tid] = (at + 1) % p.ring_tokens;
+      else
+        p.ring_len[tid] = len + 1;
+    }
     if (loader >= 0)
       for (int n = 0, j = 0; n < first; ++n) {
         load_rows(n, j);
@@ -252,7 +269,7 @@ __global__ void __launch_bounds__(32 * kSkinnyMaxWarps + kSkinnyLoaders) skinny_
         if (r < p.rows && f < p.F) {
           if constexpr (EPI == kSkinnyResidual) old[m] = __ldcg(reinterpret_cast<const uint32_t*>(p.out + (size_t)r * p.F + f));
           if constexpr (EPI == kSkinnyQkv) {
-            if (which < 2) cs[m] = __ldg(p.freqs + __ldcg(p.pos + r / p.slots) * (p.head_dim / 2) + (fi % p.head_dim) / 2);
+            if (which < 2) cs[m] = __ldg(p.freqs + pos[m] * (p.head_dim / 2) + (fi % p.head_dim) / 2);
           }
         }
       }

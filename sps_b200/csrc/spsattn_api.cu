@@ -832,7 +832,8 @@ static int decode_impl(const void* q, int nq, void* out, int out_dtype, const sp
                        int n_segments, const spsattn_extra* extras, int n_extras,
                        const spsattn_kv_append* append, bool single_launch, int S, int H, int D, int dtype,
                        float sm_scale, void* workspace, size_t workspace_bytes, int* tickets,
-                       size_t ticket_bytes, int* device_status, void* stream) {
+                       size_t ticket_bytes, int* device_status, void* stream,
+                       bool* ring_later = nullptr /* inside spsattn_decoder_step */) {
   if (!q || !out) return SPSATTN_ERR_ARG;
   if (nq != 1 && nq != 2) return SPSATTN_ERR_ARG;
   if (S <= 0 || H <= 0) return SPSATTN_ERR_ARG;
@@ -897,7 +898,11 @@ static int decode_impl(const void* q, int nq, void* out, int out_dtype, const sp
     n_chunks = (rows + prm.chunk_rows - 1) / prm.chunk_rows;
     if (n_chunks < 1) n_chunks = 1;
     prm.extras_slot = -1;
-    const bool pair_ok = single_launch && D <= 128 && n_chunks <= kPairMaxChunks;
+    bool pair_ok = single_launch && D <= 128 && n_chunks <= kPairMaxChunks;
+    if (append)        // it stores the new rows by 16 bytes
+      for (const void* ptr : {(const void*)append->br_k, (const void*)append->br_v, append->k_retained, append->v_retained,
+                              (const void*)append->nw_k, (const void*)append->nw_v, append->k_window, append->v_window})
+        pair_ok = pair_ok && aligned16(ptr);
     if (path == 3 && !pair_ok) return SPSATTN_ERR_ARG;
     prm.pair = pair_ok && (path == 3 || (path == 0 && pair_fits(S, H, D, rows)));
   }
@@ -938,6 +943,11 @@ static int decode_impl(const void* q, int nq, void* out, int out_dtype, const sp
     d.window_storage = a.window_storage;
     d.retained_storage = a.retained_storage;
     d.window_tokens = a.window_tokens > 0 ? a.window_tokens : 0;
+  }
+  if (ring_later) {
+    *ring_later = append && prm.pair && prm.app.window_tokens > 0;
+    prm.app.ring_later = *ring_later;
+    prm.early_rows = 1;
   }
   if (single_launch)
     prm.tickets = own_tickets ? reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(workspace) + records) : tickets;
@@ -1434,11 +1444,19 @@ int spsattn_decoder_step(const spsattn_decoder* d, const spsattn_token_source* s
     p.batch = d->batch;
     p.head_dim = d->head_dim;
     if ((rc = launch_skinny<kSkinnyQkv>(p, st)) != 0) return rc;
-    rc = spsattn_decode_step(d->q, d->slots, d->y, SPSATTN_DTYPE_BF16, w.segments, d->n_segments, extras, d->slots,
-                             &w.append, d->batch, d->n_head, d->head_dim, SPSATTN_DTYPE_BF16,
-                             1.0f / sqrtf((float)d->head_dim), d->workspace, d->workspace_bytes, device_status, stream);
+    bool ring_later = false;
+    rc = decode_impl(d->q, d->slots, d->y, SPSATTN_DTYPE_BF16, w.segments, d->n_segments, extras, d->slots, &w.append, true,
+                     d->batch, d->n_head, d->head_dim, SPSATTN_DTYPE_BF16, 1.0f / sqrtf((float)d->head_dim), d->workspace,
+                     d->workspace_bytes, nullptr, 0, device_status, stream, &ring_later);
     if (rc != 0) return rc;
     p = base;
+    if (ring_later) {
+      p.ring_len = w.append.nw_len;
+      p.ring_pos = w.append.nw_pos;
+      p.ring_tokens = w.append.window_tokens;
+      p.active = w.append.active;
+      p.batch = d->batch;
+    }
     p.w = reinterpret_cast<const uint16_t*>(w.c_proj);
     p.x = reinterpret_cast<const uint16_t*>(d->y);
     p.F = C;

@@ -475,6 +475,8 @@ typedef struct spsattn_token_source {
   int64_t* generated;         /* [batch, max_new] */
   int64_t* step;              /* [batch], advanced */
   uint8_t* finished;          /* [batch] */
+  unsigned long long* best;   /* [batch] or NULL: what spsattn_decoder_step leaves behind for the next choice when
+                                 its logits_out is `logits`; the caller zeroes it when it writes `logits` itself */
   int32_t max_new, stop_on_eos;
   const int64_t* token_in;    /* [batch] */
   const uint8_t* active_in;   /* [batch] */

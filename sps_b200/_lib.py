@@ -91,7 +91,7 @@ class TokenSource(C.Structure):
     """struct spsattn_token_source"""
     _fields_ = [
         ("logits", C.c_void_p), ("suppressed", C.c_void_p), ("generated", C.c_void_p), ("step", C.c_void_p),
-        ("finished", C.c_void_p), ("max_new", C.c_int32), ("stop_on_eos", C.c_int32),
+        ("finished", C.c_void_p), ("best", C.c_void_p), ("max_new", C.c_int32), ("stop_on_eos", C.c_int32),
         ("token_in", C.c_void_p), ("active_in", C.c_void_p),
     ]
 

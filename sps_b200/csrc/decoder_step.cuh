@@ -62,6 +62,10 @@ struct SkinnyParams {
   // move on (all heads of that launch have read them), for sequences of `active`
   int64_t *ring_len, *ring_pos;
   int ring_tokens;
+  // logits, if the next token is chosen on the device: the largest choice_key of each row, by atomic
+  // maximum (the start of the step set them to 0); ids whose bit in `suppressed` is set are not chosen
+  unsigned long long* best;  // [rows] or null
+  const uint32_t* suppressed;
   int* status;
 };
 
@@ -100,6 +104,17 @@ __device__ __forceinline__ uint32_t norm_pair(uint32_t x, uint32_t w, float scal
   return pack2<false>(x0 * w0, x1 * w1);
 }
 
+// Greedy choice: the first maximum; a NaN counts as the maximum, as in torch.argmax.  One 64-bit key per
+// logit, its order as an integer, then the complement of its index, so that the largest key is it.
+// Never 0.  u: bits of the logit as fp32.
+__device__ __forceinline__ unsigned long long choice_key(uint32_t u, int i, bool hidden) {
+  if ((u & 0x7fffffffu) == 0) u = 0;                          // -0 equals 0
+  uint32_t order = u & 0x80000000u ? ~u : u | 0x80000000u;
+  if ((u & 0x7fffffffu) > 0x7f800000u) order = 0xffffffffu;   // NaN
+  if (hidden) order = 0x007fffffu;                            // -inf
+  return ((unsigned long long)order << 32) | (uint32_t)~(uint32_t)i;
+}
+
 // MT: tiles of 8 input rows (1 or 2)
 template <int EPI, int MT>
 __global__ void __launch_bounds__(32 * kSkinnyMaxWarps + kSkinnyLoaders) skinny_gemm_kernel(const SkinnyParams p) {
@@ -109,6 +124,7 @@ __global__ void __launch_bounds__(32 * kSkinnyMaxWarps + kSkinnyLoaders) skinny_
   __shared__ __align__(8) uint64_t s_full[kSkinnyMaxStages], s_empty[kSkinnyMaxStages];
   __shared__ int s_abort;
   __shared__ float s_scale[kSkinnyMaxRows];
+  __shared__ unsigned long long s_best[kSkinnyMaxRows];    // logits
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int threads = blockDim.x, loader = tid - (threads - kSkinnyLoaders);     // below 0: not one
   const int g = lane >> 2, t = lane & 3;
@@ -158,6 +174,7 @@ __global__ void __launch_bounds__(32 * kSkinnyMaxWarps + kSkinnyLoaders) skinny_
   };
 
   const int loads = rounds * chunks, first = min(loads, p.stages);
+  if (EPI == kSkinnyLogits && tid < kSkinnyMaxRows) s_best[tid] = 0;
   if (loader == 0) {
     s_abort = 0;
     for (int i = 0; i < p.stages; ++i) {
@@ -254,12 +271,14 @@ __global__ void __launch_bounds__(32 * kSkinnyMaxWarps + kSkinnyLoaders) skinny_
   } else if (warp < p.warps) {
     // ------------------------------------------------------------------ products
     int st = 0, phase = 0;
+    unsigned long long best[MT] = {};
     for (int it = 0; it < rounds; ++it) {
       // lane (g, t): rows g and g + 8, outputs f and f + 1
       const int f = ((int)blockIdx.x + it * (int)gridDim.x) * per_round + warp * 8 + 2 * t;
       // what the epilogue needs besides the sums is asked for here
-      uint32_t old[MT];
+      uint32_t old[MT], hide = 0;
       float2 cs[MT];
+      if (EPI == kSkinnyLogits && p.suppressed != nullptr && f < p.F) hide = __ldg(p.suppressed + (f >> 5)) >> (f & 31);
       const int C = EPI == kSkinnyQkv ? p.F / 3 : 1, which = EPI == kSkinnyQkv ? f / C : 0, fi = f - which * C;
 #pragma unroll
       for (int m = 0; m < MT; ++m) {
@@ -375,6 +394,11 @@ __global__ void __launch_bounds__(32 * kSkinnyMaxWarps + kSkinnyLoaders) skinny_
           const bool on = p.active == nullptr || p.active[r] != 0;
           uint16_t* dst = p.out + (size_t)r * p.F + f;
           const uint32_t both = on ? pack2<false>(v0, v1) : 0u;
+          if (p.best != nullptr && on) {
+            const unsigned long long k0 = choice_key(__float_as_uint(v0), f, hide & 1u);
+            const unsigned long long k1 = f + 1 < p.F ? choice_key(__float_as_uint(v1), f + 1, hide & 2u) : 0;
+            best[m] = max(best[m], max(k0, k1));
+          }
           if (p.F % 2 == 0) {
             *reinterpret_cast<uint32_t*>(dst) = both;
           } else {
@@ -383,6 +407,17 @@ __global__ void __launch_bounds__(32 * kSkinnyMaxWarps + kSkinnyLoaders) skinny_
           }
         }
       }
+    }
+    if (EPI == kSkinnyLogits && p.best != nullptr) {
+      // one atomic per block and row: 1776 warps on one address would queue for longer than they multiply
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        best[m] = max(best[m], __shfl_xor_sync(0xffffffffu, best[m], 1));
+        best[m] = max(best[m], __shfl_xor_sync(0xffffffffu, best[m], 2));
+        if (t == 0 && g + 8 * m < p.rows) atomicMax(&s_best[g + 8 * m], best[m]);
+      }
+      asm volatile("bar.sync 2, %0;" ::"r"(32 * p.warps) : "memory");
+      if (tid < p.rows && s_best[tid] != 0) atomicMax(p.best + tid, s_best[tid]);
     }
   }
   // a step that was given up may leave copies in flight
@@ -393,7 +428,9 @@ __global__ void __launch_bounds__(32 * kSkinnyMaxWarps + kSkinnyLoaders) skinny_
 // Start of a decode step, one block per sequence: choose the token (greedy over the logits of the
 // step before, or the caller's), book-keeping of the sequence's counters, embedding of its rows.
 // Stands in for two dozen small launches of the same steps in tensor operations, which cost more
-// than the projections of a small model.
+// than the projections of a small model.  Bound: latency, a chain of dependent reads.  The choice is
+// left by the head of the step before (SkinnyParams::best): reading 50304 logits again took the block
+// 11 of its 14 us.  They are read here only behind the prefill and behind library projections.
 struct TokenStartParams {
   // greedy choice (logits null: tokens and activity come from token_in / active_in)
   const void* logits;            // [batch, vocab] bf16 or fp32
@@ -401,6 +438,7 @@ struct TokenStartParams {
   int64_t* generated;            // [batch, max_new], written at *step
   int64_t* step;                 // [batch] tokens chosen so far (advanced here)
   uint8_t* finished;             // [batch]
+  unsigned long long* best;      // [batch] largest choice_key of the row, 0: not known; or null
   int max_new, stop_on_eos;
   int choose_only;               // the last token: nothing is embedded or advanced
   const int64_t* token_in;       // [batch]
@@ -430,89 +468,76 @@ constexpr int kStartThreads = 1024;
 template <bool F32>
 __global__ void __launch_bounds__(kStartThreads) token_start_kernel(const TokenStartParams p) {
   __shared__ unsigned long long s_best[kStartThreads / 32];
-  __shared__ int64_t s_token;
-  __shared__ int s_active;
   const int b = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // Dependents are let go only after the wait: what they touch before their own wait (weights) is
   // then no longer being written by anything before this step.
   grid_dependency_wait();
   grid_launch_dependents();
 
+  // All threads read the sequence's state and come to the same choice; thread 0 writes it back at the end.
+  const int64_t n = p.choose_only ? 0 : p.processed[b];
+  const bool starts_doc = !p.choose_only && p.next_doc_start[b] != 0;
+  bool live, newly = false;
+  int64_t chosen, at = 0;
   if (p.logits != nullptr) {
-    // First maximum; a NaN counts as the maximum, as in torch.argmax.  One 64-bit key per logit: its
-    // order as an integer, then the complement of its index, so that the largest key is it.
-    unsigned long long best = 0;
-    auto take = [&](uint32_t u, int i, uint32_t hidden) {     // u: bits of the logit as fp32
-      if ((u & 0x7fffffffu) == 0) u = 0;                      // -0 equals 0
-      uint32_t order = u & 0x80000000u ? ~u : u | 0x80000000u;
-      if ((u & 0x7fffffffu) > 0x7f800000u) order = 0xffffffffu;   // NaN
-      if (hidden) order = 0x007fffffu;                        // -inf
-      const unsigned long long key = ((unsigned long long)order << 32) | (uint32_t)~(uint32_t)i;
-      best = key > best ? key : best;
-    };
-    constexpr int V = F32 ? 4 : 8, U = 4;      // logits per 16-byte load, loads in flight
-    const uint8_t* row = reinterpret_cast<const uint8_t*>(p.logits) + (size_t)b * p.vocab * (F32 ? 4 : 2);
-    if (p.vocab % V == 0) {
-      for (int i0 = tid; i0 < p.vocab / V; i0 += U * kStartThreads) {
-        uint4 u[U];
-        uint32_t hide[U];
+    live = p.finished[b] == 0;
+    at = p.step[b];
+    unsigned long long best = p.best == nullptr ? 0 : __ldcg(p.best + b);
+    if (live && best == 0) {
+      auto take = [&](uint32_t u, int i, uint32_t hidden) { best = max(best, choice_key(u, i, hidden != 0)); };
+      constexpr int V = F32 ? 4 : 8, U = 4;    // logits per 16-byte load, loads in flight
+      const uint8_t* row = reinterpret_cast<const uint8_t*>(p.logits) + (size_t)b * p.vocab * (F32 ? 4 : 2);
+      if (p.vocab % V == 0) {
+        for (int i0 = tid; i0 < p.vocab / V; i0 += U * kStartThreads) {
+          uint4 u[U];
+          uint32_t hide[U];
 #pragma unroll
-        for (int x = 0; x < U; ++x) {
-          const int i = i0 + x * kStartThreads;
-          if (i < p.vocab / V) {
-            u[x] = __ldcg(reinterpret_cast<const uint4*>(row) + i);
-            hide[x] = p.suppressed == nullptr ? 0u : p.suppressed[i * V >> 5] >> (i * V & 31);
+          for (int x = 0; x < U; ++x) {
+            const int i = i0 + x * kStartThreads;
+            if (i < p.vocab / V) {
+              u[x] = __ldcg(reinterpret_cast<const uint4*>(row) + i);
+              hide[x] = p.suppressed == nullptr ? 0u : p.suppressed[i * V >> 5] >> (i * V & 31);
+            }
+          }
+#pragma unroll
+          for (int x = 0; x < U; ++x) {
+            const int i = i0 + x * kStartThreads;
+            if (i < p.vocab / V) {
+              const uint32_t w[4] = {u[x].x, u[x].y, u[x].z, u[x].w};
+#pragma unroll
+              for (int e = 0; e < V; ++e)
+                take(F32 ? w[e * 4 / V] : e & 1 ? w[e * 4 / V] & 0xffff0000u : w[e * 4 / V] << 16, i * V + e, (hide[x] >> e) & 1u);
+            }
           }
         }
-#pragma unroll
-        for (int x = 0; x < U; ++x) {
-          const int i = i0 + x * kStartThreads;
-          if (i < p.vocab / V) {
-            const uint32_t w[4] = {u[x].x, u[x].y, u[x].z, u[x].w};
-#pragma unroll
-            for (int e = 0; e < V; ++e)
-              take(F32 ? w[e * 4 / V] : e & 1 ? w[e * 4 / V] & 0xffff0000u : w[e * 4 / V] << 16, i * V + e, (hide[x] >> e) & 1u);
-          }
-        }
+      } else {
+        for (int i = tid; i < p.vocab; i += kStartThreads)
+          take(F32 ? reinterpret_cast<const uint32_t*>(row)[i] : (uint32_t)reinterpret_cast<const uint16_t*>(row)[i] << 16, i,
+               p.suppressed == nullptr ? 0u : (p.suppressed[i >> 5] >> (i & 31)) & 1u);
       }
-    } else {
-      for (int i = tid; i < p.vocab; i += kStartThreads)
-        take(F32 ? reinterpret_cast<const uint32_t*>(row)[i] : (uint32_t)reinterpret_cast<const uint16_t*>(row)[i] << 16, i,
-             p.suppressed == nullptr ? 0u : (p.suppressed[i >> 5] >> (i & 31)) & 1u);
-    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long k = __shfl_xor_sync(0xffffffffu, best, o);
-      best = k > best ? k : best;
+      for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+      if (lane == 0) s_best[warp] = best;
+      __syncthreads();
+      best = s_best[lane];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
     }
-    if (lane == 0) s_best[warp] = best;
-    __syncthreads();
-    if (tid == 0) {
-      for (int w = 1; w < kStartThreads / 32; ++w) best = s_best[w] > best ? s_best[w] : best;
-      const bool live = p.finished[b] == 0;
-      const int64_t token = live ? (int64_t)(uint32_t)~(uint32_t)best : p.pad;
-      const int64_t at = p.step[b];
-      if (at < p.max_new) p.generated[(size_t)b * p.max_new + at] = token;
-      const bool newly = live && p.stop_on_eos && token == p.eos;
-      s_token = token;
-      s_active = live && !newly;
-      if (!p.choose_only) {
-        p.step[b] = at + 1;
-        if (newly) p.finished[b] = 1;
-      }
+    chosen = live ? (int64_t)(uint32_t)~(uint32_t)best : p.pad;
+    newly = live && p.stop_on_eos && chosen == p.eos;
+    if (p.choose_only) {
+      if (tid == 0 && at < p.max_new) p.generated[(size_t)b * p.max_new + at] = chosen;
+      return;
     }
-    if (p.choose_only) return;
-  } else if (tid == 0) {
-    s_token = p.token_in[b];
-    s_active = p.active_in[b] != 0;
+  } else {
+    chosen = p.token_in[b];
+    live = p.active_in[b] != 0;
   }
-  __syncthreads();
-  const bool active = s_active != 0;
-  const int64_t token = active ? s_token : 0;
-  const int64_t n = p.processed[b];
+  const bool active = live && !newly;
+  const int64_t token = active ? chosen : 0;
 
   // a row that starts a document forgets its caches, in every layer
-  if (active && p.next_doc_start[b] != 0) {
+  if (active && starts_doc) {
     for (int i = tid; i < p.layers * p.heads; i += kStartThreads)
       p.br_len[((size_t)(i / p.heads) * p.batch + b) * p.heads + i % p.heads] = 0;
     for (int i = tid; i < p.layers; i += kStartThreads) {
@@ -544,13 +569,19 @@ __global__ void __launch_bounds__(kStartThreads) token_start_kernel(const TokenS
   if (p.freqs_out != nullptr)
     for (int i = tid; i < p.half_dim; i += kStartThreads)
       p.freqs_out[(size_t)b * p.half_dim + i] = p.freqs[(active ? n : 0) * p.half_dim + i];
-  __syncthreads();               // everybody has read next_doc_start and processed
+  __syncthreads();               // everybody has read the state
   if (tid == 0) {
+    if (p.logits != nullptr) {
+      if (at < p.max_new) p.generated[(size_t)b * p.max_new + at] = chosen;
+      p.step[b] = at + 1;
+      if (newly) p.finished[b] = 1;
+      if (p.best != nullptr) p.best[b] = 0;
+    }
     p.active[b] = active ? 1 : 0;
     p.pos[b] = active ? n : 0;
     if (active) {
       p.processed[b] = n + 1;
-      p.next_doc_start[b] = s_token == p.eos ? 1 : 0;
+      p.next_doc_start[b] = chosen == p.eos ? 1 : 0;
     }
   }
 }

@@ -1343,6 +1343,7 @@ int launch_token_start(const spsattn_decoder* d, const spsattn_token_source* src
   p.generated = src->generated;
   p.step = src->step;
   p.finished = src->finished;
+  p.best = src->best;
   p.max_new = src->max_new;
   p.stop_on_eos = src->stop_on_eos;
   p.choose_only = choose_only;
@@ -1488,6 +1489,8 @@ int spsattn_decoder_step(const spsattn_decoder* d, const spsattn_token_source* s
   p.ssq_stride = (int64_t)d->slots * (C / 8);
   p.out = reinterpret_cast<uint16_t*>(logits_out);
   p.active = d->active;
+  p.best = source->logits == logits_out ? source->best : nullptr;
+  p.suppressed = source->suppressed;
   return launch_skinny<kSkinnyLogits>(p, st);
 }
 

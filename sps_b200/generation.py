@@ -504,7 +504,7 @@ class SPSGenerator:
         g.next_logits.copy_(next_logits)
         g.generated.fill_(d.pad_token_id)
         g.finished.fill_(False)
-        g.step_idx.zero_()
+        g.counters.zero_()
         ev[2].record()
         for _ in range(n_steps):
             if use_graph:
@@ -536,7 +536,7 @@ class SPSGenerator:
         g.step = self._step
         g.generated = torch.full((b, max_new), d.pad_token_id, device=dev, dtype=torch.long)
         g.finished = torch.zeros(b, device=dev, dtype=torch.bool)
-        g.step_idx = torch.zeros(b, device=dev, dtype=torch.long)
+        g.counters = torch.zeros((2, b), device=dev, dtype=torch.long)       # tokens chosen; keys of the next choice
         g.next_logits = torch.zeros((b, d.vocab_size), device=dev, dtype=self.param_dtype)
         words = torch.zeros((d.vocab_size + 31) // 32, dtype=torch.long)      # suppressed ids, a bit each
         ids = torch.tensor(key[4], dtype=torch.long)
@@ -544,7 +544,8 @@ class SPSGenerator:
         g.suppressed = torch.where(words >= 1 << 31, words - (1 << 32), words).to(torch.int32).to(dev)
         src = g.source = _lib.TokenSource()
         src.logits, src.suppressed = g.next_logits.data_ptr(), g.suppressed.data_ptr()
-        src.generated, src.step, src.finished = g.generated.data_ptr(), g.step_idx.data_ptr(), g.finished.data_ptr()
+        src.generated, src.step, src.finished = g.generated.data_ptr(), g.counters[0].data_ptr(), g.finished.data_ptr()
+        src.best = g.counters[1].data_ptr()
         src.max_new, src.stop_on_eos = max_new, int(key[3])
         self._session = g
         return g

@@ -84,3 +84,37 @@ def test_greedy_choice_is_the_first_unsuppressed_maximum(dtype, vocab):
     keep = [i for i in range(batch) if not (i == 2 and vocab // 2 in hidden)]     # a hidden NaN counts as hidden
     assert torch.equal(out[keep, 1].cpu(), want[keep])
     assert bool((out[:, 0] == -1).all())
+
+
+@pytest.mark.parametrize("variant,batch,heads,hidden,vocab", [
+    ("standard", 1, 1, 64, 33),           # one warp with one output past the end
+    ("reverse_sps", 8, 2, 128, 9473),     # eight rows, several rounds, odd vocabulary
+    ("standard", 13, 2, 128, 50304),      # two row tiles
+])
+def test_head_leaves_the_choice_of_the_next_token(variant, batch, heads, hidden, vocab):
+    """The key that the head leaves is that of the first unsuppressed maximum of the logits it wrote;
+    a finished row leaves none, and the start of the step takes the old ones away."""
+    import sps_b200
+    engine, dims = _engine(variant, 1, heads, hidden, 64, vocab)
+    g = torch.Generator().manual_seed(11)
+    prompt = torch.randint(0, vocab - 3, (batch, 5), generator=g)
+    hidden_ids = torch.randperm(vocab - 3, generator=g)[: vocab // 2]
+    engine.generate(prompt, 3, stop_on_eos=False, forbidden_token_ids=hidden_ids, use_graph=False)
+    s = engine._session
+    assert engine._step.fused
+    s.finished[batch // 2] = batch > 1
+    s.counters[0].zero_()
+    engine._token_body(s)
+    sps_b200.check_device_status()
+    z = s.next_logits.float()
+    z[:, hidden_ids.to(z.device)] = float("-inf")
+    z[:, dims.pad_token_id] = float("-inf")
+    if engine.n_slot == 2:
+        z[:, dims.predict_token_id] = float("-inf")
+    want = torch.stack([torch.argmax(r) for r in z])
+    got = (~s.counters[1]) & 0xffffffff
+    for r in range(batch):
+        if batch > 1 and r == batch // 2:
+            assert int(s.counters[1][r]) == 0
+        else:
+            assert int(got[r]) == int(want[r])

@@ -535,11 +535,27 @@ struct PairScratch {
   float m[4][NQ], l[4][NQ], acc[4][NQ][D];
 };
 
-__device__ __forceinline__ int live_rows_now(const DecodeSeg& sg, int s, int h, int H) {
-  long long len = __ldcg(sg.lengths + (sg.lengths_per_head ? (size_t)s * H + h : (size_t)s));
-  if (len < 0) len = 0;
-  return len < sg.max_rows ? (int)len : sg.max_rows;
-}
+// Live rows of the segments, laid end to end.  The lengths are asked for together: one at a time, each
+// behind a branch, they and the counters were 3200 of the block's 11000 clocks.
+struct PairLengths {
+  long long raw[kMaxSegments];
+  __device__ __forceinline__ void ask(const DecodeParams& prm, int s, int sh) {
+#pragma unroll
+    for (int x = 0; x < kMaxSegments; ++x) {
+      const DecodeSeg& sg = prm.seg[x];
+      raw[x] = 0;
+      if (x < prm.n_segments) raw[x] = __ldcg(sg.lengths + (sg.lengths_per_head ? sh : s));
+    }
+  }
+  __device__ __forceinline__ void starts(const DecodeParams& prm, int (&seg_start)[kMaxSegments + 1]) const {
+    seg_start[0] = 0;
+#pragma unroll
+    for (int x = 0; x < kMaxSegments; ++x) {
+      const long long len = raw[x] < 0 ? 0 : raw[x];
+      seg_start[x + 1] = seg_start[x] + (x >= prm.n_segments ? 0 : len < prm.seg[x].max_rows ? (int)len : prm.seg[x].max_rows);
+    }
+  }
+};
 
 // A lane's batch of rows r, r + 4 RPI, ... (kDecodeUnroll of them) of segment x; the next one is
 // 4 RPI kDecodeUnroll rows further on, or the first of a later segment.
@@ -581,12 +597,14 @@ __device__ __forceinline__ void pair_load(const uint16_t* base, const PairBatch&
   }
 }
 
-// `cur`, kr, vr: the chunk's first batch and its rows
+// `cur`, kr, vr: the chunk's first batch and its rows; `entries`: current-token rows in shared memory, K
+// and V in turn, copied there by the warp that reads them (asynchronously, it still has to wait)
 template <int D, int NQ, bool FP16>
 __device__ __forceinline__ void pair_chunk(const DecodeParams& prm, int s, int h, int sh,
                                            const int (&seg_start)[kMaxSegments + 1], int c_lo, int c_hi,
                                            bool with_extras, float* rec, int tid, PairScratch<D, NQ>& scratch, int bar_id,
-                                           PairBatch cur, uint4 (&kr)[kDecodeUnroll], uint4 (&vr)[kDecodeUnroll]) {
+                                           const uint4 (&q_raw)[NQ], uint32_t entries, PairBatch cur, uint4 (&kr)[kDecodeUnroll],
+                                           uint4 (&vr)[kDecodeUnroll]) {
   constexpr int LPR = D / 8;          // lanes per row
   constexpr int RPI = 32 / LPR;       // rows per warp load instruction
   constexpr int U = kDecodeUnroll;
@@ -595,20 +613,7 @@ __device__ __forceinline__ void pair_chunk(const DecodeParams& prm, int s, int h
   const int g = lane / LPR;           // row inside a load instruction
   const int dl = (lane % LPR) * 8;    // first of this lane's 8 dims
   const int off = warp * RPI + g;
-  uint4 q_raw[NQ], ek[kMaxExtras], ev[kMaxExtras];
-#pragma unroll
-  for (int qi = 0; qi < NQ; ++qi)
-    q_raw[qi] = __ldcg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(prm.q) +
-                                                      (((size_t)s * NQ + qi) * prm.H + h) * D + dl));
   const bool extras = with_extras && warp == 0;
-#pragma unroll
-  for (int e = 0; e < kMaxExtras; ++e) {
-    ek[e] = ev[e] = make_uint4(0, 0, 0, 0);
-    if (extras && e < prm.n_extras) {
-      ek[e] = __ldcg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(prm.extra_k[e]) + (size_t)sh * D + dl));
-      ev[e] = __ldcg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(prm.extra_v[e]) + (size_t)sh * D + dl));
-    }
-  }
   float q[NQ][8], m_run[NQ], l_run[NQ], acc[NQ][8];
 #pragma unroll
   for (int qi = 0; qi < NQ; ++qi) {
@@ -692,13 +697,39 @@ __device__ __forceinline__ void pair_chunk(const DecodeParams& prm, int s, int h
     cur = next;
   }
   if (extras) {
-    // one row each, in lane group 0, as batches whose other rows are masked
+    // one row each, in lane group 0, one after the other; their scores are made at once
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+    float sc[kMaxExtras][NQ];
 #pragma unroll
     for (int e = 0; e < kMaxExtras; ++e) {
       if (e >= prm.n_extras) break;
-      const uint4 zero = make_uint4(0, 0, 0, 0);
-      const uint4 k4[U] = {g == 0 ? ek[e] : zero, zero, zero, zero}, v4[U] = {g == 0 ? ev[e] : zero, zero, zero, zero};
-      compute(k4, v4, g, 1, prm.extra_mask[e], []() {});
+      float kf[8];
+      unpack8(lds16(entries + (2 * e * D + dl) * 2), kf);
+#pragma unroll
+      for (int qi = 0; qi < NQ; ++qi) {
+        float d = 0.f;
+#pragma unroll
+        for (int x = 0; x < 8; ++x) d = fmaf(q[qi][x], kf[x], d);
+#pragma unroll
+        for (int o = LPR / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+        sc[e][qi] = g == 0 && ((prm.extra_mask[e] >> qi) & 1u) ? d : -INFINITY;
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < kMaxExtras; ++e) {
+      if (e >= prm.n_extras) break;
+      float vf[8];
+      unpack8(lds16(entries + ((2 * e + 1) * D + dl) * 2), vf);
+#pragma unroll
+      for (int qi = 0; qi < NQ; ++qi) {
+        const float mx = fmaxf(m_run[qi], sc[e][qi]);
+        const float alpha = fast_exp2(m_run[qi] - mx), p = fast_exp2(sc[e][qi] - mx);
+        l_run[qi] = l_run[qi] * alpha + p;
+        m_run[qi] = mx;
+#pragma unroll
+        for (int x = 0; x < 8; ++x) acc[qi][x] = fmaf(p, vf[x], acc[qi][x] * alpha);
+      }
     }
   }
 
@@ -753,6 +784,7 @@ template <int D, int NQ, bool FP16>
 __global__ void __launch_bounds__(kPairMaxGroups * kDecodeThreads, 1) decode_pair_kernel(const DecodeParams prm) {
   __shared__ PairScratch<D, NQ> s_scratch[kPairMaxGroups];
   __shared__ float s_record[kPairMaxChunks][NQ * (D + 2)];
+  __shared__ __align__(16) uint16_t s_rows[(2 * kMaxExtras + 4) * D];     // current-token entries, rows to store
   const int sh = blockIdx.x;
   const int s = sh / prm.H, h = sh % prm.H;
   const int tid = threadIdx.x, group = tid / kDecodeThreads, gt = tid % kDecodeThreads;
@@ -761,12 +793,6 @@ __global__ void __launch_bounds__(kPairMaxGroups * kDecodeThreads, 1) decode_pai
   const DecodeAppend& ap = prm.app;
   constexpr int RPI = 32 / (D / 8);
   const int lane = gt & 31, off = (gt >> 5) * RPI + lane / (D / 8), dl = (lane % (D / 8)) * 8;
-  auto starts = [&](int (&seg_start)[kMaxSegments + 1]) {
-    seg_start[0] = 0;
-#pragma unroll
-    for (int x = 0; x < kMaxSegments; ++x)
-      seg_start[x + 1] = seg_start[x] + (x < prm.n_segments ? live_rows_now(prm.seg[x], s, h, prm.H) : 0);
-  };
   auto first_batch = [&](const int (&seg_start)[kMaxSegments + 1], int c, PairBatch& cur, uint4 (&kr)[kDecodeUnroll],
                          uint4 (&vr)[kDecodeUnroll]) {
     cur.x = 0;
@@ -785,7 +811,9 @@ __global__ void __launch_bounds__(kPairMaxGroups * kDecodeThreads, 1) decode_pai
   uint4 kr[kDecodeUnroll], vr[kDecodeUnroll];
   bool same = prm.early_rows != 0;
   if (same) {
-    starts(seg_start);
+    PairLengths lengths;
+    lengths.ask(prm, s, sh);
+    lengths.starts(prm, seg_start);
     first_batch(seg_start, group, cur, kr, vr);
   }
 #pragma unroll
@@ -805,15 +833,29 @@ __global__ void __launch_bounds__(kPairMaxGroups * kDecodeThreads, 1) decode_pai
   }
   grid_dependency_wait();
 
-  // the counters as they are before this step's update, and (a thread each) the vectors of the new rows:
-  // K and V for the retained cache, K and V for the ring
-  long long ring_len = 0, ring_pos = 0, ret_len = 0;
-  bool append = false;
+  // What the block needs from memory now is asked for at once: the queries and current-token entries, the
+  // lengths, the counters as they are before this step's update, and (a thread each) the vectors of the
+  // new rows: K and V for the retained cache, K and V for the ring.
+  uint4 q_raw[NQ];
+  PairLengths lengths;
+#pragma unroll
+  for (int qi = 0; qi < NQ; ++qi)
+    q_raw[qi] = __ldcg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(prm.q) +
+                                                      (((size_t)s * NQ + qi) * prm.H + h) * D + dl));
+  lengths.ask(prm, s, sh);
   constexpr int kRowVecs = D / 8;
-  uint4 fresh = make_uint4(0, 0, 0, 0);
+  const uint32_t entries = smem_u32(s_rows), new_rows = entries + 2 * kMaxExtras * D * 2;
+  if (tid < 32)
+    for (int i = tid; i < 2 * prm.n_extras * kRowVecs; i += 32) {
+      const int row = i / kRowVecs;
+      const void* src = (row & 1) ? prm.extra_v[row >> 1] : prm.extra_k[row >> 1];
+      copy16(entries + i * 16, reinterpret_cast<const uint16_t*>(src) + (size_t)sh * D + (i - row * kRowVecs) * 8);
+    }
+  long long ring_len = 0, ring_pos = 0, ret_len = 0;
+  int8_t active = 0;
   const int kind = tid / kRowVecs;
   if (ap.br_len != nullptr) {
-    append = ap.active[s] != 0;
+    active = __ldcg(ap.active + s);
     ret_len = __ldcg(ap.br_len + sh);
     if (ap.window_tokens > 0) {
       ring_len = __ldcg(ap.nw_len + s);
@@ -821,12 +863,12 @@ __global__ void __launch_bounds__(kPairMaxGroups * kDecodeThreads, 1) decode_pai
     }
     if (kind < (ap.window_tokens > 0 ? 4 : 2)) {
       const uint16_t* src = kind == 0 ? ap.k_retained : kind == 1 ? ap.v_retained : kind == 2 ? ap.k_window : ap.v_window;
-      fresh = __ldcg(reinterpret_cast<const uint4*>(src + (size_t)sh * D) + tid % kRowVecs);
+      copy16(new_rows + tid * 16, src + (size_t)sh * D + tid % kRowVecs * 8);
     }
   }
   {
     int now[kMaxSegments + 1];
-    starts(now);
+    lengths.starts(prm, now);
 #pragma unroll
     for (int x = 1; x <= kMaxSegments; ++x) {
       same = same && now[x] == seg_start[x];
@@ -843,7 +885,7 @@ __global__ void __launch_bounds__(kPairMaxGroups * kDecodeThreads, 1) decode_pai
       asm volatile("bar.sync %0, %1;" ::"r"(2 + group), "n"(kDecodeThreads) : "memory");
     }
     pair_chunk<D, NQ, FP16>(prm, s, h, sh, seg_start, c * prm.chunk_rows, min((c + 1) * prm.chunk_rows, n_total), c == 0,
-                            s_record[c], gt, s_scratch[group], 2 + group, cur, kr, vr);
+                            s_record[c], gt, s_scratch[group], 2 + group, q_raw, entries, cur, kr, vr);
   }
   __syncthreads();
   // merge_records on shared memory: one group of eight
@@ -867,14 +909,15 @@ __global__ void __launch_bounds__(kPairMaxGroups * kDecodeThreads, 1) decode_pai
   }
   if (ap.br_k == nullptr) return;
   // the pair's rows have all been read: its new rows may be stored
-  const bool full = ring_len >= ap.window_tokens;
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  const bool full = ring_len >= ap.window_tokens, append = active != 0;
   if (append && kind < 4) {
     const bool ring = kind >= 2;
     const long long at = ring ? (full ? ring_pos : ring_len) : ret_len;
     const int storage = ring ? ap.window_storage : ap.retained_storage;
     uint16_t* dst = kind == 0 ? ap.br_k : kind == 1 ? ap.br_v : kind == 2 ? ap.nw_k : ap.nw_v;
     if ((!ring || ap.window_tokens > 0) && at >= 0 && at < storage)
-      reinterpret_cast<uint4*>(dst + ((size_t)sh * storage + (size_t)at) * D)[tid % kRowVecs] = fresh;
+      reinterpret_cast<uint4*>(dst + ((size_t)sh * storage + (size_t)at) * D)[tid % kRowVecs] = lds16(new_rows + tid * 16);
   }
   if (tid == 0) {
     if (append && ret_len < ap.retained_storage) ap.br_len[sh] = ret_len + 1;

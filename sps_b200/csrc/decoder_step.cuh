@@ -87,9 +87,6 @@ __device__ __forceinline__ uint2 lds8(uint32_t addr) {
   return v;
 }
 
-__device__ __forceinline__ void copy16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
 // one arrival when every copy that this thread has asked for so far is complete
 __device__ __forceinline__ void copies_arrive(uint32_t bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");

@@ -11,16 +11,16 @@ __device__ __forceinline__ long long load_doc(const void* docs, int is_i64, size
                 : (long long)reinterpret_cast<const int*>(docs)[off];
 }
 
-// One block per batch row: lo[b][i] = first row of the run of equal ids containing row i
-// (inclusive max-scan of run-start positions), mono[b] = 1 iff the ids never decrease.
-// Each thread scans kItems consecutive rows, so rows up to 8192 need a single pass.
+// One block per batch row: lo[b][i] = first row of the run of equal ids containing row i, mono[b] = 1
+// iff the ids never decrease.  Bound by latency (a few thousand ids): every warp asks for the ids of 256
+// consecutive rows at once, coalesced, finds the run starts of 32 rows by a ballot, and one barrier
+// carries the last start of each warp to those after it.  (With eight neighbouring rows per thread and a
+// shuffle scan over them: 5.3 instead of 3.6 us at 3 x 3001 rows and 10.1 instead of 4.7 at 8 x 8192.)
 __global__ void __launch_bounds__(1024)
 doc_prepass_kernel(const void* docs, int is_i64, int64_t stride_b, int64_t stride_t, int N,
                    int* __restrict__ lo, int* __restrict__ mono, int* __restrict__ work_counter) {
-  constexpr int kItems = 8;
-  __shared__ int s_warp[32];
-  __shared__ int s_carry;
-  __shared__ int s_mono;
+  constexpr int kItems = 8;            // rows up to 8192 need a single pass
+  __shared__ int s_last[2][32];        // last run start of a warp's rows (two passes' worth)
   const int b = blockIdx.x;
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
@@ -29,64 +29,45 @@ doc_prepass_kernel(const void* docs, int is_i64, int64_t stride_b, int64_t strid
   grid_launch_dependents();
   const uint8_t* base =
       reinterpret_cast<const uint8_t*>(docs) + (size_t)b * stride_b * (is_i64 ? 8 : 4);
-  if (tid == 0) {
-    s_carry = 0;
-    s_mono = 1;
-    // the attention kernel that follows in the stream draws its work items from this counter
-    if (b == 0 && work_counter != nullptr) *work_counter = 0;
-  }
-  __syncthreads();
-  bool dec = false;
-  for (int c0 = 0; c0 < N; c0 += 1024 * kItems) {
-    const int i0 = c0 + tid * kItems;
-    int v[kItems];
-    long long prev = 0;
-    if (i0 > 0 && i0 - 1 < N) prev = load_doc(base, is_i64, (size_t)(i0 - 1) * stride_t);
-    int run = 0;
+  // the attention kernel that follows in the stream draws its work items from this counter
+  if (tid == 0 && b == 0 && work_counter != nullptr) *work_counter = 0;
+  int carry = 0, decreases = 0;
+  for (int c0 = 0, pass = 0; c0 < N; c0 += 1024 * kItems, pass ^= 1) {
+    const int w0 = c0 + warp * 32 * kItems;
+    long long id[kItems], edge = 0;
 #pragma unroll
     for (int x = 0; x < kItems; ++x) {
-      const int i = i0 + x;
-      if (i < N) {
-        const long long d = load_doc(base, is_i64, (size_t)i * stride_t);
-        if (i > 0) {
-          if (d != prev) run = i;
-          dec |= d < prev;
-        }
-        prev = d;
-      }
-      v[x] = run;   // inclusive max of the run starts inside this thread's span
+      const int i = w0 + x * 32 + lane;
+      id[x] = i < N ? load_doc(base, is_i64, (size_t)i * stride_t) : 0;
     }
-    int tot = run;
+    if (lane == 0 && w0 > 0 && w0 < N) edge = load_doc(base, is_i64, (size_t)(w0 - 1) * stride_t);
+    int start[kItems], last = 0;       // run starts as far as this warp's rows tell
+    bool dec = false;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int u = __shfl_up_sync(0xffffffffu, tot, o);
-      if (lane >= o) tot = max(tot, u);
+    for (int x = 0; x < kItems; ++x) {
+      const int i = w0 + x * 32 + lane;
+      long long prev = __shfl_up_sync(0xffffffffu, id[x], 1);
+      const long long tail = x > 0 ? __shfl_sync(0xffffffffu, id[x > 0 ? x - 1 : 0], 31) : edge;
+      if (lane == 0) prev = tail;
+      const bool inside = i > 0 && i < N;
+      dec |= inside && id[x] < prev;
+      const uint32_t starts = __ballot_sync(0xffffffffu, inside && id[x] != prev);
+      const uint32_t upto = starts & (0xffffffffu >> (31 - lane));
+      start[x] = upto ? i - lane + 31 - __clz(upto) : last;
+      if (starts) last = w0 + x * 32 + 31 - __clz(starts);
     }
-    if (lane == 31) s_warp[warp] = tot;
-    __syncthreads();
-    if (warp == 0) {
-      int wv = s_warp[lane];
+    if (lane == 0) s_last[pass][warp] = last;
+    decreases |= __syncthreads_or(dec);
+    const int of_warp = s_last[pass][lane];
+    const int before = max(carry, __reduce_max_sync(0xffffffffu, lane < warp ? of_warp : 0));
+    carry = max(carry, __reduce_max_sync(0xffffffffu, of_warp));
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int u = __shfl_up_sync(0xffffffffu, wv, o);
-        if (lane >= o) wv = max(wv, u);
-      }
-      s_warp[lane] = wv;
+    for (int x = 0; x < kItems; ++x) {
+      const int i = w0 + x * 32 + lane;
+      if (i < N) lo[(size_t)b * N + i] = max(start[x], before);
     }
-    __syncthreads();
-    int pre = __shfl_up_sync(0xffffffffu, tot, 1);   // everything before this thread in its warp
-    if (lane == 0) pre = 0;
-    pre = max(pre, max(s_carry, warp > 0 ? s_warp[warp - 1] : 0));
-#pragma unroll
-    for (int x = 0; x < kItems; ++x)
-      if (i0 + x < N) lo[(size_t)b * N + i0 + x] = max(v[x], pre);
-    __syncthreads();
-    if (tid == 1023) s_carry = max(tot, pre);
-    __syncthreads();
   }
-  if (dec) s_mono = 0;
-  __syncthreads();
-  if (tid == 0) mono[b] = s_mono;
+  if (tid == 0) mono[b] = decreases ? 0 : 1;
 }
 
 // Test hook for the bounded waits: one warp waits, with the given limit, on an mbarrier that

@@ -377,3 +377,23 @@ def test_rope_cast_feeds_the_attention_kernel_without_copies():
     _ulp_close(qr, q_ref)
     ref = orc.prefill_attention(qr.cpu(), kr.cpu(), vr.cpu(), 1 / math.sqrt(D), temporary_window=w, docs=docs.cpu())
     _check(out, ref)
+
+
+@pytest.mark.parametrize("n", [1153, 2049, 8192, 8500])
+def test_document_starts_across_warps_and_passes(n):
+    """The pre-pass finds the document starts per 32 rows, per warp of 256 and per pass of 8192: seen
+    through causal attention with equal scores, where row i is the mean over its i - start + 1 keys.
+    Row 1 has one document throughout, row 2 ids that go down (compared id by id) at the very end."""
+    from sps_b200 import attention
+    rng = np.random.default_rng(n)
+    docs = np.cumsum(rng.random((3, n)) < 0.004, axis=1)
+    docs[1] = 5
+    docs[2, -1] = -1
+    starts = np.stack([orc.run_starts(d) for d in docs])
+    zero = torch.zeros(3, 1, n, 64, dtype=torch.bfloat16, device=_dev())
+    v = torch.from_numpy(starts == np.arange(n)).to(_dev()).to(torch.bfloat16)[:, None, :, None].expand(3, 1, n, 64)
+    out = attention.full_attention(zero, zero, v.contiguous(), 0.125, documents_idx_BxT=torch.from_numpy(docs).to(_dev()))
+    want = torch.from_numpy(1.0 / (np.arange(n) - starts + 1))
+    # probabilities 1 and a whole-number sum are exact: one division and the rounding to bf16
+    err = (out[:, 0].double().cpu() - want[:, :, None]).abs() / want[:, :, None]
+    assert float(err.max()) <= 2.0 ** -8

@@ -108,24 +108,30 @@ struct DeltaStrides {
 };
 struct BwdPrepareParams {
   const void *o, *d_o;
-  float* delta;
-  long long rows;         // B * H * N
+  float* delta;           // [B, H, N]
   int H, N;
   DeltaStrides st;
   const int* lo;          // run starts [B, N] or null
   int* hi;                // run ends [B, N]
   long long ids;          // B * N, 0 without documents
-  unsigned delta_blocks;  // blocks from here on work on the run ends
+  unsigned run_blocks;    // blocks before this one work on the run ends
+  unsigned per_head;      // blocks of one (batch, head)
 };
+constexpr int kPrepareRows = 4;   // rows per thread
+__host__ __device__ constexpr int prepare_block_rows(int D) { return 256 / (D / 8) * kPrepareRows; }
 
-// Bound: HBM (O and dO are read once: 8.4 us at [4, 12, 4096, 64]).  One launch for the row sums and
-// for hi[b][i] = last row of the run of equal document ids that contains row i: the first later row
-// whose run starts after i, minus one (lo[b][.] is a non-decreasing step function).
+// Bound: HBM (O and dO are read once).  One launch for the row sums and for hi[b][i] = last row of the
+// run of equal document ids that contains row i: the first later row whose run starts after i, minus one
+// (lo[b][.] is a non-decreasing step function); those blocks come first, a search of a dozen dependent
+// reads must not be the end of the launch.  A block stays inside one (batch, head), so that rows are
+// found without a division, and a thread has four rows in flight: with one row and two 64-bit divisions
+// per thread the arithmetic took longer than the reads (13.6 instead of 8.5 us at [4, 12, 4096, 64], of
+// which 7.9 are the reads at the copy bandwidth).
 template <bool FP16, int D>
 __global__ void __launch_bounds__(256) bwd_prepare_kernel(const BwdPrepareParams p) {
   grid_launch_dependents();       // the dK/dV kernel waits before it reads what this one writes
-  if (blockIdx.x >= p.delta_blocks) {
-    const long long g = (long long)(blockIdx.x - p.delta_blocks) * 256 + threadIdx.x;
+  if (blockIdx.x < p.run_blocks) {
+    const long long g = (long long)blockIdx.x * 256 + threadIdx.x;
     if (g >= p.ids) return;
     const int i = (int)(g % p.N);
     const int* lo_b = p.lo + (g - i);
@@ -137,19 +143,27 @@ __global__ void __launch_bounds__(256) bwd_prepare_kernel(const BwdPrepareParams
     p.hi[g] = a - 1;
     return;
   }
-  constexpr int TPR = D / 8;                  // threads per row (8 or 16)
-  const long long r = ((long long)blockIdx.x * 256 + threadIdx.x) / TPR;
+  constexpr int TPR = D / 8, U = kPrepareRows;    // threads per row (8 or 16)
+  const unsigned block = blockIdx.x - p.run_blocks, bh = block / p.per_head, bb = bh / p.H, hh = bh - bb * p.H;
+  const int i0 = (int)(block - bh * p.per_head) * prepare_block_rows(D) + (int)threadIdx.x / TPR;
   const int part = threadIdx.x % TPR;
-  float acc = 0.f;
-  if (r < p.rows) {
-    const long long bh = r / p.N;
-    const int i = (int)(r - bh * p.N);
-    const long long bb = bh / p.H, hh = bh - bb * p.H;
-    const uint4 a = reinterpret_cast<const uint4*>(
-        reinterpret_cast<const uint16_t*>(p.o) + bb * p.st.o[0] + hh * p.st.o[1] + (long long)i * p.st.o[2])[part];
-    const uint4 g = reinterpret_cast<const uint4*>(
-        reinterpret_cast<const uint16_t*>(p.d_o) + bb * p.st.g[0] + hh * p.st.g[1] + (long long)i * p.st.g[2])[part];
-    const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, gw[4] = {g.x, g.y, g.z, g.w};
+  const uint16_t* o = reinterpret_cast<const uint16_t*>(p.o) + bb * p.st.o[0] + hh * p.st.o[1] + part * 8;
+  const uint16_t* d_o = reinterpret_cast<const uint16_t*>(p.d_o) + bb * p.st.g[0] + hh * p.st.g[1] + part * 8;
+  uint4 a[U], g[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int i = i0 + u * (256 / TPR);
+    a[u] = g[u] = make_uint4(0, 0, 0, 0);
+    if (i < p.N) {
+      a[u] = *reinterpret_cast<const uint4*>(o + i * p.st.o[2]);
+      g[u] = *reinterpret_cast<const uint4*>(d_o + i * p.st.g[2]);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int i = i0 + u * (256 / TPR);
+    const uint32_t aw[4] = {a[u].x, a[u].y, a[u].z, a[u].w}, gw[4] = {g[u].x, g[u].y, g[u].z, g[u].w};
+    float acc = 0.f;
 #pragma unroll
     for (int x = 0; x < 4; ++x) {
       float a0, a1, b0, b1;
@@ -157,10 +171,10 @@ __global__ void __launch_bounds__(256) bwd_prepare_kernel(const BwdPrepareParams
       unpack2<FP16>(gw[x], b0, b1);
       acc = fmaf(a0, b0, fmaf(a1, b1, acc));
     }
-  }
 #pragma unroll
-  for (int off = TPR / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-  if (part == 0 && r < p.rows) p.delta[r] = acc;
+    for (int off = TPR / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    if (part == 0 && i < p.N) p.delta[(size_t)bh * p.N + i] = acc;
+  }
 }
 
 struct alignas(16) BwdMeta {   // per streamed query tile in kDKV mode: one entry per column

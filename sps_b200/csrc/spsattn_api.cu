@@ -642,15 +642,15 @@ static int prefill_bwd_impl(const void* q, const void* k, const void* v, const v
   pp.o = o;
   pp.d_o = d_o;
   pp.delta = delta;
-  pp.rows = (long long)B * H * N;
   pp.H = H;
   pp.N = N;
   pp.st = {{so.b, so.h, so.n}, {sg.b, sg.h, sg.n}};
   pp.lo = lo;
   pp.hi = hi;
   pp.ids = lo != nullptr ? (long long)B * N : 0;
-  pp.delta_blocks = (unsigned)((pp.rows * (D / 8) + 255) / 256);
-  const unsigned pgrid = pp.delta_blocks + (unsigned)((pp.ids + 255) / 256);
+  pp.run_blocks = (unsigned)((pp.ids + 255) / 256);
+  pp.per_head = (unsigned)((N + prepare_block_rows(D) - 1) / prepare_block_rows(D));
+  const unsigned pgrid = pp.run_blocks + (unsigned)(B * H) * pp.per_head;
   if (D == 64) {
     if (fp16) bwd_prepare_kernel<true, 64><<<pgrid, 256, 0, st>>>(pp);
     else bwd_prepare_kernel<false, 64><<<pgrid, 256, 0, st>>>(pp);

@@ -32,7 +32,7 @@ struct PrefillParams {
   const void* docs;      // [B,N] ids or null
   int64_t doc_stride_b, doc_stride_t;
   int doc_is_i64;
-  int scan_docs;         // no pre-pass: every block works its document starts out from the ids
+  int scan_docs;         // host: take the kernel that scans the ids itself
   const int* lo;         // [B,N] run starts (pre-pass, or the caller's) or null
   const int* mono;       // [B] 1 when ids of the row are non-decreasing, or null
   int B, H, N;
@@ -182,7 +182,9 @@ __device__ __forceinline__ void softmax_arrive(uint32_t bar, int lane) {
 }
 #endif
 
-template <int D, bool FP16>
+// kScan: no pre-pass, every block works its document starts out from the ids (a kernel of its own: the
+// branch alone cost the others 1 %, 342 against 339 us at [8, 12, 8192, 64])
+template <int D, bool FP16, bool kScan>
 __global__ void __launch_bounds__(kPrefillThreads, PrefillCfg<D>::kBlocksPerSM)
 prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const PrefillParams prm) {
@@ -194,8 +196,8 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   __shared__ uint32_t s_tmem_base;
   __shared__ uint32_t s_tmem_p;
   __shared__ int s_abort;
-  __shared__ int s_lo[kTileM];         // scan_docs: run starts of the block's rows
-  __shared__ int s_scan[kPrefillThreads / 32 + 1];
+  __shared__ int s_lo[kScan ? kTileM : 1];         // run starts of the block's rows
+  __shared__ int s_scan[kScan ? kPrefillThreads / 32 + 1 : 1];
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
@@ -263,7 +265,7 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     tmem_relinquish();
     if (lane == 0) SPS_TRACE(6, 15);
   }
-  if (prm.scan_docs) {
+  if constexpr (kScan) {
     // Short rows (up to kScanRows) without a pre-pass launch, which costs more than it does: the ids
     // before and inside this block's rows, kScanItems per thread.  Rows see no later key, so whether
     // the ids decrease matters only up to here.
@@ -319,9 +321,9 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     // whether or not the ids turn out monotone: the table exists whenever ids were given)
     int st_word = 0;
     if (slot == 0 && prm.status != nullptr) st_word = *reinterpret_cast<volatile int*>(prm.status);
-    const int mono_b = prm.scan_docs ? !s_scan[kPrefillThreads / 32] : (has_docs && prm.mono != nullptr) ? prm.mono[b] : 1;
+    const int mono_b = kScan ? !s_scan[kScan ? kPrefillThreads / 32 : 0] : (has_docs && prm.mono != nullptr) ? prm.mono[b] : 1;
     int lo0 = 0, lo1 = 0;
-    if (prm.scan_docs) {
+    if constexpr (kScan) {
       lo0 = s_lo[0];
       lo1 = s_lo[min(kTileM - 1, prm.N - 1 - i0)];
     } else if (has_docs) {
@@ -512,7 +514,7 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       const bool general = s_plan.general_docs != 0;
       int lo_i = 0;
       if (!general && i < prm.N) {
-        if (prm.scan_docs) lo_i = s_lo[row];
+        if constexpr (kScan) lo_i = s_lo[row];
         else if (has_docs) lo_i = prm.lo[(size_t)b * prm.N + i];
       }
       int kmin_s[2], kmax_s[2];

@@ -147,14 +147,14 @@ int multiprocessors() {
   return sms;
 }
 
-template <int D, bool FP16>
-int launch_prefill_sm100(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
+template <int D, bool FP16, bool kScan>
+int launch_prefill_kernel(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                          const PrefillParams& prm, cudaStream_t st) {
   using Cfg = PrefillCfg<D>;
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(prefill_sm100_kernel<D, FP16>,
+    attr_err = cudaFuncSetAttribute(prefill_sm100_kernel<D, FP16, kScan>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
   });
   if (attr_err != cudaSuccess) return (int)attr_err;
@@ -179,8 +179,15 @@ int launch_prefill_sm100(const CUtensorMap& tq, const CUtensorMap& tk, const CUt
 #else
   cfg.numAttrs = prm.mono != nullptr ? 1 : 0;
 #endif
-  const cudaError_t le = cudaLaunchKernelEx(&cfg, prefill_sm100_kernel<D, FP16>, tq, tk, tv, prm);
+  const cudaError_t le = cudaLaunchKernelEx(&cfg, prefill_sm100_kernel<D, FP16, kScan>, tq, tk, tv, prm);
   return le != cudaSuccess ? (int)le : (int)cudaGetLastError();
+}
+
+template <int D, bool FP16>
+int launch_prefill_sm100(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
+                         const PrefillParams& prm, cudaStream_t st) {
+  return prm.scan_docs ? launch_prefill_kernel<D, FP16, true>(tq, tk, tv, prm, st)
+                       : launch_prefill_kernel<D, FP16, false>(tq, tk, tv, prm, st);
 }
 
 // Persistent launch: two blocks per SM draw the (batch, head, query tile) items from

@@ -16,7 +16,8 @@
 //     per lane (rows are padded to 32 bytes past a multiple of 128: no bank conflicts; a lane's four
 //     elements are neighbours, as the order inside the 16 columns of one product is free).
 //     tcgen05 was slower here (25-45 clk to issue each product of M = 64, a commit and a read of
-//     tensor memory at the end: 490 against 290 us for a token of the model above).
+//     tensor memory at the end: 490 against 375 us for a token of the model above when it was tried;
+//     297 now, 566 with library projections and separate kernels).
 // The contraction of one output is one chain of products in ascending k, never split, with results
 // rounded to bf16 where the separate kernels (library GEMM, model_glue.cuh, rope.cuh) round theirs and
 // the norm's sums in the order of add_rmsnorm_kernel: a step's logits are the same bits as theirs.

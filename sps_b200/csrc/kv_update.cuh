@@ -26,7 +26,7 @@ struct KvUpdateParams {
 
 // Bound: latency (a few MB at most).  New rows and counters are asked for together, and the launch is a
 // programmatic dependent of the attention before it, which it waits for only here: with 128
-// sequences of 16 x 64 the pair takes 209 + 10 us instead of 209 + 15.
+// sequences of 16 x 64 attention and update take 219 us instead of 226 (the attention alone 211).
 template <typename V>
 __global__ void __launch_bounds__(256) kv_update_kernel(const KvUpdateParams p) {
   const int s = blockIdx.x, tid = threadIdx.x;

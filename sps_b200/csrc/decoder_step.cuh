@@ -17,7 +17,7 @@
 //     elements are neighbours, as the order inside the 16 columns of one product is free).
 //     tcgen05 was slower here (25-45 clk to issue each product of M = 64, a commit and a read of
 //     tensor memory at the end: 490 against 375 us for a token of the model above when it was tried;
-//     297 now, 566 with library projections and separate kernels).
+//     295 now, 566 with library projections and separate kernels).
 // The contraction of one output is one chain of products in ascending k, never split, with results
 // rounded to bf16 where the separate kernels (library GEMM, model_glue.cuh, rope.cuh) round theirs and
 // the norm's sums in the order of add_rmsnorm_kernel: a step's logits are the same bits as theirs.
@@ -191,6 +191,13 @@ __global__ void __launch_bounds__(32 * kSkinnyMaxWarps + kSkinnyLoaders) skinny_
 
   // ------------------------------------------------------------------ input rows
   int64_t pos[MT] = {};                // of the lane's rows (q, k, v)
+  // q, k, v: which of them output f belongs to and its pair inside a head; the remainder of the first
+  // round is taken before the wait
+  const int C = EPI == kSkinnyQkv ? p.F / 3 : 1;
+  auto part_of = [&](int f) { return EPI == kSkinnyQkv ? (f >= C) + (f >= 2 * C) : 0; };
+  auto pair_of = [&](int f) { return EPI == kSkinnyQkv ? (f - part_of(f) * C) % p.head_dim / 2 : 0; };
+  const int first_pair = pair_of((int)blockIdx.x * per_round + warp * 8 + 2 * t);
+  const int two = p.slots - 1;         // rows of a sequence: 1 or 2
   if constexpr (kNorm) {
     // a thread takes one vector of 8 columns (at most 256 of them) of every `at_once`-th row
     constexpr int kOwn = 4;            // rows a thread has in flight
@@ -203,7 +210,7 @@ __global__ void __launch_bounds__(32 * kSkinnyMaxWarps + kSkinnyLoaders) skinny_
     // (asked for here so that the rotary factors can be asked for as soon as the products start)
     if (EPI == kSkinnyQkv && warp < p.warps) {
 #pragma unroll
-      for (int m = 0; m < MT; ++m) pos[m] = g + 8 * m < p.rows ? __ldcg(p.pos + (g + 8 * m) / p.slots) : 0;
+      for (int m = 0; m < MT; ++m) pos[m] = g + 8 * m < p.rows ? __ldcg(p.pos + ((g + 8 * m) >> two)) : 0;
     }
     const uint16_t* xp = p.x + (size_t)sub * p.x_stride + i * 8;
     const int64_t x_step = (int64_t)at_once * p.x_stride;
@@ -216,10 +223,14 @@ __global__ void __launch_bounds__(32 * kSkinnyMaxWarps + kSkinnyLoaders) skinny_
       float part[8], sum = 0.f;
 #pragma unroll
       for (int w = 0; w < 8; ++w) part[w] = w * 32 + lane < vecs ? __ldcg(p.ssq + r * p.ssq_stride + w * 32 + lane) : 0.f;
+      auto butterfly = [&](int from) {       // four at a time: rows of up to 1024 columns have no more
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1)
+        for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-        for (int w = 0; w < 8; ++w) part[w] += __shfl_xor_sync(0xffffffffu, part[w], o);
+          for (int w = from; w < from + 4; ++w) part[w] += __shfl_xor_sync(0xffffffffu, part[w], o);
+      };
+      butterfly(0);
+      if (vecs > 128) butterfly(4);
 #pragma unroll
       for (int w = 0; w < 8; ++w) sum += part[w];
       if (lane == 0) s_scale[r] = rsqrtf(sum / (float)p.K + p.eps);
@@ -277,7 +288,7 @@ __global__ void __launch_bounds__(32 * kSkinnyMaxWarps + kSkinnyLoaders) skinny_
       uint32_t old[MT], hide = 0;
       float2 cs[MT];
       if (EPI == kSkinnyLogits && p.suppressed != nullptr && f < p.F) hide = __ldg(p.suppressed + (f >> 5)) >> (f & 31);
-      const int C = EPI == kSkinnyQkv ? p.F / 3 : 1, which = EPI == kSkinnyQkv ? f / C : 0, fi = f - which * C;
+      const int which = part_of(f), fi = f - which * C;
 #pragma unroll
       for (int m = 0; m < MT; ++m) {
         const int r = g + 8 * m;
@@ -286,7 +297,7 @@ __global__ void __launch_bounds__(32 * kSkinnyMaxWarps + kSkinnyLoaders) skinny_
         if (r < p.rows && f < p.F) {
           if constexpr (EPI == kSkinnyResidual) old[m] = __ldcg(reinterpret_cast<const uint32_t*>(p.out + (size_t)r * p.F + f));
           if constexpr (EPI == kSkinnyQkv) {
-            if (which < 2) cs[m] = __ldg(p.freqs + pos[m] * (p.head_dim / 2) + (fi % p.head_dim) / 2);
+            if (which < 2) cs[m] = __ldg(p.freqs + pos[m] * (p.head_dim / 2) + (it == 0 ? first_pair : pair_of(f)));
           }
         }
       }
@@ -363,7 +374,7 @@ __global__ void __launch_bounds__(32 * kSkinnyMaxWarps + kSkinnyLoaders) skinny_
               v0 = __fsub_rn(__fmul_rn(a, cs[m].x), __fmul_rn(b, cs[m].y));
               v1 = __fadd_rn(__fmul_rn(a, cs[m].y), __fmul_rn(b, cs[m].x));
             }
-            const int bi = r / p.slots, slot = r - bi * p.slots;
+            const int bi = r >> two, slot = r & two;
             uint16_t* dst = which == 0 ? p.q + (size_t)r * C
                                        : (which == 1 ? p.k : p.v) + ((size_t)slot * p.batch + bi) * C;
             *reinterpret_cast<uint32_t*>(dst + fi) = pack2<false>(v0, v1);

@@ -64,9 +64,11 @@ extern "C" {
 #define SPSATTN_ERR_TOO_LARGE (-7)  /* size beyond a documented maximum */
 #define SPSATTN_ERR_SCRATCH_LIMIT (-8) /* needs more scratch than the built-in static buffer holds */
 
-/* device_status codes written by kernels (0 = ok) */
+/* bits of the device_status word that kernels set (0 = ok); only WAIT_EXPIRED makes other blocks and
+ * later launches give up */
 #define SPSATTN_STATUS_WAIT_EXPIRED 1
-#define SPSATTN_STATUS_BAD_TOKEN 2      /* a decode step was given a token id outside the vocabulary */
+#define SPSATTN_STATUS_BAD_TOKEN 2      /* a decode step was given a token id outside the vocabulary; the sequence
+                                           was taken as inactive */
 
 const char* spsattn_strerror(int code);
 int spsattn_version(void);
@@ -348,7 +350,7 @@ int spsattn_debug_prefill_path(int path);
  * nobody arrives at (no copy or tensor-core operation in flight), with a limit of `limit_ns`
  * nanoseconds (at most 1e9).  The wait gives up, writes SPSATTN_STATUS_WAIT_EXPIRED to
  * *device_status as the attention kernels do, sets device_result[0] = 1 (when given) and the
- * block ends normally.  While the status word is non-zero the tensor-core attention kernels
+ * block ends normally.  While the status word holds that bit the tensor-core attention kernels
  * return without computing; the caller clears it.  No counterpart in the reference. */
 int spsattn_debug_wait_expiry(int* device_status, unsigned long long limit_ns, int* device_result,
                               void* stream);

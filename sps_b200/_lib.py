@@ -17,7 +17,7 @@ PARITY_EVEN, PARITY_ODD, PARITY_NONE = 0, 1, -1
 NO_WINDOW = -2147483648
 NOALLOC_SCRATCH_BYTES = 16 << 20
 FLAG_PERSISTENT_Q_SKIPS_TEMPORARY = 1
-STATUS_BAD_TOKEN = 2
+STATUS_WAIT_EXPIRED, STATUS_BAD_TOKEN = 1, 2
 
 EXPORTS = (
     "spsattn_version", "spsattn_strerror",

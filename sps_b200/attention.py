@@ -20,19 +20,21 @@ import torch
 from . import _lib
 
 def _status(device: torch.device) -> torch.Tensor:
-    """Per-device int32 word that kernels set when a bounded wait expires."""
+    """Per-device int32 word of STATUS bits: a bounded wait that expired, an input outside its range."""
     return _lib.native().status_word(device.index if device.index is not None else torch.cuda.current_device())
 
 
 def check_device_status(device=None) -> None:
-    """Synchronise and raise if any kernel reported a failure (a bounded wait that expired)."""
+    """Synchronise and raise if any kernel reported a failure (a bounded wait that expired, a token id
+    outside the vocabulary)."""
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     word = _status(dev)
     code = int(word.item())
     if code != 0:
         word.zero_()
-        what = "a token id outside the vocabulary" if code == _lib.STATUS_BAD_TOKEN else "a bounded wait expired"
-        raise _lib.SpsAttnError(f"device reported status {code} ({what})")
+        what = [text for bit, text in ((_lib.STATUS_WAIT_EXPIRED, "a bounded wait expired"),
+                                       (_lib.STATUS_BAD_TOKEN, "a token id outside the vocabulary")) if code & bit]
+        raise _lib.SpsAttnError(f"device reported status {code} ({', '.join(what)})")
 
 
 def _dtype_code(t: torch.Tensor) -> int:

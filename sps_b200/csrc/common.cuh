@@ -131,6 +131,12 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
+// Whether a wait has expired in another block or an earlier launch.  (The word also carries errors of a
+// caller's input, which concern that call alone.)
+__device__ __forceinline__ bool wait_has_expired(const int* status) {
+  return status != nullptr && (*reinterpret_cast<const volatile int*>(status) & SPSATTN_STATUS_WAIT_EXPIRED) != 0;
+}
+
 // Every wait in the kernels is bounded: after kWaitLimitNs of wall time, or as soon as another
 // block has reported a failure, the wait gives up, records SPSATTN_STATUS_WAIT_EXPIRED in the
 // caller's status word (when given) and raises the block-local abort flag.  The caller then
@@ -144,7 +150,7 @@ __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volat
     if (mbar_try_wait(bar, parity)) return true;
     if ((it & 63u) == 63u) {
       if (*abort_flag) return false;
-      if (status != nullptr && *reinterpret_cast<volatile int*>(status) != 0) {
+      if (wait_has_expired(status)) {
         *abort_flag = 1;
         return false;
       }
@@ -152,7 +158,7 @@ __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volat
     }
   }
   *abort_flag = 1;
-  if (status != nullptr) atomicExch(status, SPSATTN_STATUS_WAIT_EXPIRED);
+  if (status != nullptr) atomicOr(status, SPSATTN_STATUS_WAIT_EXPIRED);
   return false;
 }
 

@@ -163,7 +163,7 @@ decode_tc_kernel(const __grid_constant__ DecodeMaps maps, const DecodeParams prm
     const uint32_t qmask = prm.seg[seg].query_mask;
 
     if (tid == 0)
-      s_abort = (prm.status != nullptr && *reinterpret_cast<volatile int*>(prm.status) != 0) ? 1 : 0;
+      s_abort = wait_has_expired(prm.status) ? 1 : 0;
     // The nq query rows go into the padded query tile (K-major, 128-byte swizzle: 16-byte chunk ch
     // of row r of a 64-wide sub-tile sits at r * 128 + ((ch ^ (r & 7)) << 4)).  Its other rows,
     // and rows >= nq of P, are left as they are: they only produce score columns and accumulator

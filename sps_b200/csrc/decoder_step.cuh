@@ -307,8 +307,8 @@ __global__ void __launch_bounds__(32 * kSkinnyMaxWarps + kSkinnyLoaders) skinny_
 #pragma unroll
         for (int e = 0; e < 4; ++e) c[x][e] = 0.f;
       for (int j = 0; j < chunks; ++j) {
-        // (a wait that gives up does not leave the loop: the waits after it return at once, the
-        // results are discarded, and the warp stays whole without a vote per stage)
+        // (a wait that gives up does not leave the loop: the waits after it return at once, and the warp
+        // stays whole without a vote per stage; what is stored then is wrong, and the status word says so)
         mbar_wait(full0 + 8 * st, phase, abort_flag, p.status);
         __syncwarp();
         const uint32_t wb = smem + st * stage_bytes + (warp * R + g) * pitch + t * 8;
@@ -542,8 +542,12 @@ __global__ void __launch_bounds__(kStartThreads) token_start_kernel(const TokenS
     chosen = p.token_in[b];
     live = p.active_in[b] != 0;
   }
-  const bool active = live && !newly;
+  // A caller's id outside the vocabulary is reported, and its sequence sits the step out.
+  const bool wanted = live && !newly;
+  const bool known = chosen >= 0 && chosen < p.vocab && (p.slots == 1 || (p.predict >= 0 && p.predict < p.vocab));
+  const bool active = wanted && known;
   const int64_t token = active ? chosen : 0;
+  if (wanted && !known && tid == 0 && p.status != nullptr) atomicOr(p.status, SPSATTN_STATUS_BAD_TOKEN);
 
   // a row that starts a document forgets its caches, in every layer
   if (active && starts_doc) {
@@ -559,10 +563,7 @@ __global__ void __launch_bounds__(kStartThreads) token_start_kernel(const TokenS
     const int slot = idx / (p.C / V), i = idx - slot * (p.C / V);
     const int64_t id = slot == 0 ? token : p.predict;
     uint4 u = make_uint4(0, 0, 0, 0);
-    if (id >= 0 && id < p.vocab)
-      u = reinterpret_cast<const uint4*>(p.wte)[(size_t)id * (p.C / V) + i];
-    else if (p.status != nullptr)
-      atomicExch(p.status, SPSATTN_STATUS_BAD_TOKEN);
+    if (id >= 0 && id < p.vocab) u = reinterpret_cast<const uint4*>(p.wte)[(size_t)id * (p.C / V) + i];
     reinterpret_cast<uint4*>(p.x)[((size_t)b * p.slots + slot) * (p.C / V) + i] = u;
     if (!F32 && p.ssq != nullptr) {
       float f[8], sq = 0.f;

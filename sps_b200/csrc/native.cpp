@@ -107,7 +107,7 @@ int dtype_code(const Tensor& t) {
 
 constexpr int kMaxDevices = 64;
 
-// One int32 word per device that kernels set when a bounded wait expires; lives as long as the process.
+// One int32 word of SPSATTN_STATUS bits per device; lives as long as the process.
 const Tensor& status_word(int device) {
   static std::once_flag once[kMaxDevices];
   static Tensor* words[kMaxDevices];

@@ -254,7 +254,7 @@ prefill_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid
   const int* lo_b = (has_docs && !general) ? prm.lo + (size_t)b * prm.N : nullptr;
 
   if (tid == 0) {
-    s_abort = (prm.status != nullptr && *reinterpret_cast<volatile int*>(prm.status) != 0) ? 1 : 0;
+    s_abort = wait_has_expired(prm.status) ? 1 : 0;
     if constexpr (!kDKV) {
       BlockPlan bp;
       bp.general_docs = general ? 1 : 0;

@@ -319,8 +319,7 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const int slot = tid >> 5;
     // the global words the plan needs are asked for together (the document starts are read
     // whether or not the ids turn out monotone: the table exists whenever ids were given)
-    int st_word = 0;
-    if (slot == 0 && prm.status != nullptr) st_word = *reinterpret_cast<volatile int*>(prm.status);
+    const bool expired = slot == 0 && wait_has_expired(prm.status);
     const int mono_b = kScan ? !s_scan[kScan ? kPrefillThreads / 32 : 0] : (has_docs && prm.mono != nullptr) ? prm.mono[b] : 1;
     int lo0 = 0, lo1 = 0;
     if constexpr (kScan) {
@@ -341,7 +340,7 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     s_plan.stream_id[slot] = stream;
     if (slot == 0) {
       // a failure reported by an earlier block turns every later block into a no-op
-      s_abort = st_word != 0 ? 1 : 0;
+      s_abort = expired ? 1 : 0;
       s_plan.general_docs = mono_b == 0 ? 1 : 0;
       s_plan.n_streams = two ? 2 : 1;
     }

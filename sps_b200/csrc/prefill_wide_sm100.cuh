@@ -509,7 +509,7 @@ prefill_wide_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
 
   if (tid == 0)
     // a failure reported by an earlier launch or block turns this block into a no-op
-    s_abort = (prm.status != nullptr && *reinterpret_cast<volatile int*>(prm.status) != 0) ? 1 : 0;
+    s_abort = wait_has_expired(prm.status) ? 1 : 0;
   if (warp == 4) {
     if (lane == 0) {
       for (int s = 0; s < 2; ++s) {

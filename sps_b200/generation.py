@@ -428,7 +428,8 @@ class SPSGenerator:
         the reference returns them (inference.py:485).  Raises ValueError, like the reference
         (inference.py:384-389), when a row could already hold as many tokens as the rotary table
         or the caches take: past that point the position lookup would read out of range and the
-        cache append would be dropped."""
+        cache append would be dropped.  A row whose token id is outside the vocabulary sits the step out
+        like an inactive one, and ``check_device_status`` or the next ``prefill`` raises."""
         limit = min(self.dims.block_size, state.max_tokens)
         if state.host_tokens >= limit:
             raise ValueError(f"Cannot decode another token: up to {state.host_tokens} tokens are processed "
@@ -447,7 +448,7 @@ class SPSGenerator:
         with torch.cuda.device(self.device):
             self._step_body(source, logits)
         if not s.fused:
-            logits.masked_fill_(~active.unsqueeze(1), 0)
+            logits.masked_fill_((s.active_i8 == 0).unsqueeze(1), 0)
         return logits
 
     # ------------------------------------------------------------------ generation

@@ -51,6 +51,46 @@ def test_fused_step_matches_the_separate_kernels(variant, batch, heads, hidden, 
         assert torch.equal(getattr(states[0], name), getattr(states[1], name)), name
 
 
+@pytest.mark.parametrize("fused", [True, False])
+@pytest.mark.parametrize("bad", [-1, 200, 1 << 40])
+def test_a_token_outside_the_vocabulary_concerns_its_row_alone(fused, bad):
+    """The row sits the step out as if it were inactive, the check raises, and an attention call before
+    the check still gives its numbers (a tensor-core kernel asks the status word before it starts)."""
+    import sps_b200
+    from sps_b200 import _lib
+    engine, dims = _engine("sps", 2, 2, 128, 80, 200)
+    g = torch.Generator().manual_seed(17)
+    prompt = torch.randint(0, 197, (4, 9), generator=g)
+    good = torch.randint(0, 197, (4,), generator=g)
+    q, k, v = (torch.randn(1, 2, 256, 64, generator=g).bfloat16().cuda() for _ in range(3))
+    want = sps_b200.sps_sliding_attention(q, k, v, 0.125, 8)
+    outs, states = [], []
+    for given in (bad, None):
+        state, _ = engine.prefill(prompt, 8)
+        engine._bind_step(state)
+        engine._step.fused = fused
+        token, active = good.clone(), torch.ones(4, dtype=torch.bool)
+        if given is None:
+            active[1] = False
+        else:
+            token[1] = given
+        logits = [engine.decode_one_token(state, token, active)]
+        if given is not None:
+            assert torch.equal(sps_b200.sps_sliding_attention(q, k, v, 0.125, 8), want)
+            with pytest.raises(_lib.SpsAttnError, match="vocabulary"):
+                sps_b200.check_device_status()
+        active[1] = True
+        logits.append(engine.decode_one_token(state, good, active))
+        sps_b200.check_device_status()
+        outs.append(logits)
+        states.append(state)
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
+    assert bool((outs[0][0][1] == 0).all())
+    for name in ("br_k", "br_v", "br_len", "nw_k", "nw_v", "nw_len", "nw_pos", "processed_tokens", "next_doc_start"):
+        assert torch.equal(getattr(states[0], name), getattr(states[1], name)), name
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("vocab", [7, 64, 1003, 50304])
 def test_greedy_choice_is_the_first_unsuppressed_maximum(dtype, vocab):

@@ -430,9 +430,9 @@ int spsattn_swiglu(const void* gate_up, void* y, int dtype, long long rows, int 
  *   or the caller's), counters, embedding; parameters and activations in `param_dtype`.
  * spsattn_decoder_choose: the greedy choice alone (the last token of a generation).
  * spsattn_decoder_step: start, every layer's projections around spsattn_decode_step, and the head on
- *   the prediction slot, each launch a programmatic dependent of the one before it.  For sizes that
+ *   the prediction slot, each launch a programmatic dependent of the one before it.  For decoders that
  *   spsattn_decoder_step_supported takes (1 = yes): bf16, batch * slots <= 16 rows, hidden and
- *   intermediate multiples of 16, hidden <= 2048.
+ *   intermediate multiples of 16, hidden <= 2048, weights (wte apart) and step buffers 16-byte aligned.
  * ------------------------------------------------------------------------------------------- */
 typedef struct spsattn_decoder_layer {
   const void* attn_norm;      /* [C] */

@@ -466,6 +466,7 @@ struct TokenStartParams {
   float2* freqs_out;             // [batch, half_dim]: the sequence's row, or null
   int half_dim;
   const void* wte;               // [vocab, C] bf16 or fp32
+  int wte_wide;                  // 16-byte aligned
   void* x;                       // [batch * slots, C]
   float* ssq;                    // [batch * slots, C / 8] sums of squares of 8 elements each, or null (bf16 only)
   int slots, C;
@@ -563,7 +564,19 @@ __global__ void __launch_bounds__(kStartThreads) token_start_kernel(const TokenS
     const int slot = idx / (p.C / V), i = idx - slot * (p.C / V);
     const int64_t id = slot == 0 ? token : p.predict;
     uint4 u = make_uint4(0, 0, 0, 0);
-    if (id >= 0 && id < p.vocab) u = reinterpret_cast<const uint4*>(p.wte)[(size_t)id * (p.C / V) + i];
+    if (id >= 0 && id < p.vocab) {
+      const size_t at = (size_t)id * (p.C / V) + i;
+      if (p.wte_wide) {
+        u = reinterpret_cast<const uint4*>(p.wte)[at];
+      } else if constexpr (F32) {
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(p.wte) + at * V;
+        u = make_uint4(w[0], w[1], w[2], w[3]);
+      } else {
+        const uint16_t* w = reinterpret_cast<const uint16_t*>(p.wte) + at * V;
+        u = make_uint4(w[0] | (uint32_t)w[1] << 16, w[2] | (uint32_t)w[3] << 16, w[4] | (uint32_t)w[5] << 16,
+                       w[6] | (uint32_t)w[7] << 16);
+      }
+    }
     reinterpret_cast<uint4*>(p.x)[((size_t)b * p.slots + slot) * (p.C / V) + i] = u;
     if (!F32 && p.ssq != nullptr) {
       float f[8], sq = 0.f;

@@ -7,6 +7,7 @@
 #include <string.h>
 
 #include <atomic>
+#include <initializer_list>
 #include <mutex>
 #include <utility>
 
@@ -46,7 +47,8 @@ EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+inline bool aligned(const void* p, unsigned bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
+inline bool aligned16(const void* p) { return aligned(p, 16); }
 
 inline int clamp_window(long long w, int n) {
   if (w < 0) return -1;
@@ -1364,7 +1366,7 @@ int launch_token_start(const spsattn_decoder* d, const spsattn_token_source* src
     if (!d->processed || !d->next_doc_start || !d->nw_len || !d->nw_pos || !d->br_len || !d->active || !d->pos ||
         !d->wte || !d->x || d->n_layer <= 0 || d->n_head <= 0 || d->hidden <= 0 || d->slots < 1 || d->slots > 2)
       return SPSATTN_ERR_ARG;
-    if (d->hidden % (f32 ? 4 : 8) || !aligned16(d->wte) || !aligned16(d->x)) return SPSATTN_ERR_ALIGN;
+    if (d->hidden % (f32 ? 4 : 8) || !aligned(d->wte, f32 ? 4 : 2) || !aligned16(d->x)) return SPSATTN_ERR_ALIGN;
     p.processed = d->processed;
     p.next_doc_start = d->next_doc_start;
     p.nw_len = d->nw_len;
@@ -1379,6 +1381,7 @@ int launch_token_start(const spsattn_decoder* d, const spsattn_token_source* src
     p.freqs_out = reinterpret_cast<float2*>(d->freqs_out);
     p.half_dim = d->head_dim / 2;
     p.wte = d->wte;
+    p.wte_wide = aligned16(d->wte);
     p.x = d->x;
     p.ssq = d->ssq;
     p.slots = d->slots;
@@ -1387,6 +1390,32 @@ int launch_token_start(const spsattn_decoder* d, const spsattn_token_source* src
   }
   return f32 ? launch_dependent(token_start_kernel<true>, dim3((unsigned)d->batch), dim3(kStartThreads), 0, st, p)
              : launch_dependent(token_start_kernel<false>, dim3((unsigned)d->batch), dim3(kStartThreads), 0, st, p);
+}
+
+// sizes that the fused step takes
+bool fused_step_sizes(const spsattn_decoder* d) {
+  if (!d || d->param_dtype != SPSATTN_DTYPE_BF16 || d->batch <= 0 || d->n_layer <= 0) return false;
+  if ((d->slots != 1 && d->slots != 2) || d->n_head <= 0 || d->vocab <= 0) return false;
+  if (d->hidden != d->n_head * d->head_dim || d->batch * d->slots > kSkinnyMaxRows) return false;
+  // the norm's sums are those of a row of at most 256 vectors
+  return d->hidden % 16 == 0 && d->hidden <= kSkinnyMaxCols && d->intermediate > 0 && d->intermediate % 16 == 0;
+}
+
+// what its kernels move by 16 bytes (weights may be views into a buffer of the caller's)
+int fused_step_pointers(const spsattn_decoder* d) {
+  if (!d->layers || !d->ssq || !d->freqs || !d->pos || !d->active) return SPSATTN_ERR_ARG;
+  int rc = aligned(d->ssq, 4) && aligned(d->freqs, 8) ? 0 : SPSATTN_ERR_ALIGN;
+  auto check = [&rc](std::initializer_list<const void*> ptrs) {
+    for (const void* p : ptrs)
+      if (!p) rc = SPSATTN_ERR_ARG;
+      else if (rc == 0 && !aligned16(p)) rc = SPSATTN_ERR_ALIGN;
+  };
+  check({d->lm_head, d->out_norm, d->x, d->q, d->k2, d->v2, d->y, d->mlp_hidden});
+  for (int l = 0; l < d->n_layer; ++l) {
+    const spsattn_decoder_layer& w = d->layers[l];
+    check({w.attn_norm, w.c_attn, w.c_proj, w.mlp_norm, w.gate_up, w.down});
+  }
+  return rc;
 }
 
 }  // namespace
@@ -1403,19 +1432,18 @@ int spsattn_decoder_choose(const spsattn_decoder* d, const spsattn_token_source*
 }
 
 int spsattn_decoder_step_supported(const spsattn_decoder* d) {
-  if (!d || d->param_dtype != SPSATTN_DTYPE_BF16 || d->batch <= 0 || d->n_layer <= 0) return 0;
-  if ((d->slots != 1 && d->slots != 2) || d->n_head <= 0 || d->vocab <= 0) return 0;
-  if (d->hidden != d->n_head * d->head_dim || d->batch * d->slots > kSkinnyMaxRows) return 0;
-  // the norm's sums are those of a row of at most 256 vectors
-  return d->hidden % 16 == 0 && d->hidden <= kSkinnyMaxCols && d->intermediate > 0 && d->intermediate % 16 == 0 ? 1 : 0;
+  return fused_step_sizes(d) && fused_step_pointers(d) == 0 ? 1 : 0;
 }
 
 int spsattn_decoder_step(const spsattn_decoder* d, const spsattn_token_source* source, void* logits_out,
                          int* device_status, void* stream) {
-  if (!spsattn_decoder_step_supported(d) || !logits_out || !d->layers || !d->ssq) return SPSATTN_ERR_ARG;
+  if (!fused_step_sizes(d) || !source || !logits_out) return SPSATTN_ERR_ARG;
   if (d->n_segments < 1 || d->n_segments > 2) return SPSATTN_ERR_ARG;
+  int rc = fused_step_pointers(d);
+  if (rc == 0 && !aligned(logits_out, 4)) rc = SPSATTN_ERR_ALIGN;
+  if (rc != 0) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  int rc = launch_token_start(d, source, false, device_status, st);
+  rc = launch_token_start(d, source, false, device_status, st);
   if (rc != 0) return rc;
   const int C = d->hidden, I = d->intermediate, rows = d->batch * d->slots;
   // every slot sees the step's input row, only the <predict> slot its own (decode_attention.py:354-361)

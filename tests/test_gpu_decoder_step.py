@@ -51,6 +51,38 @@ def test_fused_step_matches_the_separate_kernels(variant, batch, heads, hidden, 
         assert torch.equal(getattr(states[0], name), getattr(states[1], name)), name
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_weights_at_any_element_of_a_flat_buffer(dtype):
+    """Projections, embedding and head as views at odd elements: the step runs, by library projections."""
+    import sps_b200
+    from sps_b200.generation import random_state_dict
+    _, dims = _engine("sps", 2, 2, 128, 80, 200)
+    sd = random_state_dict(dims, seed=3, dtype=dtype)
+    flat = torch.empty(1 + sum(w.numel() + 1 for w in sd.values()), device="cuda", dtype=dtype)
+    views, at = {}, 1
+    for name, w in sd.items():
+        if "norm" in name:
+            views[name] = w
+            continue
+        at += 1 - at % 2                                   # an odd element
+        views[name] = flat[at:at + w.numel()].view(w.shape).copy_(w)
+        at += w.numel()
+    g = torch.Generator().manual_seed(7)
+    prompt, tokens = torch.randint(0, 197, (3, 9), generator=g), torch.randint(0, 197, (2, 3), generator=g)
+    outs = []
+    for params in (sd, views):
+        engine = sps_b200.SPSGenerator(params, dims, variant="sps", param_dtype=dtype)
+        state, logits = engine.prefill(prompt, 4)
+        engine._bind_step(state)
+        assert engine._step.fused == (params is sd and dtype == torch.bfloat16)
+        engine._step.fused = False
+        outs.append([logits.float()] + [engine.decode_one_token(state, t, torch.ones(3, dtype=torch.bool)).float() for t in tokens])
+    sps_b200.check_device_status()
+    for a, b in zip(*outs):
+        # the library may take another algorithm for such operands: bf16 projections, as above
+        assert float((a - b).norm()) <= 2.0 ** -6 * float(b.norm())
+
+
 @pytest.mark.parametrize("fused", [True, False])
 @pytest.mark.parametrize("bad", [-1, 200, 1 << 40])
 def test_a_token_outside_the_vocabulary_concerns_its_row_alone(fused, bad):

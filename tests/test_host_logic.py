@@ -306,3 +306,49 @@ def test_balanced_partition_and_grouped_block_order():
         # inside a group the tile number never increases
         first_group = [t for p, t in seen[:min(group, n_pairs) * n_qtiles]]
         assert first_group == sorted(first_group, reverse=True)
+
+
+def test_the_fused_decode_step_is_refused_for_weights_that_it_cannot_address():
+    """Its kernels copy by 16 bytes; weights may be views into a flat buffer, at any element."""
+    lib = _lib.load()
+
+    def decoder():
+        layers = (_lib.DecoderLayer * 2)()
+        for la in layers:
+            for name in ("attn_norm", "c_attn", "c_proj", "mlp_norm", "gate_up", "down"):
+                setattr(la, name, 4096)
+        d = _lib.Decoder()
+        d.n_layer, d.batch, d.slots, d.n_head, d.head_dim = 2, 3, 2, 2, 64
+        d.hidden, d.intermediate, d.vocab, d.n_segments = 128, 80, 200, 1
+        d.param_dtype, d.layers = _lib.DTYPE_BF16, layers
+        for name in ("wte", "lm_head", "out_norm", "freqs", "processed", "next_doc_start", "nw_len", "nw_pos", "br_len",
+                     "active", "pos", "x", "q", "k2", "v2", "y", "mlp_hidden", "ssq"):
+            setattr(d, name, 4096)
+        return d, layers
+
+    d, _ = decoder()
+    assert lib.spsattn_decoder_step_supported(ctypes.byref(d)) == 1
+    source = _lib.TokenSource()
+    source.token_in, source.active_in = 4096, 4096
+
+    def refused(d, code):
+        assert lib.spsattn_decoder_step_supported(ctypes.byref(d)) == 0
+        assert lib.spsattn_decoder_step(ctypes.byref(d), ctypes.byref(source), 4096, None, None) == code
+
+    for name in ("lm_head", "out_norm", "x", "q", "k2", "v2", "y", "mlp_hidden"):
+        for value, code in ((4098, -3), (None, -1)):
+            d, keep = decoder()
+            setattr(d, name, value)
+            refused(d, code)
+    for name in ("attn_norm", "c_attn", "c_proj", "mlp_norm", "gate_up", "down"):
+        for value, code in ((4098, -3), (None, -1)):
+            d, layers = decoder()
+            setattr(layers[1], name, value)
+            refused(d, code)
+    for name in ("ssq", "freqs", "pos", "active"):
+        d, keep = decoder()
+        setattr(d, name, None)
+        refused(d, -1)
+    d, keep = decoder()
+    d.wte = 4098                                     # read by elements where it has to be
+    assert lib.spsattn_decoder_step_supported(ctypes.byref(d)) == 1

@@ -16,6 +16,7 @@
 #include "decode.cuh"
 #include "decode_sm100.cuh"
 #include "decoder_step.cuh"
+#include "device_once.h"
 #include "kv_update.cuh"
 #include "model_glue.cuh"
 #include "prefill_aux.cuh"
@@ -139,6 +140,17 @@ int launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, c
   return (int)cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
+// Lets a kernel ask for `bytes` of dynamic shared memory on the current device (the limit is the device's own).
+template <typename K>
+int allow_shared_memory(std::atomic<uint64_t>& sized, K kernel, int bytes) {
+  int dev = 0;
+  const cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return (int)e;
+  return once_per_device(sized, dev, [&] {
+    return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  });
+}
+
 int multiprocessors() {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 148;
@@ -153,13 +165,8 @@ template <int D, bool FP16, bool kScan>
 int launch_prefill_kernel(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                          const PrefillParams& prm, cudaStream_t st) {
   using Cfg = PrefillCfg<D>;
-  static std::once_flag once;
-  static cudaError_t attr_err = cudaSuccess;
-  std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(prefill_sm100_kernel<D, FP16, kScan>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
-  });
-  if (attr_err != cudaSuccess) return (int)attr_err;
+  static std::atomic<uint64_t> sized{0};
+  if (const int rc = allow_shared_memory(sized, prefill_sm100_kernel<D, FP16, kScan>, Cfg::kSmemBytes)) return rc;
   const long long blocks = (long long)prm.n_qtiles * prm.B * prm.H;
   if (blocks <= 0 || blocks > 0x7fffffffLL) return SPSATTN_ERR_TOO_LARGE;
   // With document ids the kernel just before this one in the stream is the pre-pass (8 blocks of
@@ -197,13 +204,8 @@ int launch_prefill_sm100(const CUtensorMap& tq, const CUtensorMap& tk, const CUt
 template <bool FP16>
 int launch_prefill_wide(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                         const PrefillParams& prm, cudaStream_t st) {
-  static std::once_flag once;
-  static cudaError_t attr_err = cudaSuccess;
-  std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(prefill_wide_sm100_kernel<FP16>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg::kSmemBytes);
-  });
-  if (attr_err != cudaSuccess) return (int)attr_err;
+  static std::atomic<uint64_t> sized{0};
+  if (const int rc = allow_shared_memory(sized, prefill_wide_sm100_kernel<FP16>, WideCfg::kSmemBytes)) return rc;
   const long long items = (long long)prm.n_qtiles * prm.B * prm.H;
   if (items <= 0 || items > 0x7fffffffLL) return SPSATTN_ERR_TOO_LARGE;
   int dev = 0, sms = 0;
@@ -228,13 +230,8 @@ template <int D, bool FP16, int MODE>
 int launch_prefill_bwd(const CUtensorMap& x0, const CUtensorMap& x1, const CUtensorMap& y0,
                        const CUtensorMap& y1, const BwdParams& prm, cudaStream_t st) {
   using Cfg = BwdCfg<D, MODE>;
-  static std::once_flag once;
-  static cudaError_t attr_err = cudaSuccess;
-  std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(prefill_bwd_sm100_kernel<D, FP16, MODE>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
-  });
-  if (attr_err != cudaSuccess) return (int)attr_err;
+  static std::atomic<uint64_t> sized{0};
+  if (const int rc = allow_shared_memory(sized, prefill_bwd_sm100_kernel<D, FP16, MODE>, Cfg::kSmemBytes)) return rc;
   const long long blocks = (long long)prm.n_xtiles * prm.B * prm.H;
   if (blocks <= 0 || blocks > 0x7fffffffLL) return SPSATTN_ERR_TOO_LARGE;
   return launch_dependent(prefill_bwd_sm100_kernel<D, FP16, MODE>, dim3((unsigned)blocks), dim3(Cfg::kThreads),
@@ -376,13 +373,8 @@ int encode_cache_map(CUtensorMap* tm, const void* ptr, const spsattn_segment& sg
 template <int D, int NQ, bool FP16>
 int launch_decode_tc(const DecodeMaps& maps, const DecodeParams& prm, cudaStream_t st) {
   using Cfg = DecodeTcCfg<D>;
-  static std::once_flag once;
-  static cudaError_t attr_err = cudaSuccess;
-  std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(decode_tc_kernel<D, NQ, FP16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    Cfg::kSmemBytes);
-  });
-  if (attr_err != cudaSuccess) return (int)attr_err;
+  static std::atomic<uint64_t> sized{0};
+  if (const int rc = allow_shared_memory(sized, decode_tc_kernel<D, NQ, FP16>, Cfg::kSmemBytes)) return rc;
   // one block per chunk of a long segment; the record slot of the current-token entries and short
   // segments has no block of its own (slot 0's block fills it)
   int blocks_y = 0;
@@ -1326,14 +1318,8 @@ int launch_skinny(SkinnyParams p, cudaStream_t st) {
   }
   const int busy = 32 * p.warps + kSkinnyLoaders, threads = busy < kSkinnyMinThreads ? kSkinnyMinThreads : busy;
   auto* kernel = p.rows <= 8 ? skinny_gemm_kernel<EPI, 1> : skinny_gemm_kernel<EPI, 2>;
-  static std::once_flag once;
-  static cudaError_t attr_err = cudaSuccess;
-  std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(skinny_gemm_kernel<EPI, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (attr_err == cudaSuccess)
-      attr_err = cudaFuncSetAttribute(skinny_gemm_kernel<EPI, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  });
-  if (attr_err != cudaSuccess) return (int)attr_err;
+  static std::atomic<uint64_t> sized[2] = {};
+  if (const int rc = allow_shared_memory(sized[p.rows > 8], kernel, 200 * 1024)) return rc;
   return launch_dependent(kernel, dim3((unsigned)blocks), dim3((unsigned)threads), (size_t)(ring + fixed), st, p);
 }
 

@@ -352,3 +352,31 @@ def test_the_fused_decode_step_is_refused_for_weights_that_it_cannot_address():
     d, keep = decoder()
     d.wte = 4098                                     # read by elements where it has to be
     assert lib.spsattn_decoder_step_supported(ctypes.byref(d)) == 1
+
+
+def test_settings_are_made_once_on_every_device(tmp_path):
+    """The limit of a kernel's shared memory belongs to a device: the second one needs it too, and a
+    failure is tried again."""
+    import subprocess
+    source = tmp_path / "once.cpp"
+    source.write_text(r"""
+#include "device_once.h"
+#include <cstdio>
+#include <initializer_list>
+int main() {
+  std::atomic<uint64_t> done{0};
+  int calls = 0;
+  auto ok = [&] { ++calls; return 0; };
+  for (int device : {0, 0, 1, 63, 63, 1, 64, 64, -1}) std::printf("%d ", (spsattn::once_per_device(done, device, ok), calls));
+  calls = 0;
+  for (int rc : {98, 0, 98}) std::printf("%d ", spsattn::once_per_device(done, 5, [&] { return rc; }));
+}
+""")
+    exe = tmp_path / "once"
+    csrc = os.path.join(ROOT, "sps_b200", "csrc")
+    subprocess.run(["g++", "-std=c++17", "-I", csrc, str(source), "-o", str(exe)], check=True)
+    out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout
+    assert [int(x) for x in out.split()] == [1, 1, 2, 3, 3, 3, 4, 5, 6, 98, 0, 0]
+    # no launcher keeps such a setting by a flag of the process (the encoder lookup is the process's own)
+    api = open(os.path.join(csrc, "spsattn_api.cu")).read()
+    assert api.count("std::call_once") == 1 and api.count("cudaFuncSetAttribute(") == 1

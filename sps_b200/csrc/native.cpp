@@ -256,8 +256,11 @@ struct PrefillAttention : public torch::autograd::Function<PrefillAttention> {
   static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v,
                         const MaskArgs& m, const optional<Tensor>& docs) {
     Forward r = prefill_forward(q, k, v, m, docs, true, c10::nullopt);
-    ctx->save_for_backward({q, k, v, r.o, r.lse, r.ws});
+    ctx->save_for_backward({q, k, v, r.o, r.lse});
     if (docs.has_value()) ctx->saved_data["docs"] = *docs;
+    // not a saved tensor: hooks on those may give back other values (compressed ones, say), and these
+    // are row indices
+    if (r.ws.defined()) ctx->saved_data["runs"] = r.ws;
     ctx->saved_data["scale"] = m.sm_scale;
     ctx->saved_data["mask"] = std::vector<int64_t>{m.parity, m.temporary_window, m.persistent_window, m.flags,
                                                    (int64_t)m.has_persistent_window};
@@ -269,13 +272,16 @@ struct PrefillAttention : public torch::autograd::Function<PrefillAttention> {
     const auto saved = ctx->get_saved_variables();
     const auto mask = ctx->saved_data["mask"].toIntVector();
     MaskArgs m{ctx->saved_data["scale"].toDouble(), mask[0], mask[1], mask[2], mask[3], mask[4] != 0};
-    optional<Tensor> docs;
-    const auto it = ctx->saved_data.find("docs");
-    if (it != ctx->saved_data.end()) docs = it->second.toTensor();
+    auto kept = [ctx](const char* name) {
+      const auto it = ctx->saved_data.find(name);
+      return it == ctx->saved_data.end() ? optional<Tensor>() : it->second.toTensor();
+    };
+    const optional<Tensor> docs = kept("docs"), runs = kept("runs");
     torch::autograd::variable_list out(5);
     try {
       const at::AutoGradMode no_grad(false);
-      Gradients g = prefill_backward(saved[0], saved[1], saved[2], saved[3], saved[4], grads[0].detach(), m, docs, saved[5]);
+      Gradients g = prefill_backward(saved[0], saved[1], saved[2], saved[3], saved[4], grads[0].detach(), m, docs,
+                                     runs.value_or(Tensor()));
       out[0] = g.dq;
       out[1] = g.dk;
       out[2] = g.dv;

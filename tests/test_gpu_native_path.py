@@ -40,3 +40,20 @@ def test_a_second_differentiation_is_refused():
     (dq,) = torch.autograd.grad(o, q, d_o, create_graph=True)
     with pytest.raises(RuntimeError):
         dq.float().sum().backward()
+
+
+def test_hooks_on_saved_tensors_see_the_operands_and_results_alone():
+    """Hooks may give back other values than they were given; what the forward found out about the
+    documents (row indices) is none of their business."""
+    import sps_b200
+    q, k, v = (torch.randn(1, 2, 64, 64, device="cuda", dtype=torch.bfloat16, requires_grad=True) for _ in range(3))
+    docs = torch.arange(64, device="cuda").div(8, rounding_mode="floor").unsqueeze(0)
+    packed, grads = [], []
+    for hooked in (False, True):
+        pack = lambda x: (packed.append(x.dtype), x)[1]
+        with torch.autograd.graph.saved_tensors_hooks(pack if hooked else (lambda x: x), lambda x: x):
+            o = sps_b200.sps_sliding_attention(q, k, v, 1 / math.sqrt(64), 8, documents_idx_BxT=docs)
+            grads.append(torch.autograd.grad(o, (q, k, v), torch.ones_like(o)))
+    assert packed == [torch.bfloat16] * 4 + [torch.float32]
+    for a, b in zip(*grads):
+        assert torch.equal(a, b)

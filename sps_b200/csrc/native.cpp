@@ -3,7 +3,9 @@
 // (sps_b200._native).  A small attention call is bound by its host path, not by its kernels: the
 // same steps in Python with ctypes took 32-38 us per forward call and about 40 us more per
 // backward, against 8-13 us of kernel time.  Functions take positional arguments only and raise what
-// their Python wrappers document; nothing here synchronises.
+// their Python wrappers document; nothing here synchronises.  Whatever may launch or allocate runs without
+// the interpreter lock (a launch blocks while its stream's queue is full, and what empties the queue may
+// need another Python thread).
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -86,6 +88,19 @@ bool bool_arg(PyObject* o) {
 at::ScalarType dtype_arg(PyObject* o) {
   if (!THPDtype_Check(o)) fail(PyExc_TypeError, "expected a torch.dtype");
   return reinterpret_cast<THPDtype*>(o)->scalar_type;
+}
+
+struct Unlocked {         // the interpreter lock is given up while one of these lives
+  PyThreadState* state = PyEval_SaveThread();
+  Unlocked() = default;
+  Unlocked(const Unlocked&) = delete;
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
+
+template <typename F>
+auto unlocked(F&& f) {
+  const Unlocked u;
+  return f();
 }
 
 struct PyRef {            // owned reference
@@ -337,9 +352,9 @@ PyObject* prefill_impl(PyObject* const* a, Py_ssize_t n) {
   const optional<Tensor> out = optional_tensor(a[10], "out");
   if (needs_grad({&q, &k, &v})) {
     if (q.dim() != 4 || !backward_head_dim(q.size(3)) || return_lse || out.has_value()) forward_only({&q, &k, &v});
-    return THPVariable_Wrap(PrefillAttention::apply(q, k, v, m, docs));
+    return THPVariable_Wrap(unlocked([&] { return PrefillAttention::apply(q, k, v, m, docs); }));
   }
-  Forward r = prefill_forward(q, k, v, m, docs, return_lse, out);
+  Forward r = unlocked([&] { return prefill_forward(q, k, v, m, docs, return_lse, out); });
   if (!return_lse) return out.has_value() ? Py_NewRef(a[10]) : THPVariable_Wrap(std::move(r.o));
   PyRef o(out.has_value() ? Py_NewRef(a[10]) : THPVariable_Wrap(std::move(r.o)));
   PyRef lse(THPVariable_Wrap(std::move(r.lse)));
@@ -351,9 +366,11 @@ PyObject* prefill_backward_impl(PyObject* const* a, Py_ssize_t n) {
   if (n != 12) fail(PyExc_TypeError, "prefill_backward takes 12 arguments");
   const Tensor& q = tensor_arg(a[0], "q");
   if (q.dim() != 4) fail(PyExc_ValueError, "q must be [B, H, N, D]");
-  Gradients g = prefill_backward(q, tensor_arg(a[1], "k"), tensor_arg(a[2], "v"), tensor_arg(a[3], "o"),
-                                 tensor_arg(a[4], "lse"), tensor_arg(a[5], "d_o"), mask_args(a + 6),
-                                 optional_tensor(a[11], "document ids"));
+  const Tensor &k = tensor_arg(a[1], "k"), &v = tensor_arg(a[2], "v"), &o = tensor_arg(a[3], "o"),
+               &lse = tensor_arg(a[4], "lse"), &d_o = tensor_arg(a[5], "d_o");
+  const MaskArgs m = mask_args(a + 6);
+  const optional<Tensor> docs = optional_tensor(a[11], "document ids");
+  Gradients g = unlocked([&] { return prefill_backward(q, k, v, o, lse, d_o, m, docs); });
   PyRef dq(THPVariable_Wrap(std::move(g.dq))), dk(THPVariable_Wrap(std::move(g.dk))), dv(THPVariable_Wrap(std::move(g.dv)));
   return PyTuple_Pack(3, dq.p, dk.p, dv.p);
 }
@@ -424,9 +441,9 @@ struct DecodeCall {
     if (q.dim() != 4) fail(PyExc_ValueError, "q must be [S, nq, H, D]");
     forward_only({&q});
     s = q.size(0), nq = q.size(1), h = q.size(2), d = q.size(3);
-    if (!q.is_contiguous()) q = q.contiguous();
+    if (!q.is_contiguous()) q = unlocked([&] { return q.contiguous(); });
     dtype_code(q);
-    keep.reserve(12);
+    keep.reserve(16);
   }
 
   void add_segment(PyObject* seg, unsigned mask) {
@@ -438,12 +455,13 @@ struct DecodeCall {
     forward_only({&k, &v});
     Tensor lengths = attr_tensor(seg, nm.lengths);
     if (lengths.device() != q.device()) fail(PyExc_RuntimeError, "Segment lengths must live on the same device as query");
-    if (lengths.scalar_type() != at::kLong) lengths = lengths.to(at::kLong);
-    if (!lengths.is_contiguous()) lengths = lengths.contiguous();
+    if (lengths.scalar_type() != at::kLong || !lengths.is_contiguous())
+      lengths = unlocked([&] { return lengths.to(at::kLong).contiguous(); });
     const int packed = g_packed_type ? PyObject_IsInstance(seg, g_packed_type) : 0;
     if (packed < 0) throw python_error();
     if (packed) {
-      Tensor off = attr_tensor(seg, nm.seq_offset).to(at::kLong).contiguous();
+      Tensor off = attr_tensor(seg, nm.seq_offset);
+      if (off.scalar_type() != at::kLong || !off.is_contiguous()) off = unlocked([&] { return off.to(at::kLong).contiguous(); });
       st.seq_offset = off.data_ptr<int64_t>();
       keep.push_back(std::move(off));
       st.head_stride = attr_int(seg, nm.head_stride);
@@ -481,7 +499,10 @@ struct DecodeCall {
     st.lengths = lengths.data_ptr<int64_t>();
     st.lengths_per_head = lengths.dim() == 2;
     st.query_mask = mask;
+    // the caches too: without the lock nothing else holds the segment's attributes to the launch
     keep.push_back(std::move(lengths));
+    keep.push_back(k);
+    keep.push_back(v);
     ++n_segs;
   }
 
@@ -493,8 +514,8 @@ struct DecodeCall {
       if (x->dim() != 3 || x->size(0) != s || x->size(1) != h || x->size(2) != d)
         fail(PyExc_RuntimeError, "Current-token K/V tensors must have shape " + c10::str(at::IntArrayRef({s, h, d})) +
                                      ", got " + c10::str(x->sizes()));
-      if (x->scalar_type() != q.scalar_type()) *x = x->to(q.scalar_type());
-      if (!x->is_contiguous()) *x = x->contiguous();
+      if (x->scalar_type() != q.scalar_type() || !x->is_contiguous())
+        *x = unlocked([&] { return x->to(q.scalar_type()).contiguous(); });
     }
     spsattn_extra& e = extras[n_extras++];
     e = spsattn_extra{};
@@ -506,6 +527,7 @@ struct DecodeCall {
   }
 
   Tensor launch(double scale) {
+    const Unlocked u;
     const c10::cuda::CUDAGuard guard(q.device());
     void* stream = stream_of(q);
     Tensor out = at::detail::empty_cuda({s, nq, h, d}, at::kFloat, q.device(), c10::nullopt);
@@ -562,7 +584,7 @@ PyObject* decode_q2_impl(PyObject* const* a, Py_ssize_t n) {
   if (q.size(3) <= 0 || q.size(3) > 256)
     fail(PyExc_RuntimeError, "Unsupported SPS-family q2 attention head_dim=" + std::to_string(q.size(3)));
   const at::ScalarType dt = dtype_arg(a[6]);
-  if (q.scalar_type() != dt) q = q.to(dt);
+  if (q.scalar_type() != dt) q = unlocked([&] { return q.to(dt); });
   DecodeCall call(q);
   for (Py_ssize_t i = 0; i < segs.n; ++i) call.add_segment(segs[i], 0xFF);
   call.add_extra(tensor_arg(a[2], "normal k"), tensor_arg(a[3], "normal v"), 3);
@@ -577,7 +599,7 @@ PyObject* decode_q1_impl(PyObject* const* a, Py_ssize_t n) {
   if (segs.n > 3) fail(PyExc_RuntimeError, "q1 attention supports at most 3 segments, got " + std::to_string(segs.n));
   Tensor q = tensor_arg(a[0], "q");
   const at::ScalarType dt = dtype_arg(a[3]);
-  if (q.scalar_type() != dt) q = q.to(dt);
+  if (q.scalar_type() != dt) q = unlocked([&] { return q.to(dt); });
   if (q.dim() != 3) fail(PyExc_ValueError, "q must be [B, H, D]");
   DecodeCall call(q.unsqueeze(1));
   for (Py_ssize_t i = 0; i < segs.n; ++i) call.add_segment(segs[i], 0xFF);
@@ -608,11 +630,11 @@ PyObject* kv_update_impl(PyObject* const* a, Py_ssize_t n) {
               br_len.is_contiguous(),
           "br_len must be contiguous int64 [B, H]");
   // a bool tensor holds the 0 / 1 bytes that the kernel reads
-  if (active.scalar_type() != at::kChar && active.scalar_type() != at::kBool) active = active.to(at::kChar);
-  if (!active.is_contiguous()) active = active.contiguous();
+  if ((active.scalar_type() != at::kChar && active.scalar_type() != at::kBool) || !active.is_contiguous())
+    active = unlocked([&] { return active.to(active.scalar_type() == at::kBool ? at::kBool : at::kChar).contiguous(); });
   auto row = [](Tensor& x, const Tensor& like) {
-    if (x.scalar_type() != like.scalar_type()) x = x.to(like.scalar_type());
-    if (!x.is_contiguous()) x = x.contiguous();
+    if (x.scalar_type() != like.scalar_type() || !x.is_contiguous())
+      x = unlocked([&] { return x.to(like.scalar_type()).contiguous(); });
   };
   row(kr, br_k);
   row(vr, br_v);
@@ -635,12 +657,14 @@ PyObject* kv_update_impl(PyObject* const* a, Py_ssize_t n) {
     nw_k_ptr = nw_k.data_ptr(), nw_v_ptr = nw_v.data_ptr();
     nw_len_ptr = nw_len.data_ptr<int64_t>(), nw_pos_ptr = nw_pos.data_ptr<int64_t>();
   }
-  const c10::cuda::CUDAGuard guard(br_k.device());
-  const int rc = spsattn_kv_update(
-      nw_k_ptr, nw_v_ptr, nw_len_ptr, nw_pos_ptr, br_k.data_ptr(), br_v.data_ptr(), br_len.data_ptr<int64_t>(),
-      kw.defined() ? kw.data_ptr() : nullptr, vw.defined() ? vw.data_ptr() : nullptr, kr.data_ptr(), vr.data_ptr(),
-      reinterpret_cast<const int8_t*>(active.data_ptr()), b, h, d, storage, br_k.size(2), (int)window_tokens,
-      (int)br_k.element_size(), stream_of(br_k));
+  const int rc = unlocked([&] {
+    const c10::cuda::CUDAGuard guard(br_k.device());
+    return spsattn_kv_update(
+        nw_k_ptr, nw_v_ptr, nw_len_ptr, nw_pos_ptr, br_k.data_ptr(), br_v.data_ptr(), br_len.data_ptr<int64_t>(),
+        kw.defined() ? kw.data_ptr() : nullptr, vw.defined() ? vw.data_ptr() : nullptr, kr.data_ptr(), vr.data_ptr(),
+        reinterpret_cast<const int8_t*>(active.data_ptr()), b, h, d, storage, br_k.size(2), (int)window_tokens,
+        (int)br_k.element_size(), stream_of(br_k));
+  });
   check_rc(rc, "spsattn_kv_update");
   Py_RETURN_NONE;
 }
@@ -651,7 +675,8 @@ PyObject* kv_update_impl(PyObject* const* a, Py_ssize_t n) {
 
 PyObject* status_word_impl(PyObject* const* a, Py_ssize_t n) {
   if (n != 1) fail(PyExc_TypeError, "status_word takes 1 argument");
-  return THPVariable_Wrap(status_word((int)int_arg(a[0])));
+  const int device = (int)int_arg(a[0]);
+  return THPVariable_Wrap(unlocked([&] { return status_word(device); }));
 }
 
 // setup(SpsAttnError, PackedKVSegment)

@@ -88,39 +88,32 @@ PyObject* engine_scan_impl(PyObject* const* a, Py_ssize_t n) {
   const Tensor& ids = tensor_arg(a[1], "ids");
   require(ids.is_cuda() && ids.dim() == 2 && ids.scalar_type() == at::kLong && ids.is_contiguous(), "ids must be contiguous int64 [B, T]");
   const int64_t b = ids.size(0), t = ids.size(1), rows = t * m.slots;
-  const c10::cuda::CUDAGuard guard(ids.device());
-  auto make = [&](at::IntArrayRef shape, at::ScalarType type) {
-    return at::detail::empty_cuda(shape, type, ids.device(), c10::nullopt);
-  };
-  Tensor ids2 = make({b, rows}, at::kLong), pos2 = make({b, rows}, at::kLong), runs = make({b, rows}, at::kInt);
-  Tensor mask = make({b, t}, at::kByte), real = make({b}, at::kLong), ends = make({b}, at::kByte), flags = make({4}, at::kLong);
-  check_rc(spsattn_prompt_scan(ids.data_ptr<int64_t>(), (int)b, (int)t, (int)m.slots, int_arg(a[2]), int_arg(a[3]), int_arg(a[4]),
-                               bool_arg(a[5]), ids2.data_ptr<int64_t>(), pos2.data_ptr<int64_t>(), runs.data_ptr<int>(),
-                               mask.data_ptr<uint8_t>(), real.data_ptr<int64_t>(), ends.data_ptr<uint8_t>(),
-                               flags.data_ptr<int64_t>(), status_ptr(ids), stream_of(ids)),
-           "spsattn_prompt_scan");
+  const long long eos = int_arg(a[2]), pad = int_arg(a[3]), predict = int_arg(a[4]);
+  const bool empty_after_eos = bool_arg(a[5]);
+  Tensor ids2, pos2, runs, mask, real, ends, flags;
+  unlocked([&] {
+    const c10::cuda::CUDAGuard guard(ids.device());
+    auto make = [&](at::IntArrayRef shape, at::ScalarType type) {
+      return at::detail::empty_cuda(shape, type, ids.device(), c10::nullopt);
+    };
+    ids2 = make({b, rows}, at::kLong), pos2 = make({b, rows}, at::kLong), runs = make({b, rows}, at::kInt);
+    mask = make({b, t}, at::kByte), real = make({b}, at::kLong), ends = make({b}, at::kByte), flags = make({4}, at::kLong);
+    check_rc(spsattn_prompt_scan(ids.data_ptr<int64_t>(), (int)b, (int)t, (int)m.slots, eos, pad, predict, empty_after_eos,
+                                 ids2.data_ptr<int64_t>(), pos2.data_ptr<int64_t>(), runs.data_ptr<int>(),
+                                 mask.data_ptr<uint8_t>(), real.data_ptr<int64_t>(), ends.data_ptr<uint8_t>(),
+                                 flags.data_ptr<int64_t>(), status_ptr(ids), stream_of(ids)),
+             "spsattn_prompt_scan");
+  });
   PyRef r0(THPVariable_Wrap(ids2)), r1(THPVariable_Wrap(pos2)), r2(THPVariable_Wrap(runs)), r3(THPVariable_Wrap(mask)),
       r4(THPVariable_Wrap(real)), r5(THPVariable_Wrap(ends)), r6(THPVariable_Wrap(flags));
   return PyTuple_Pack(7, r0.p, r1.p, r2.p, r3.p, r4.p, r5.p, r6.p);
 }
 
-// engine_prefill(model, ids2 [B, N], pos2 [B, N], docs [B, N] int64 | run_start [B, N] int32,
-//                caches (nw_k, nw_v, nw_len, nw_pos, br_k, br_v, br_len) or None, doc_mask or None)
-//   -> final-norm hidden states [B, N, C]; the caches of all layers filled on the way
-PyObject* engine_prefill_impl(PyObject* const* a, Py_ssize_t n) {
-  if (n != 6) fail(PyExc_TypeError, "engine_prefill takes 6 arguments");
-  const EngineModel& m = engine_arg(a[0]);
-  const Tensor &ids2 = tensor_arg(a[1], "ids2"), &pos2 = tensor_arg(a[2], "pos2"), &docs = tensor_arg(a[3], "documents");
+// Final-norm hidden states [B, N, C] of doubled ids; the caches of all layers (none: empty) filled on the way.
+Tensor prefill_chain(const EngineModel& m, const Tensor& ids2, const Tensor& pos2, const Tensor& docs, const std::vector<Tensor>& caches,
+                     const Tensor& mask) {
   const int64_t b = ids2.size(0), rows = ids2.size(1), all = b * rows, C = m.C, H = m.heads, D = m.head_dim;
   const bool runs = docs.scalar_type() == at::kInt;
-  require(docs.dim() == 2 && docs.size(0) == b && docs.size(1) == rows && docs.is_contiguous(), "documents must be contiguous [B, N]");
-  std::vector<Tensor> caches;
-  Tensor mask;
-  if (a[4] != Py_None) {
-    caches = tensor_list(a[4], false);
-    require(caches.size() == 7, "seven cache tensors are needed");
-    mask = tensor_arg(a[5], "doc_mask");
-  }
   const c10::cuda::CUDAGuard guard(ids2.device());
   void* stream = stream_of(ids2);
   int* status = status_ptr(ids2);
@@ -181,7 +174,25 @@ PyObject* engine_prefill_impl(PyObject* const* a, Py_ssize_t n) {
     check_rc(rc, "spsattn_prefill_fwd");
     block_tail(m, l, m.f32() ? y.to(pt) : y, x, xn, delta, gate_up, hidden, stream);
   }
-  return THPVariable_Wrap(xn.view({b, rows, C}));
+  return xn.view({b, rows, C});
+}
+
+// engine_prefill(model, ids2 [B, N], pos2 [B, N], docs [B, N] int64 | run_start [B, N] int32,
+//                caches (nw_k, nw_v, nw_len, nw_pos, br_k, br_v, br_len) or None, doc_mask or None)
+//   -> final-norm hidden states [B, N, C]; the caches of all layers filled on the way
+PyObject* engine_prefill_impl(PyObject* const* a, Py_ssize_t n) {
+  if (n != 6) fail(PyExc_TypeError, "engine_prefill takes 6 arguments");
+  const EngineModel& m = engine_arg(a[0]);
+  const Tensor &ids2 = tensor_arg(a[1], "ids2"), &pos2 = tensor_arg(a[2], "pos2"), &docs = tensor_arg(a[3], "documents");
+  require(docs.dim() == 2 && docs.sizes() == ids2.sizes() && docs.is_contiguous(), "documents must be contiguous [B, N]");
+  std::vector<Tensor> caches;
+  Tensor mask;
+  if (a[4] != Py_None) {
+    caches = tensor_list(a[4], false);
+    require(caches.size() == 7, "seven cache tensors are needed");
+    mask = tensor_arg(a[5], "doc_mask");
+  }
+  return THPVariable_Wrap(unlocked([&] { return prefill_chain(m, ids2, pos2, docs, caches, mask); }));
 }
 
 // engine_step(model, decoder address, source address, rope groups address, buffers (x, xn, delta, qkv, y,
@@ -197,31 +208,33 @@ PyObject* engine_step_impl(PyObject* const* a, Py_ssize_t n) {
   require(d && source && groups && buf.size() == 8, "engine_step needs its argument blocks and eight buffers");
   Tensor &x = buf[0], &xn = buf[1], &delta = buf[2], &qkv = buf[3], &y = buf[4], &gate_up = buf[5], &hidden = buf[6], &fc = buf[7];
   Tensor logits = tensor_arg(a[5], "logits");
-  const c10::cuda::CUDAGuard guard(x.device());
-  void* stream = stream_of(x);
-  int* status = status_ptr(x);
-  const int ns = d->slots, b = d->batch;
-  const int64_t C = m.C, D = m.head_dim;
-  check_rc(spsattn_decoder_start(d, source, status, stream), "spsattn_decoder_start");
-  spsattn_extra extras[2] = {};
-  for (int s = 0; s < ns; ++s) {
-    extras[s].k = reinterpret_cast<const uint16_t*>(d->k2) + (size_t)s * b * C;
-    extras[s].v = reinterpret_cast<const uint16_t*>(d->v2) + (size_t)s * b * C;
-    extras[s].query_mask = s == 0 ? (1u << ns) - 1 : 2u;
-  }
-  norm_into(m, x, nullptr, m.attn_norm[0], xn, stream);
-  for (int l = 0; l < m.layers(); ++l) {
-    const spsattn_decoder_layer& w = d->layers[l];
-    at::mm_out(qkv, xn, m.c_attn[l]);
-    check_rc(spsattn_qkv_rope_cast(qkv.data_ptr(), m.f32() ? 2 : 0, 3 * ns * C, 0, D, fc.data_ptr<float>(), D / 2, groups, 3 * ns,
-                                   SPSATTN_DTYPE_BF16, b, 1, (int)m.heads, (int)D, stream),
-             "spsattn_qkv_rope_cast");
-    check_rc(spsattn_decode_step(d->q, ns, d->y, SPSATTN_DTYPE_BF16, w.segments, d->n_segments, extras, ns, &w.append, b,
-                                 (int)m.heads, (int)D, SPSATTN_DTYPE_BF16, (float)(1.0 / std::sqrt((double)D)), d->workspace,
-                                 d->workspace_bytes, status, stream),
-             "spsattn_decode_step");
-    block_tail(m, l, m.f32() ? y.to(x.scalar_type()) : y, x, xn, delta, gate_up, hidden, stream);
-  }
-  at::mm_out(logits, xn.view({b, ns, C}).select(1, d->pred_slot), m.lm_head);
+  unlocked([&] {
+    const c10::cuda::CUDAGuard guard(x.device());
+    void* stream = stream_of(x);
+    int* status = status_ptr(x);
+    const int ns = d->slots, b = d->batch;
+    const int64_t C = m.C, D = m.head_dim;
+    check_rc(spsattn_decoder_start(d, source, status, stream), "spsattn_decoder_start");
+    spsattn_extra extras[2] = {};
+    for (int s = 0; s < ns; ++s) {
+      extras[s].k = reinterpret_cast<const uint16_t*>(d->k2) + (size_t)s * b * C;
+      extras[s].v = reinterpret_cast<const uint16_t*>(d->v2) + (size_t)s * b * C;
+      extras[s].query_mask = s == 0 ? (1u << ns) - 1 : 2u;
+    }
+    norm_into(m, x, nullptr, m.attn_norm[0], xn, stream);
+    for (int l = 0; l < m.layers(); ++l) {
+      const spsattn_decoder_layer& w = d->layers[l];
+      at::mm_out(qkv, xn, m.c_attn[l]);
+      check_rc(spsattn_qkv_rope_cast(qkv.data_ptr(), m.f32() ? 2 : 0, 3 * ns * C, 0, D, fc.data_ptr<float>(), D / 2, groups, 3 * ns,
+                                     SPSATTN_DTYPE_BF16, b, 1, (int)m.heads, (int)D, stream),
+               "spsattn_qkv_rope_cast");
+      check_rc(spsattn_decode_step(d->q, ns, d->y, SPSATTN_DTYPE_BF16, w.segments, d->n_segments, extras, ns, &w.append, b,
+                                   (int)m.heads, (int)D, SPSATTN_DTYPE_BF16, (float)(1.0 / std::sqrt((double)D)), d->workspace,
+                                   d->workspace_bytes, status, stream),
+               "spsattn_decode_step");
+      block_tail(m, l, m.f32() ? y.to(x.scalar_type()) : y, x, xn, delta, gate_up, hidden, stream);
+    }
+    at::mm_out(logits, xn.view({b, ns, C}).select(1, d->pred_slot), m.lm_head);
+  });
   Py_RETURN_NONE;
 }

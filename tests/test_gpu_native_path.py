@@ -57,3 +57,67 @@ def test_hooks_on_saved_tensors_see_the_operands_and_results_alone():
     assert packed == [torch.bfloat16] * 4 + [torch.float32]
     for a, b in zip(*grads):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("call", ["prefill", "backward", "decode", "kv_update", "engine"])
+def test_other_threads_run_while_a_launch_waits_for_room_in_its_queue(call):
+    """A launch blocks while its stream's queue is full.  What empties the queue may depend on another
+    Python thread (a collective's other rank), so the interpreter lock must not be held meanwhile."""
+    import threading
+    import time
+    import sps_b200
+    from sps_b200.attention import prefill_attention_backward
+    bf = torch.bfloat16
+    rnd = lambda *s: torch.randn(s, device="cuda").to(bf)
+    if call in ("prefill", "backward"):
+        q, k, v = (rnd(1, 1, 64, 64).requires_grad_(call == "backward") for _ in range(3))
+        with torch.no_grad():
+            o, lse = sps_b200.prefill_attention(q, k, v, 0.125, persistent_parity=0, temporary_window=8, return_lse=True)
+        run = ((lambda: sps_b200.sps_sliding_attention(q, k, v, 0.125, 8)) if call == "prefill" else
+               (lambda: prefill_attention_backward(q.detach(), k.detach(), v.detach(), o, lse, o, 0.125,
+                                                   persistent_parity=0, temporary_window=8)))
+    elif call == "decode":
+        q, seg = rnd(1, 1, 64), sps_b200.KVSegment(rnd(1, 1, 8, 64), rnd(1, 1, 8, 64), torch.tensor([8], device="cuda"))
+        run = lambda: sps_b200.masked_kv_attention(q, [seg], attn_dtype=bf)
+    elif call == "kv_update":
+        k, v, row = rnd(1, 1, 8, 64), rnd(1, 1, 8, 64), rnd(1, 1, 64)
+        length, active = torch.zeros(1, 1, dtype=torch.long, device="cuda"), torch.ones(1, dtype=torch.bool, device="cuda")
+        run = lambda: sps_b200.fused_sps_kv_update(
+            nw_k=None, nw_v=None, nw_len=None, nw_pos=None, br_k=k, br_v=v, br_len=length, k_window_BxHxD=None,
+            v_window_BxHxD=None, k_retained_BxHxD=row, v_retained_BxHxD=row, active_mask_B=active, window_tokens=0)
+    else:
+        from sps_b200.generation import random_state_dict
+        dims = sps_b200.SPSDims(block_size=64, vocab_size=200, n_layer=4, n_head=2, hidden_size=128, intermediate_size=80,
+                                eos_token_id=197, pad_token_id=199, predict_token_id=198)
+        engine = sps_b200.SPSGenerator(random_state_dict(dims), dims)
+        ext, model = engine._native()
+        ids = torch.randint(0, 197, (2, 16), device="cuda")
+        pos = torch.arange(16, device="cuda").expand(2, -1)
+        docs = torch.zeros(2, 16, dtype=torch.long, device="cuda")
+        run = lambda: ext.engine_prefill(model, ids, pos, docs, None, None)
+    run()
+    torch.cuda.synchronize()
+    gaps, done = [0.0], threading.Event()
+
+    def tick():
+        last = time.perf_counter()
+        while not done.is_set():
+            time.sleep(0.002)
+            now = time.perf_counter()
+            gaps[0] = max(gaps[0], now - last)
+            last = now
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    try:
+        torch.cuda._sleep(int(2e9))                       # about a second of the GPU
+        began = time.perf_counter()
+        for _ in range(6000 if call != "engine" else 200):    # some thousands of launches: more than a queue holds
+            run()
+        blocked = time.perf_counter() - began
+        torch.cuda.synchronize()
+    finally:
+        done.set()
+        thread.join()
+    assert blocked > 0.5                                   # the queue was full
+    assert gaps[0] < 0.3

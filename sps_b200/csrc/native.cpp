@@ -45,6 +45,14 @@ PyObject* g_packed_type = nullptr;     // sps_b200.decode.PackedKVSegment
 
 [[noreturn]] void fail(PyObject* type, const std::string& message) { throw PyError{type, message}; }
 
+// As the exception that torch carries through its own code; the interpreter lock is held.
+[[noreturn]] void raise(const PyError& e) {
+  PyErr_SetString(e.type ? e.type : PyExc_RuntimeError, e.message.c_str());
+  python_error err;
+  err.persist();
+  throw err;
+}
+
 void require(bool ok, const char* message) {
   if (!ok) fail(PyExc_AssertionError, message);
 }
@@ -302,10 +310,7 @@ struct PrefillAttention : public torch::autograd::Function<PrefillAttention> {
       out[2] = g.dv;
     } catch (const PyError& e) {          // runs on an autograd thread: hand the exception over
       pybind11::gil_scoped_acquire gil;
-      PyErr_SetString(e.type, e.message.c_str());
-      python_error err;
-      err.persist();
-      throw err;
+      raise(e);
     }
     if (at::GradMode::is_enabled() && grads[0].requires_grad()) {
       auto twice = std::make_shared<torch::autograd::DelayedError>(
@@ -689,18 +694,13 @@ PyObject* setup_impl(PyObject* const* a, Py_ssize_t n) {
 
 template <PyObject* (*F)(PyObject* const*, Py_ssize_t)>
 PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS          // torch's errors (out of memory, say) as torch's own functions raise them
   try {
     return F(args, n);
   } catch (const PyError& e) {
-    PyErr_SetString(e.type ? e.type : PyExc_RuntimeError, e.message.c_str());
-  } catch (python_error& e) {
-    e.restore();
-  } catch (const c10::Error& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
+    raise(e);
   }
-  return nullptr;
+  END_HANDLE_TH_ERRORS
 }
 
 #define SPS_ENTRY(name, fn) \

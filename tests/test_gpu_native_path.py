@@ -121,3 +121,17 @@ def test_other_threads_run_while_a_launch_waits_for_room_in_its_queue(call):
         thread.join()
     assert blocked > 0.5                                   # the queue was full
     assert gaps[0] < 0.3
+
+
+def test_running_out_of_memory_raises_torchs_error():
+    """Programs that look for a batch that fits catch it by its type."""
+    import sps_b200
+    one = torch.zeros(1, 1, 1, 64, device="cuda", dtype=torch.bfloat16)
+    q = one.expand(1, 1, 1 << 40, 64)                      # its copy would take 128 TB
+    with pytest.raises(torch.OutOfMemoryError):
+        sps_b200.full_attention(q, q, q, 0.125)
+    seg = sps_b200.KVSegment(one, one, torch.tensor([1], device="cuda"))
+    with pytest.raises(torch.OutOfMemoryError):
+        sps_b200.masked_kv_attention(one[0].expand(1 << 40, 1, 64), [seg], attn_dtype=torch.bfloat16)
+    with pytest.raises(TypeError):
+        sps_b200.masked_kv_attention(one[0], 3, attn_dtype=torch.bfloat16)

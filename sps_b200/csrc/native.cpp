@@ -20,6 +20,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <limits>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -75,10 +76,17 @@ optional<Tensor> optional_tensor(PyObject* o, const char* name) {
   return tensor_arg(o, name);
 }
 
-long long int_arg(PyObject* o) {
-  const long long v = PyLong_AsLongLong(o);
+// int(o); with `saturate`, a value past the range of 64 bits is its end (a window longer than any row)
+long long int_arg(PyObject* o, bool saturate = false) {
+  PyObject* whole = PyLong_CheckExact(o) ? Py_NewRef(o) : PyNumber_Long(o);
+  if (!whole) throw python_error();
+  int past = 0;
+  const long long v = PyLong_AsLongLongAndOverflow(whole, &past);
+  Py_DECREF(whole);
   if (v == -1 && PyErr_Occurred()) throw python_error();
-  return v;
+  if (past == 0) return v;
+  if (!saturate) fail(PyExc_OverflowError, "the number does not fit 64 bits");
+  return past > 0 ? std::numeric_limits<long long>::max() : std::numeric_limits<long long>::min();
 }
 
 double float_arg(PyObject* o) {
@@ -340,9 +348,9 @@ MaskArgs mask_args(PyObject* const* a) {     // sm_scale, parity, temporary, per
   MaskArgs m;
   m.sm_scale = float_arg(a[0]);
   m.parity = int_arg(a[1]);
-  m.temporary_window = int_arg(a[2]);
+  m.temporary_window = int_arg(a[2], true);
   m.has_persistent_window = a[3] != Py_None;
-  m.persistent_window = m.has_persistent_window ? int_arg(a[3]) : 0;
+  m.persistent_window = m.has_persistent_window ? int_arg(a[3], true) : 0;
   m.flags = int_arg(a[4]);
   return m;
 }
@@ -427,8 +435,7 @@ Tensor attr_tensor(PyObject* o, PyObject* name) {
 
 long long attr_int(PyObject* o, PyObject* name) {
   const PyRef r(PyObject_GetAttr(o, name));
-  const PyRef i(PyNumber_Long(r.p));
-  return int_arg(i.p);
+  return int_arg(r.p);
 }
 
 constexpr int kSegmentLimit = 16, kExtraLimit = 16;    // beyond the library's own limits, which it checks itself
@@ -488,8 +495,7 @@ struct DecodeCall {
       if (max_t > 0) {
         const PyRef cap(PyObject_GetAttr(seg, nm.max_len_cap));
         if (cap.p != Py_None) {
-          const PyRef whole(PyNumber_Long(cap.p));
-          const long long c = int_arg(whole.p);
+          const long long c = int_arg(cap.p, true);
           if (c < 0) fail(PyExc_ValueError, "KVSegment.max_len_cap must be non-negative, got " + std::to_string(c));
           scan = std::max<int64_t>(1, std::min<int64_t>(max_t, c));
         }

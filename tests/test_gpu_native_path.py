@@ -135,3 +135,35 @@ def test_running_out_of_memory_raises_torchs_error():
         sps_b200.masked_kv_attention(one[0].expand(1 << 40, 1, 64), [seg], attn_dtype=torch.bfloat16)
     with pytest.raises(TypeError):
         sps_b200.masked_kv_attention(one[0], 3, attn_dtype=torch.bfloat16)
+
+
+def test_numbers_of_any_type_that_int_takes():
+    import numpy as np
+    import sps_b200
+    bf = torch.bfloat16
+    q, k, v = (torch.randn(1, 2, 96, 64, device="cuda").to(bf) for _ in range(3))
+    call = lambda tw, pw, **kw: sps_b200.prefill_attention(q, k, v, 0.125, temporary_window=tw, persistent_window=pw,
+                                                           **{"persistent_parity": 0, **kw})
+    want = call(5, 9)
+    for tw, pw in ((5.0, 9.7), (np.int32(5), np.float64(9)), (torch.tensor(5), torch.tensor(9.0, device="cuda"))):
+        assert torch.equal(call(tw, pw, persistent_parity=np.float32(0), mask_flags=0.0), want)
+    for long in (1 << 70, -(1 << 70)):
+        assert torch.equal(call(long, long), call(200 if long > 0 else -1, 200 if long > 0 else -1))
+    with pytest.raises((TypeError, ValueError)):
+        call(5, "nine")
+    # decode: query masks, the scan limit of a segment; cache update: ring size
+    kc, vc = torch.randn(1, 2, 8, 64, device="cuda").to(bf), torch.randn(1, 2, 8, 64, device="cuda").to(bf)
+    qd, e = torch.randn(1, 2, 2, 64, device="cuda").to(bf), torch.randn(1, 2, 64, device="cuda").to(bf)
+    seg = lambda cap: sps_b200.KVSegment(kc, vc, torch.tensor([8], device="cuda"), max_len_cap=cap)
+    want = sps_b200.decode_attention(qd, [seg(4)], [(e, e, 2)], segment_query_masks=[1])
+    assert torch.equal(sps_b200.decode_attention(qd, [seg(4.0)], [(e, e, 2.0)], segment_query_masks=[np.float64(1)]), want)
+    assert torch.equal(sps_b200.decode_attention(qd, [seg(1 << 70)], []), sps_b200.decode_attention(qd, [seg(None)], []))
+    lens = []
+    for window in (4, 4.0):
+        ring = torch.zeros(1, dtype=torch.long, device="cuda")
+        sps_b200.fused_sps_kv_update(
+            nw_k=kc.clone(), nw_v=vc.clone(), nw_len=ring, nw_pos=torch.zeros_like(ring), br_k=kc.clone(), br_v=vc.clone(),
+            br_len=torch.zeros(1, 2, dtype=torch.long, device="cuda"), k_window_BxHxD=e, v_window_BxHxD=e, k_retained_BxHxD=e,
+            v_retained_BxHxD=e, active_mask_B=torch.ones(1, dtype=torch.bool, device="cuda"), window_tokens=window)
+        lens.append(int(ring))
+    assert lens == [1, 1]

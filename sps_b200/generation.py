@@ -438,10 +438,9 @@ class SPSGenerator:
         if self._step is None or self._step.state is not state:
             self._bind_step(state)
         s = self._step
-        token = token_B.to(self.device, torch.long).contiguous()
-        active = active_B.to(self.device, torch.bool).contiguous()
-        if token.shape != (s.b,) or active.shape != (s.b,):
-            raise ValueError(f"token and active must have shape {(s.b,)}")
+        # one value may stand for all rows
+        token = token_B.to(self.device, torch.long).expand(s.b).contiguous()
+        active = active_B.to(self.device, torch.bool).expand(s.b).contiguous()
         source = _lib.TokenSource()
         source.token_in, source.active_in = token.data_ptr(), active.data_ptr()
         logits = torch.empty((s.b, self.dims.vocab_size), device=self.device, dtype=self.param_dtype)

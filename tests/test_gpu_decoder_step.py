@@ -83,6 +83,21 @@ def test_weights_at_any_element_of_a_flat_buffer(dtype):
         assert float((a - b).norm()) <= 2.0 ** -6 * float(b.norm())
 
 
+def test_one_token_or_flag_for_all_rows():
+    engine, _ = _engine("sps", 1, 2, 128, 80, 200)
+    prompt = torch.randint(0, 197, (3, 9), generator=torch.Generator().manual_seed(5))
+    full = lambda x: torch.full((3,), x)
+    state, _ = engine.prefill(prompt, 8)
+    want = engine.decode_one_token(state, full(11), full(True))
+    for token, active in ((torch.tensor(11), torch.tensor(True)), (torch.tensor([11.0]), torch.tensor([1])),
+                          (full(11).int(), torch.tensor(True, device="cuda"))):
+        state, _ = engine.prefill(prompt, 8)
+        assert torch.equal(engine.decode_one_token(state, token, active), want)
+    for token in (torch.zeros(2, dtype=torch.long), torch.zeros(1, 3, dtype=torch.long), torch.zeros(3, 1, dtype=torch.long)):
+        with pytest.raises(RuntimeError):
+            engine.decode_one_token(state, token, full(True))
+
+
 @pytest.mark.parametrize("fused", [True, False])
 @pytest.mark.parametrize("bad", [-1, 200, 1 << 40])
 def test_a_token_outside_the_vocabulary_concerns_its_row_alone(fused, bad):

@@ -118,6 +118,15 @@ def left_padded_position_ids(idx: Tensor, pad: int) -> Tensor:
     return torch.where(real, pos, torch.zeros_like(pos))
 
 
+def suppressed_words(ids, vocab_size: int) -> Tensor:
+    """int32 [(vocab_size + 31) // 32]: a bit per token id that is never chosen.  Ids below 0 count from the
+    end of the vocabulary, as an index does (a model without a pad token has -1 for it)."""
+    ids = torch.tensor(sorted({i + vocab_size if i < 0 else i for i in ids}), dtype=torch.long)
+    words = torch.zeros((vocab_size + 31) // 32, dtype=torch.long)
+    words.index_add_(0, ids >> 5, torch.ones_like(ids) << (ids & 31))
+    return torch.where(words >= 1 << 31, words - (1 << 32), words).to(torch.int32)
+
+
 def _validate_left_padded(idx: Tensor, pad: int, context: str) -> None:
     """model.py:39-57 (pads only on the left, at least one real token per row)."""
     real = idx != pad
@@ -538,10 +547,7 @@ class SPSGenerator:
         g.finished = torch.zeros(b, device=dev, dtype=torch.bool)
         g.counters = torch.zeros((2, b), device=dev, dtype=torch.long)       # tokens chosen; keys of the next choice
         g.next_logits = torch.zeros((b, d.vocab_size), device=dev, dtype=self.param_dtype)
-        words = torch.zeros((d.vocab_size + 31) // 32, dtype=torch.long)      # suppressed ids, a bit each
-        ids = torch.tensor(key[4], dtype=torch.long)
-        words.index_add_(0, ids >> 5, torch.ones_like(ids) << (ids & 31))
-        g.suppressed = torch.where(words >= 1 << 31, words - (1 << 32), words).to(torch.int32).to(dev)
+        g.suppressed = suppressed_words(key[4], d.vocab_size).to(dev)
         src = g.source = _lib.TokenSource()
         src.logits, src.suppressed = g.next_logits.data_ptr(), g.suppressed.data_ptr()
         src.generated, src.step, src.finished = g.generated.data_ptr(), g.counters[0].data_ptr(), g.finished.data_ptr()

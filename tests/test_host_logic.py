@@ -380,3 +380,18 @@ int main() {
     # no launcher keeps such a setting by a flag of the process (the encoder lookup is the process's own)
     api = open(os.path.join(csrc, "spsattn_api.cu")).read()
     assert api.count("std::call_once") == 1 and api.count("cudaFuncSetAttribute(") == 1
+
+
+@pytest.mark.parametrize("vocab,ids", [(7, (0, 6)), (64, (31, 32, 63)), (1003, (-1, 5, 1002, -1003)), (50304, (-50304, 0, 31, -2))])
+def test_suppressed_ids_as_bits(vocab, ids):
+    """Ids below 0 count from the end, as the index of a tensor does; each id once, however it is written."""
+    from sps_b200.generation import suppressed_words
+    words = suppressed_words(ids, vocab)
+    assert words.dtype == torch.int32 and words.numel() == (vocab + 31) // 32
+    got = [i for i in range(vocab) if (int(words[i >> 5]) >> (i & 31)) & 1]
+    mask = torch.zeros(vocab, dtype=torch.bool)
+    mask[list(ids)] = True
+    assert got == mask.nonzero().flatten().tolist()
+    for wrong in (-vocab - 1, 32 * words.numel()):
+        with pytest.raises((IndexError, RuntimeError)):
+            suppressed_words((wrong,), vocab)

@@ -457,9 +457,14 @@ static int prefill_impl(const void* q, const void* k, const void* v, void* o, fl
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 
   int *lo = nullptr, *mono = nullptr;
-  // Short rows: the blocks scan the ids themselves (prefill of [2, 8, 512, 64] 13.6 -> 10.3 us), unless
-  // a backward will want the pre-pass's output.
-  const bool scan = doc_ids != nullptr && N <= kScanRows && lse == nullptr && g_prefill_path.load() != 2;
+  // Short rows: the blocks scan the ids themselves, unless a backward will want the pre-pass's output.
+  // That saves the pre-pass's 1.7 us and costs every block some hundred clocks, so it pays for few
+  // blocks: 11.0 against 12.7 us at [1, 16, 512, 64], 20.3 / 20.4 at [4, 16, 1024, 64] (512 blocks), 33.5 /
+  // 32.4 at 1024 blocks and 228 / 209 at 8192; head_dim 128 crosses between 768 and 1024 blocks, 256
+  // between 384 and 576.
+  const long long blocks = (long long)B * H * ((N + kTileM - 1) / kTileM);
+  const bool scan = doc_ids != nullptr && N <= kScanRows && lse == nullptr && g_prefill_path.load() != 2 &&
+                    (blocks <= 4LL * multiprocessors() || workspace == nullptr);
   int rc = run_doc_prepass(scan ? nullptr : doc_ids, doc_is_i64, doc_stride_b, doc_stride_t, B, N, workspace,
                            workspace_bytes, &lo, &mono, st);
   if (rc != 0) return rc;

@@ -397,3 +397,20 @@ def test_document_starts_across_warps_and_passes(n):
     # probabilities 1 and a whole-number sum are exact: one division and the rounding to bf16
     err = (out[:, 0].double().cpu() - want[:, :, None]).abs() / want[:, :, None]
     assert float(err.max()) <= 2.0 ** -8
+
+
+@pytest.mark.parametrize("b,h,n", [(37, 16, 128), (38, 16, 128), (4, 16, 1152), (6, 11, 1152), (1, 3, 1152), (1, 3, 1154)])
+@pytest.mark.parametrize("ordered", [True, False])
+def test_document_ids_scanned_by_the_blocks_or_by_the_pre_pass(b, h, n, ordered):
+    """Few blocks with short rows scan the ids themselves, unless a log-sum-exp is asked for: both sides
+    of the border (four blocks per SM, 1152 rows) against the pre-pass, the same bits."""
+    import sps_b200
+    g = torch.Generator().manual_seed(b + n)
+    q, k, v = (torch.randn(b, h, n, 64, generator=g).bfloat16().cuda() for _ in range(3))
+    docs = torch.randint(0, 9, (b, n // 2), generator=g)
+    if ordered:
+        docs = docs.sort(dim=1).values
+    docs = docs.repeat_interleave(2, dim=1).cuda()
+    call = lambda lse: sps_b200.prefill_attention(q, k, v, 0.125, persistent_parity=0, temporary_window=16,
+                                                  documents_idx=docs, return_lse=lse)
+    assert torch.equal(call(False), call(True)[0])

@@ -31,21 +31,27 @@ struct RopeParams {
   int heads_per_group;         // H = n_groups * heads_per_group
   int out_fp16;
   int B, N, H, D;
+  // launch: rows that a thread walks down; rows side by side in a block, and their number as batches and rows
+  int walk, side, step_b, step_n;
 };
 
-// Bound: HBM.  A thread keeps its place in the row (head, group, eight elements) and walks down
-// `rows_per_block` rows, two loads in flight, so that nothing is divided per element: one flat index
-// per vector reached half of the bandwidth (65536 rows of 6144: 440 -> 283 us, 5.7 TB/s).
-// X_DTYPE: 0 bf16, 1 fp16, 2 fp32
-template <int X_DTYPE>
-__global__ void __launch_bounds__(256, 4) rope_cast_kernel(const RopeParams p, int rows_per_block) {
+// Bound: HBM.  A thread keeps its place in the row (head, group, eight elements) and walks down `walk`
+// rows, two loads in flight, so that nothing is divided per element: one flat index per vector
+// reached half of the bandwidth (65536 rows of 6144: 440 -> 283 us, 5.7 TB/s).
+// X_DTYPE: 0 bf16, 1 fp16, 2 fp32.  kSide: many narrow rows, `side` of them next to one another in a block;
+// with a row per block, 65536 rows of one head of 16 took 30 us, now 2.9 (a kernel of its own: the general
+// step from row to row alone cost wide fp32 rows 20 %, 72 -> 86 us for 32768 rows of 2304).
+template <int X_DTYPE, bool kSide>
+__global__ void __launch_bounds__(256, 4) rope_cast_kernel(const RopeParams p) {
   grid_dependency_wait();
   const int vec_per_head = p.D / 8, vecs = p.H * vec_per_head;
-  const long long row0 = (long long)blockIdx.x * rows_per_block;
-  const int count = (int)min((long long)rows_per_block, (long long)p.B * p.N - row0);
+  const int side = kSide ? p.side : 1, mine = kSide ? (int)threadIdx.x / vecs : 0;
+  if (mine >= side) return;
+  const long long row0 = (long long)blockIdx.x * p.walk * side + mine;
+  const int count = (int)min((long long)p.walk, ((long long)p.B * p.N - row0 + side - 1) / side);
   const int b0 = (int)(row0 / p.N), n0 = (int)(row0 - (long long)b0 * p.N);
   constexpr int kBytes = X_DTYPE == 2 ? 4 : 2, kLoads = kBytes / 2;      // 16-byte loads per vector
-  for (int v = blockIdx.y * 256 + threadIdx.x; v < vecs; v += gridDim.y * 256) {
+  for (int v = kSide ? threadIdx.x - mine * vecs : blockIdx.y * 256 + threadIdx.x; v < vecs; v += kSide ? vecs : gridDim.y * 256) {
     const int h = v / vec_per_head, x8 = v - h * vec_per_head;
     const int gi = h / p.heads_per_group, hg = h - gi * p.heads_per_group;
     RopeGroup grp = p.group[0];   // selected without indexing the parameter block dynamically
@@ -75,7 +81,12 @@ __global__ void __launch_bounds__(256, 4) rope_cast_kernel(const RopeParams p, i
           cs[u][0] = __ldg(fr);
           cs[u][1] = __ldg(fr + 1);
         }
-        if (++n == p.N) n = 0, ++b;
+        if constexpr (kSide) {
+          b += p.step_b;
+          if ((n += p.step_n) >= p.N) n -= p.N, ++b;
+        } else if (++n == p.N) {
+          n = 0, ++b;
+        }
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {

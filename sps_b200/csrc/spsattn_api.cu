@@ -9,6 +9,7 @@
 #include <atomic>
 #include <initializer_list>
 #include <mutex>
+#include <type_traits>
 #include <utility>
 
 #include "../../include/spsattn.h"
@@ -1081,16 +1082,26 @@ static int rope_impl(const void* x, int x_dtype, int64_t xs_b, int64_t xs_n, int
   p.N = N;
   p.H = heads_per_group * n_groups;
   p.D = D;
-  // eight rows per block once that still leaves several blocks per SM, and one block per 256 vectors of a row
+  // One block per 256 vectors of a row, or as many rows as 256 threads take where rows of at most 64
+  // vectors are many (rows of 96 gain in bf16, 24 -> 21 us for 32768 of them, but lose in fp32, 29 -> 31; few
+  // rows have an SM each); eight rows under one another once that still leaves several blocks per SM.
+  const int vecs = p.H * (D / 8);
   const long long rows = (long long)B * N;
-  const int rows_per_block = rows >= 148LL * 32 ? 8 : rows >= 148LL * 8 ? 4 : 1;
-  const long long blocks = (rows + rows_per_block - 1) / rows_per_block;
+  p.side = vecs <= 64 && rows >= 148LL * 8 ? 256 / vecs : 1;
+  p.step_b = p.side / N;
+  p.step_n = p.side % N;
+  const long long row_sets = (rows + p.side - 1) / p.side;
+  p.walk = row_sets >= 148LL * 32 ? 8 : row_sets >= 148LL * 8 ? 4 : 1;
+  const long long blocks = (row_sets + p.walk - 1) / p.walk;
   if (blocks > 0x7fffffffLL) return SPSATTN_ERR_TOO_LARGE;
-  const unsigned across = (unsigned)((p.H * (D / 8) + 255) / 256);
+  const unsigned across = (unsigned)((vecs + 255) / 256);
   const dim3 grid((unsigned)blocks, across < 65535u ? across : 65535u);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  auto* kernel = x_dtype == 2 ? rope_cast_kernel<2> : x_dtype == 1 ? rope_cast_kernel<1> : rope_cast_kernel<0>;
-  return launch_dependent(kernel, grid, dim3(256), 0, st, p, rows_per_block);
+  auto pick = [x_dtype](auto side) {
+    constexpr bool kSide = decltype(side)::value;
+    return x_dtype == 2 ? rope_cast_kernel<2, kSide> : x_dtype == 1 ? rope_cast_kernel<1, kSide> : rope_cast_kernel<0, kSide>;
+  };
+  return launch_dependent(p.side > 1 ? pick(std::true_type()) : pick(std::false_type()), grid, dim3(256), 0, st, p);
 }
 
 int spsattn_rope_cast(const void* x, int x_dtype, int64_t x_stride_b, int64_t x_stride_n,

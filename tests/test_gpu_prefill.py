@@ -414,3 +414,24 @@ def test_document_ids_scanned_by_the_blocks_or_by_the_pre_pass(b, h, n, ordered)
     call = lambda lse: sps_b200.prefill_attention(q, k, v, 0.125, persistent_parity=0, temporary_window=16,
                                                   documents_idx=docs, return_lse=lse)
     assert torch.equal(call(False), call(True)[0])
+
+
+@pytest.mark.parametrize("B,N,H,D", [(1, 1, 1, 16), (3, 700, 1, 16), (700, 3, 2, 16), (1183, 1, 8, 64), (1184, 1, 8, 64), (2, 1031, 9, 64),
+                                     (2, 103, 17, 64), (1, 1300, 1, 256), (3, 11, 48, 128), (2, 60, 36, 64), (1, 65536, 1, 16)])
+@pytest.mark.parametrize("xdt", [torch.bfloat16, torch.float16, torch.float32])
+def test_rope_cast_of_narrow_and_wide_rows(B, N, H, D, xdt):
+    """Rows side by side in a block (up to 64 vectors, from 1184 rows on) and blocks for parts of a row;
+    every row its own batch, a batch shorter than the rows of a block, walks of 1, 4 and 8 rows."""
+    import sps_b200
+    from oracle import sps_oracle as orc
+    g = torch.Generator().manual_seed(N + H)
+    x = torch.randn(B, N, H, D, generator=g).to(xdt)
+    angle = torch.randn(B, N, D // 2, generator=g)
+    fc = torch.polar(torch.ones_like(angle), angle)
+    for freqs in (fc, None):
+        got = sps_b200.rope_cast(x.cuda(), None if freqs is None else freqs.cuda())
+        want = orc.rope_cast(x, freqs).float()
+        # the oracle rounds to the input's type before bf16 and may fuse a product with a sum: one unit of
+        # the last place, or of fp32 sums of values below 8 where the two products cancel
+        diff = (got.transpose(1, 2).float().cpu() - want).abs()
+        assert bool((diff <= 2.0 ** -7 * want.abs() + 2.0 ** -20).all())

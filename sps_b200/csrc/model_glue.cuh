@@ -29,10 +29,11 @@ __device__ __forceinline__ float round_bf16(float f) {
 // reference's bf16 tensors round; false: everything fp32.  A row of up to 256 * kRowVecs vectors
 // stays in registers between the sum of squares and the scaling (one read of x); longer rows are
 // read again.
-// kRowVecs: 1 for rows of up to 256 vectors (registers for six blocks per SM: 174 us against 202 with five), 4 for longer ones.
-
-template <bool BF16, int kRowVecs>
-__global__ void __launch_bounds__(256, kRowVecs == 1 ? 6 : 2) add_rmsnorm_kernel(const RmsNormParams p) {
+// kAhead: a block has its next row on the way while it works on this one.  That takes registers (with
+// kRowVecs 1 six blocks per SM still fit, 174 us against 202 with five; with 4 only two), which wide rows
+// need for more blocks: without it 65536 bf16 rows of 4096 357 -> 260 us, 16384 fp32 rows of 8192 310 -> 177.
+template <bool BF16, int kRowVecs, bool kAhead>
+__global__ void __launch_bounds__(256, kRowVecs == 1 ? 6 : kAhead ? 2 : 4) add_rmsnorm_kernel(const RmsNormParams p) {
   constexpr int V = BF16 ? 8 : 4;   // elements per 16-byte access
   __shared__ float s_part[2][8];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -78,9 +79,8 @@ __global__ void __launch_bounds__(256, kRowVecs == 1 ? 6 : 2) add_rmsnorm_kernel
     py[at] = pack(r);
   };
 
-  // Bound: HBM.  A block has its next row on the way while it works on this one, and synchronises once
-  // per row (every thread adds the eight warp sums itself, in the same order): 65536 rows of 2048
-  // with delta 250 -> 174 us, 6.2 TB/s.
+  // Bound: HBM.  A block synchronises once per row (every thread adds the eight warp sums itself, in the
+  // same order): 65536 rows of 2048 with delta 250 -> 174 us, 6.2 TB/s.
   grid_dependency_wait();
   uint4 nx[kRowVecs], nd[kRowVecs];
   auto fetch = [&](long long row) {
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(256, kRowVecs == 1 ? 6 : 2) add_rmsnorm_kernel
       }
     }
   };
-  fetch(blockIdx.x);
+  if constexpr (kAhead) fetch(blockIdx.x);
   int buf = 0;
   for (long long row = blockIdx.x; row < p.rows; row += gridDim.x, buf ^= 1) {
     const size_t base = (size_t)row * n_vec;
@@ -105,12 +105,13 @@ __global__ void __launch_bounds__(256, kRowVecs == 1 ? 6 : 2) add_rmsnorm_kernel
       for (int k = 0; k < kRowVecs; ++k) {
         const int i = tid + k * 256;
         if (i < n_vec) {
-          sum(base + i, nx[k], nd[k], kept[k]);
+          if constexpr (kAhead) sum(base + i, nx[k], nd[k], kept[k]);
+          else sum(base + i, px[base + i], p.delta != nullptr ? pd[base + i] : make_uint4(0, 0, 0, 0), kept[k]);
 #pragma unroll
           for (int e = 0; e < V; ++e) ss = fmaf(kept[k][e], kept[k][e], ss);
         }
       }
-      fetch(row + gridDim.x);
+      if constexpr (kAhead) fetch(row + gridDim.x);
     } else {
       for (int i = tid; i < n_vec; i += 256) {
         float f[V];

@@ -1267,9 +1267,15 @@ int spsattn_add_rmsnorm(void* x, const void* delta, const void* weight, void* y,
   p.eps = eps;
   const unsigned blocks = (unsigned)(rows < 148LL * 16 ? rows : 148LL * 16);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const bool one = C / vec <= 256;
-  auto* kernel = dtype == SPSATTN_DTYPE_BF16 ? (one ? add_rmsnorm_kernel<true, 1> : add_rmsnorm_kernel<true, 4>)
-                                             : (one ? add_rmsnorm_kernel<false, 1> : add_rmsnorm_kernel<false, 4>);
+  // Rows of at most 256 vectors: one per thread, the next row under way.  Wider ones: so too where two
+  // blocks per SM hold all rows (149 bf16 rows of 8192 with delta: 3.4 against 3.9 us) and for fp32 up to 1024
+  // vectors (65536 rows of 2056: 237 us, 259 with the next row not under way); other rows leave it, so
+  // that four blocks fit an SM.
+  const int vecs = C / vec;
+  const bool bf16 = dtype == SPSATTN_DTYPE_BF16, ahead = rows <= 2 * 148 || (!bf16 && vecs <= 1024);
+  auto* kernel = vecs <= 256 ? (bf16 ? add_rmsnorm_kernel<true, 1, true> : add_rmsnorm_kernel<false, 1, true>)
+                 : ahead     ? (bf16 ? add_rmsnorm_kernel<true, 4, true> : add_rmsnorm_kernel<false, 4, true>)
+                             : (bf16 ? add_rmsnorm_kernel<true, 4, false> : add_rmsnorm_kernel<false, 4, false>);
   return launch_dependent(kernel, dim3(blocks), dim3(256), 0, st, p);
 }
 

@@ -74,6 +74,29 @@ def test_add_rmsnorm_matches_the_reference_ops(dtype):
     assert torch.equal(x2, x)
 
 
+@pytest.mark.parametrize("rows", [1, 296, 297, 2500])
+@pytest.mark.parametrize("dtype,c", [(torch.bfloat16, 2048), (torch.bfloat16, 2056), (torch.bfloat16, 8192), (torch.bfloat16, 8200),
+                                     (torch.float32, 1024), (torch.float32, 1028), (torch.float32, 4096), (torch.float32, 4100)])
+def test_add_rmsnorm_of_rows_wider_than_a_block(dtype, c, rows):
+    """Each form of the kernel at its borders: 256 and 1024 vectors a row, 296 rows, several rows a block."""
+    from sps_b200 import _lib
+    lib, dev = _lib.load(), _dev()
+    g = torch.Generator(device=dev).manual_seed(c + rows)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=dev).to(dtype)
+    x, delta, w = rnd(rows, c), rnd(rows, c), (1 + 0.1 * rnd(c).float()).to(dtype)
+    code = _lib.DTYPE_BF16 if dtype == torch.bfloat16 else _lib.DTYPE_FP32
+    for d in (delta, None):
+        x_ref = x + d if d is not None else x
+        xf = x_ref.float()
+        y_ref = (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + 1e-6)).type_as(x_ref) * w
+        xx, y = x.clone(), torch.empty_like(x)
+        _lib.check(lib.spsattn_add_rmsnorm(xx.data_ptr(), None if d is None else d.data_ptr(), w.data_ptr(), y.data_ptr(), code,
+                                           rows, c, 1e-6, torch.cuda.current_stream().cuda_stream), "add_rmsnorm")
+        assert torch.equal(xx, x_ref)
+        # sums in another order: a step of 2^-7 in the first bf16 rounding and one in the second
+        torch.testing.assert_close(y.float(), y_ref.float(), atol=1e-6, rtol=2 ** -6 if dtype == torch.bfloat16 else 1e-5)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_swiglu_matches_the_reference_ops(dtype):
     from sps_b200 import _lib

@@ -20,14 +20,22 @@
 // by the document / window / parity rule are never loaded or multiplied.
 #pragma once
 
+#include <cfloat>
+
 #include "common.cuh"
 #include "mask.cuh"
 
 namespace spsattn {
 
+struct PrefillOperand {
+  const uint16_t* p;
+  int64_t stride_b, stride_h, stride_n;         // elements
+};
+
 struct PrefillParams {
   void* o;               // rows of D contiguous elements, addressed with the strides below
   int64_t o_stride_b, o_stride_h, o_stride_n;   // elements
+  PrefillOperand q, k, v;                       // what the tensor maps cover (finite_row)
   float* lse;            // [B,H,N] or null
   const void* docs;      // [B,N] ids or null
   int64_t doc_stride_b, doc_stride_t;
@@ -182,12 +190,77 @@ __device__ __forceinline__ void softmax_arrive(uint32_t bar, int lane) {
 }
 #endif
 
+// One row again, by a warp, on the CUDA cores: its visible keys alone.  The products multiply a hidden key's
+// value row by a probability of 0, which is not 0 where that row holds an infinity or NaN.  Head dims 16,
+// 32 and 256 keep such rows out of the others' results (they did before they came to the tensor
+// cores); only rows whose result is not finite come here.  m, l: the row's maximum (raw score) and sum.
+template <int D, bool FP16>
+__device__ __noinline__ void finite_row(const PrefillParams& prm, int b, int h, int i, int lo_i, const uint8_t* docs_b,
+                                        long long my_doc, float m, float l, int lane) {
+  constexpr int E = (D + 31) / 32;
+  auto element = [](const PrefillOperand& x, int64_t at) {
+    float f, unused;
+    unpack2<FP16>((uint32_t)x.p[at], f, unused);
+    return f;
+  };
+  auto start = [&](const PrefillOperand& x, int64_t r) { return b * x.stride_b + h * x.stride_h + r * x.stride_n; };
+  const float c = prm.scale_log2;
+  float q[E], acc[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    q[e] = lane + 32 * e < D ? element(prm.q, start(prm.q, i) + lane + 32 * e) : 0.f;
+    acc[e] = 0.f;
+  }
+  for (int p = 0; p < prm.mask.ks; ++p) {
+    int kmin, kmax;
+    row_interval(prm.mask, i, lo_i, p, kmin, kmax);
+    constexpr int U = 4;                 // keys in flight
+    for (int k0 = max(kmin, 0); k0 <= kmax; k0 += U) {
+      bool on[U];
+      float s[U], v[U][E];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int j = prm.mask.ks * min(k0 + u, kmax) + p;
+        on[u] = k0 + u <= kmax;
+        if (docs_b != nullptr) {
+          const size_t off = (size_t)j * prm.doc_stride_t;
+          on[u] = on[u] && my_doc == (prm.doc_is_i64 ? reinterpret_cast<const long long*>(docs_b)[off]
+                                                     : (long long)reinterpret_cast<const int*>(docs_b)[off]);
+        }
+        const int64_t kr = start(prm.k, j) + lane, vr = start(prm.v, j) + lane;
+        s[u] = 0.f;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          const bool in = on[u] && lane + 32 * e < D;
+          v[u][e] = in ? element(prm.v, vr + 32 * e) : 0.f;
+          if (in) s[u] = fmaf(q[e], element(prm.k, kr + 32 * e), s[u]);
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int u = 0; u < U; ++u) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const float pr = on[u] ? fast_exp2((s[u] - m) * c) : 0.f;
+#pragma unroll
+        for (int e = 0; e < E; ++e) acc[e] = fmaf(pr, v[u][e], acc[e]);
+      }
+    }
+  }
+  const float inv_l = l > 0.f ? 1.0f / l : 0.f;
+  uint16_t* o = reinterpret_cast<uint16_t*>(prm.o) + b * prm.o_stride_b + h * prm.o_stride_h + i * prm.o_stride_n;
+#pragma unroll
+  for (int e = 0; e < E; ++e)
+    if (lane + 32 * e < D) o[lane + 32 * e] = (uint16_t)(pack2<FP16>(acc[e] * inv_l, 0.f) & 0xffffu);
+}
+
 // kScan: no pre-pass, every block works its document starts out from the ids (a kernel of its own: the
 // branch alone cost the others 1 %, 342 against 339 us at [8, 12, 8192, 64])
 template <int D, bool FP16, bool kScan>
 __global__ void __launch_bounds__(kPrefillThreads, PrefillCfg<D>::kBlocksPerSM)
 prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                     const __grid_constant__ CUtensorMap tm_v, const PrefillParams prm) {
+                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ PrefillParams prm) {
   using Cfg = PrefillCfg<D>;
   constexpr int kOChunk = D < 32 ? D : 32;      // columns of O a thread moves at a time
   extern __shared__ uint8_t smem_raw[];
@@ -749,6 +822,7 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       }
 
       // ---------------------------------------------------------------- epilogue
+      float2 all0 = make_float2(0.f, 0.f), all1 = all0;    // sums of the row's elements: finite if they are
       if (ok) ok = mbar_wait(bar_pv_done, (n_tiles - 1) & 1, abort_flag, prm.status);
       if (ok) {
         tc_fence_after();
@@ -770,11 +844,28 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
               u.w = pack2<FP16>(__uint_as_float(r[e + 6]) * inv_l, __uint_as_float(r[e + 7]) * inv_l);
               *reinterpret_cast<uint4*>(o_row + (q4 * kOChunk + e) * 2) = u;
             }
+            if constexpr (Cfg::kPLo) {
+#pragma unroll
+              for (int e = 0; e < kOChunk; e += 4) {
+                all0 = __fadd2_rn(all0, make_float2(__uint_as_float(r[e]), __uint_as_float(r[e + 1])));
+                all1 = __fadd2_rn(all1, make_float2(__uint_as_float(r[e + 2]), __uint_as_float(r[e + 3])));
+              }
+            }
           }
         }
         if (prm.lse != nullptr && i < prm.N)
           prm.lse[(size_t)bh * prm.N + i] = l_run > 0.f ? m_run * c + log2f(l_run) : -INFINITY;
         tc_fence_before();
+      }
+      if constexpr (Cfg::kPLo) {
+        // (scores that are not finite themselves leave no row to save)
+        const bool odd = !(fabsf(all0.x + all0.y + all1.x + all1.y) <= FLT_MAX);
+        for (uint32_t left = __ballot_sync(0xffffffffu, ok && odd && l_run <= FLT_MAX); left != 0; left &= left - 1) {
+          const int src = __ffs(left) - 1;
+          finite_row<D, FP16>(prm, b, h, i - lane + src, __shfl_sync(0xffffffffu, lo_i, src), docs_b,
+                              __shfl_sync(0xffffffffu, my_doc, src), __shfl_sync(0xffffffffu, m_run, src),
+                              __shfl_sync(0xffffffffu, l_run, src), lane);
+        }
       }
     }
   } else if (!bail && warp < 4) {

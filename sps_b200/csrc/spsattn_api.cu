@@ -487,6 +487,9 @@ static int prefill_impl(const void* q, const void* k, const void* v, void* o, fl
   prm.o_stride_b = so.b;
   prm.o_stride_h = so.h;
   prm.o_stride_n = so.n;
+  prm.q = {reinterpret_cast<const uint16_t*>(q), sq.b, sq.h, sq.n};
+  prm.k = {reinterpret_cast<const uint16_t*>(k), sk.b, sk.h, sk.n};
+  prm.v = {reinterpret_cast<const uint16_t*>(v), sv.b, sv.h, sv.n};
   prm.lse = lse;
   prm.docs = doc_ids;
   prm.doc_stride_b = doc_stride_b;

@@ -123,6 +123,12 @@ bool strides_ok(Strides st, int D) {
   return st.n >= D && st.h >= D && st.b >= D && (st.n % 8) == 0 && (st.h % 8) == 0 && (st.b % 8) == 0;
 }
 
+// The code of a launch that did not come about, which is then not left for a later call to find.
+int launch_code(cudaError_t e) {
+  if (e != cudaSuccess) cudaGetLastError();
+  return (int)e;
+}
+
 // A launch that may start while the kernel before it in the stream is still running; the kernel waits
 // (grid_dependency_wait) before it touches anything that one writes.
 template <typename... P, typename... A>
@@ -138,7 +144,7 @@ int launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, c
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+  return launch_code(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...));
 }
 
 // Lets a kernel ask for `bytes` of dynamic shared memory on the current device (the limit is the device's own).
@@ -148,7 +154,7 @@ int allow_shared_memory(std::atomic<uint64_t>& sized, K kernel, int bytes) {
   const cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return (int)e;
   return once_per_device(sized, dev, [&] {
-    return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    return launch_code(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   });
 }
 
@@ -189,8 +195,7 @@ int launch_prefill_kernel(const CUtensorMap& tq, const CUtensorMap& tk, const CU
 #else
   cfg.numAttrs = prm.mono != nullptr ? 1 : 0;
 #endif
-  const cudaError_t le = cudaLaunchKernelEx(&cfg, prefill_sm100_kernel<D, FP16, kScan>, tq, tk, tv, prm);
-  return le != cudaSuccess ? (int)le : (int)cudaGetLastError();
+  return launch_code(cudaLaunchKernelEx(&cfg, prefill_sm100_kernel<D, FP16, kScan>, tq, tk, tv, prm));
 }
 
 template <int D, bool FP16>

@@ -193,6 +193,10 @@ def native():
     global _native
     if _native is None:
         load()                                   # the library that it calls, with its own message when missing
+        from . import build
+        if build.built_against() not in (None, build.native_interfaces()):
+            raise SpsAttnError(f"sps_b200/_native.so was built against {build.built_against()}, this is "
+                               f"{build.native_interfaces()}: python -m sps_b200.build")
         try:
             from . import _native as ext
         except ImportError as e:

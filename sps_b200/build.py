@@ -13,11 +13,13 @@ import os
 import subprocess
 import sys
 import sysconfig
+from typing import Optional
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libspsattn.so")
 NATIVE_PATH = os.path.join(PKG_DIR, "_native.so")
+NATIVE_STAMP = os.path.join(PKG_DIR, "_native.stamp")     # what _native.so was built against
 ABI_HEADER = os.path.join("..", "..", "include", "spsattn.h")
 SOURCES = ["spsattn_api.cu"]
 HEADERS = ["common.cuh", "mask.cuh", "prefill_sm100.cuh", "prefill_wide_sm100.cuh", "prefill_bwd_sm100.cuh", "prefill_aux.cuh", "decode.cuh", "decode_sm100.cuh",
@@ -39,8 +41,33 @@ def _stale(target: str, sources) -> bool:
     return any(os.path.getmtime(d) > built for d in deps if os.path.exists(d))
 
 
+def native_interfaces() -> str:
+    """The C++ interfaces that the extension depends on besides its sources: an extension built against
+    another torch or Python fails to load, or worse."""
+    import torch
+    return f"torch {torch.__version__}, Python {sys.version_info.major}.{sys.version_info.minor}"
+
+
+def built_against() -> Optional[str]:
+    """``native_interfaces()`` as they were when the extension was built; None when that is not known."""
+    try:
+        with open(NATIVE_STAMP) as f:
+            return f.read()
+    except OSError:
+        return None
+
+
+def _library_stale() -> bool:
+    return _stale(LIB_PATH, SOURCES + HEADERS)
+
+
+def _native_stale() -> bool:
+    return (_stale(NATIVE_PATH, NATIVE_SOURCES + NATIVE_HEADERS + [ABI_HEADER])
+            or built_against() != native_interfaces())
+
+
 def is_stale() -> bool:
-    return _stale(LIB_PATH, SOURCES + HEADERS) or _stale(NATIVE_PATH, NATIVE_SOURCES + NATIVE_HEADERS + [ABI_HEADER])
+    return _library_stale() or _native_stale()
 
 
 def _run(cmd, verbose: bool) -> None:
@@ -77,12 +104,14 @@ def _build_native(verbose: bool) -> None:
     cmd += ["-L" + PKG_DIR, "-lspsattn", "-Wl,-rpath,$ORIGIN", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda",
             "-ltorch", "-ltorch_python", "-lcudart"]
     _run(cmd, verbose)
+    with open(NATIVE_STAMP, "w") as f:
+        f.write(native_interfaces())
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    if force or _stale(LIB_PATH, SOURCES + HEADERS):
+    if force or _library_stale():
         _build_library(verbose)
-    if force or _stale(NATIVE_PATH, NATIVE_SOURCES + NATIVE_HEADERS + [ABI_HEADER]):
+    if force or _native_stale():
         _build_native(verbose)
     return LIB_PATH
 

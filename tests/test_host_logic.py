@@ -395,3 +395,16 @@ def test_suppressed_ids_as_bits(vocab, ids):
     for wrong in (-vocab - 1, 32 * words.numel()):
         with pytest.raises((IndexError, RuntimeError)):
             suppressed_words((wrong,), vocab)
+
+
+def test_an_extension_built_against_another_torch_is_rebuilt_and_not_loaded(tmp_path, monkeypatch):
+    from sps_b200 import build
+    assert not build.is_stale() and build.built_against() == build.native_interfaces()
+    stamp = tmp_path / "stamp"
+    monkeypatch.setattr(build, "NATIVE_STAMP", str(stamp))
+    assert build.is_stale()                                    # not known: rebuilt, but it may load
+    stamp.write_text("torch 1.0, Python 3.12")
+    assert build._native_stale() and not build._library_stale()
+    monkeypatch.setattr(_lib, "_native", None)
+    with pytest.raises(_lib.SpsAttnError, match="built against torch 1.0"):
+        _lib.native()

@@ -7,12 +7,12 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def _engine(variant, layers, heads, hidden, inter, vocab, seed=3):
+def _engine(variant, layers, heads, hidden, inter, vocab, seed=3, block=64, window=5):
     import sps_b200
     from sps_b200.generation import random_state_dict
-    dims = sps_b200.SPSDims(block_size=64, vocab_size=vocab, n_layer=layers, n_head=heads, hidden_size=hidden,
+    dims = sps_b200.SPSDims(block_size=block, vocab_size=vocab, n_layer=layers, n_head=heads, hidden_size=hidden,
                             intermediate_size=inter, eos_token_id=vocab - 3, pad_token_id=vocab - 1,
-                            predict_token_id=vocab - 2, window_size=5)
+                            predict_token_id=vocab - 2, window_size=window)
     return sps_b200.SPSGenerator(random_state_dict(dims, seed=seed), dims, variant=variant), dims
 
 
@@ -49,6 +49,59 @@ def test_fused_step_matches_the_separate_kernels(variant, batch, heads, hidden, 
         assert bool((a[~active] == 0).all())
     for name in ("br_len", "nw_len", "nw_pos", "processed_tokens", "next_doc_start"):
         assert torch.equal(getattr(states[0], name), getattr(states[1], name)), name
+
+
+@pytest.mark.parametrize("variant,batch,heads,hidden,prompt,window", [
+    ("reverse_sps", 2, 3, 192, 250, 16),      # one block per pair: three chunks, three groups of threads
+    ("sps", 1, 4, 256, 330, 32),              # the same, the last rows of its range
+    ("standard", 3, 2, 256, 250, 5),          # no ring
+    ("sps", 3, 4, 256, 600, 64),              # the split kernel, and it alone advances the ring
+    ("standard", 16, 32, 2048, 300, 5),       # the tensor-core kernel
+    ("sps", 8, 32, 2048, 300, 200),           # the same with a ring that it streams
+])
+def test_fused_step_on_long_caches(variant, batch, heads, hidden, prompt, window):
+    """Each decode attention kernel inside the step's chain of launches, against the same kernel behind
+    separate ones: ring full and wrapping, a row that leaves a long cache for a new document."""
+    import sps_b200
+    steps = 4
+    engine, dims = _engine(variant, 2, heads, hidden, 256, 500, block=prompt + 8, window=window)
+    g = torch.Generator().manual_seed(prompt)
+    ids = torch.randint(0, 497, (batch, prompt), generator=g)
+    tokens = torch.randint(0, 497, (steps, batch), generator=g)
+    tokens[1, 0] = dims.eos_token_id                       # row 0 starts a new document in the third step
+    active = torch.ones(batch, dtype=torch.bool)
+    if batch > 2:
+        active[2] = False
+    outs, states = [], []
+    for fused in (True, False):
+        state, _ = engine.prefill(ids, 8)
+        engine._bind_step(state)
+        assert engine._step.fused
+        engine._step.fused = fused
+        outs.append([engine.decode_one_token(state, t, active).float() for t in tokens])
+        states.append(state)
+    sps_b200.check_device_status()
+    for a, b in zip(*outs):
+        assert float((a - b).norm()) <= 2.0 ** -6 * float(b.norm())          # as above
+    for name in ("br_len", "nw_len", "nw_pos", "processed_tokens", "next_doc_start"):
+        assert torch.equal(getattr(states[0], name), getattr(states[1], name)), name
+    assert states[0].br_len[:, 0].unique().tolist() == [2]
+    for name in ("br_k", "br_v"):
+        a, b = getattr(states[0], name), getattr(states[1], name)
+        written = torch.zeros(batch, a.shape[3], dtype=torch.bool)           # by the steps
+        written[1:, prompt:prompt + steps] = True
+        written[0, prompt:prompt + 2] = written[0, :2] = True
+        written[~active] = False
+        written = written.cuda()
+        keep = lambda x, rows: x.transpose(2, 3)[:, rows]                    # [L, rows, H, D]
+        assert torch.equal(keep(a, ~written), keep(b, ~written))
+        a, b = keep(a, written).float(), keep(b, written).float()
+        assert bool((b.norm(dim=-1) > 0).all())
+        # row by row: a row in a wrong place is as far off as its own norm
+        assert bool(((a - b).norm(dim=-1) <= 2.0 ** -4 * b.norm(dim=-1)).all())
+    for name in ("nw_k", "nw_v"):
+        a, b = getattr(states[0], name).float(), getattr(states[1], name).float()
+        assert bool(((a - b).norm(dim=-1) <= 2.0 ** -4 * b.norm(dim=-1)).all())
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])

@@ -7,8 +7,8 @@ triton_reverse_sps_flash_attention.py:827-853 and triton_full_flash_attention.py
 model classes can call them unchanged (see ``sps_b200.install``).  For head_dim 64 and 128 they
 are differentiable like the reference's ``torch.autograd.Function``s (backward:
 triton_sps_flash_attention.py:623-720); the other head dims are forward only.
-All compute happens in libspsattn.so (tcgen05 / TMA kernels for head_dim 64 and 128), the host
-path in native code as well (csrc/native.cpp).
+All compute happens in libspsattn.so (tcgen05 / TMA kernels for every head_dim), the host path in
+native code as well (csrc/native.cpp).
 """
 
 from __future__ import annotations

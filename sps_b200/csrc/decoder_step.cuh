@@ -18,10 +18,11 @@
 //     tcgen05 was slower here (25-45 clk to issue each product of M = 64, a commit and a read of
 //     tensor memory at the end: 490 against 375 us for a token of the model above when it was tried;
 //     295 now, 566 with library projections and separate kernels).
-// The contraction of one output is one chain of products in ascending k, never split, with results
+// The contraction of one output is one chain of products, sixteen columns at a time in ascending k, never split, with results
 // rounded to bf16 where the separate kernels (library GEMM, model_glue.cuh, rope.cuh) round theirs and
-// the norm's sums in the order of add_rmsnorm_kernel: a step's logits are the same bits as theirs.
-// (Rounding flips spread: with the contraction split over eight warps the logits of a 24-layer model
+// the norm's sums in the order of add_rmsnorm_kernel.  A step's logits were the same bits as theirs at nine
+// of eleven sizes with CUDA 12.9's library; at vocabularies of 1001 and 9473, where the library takes another
+// algorithm for the head, 2e-6 and 1e-4 of their norm apart.  (Rounding flips spread: with the contraction split over eight warps the logits of a 24-layer model
 // moved by 3 % of their norm.)
 #pragma once
 
@@ -31,6 +32,10 @@
 namespace spsattn {
 
 enum SkinnyEpilogue { kSkinnyQkv = 0, kSkinnyResidual = 1, kSkinnySwiglu = 2, kSkinnyLogits = 3 };
+// us per token against library projections (prompt 100, captured): 768 columns, 12 layers 8 rows 302 / 473, 16
+// rows 375 / 470 (library with 18: 460); 1024 columns 347 / 536, 416 / 532; 2048 columns, 24 layers 1289 / 1681,
+// 12 rows 1491 / 1518, 16 rows 1643 / 1534.  Above 16 rows a third tile of rows would be needed; past 1024
+// columns the library is already ahead from 13 rows on.
 constexpr int kSkinnyMaxRows = 16;
 constexpr int kSkinnyMaxCols = 2048;   // of a normalised input: one vector of 8 per thread of add_rmsnorm_kernel
 constexpr int kSkinnyMaxStages = 16;

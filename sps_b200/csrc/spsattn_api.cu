@@ -273,7 +273,9 @@ static int decode_chunk_rows(int S, int H, long long max_rows_total) {
 // One block per (sequence, head) (decode_pair_kernel) where its rows and those of its neighbours on the
 // SM are read in less than the tickets and records of the split form cost.  Measured: 64 rows 5.6 ->
 // 4.3 us and 200 rows 6.2 -> 5.2 us at 2 x 12 x 64; even at 400 rows; slower where an SM has several
-// pairs of 200 rows of 128.
+// pairs of 200 rows of 128.  `rows` is what the caches hold at most: live lengths are on the device.  Inside
+// a fused decode step the pair form also reads its first rows before its wait, which the split form does
+// not: at 320 live rows a token of 12 layers x 768 takes 295 us with capacity 384 and 343 with 388.
 static bool pair_fits(int S, int H, int D, long long rows) {
   const long long pairs = (long long)S * H, per_sm = (pairs + 147) / 148;
   return rows <= 384 && per_sm * rows * D * 4 <= 224 * 1024;
@@ -895,7 +897,7 @@ static int decode_impl(const void* q, int nq, void* out, int out_dtype, const sp
   if ((path == 2 && !tc_ok) || (path == 3 && D > 128)) return SPSATTN_ERR_ARG;
   // automatic choice: the tensor-core kernel when whole segments, one block each, already fill
   // the machine (two blocks per SM): then every block streams a long run of tiles, merges in
-  // shared memory and its start-up is amortised (90 % of the copy bandwidth at 128 sequences x 16
+  // shared memory and its start-up is amortised (86-90 % of the copy bandwidth at 128 sequences x 16
   // heads x 64, 5.1 TB/s against 4.4 at 32 x 16 x 128).  With fewer (sequence, head) pairs the
   // segments have to be cut into short chunks and the CUDA-core kernel, with its 740 small
   // resident blocks, is the better fit.

@@ -17,11 +17,11 @@ synchronisation, allocation or Python between tokens.  Reference behaviour being
   * Standard   src/modeling/models/full_attention_model.py:506-740 (one row per token, the cache holds
                the current document, one query per step)
 
-What runs where: the projections and the head are library GEMMs (``torch.mm``); everything else
-on the per-token chain is a kernel of libspsattn.so — residual add + RMSNorm, rotary + cast of
-the fused projection into the attention operands, the segmented decode attention with the cache
-update folded into its merge pass, the SwiGLU gate — plus a handful of small integer torch ops per
-token (not per layer) for the token/position bookkeeping.  Parameters are bf16 (as the reference
+What runs where: a decode step of up to 16 rows in bf16 is a chain of kernels of libspsattn.so alone
+(``spsattn_decoder_step``: choice of the token, counters, embedding; projections fused with their norms, rotary
+embedding, gate and residual; segmented decode attention with the cache update; head).  In the prompt
+prefill and in larger steps, or fp32 ones, the projections and the head are library GEMMs, issued with the
+other kernels from native code (csrc/native_engine.h).  Parameters are bf16 (as the reference
 generates on CUDA) or fp32; the attention operands and caches are bf16 either way.
 """
 

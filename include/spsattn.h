@@ -431,8 +431,9 @@ int spsattn_swiglu(const void* gate_up, void* y, int dtype, long long rows, int 
  * spsattn_decoder_choose: the greedy choice alone (the last token of a generation).
  * spsattn_decoder_step: start, every layer's projections around spsattn_decode_step, and the head on
  *   the prediction slot, each launch a programmatic dependent of the one before it.  For decoders that
- *   spsattn_decoder_step_supported takes (1 = yes): bf16, batch * slots <= 16 rows, hidden and
- *   intermediate multiples of 16, hidden <= 2048, weights (wte apart) and step buffers 16-byte aligned.
+ *   spsattn_decoder_step_supported takes (1 = yes): bf16, batch <= 16, hidden <= 2048, weights (wte
+ *   apart) and step buffers 16-byte aligned; batch * slots <= 16 rows with hidden and intermediate
+ *   multiples of 16, or any of them with multiples of 64, head_dim of 16, and freqs_out.
  * ------------------------------------------------------------------------------------------- */
 typedef struct spsattn_decoder_layer {
   const void* attn_norm;      /* [C] */
@@ -488,6 +489,12 @@ int spsattn_decoder_start(const spsattn_decoder* d, const spsattn_token_source* 
                           void* stream);
 int spsattn_decoder_choose(const spsattn_decoder* d, const spsattn_token_source* source, void* stream);
 int spsattn_decoder_step_supported(const spsattn_decoder* d);
+/* The layers of a step between its start and its head, for at most 64 rows of any batch (bf16, hidden and
+ * intermediate multiples of 64, head_dim of 16, freqs_out, pointers at 16-byte boundaries): the residual
+ * stream in x moves on through all layers, xn [rows, C] receives its final norm.
+ * spsattn_decoder_blocks_supported: 1 = yes. */
+int spsattn_decoder_blocks_supported(const spsattn_decoder* d);
+int spsattn_decoder_blocks(const spsattn_decoder* d, void* xn, int* device_status, void* stream);
 /* logits_out: [batch, vocab] bf16, zeros for inactive sequences. */
 int spsattn_decoder_step(const spsattn_decoder* d, const spsattn_token_source* source, void* logits_out,
                          int* device_status, void* stream);

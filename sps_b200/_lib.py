@@ -27,7 +27,7 @@ EXPORTS = (
     "spsattn_decode_step_workspace_bytes", "spsattn_decode_step", "spsattn_decode_step_tickets",
     "spsattn_qkv_rope_cast",
     "spsattn_add_rmsnorm", "spsattn_swiglu", "spsattn_debug_decode_path", "spsattn_debug_prefill_path", "spsattn_debug_wait_expiry",
-    "spsattn_decoder_start", "spsattn_decoder_choose", "spsattn_decoder_step_supported", "spsattn_decoder_step",
+    "spsattn_decoder_start", "spsattn_decoder_choose", "spsattn_decoder_step_supported", "spsattn_decoder_blocks", "spsattn_decoder_blocks_supported", "spsattn_decoder_step",
     "spsattn_prefill_bwd_workspace_bytes", "spsattn_prefill_bwd", "spsattn_prefill_bwd_strided", "spsattn_prefill_bwd_after",
 )
 
@@ -171,6 +171,10 @@ def load() -> C.CDLL:
     lib.spsattn_decoder_choose.argtypes = [C.POINTER(Decoder), C.POINTER(TokenSource), vp]
     lib.spsattn_decoder_step_supported.restype = i32
     lib.spsattn_decoder_step_supported.argtypes = [C.POINTER(Decoder)]
+    lib.spsattn_decoder_blocks_supported.restype = i32
+    lib.spsattn_decoder_blocks_supported.argtypes = [C.POINTER(Decoder)]
+    lib.spsattn_decoder_blocks.restype = i32
+    lib.spsattn_decoder_blocks.argtypes = [C.POINTER(Decoder), vp, vp, vp]
     lib.spsattn_decoder_step.restype = i32
     lib.spsattn_decoder_step.argtypes = [C.POINTER(Decoder), C.POINTER(TokenSource), vp, vp, vp]
     lib.spsattn_debug_decode_path.restype = i32

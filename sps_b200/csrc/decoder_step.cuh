@@ -32,10 +32,8 @@
 namespace spsattn {
 
 enum SkinnyEpilogue { kSkinnyQkv = 0, kSkinnyResidual = 1, kSkinnySwiglu = 2, kSkinnyLogits = 3 };
-// us per token against library projections (prompt 100, captured): 768 columns, 12 layers 8 rows 302 / 473, 16
-// rows 375 / 470 (library with 18: 460); 1024 columns 347 / 536, 416 / 532; 2048 columns, 24 layers 1289 / 1681,
-// 12 rows 1491 / 1518, 16 rows 1643 / 1534.  Above 16 rows a third tile of rows would be needed; past 1024
-// columns the library is already ahead from 13 rows on.
+// Taken up to 8 rows; from 9 on only where the projections of decoder_rows.cuh do not take the sizes
+// (rows_preferred has both sides measured), and for the head.
 constexpr int kSkinnyMaxRows = 16;
 constexpr int kSkinnyMaxCols = 2048;   // of a normalised input: one vector of 8 per thread of add_rmsnorm_kernel
 constexpr int kSkinnyMaxStages = 16;

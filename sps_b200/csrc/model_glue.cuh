@@ -19,6 +19,7 @@ struct RmsNormParams {
   long long rows;
   int C;
   float eps;
+  int let_go;          // dependents may start at once: they wait themselves before they read y
 };
 
 __device__ __forceinline__ float round_bf16(float f) {
@@ -81,6 +82,7 @@ __global__ void __launch_bounds__(256, kRowVecs == 1 ? 6 : kAhead ? 2 : 4) add_r
 
   // Bound: HBM.  A block synchronises once per row (every thread adds the eight warp sums itself, in the
   // same order): 65536 rows of 2048 with delta 250 -> 174 us, 6.2 TB/s.
+  if (p.let_go) grid_launch_dependents();
   grid_dependency_wait();
   uint4 nx[kRowVecs], nd[kRowVecs];
   auto fetch = [&](long long row) {

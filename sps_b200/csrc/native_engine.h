@@ -196,9 +196,10 @@ PyObject* engine_prefill_impl(PyObject* const* a, Py_ssize_t n) {
 }
 
 // engine_step(model, decoder address, source address, rope groups address, buffers (x, xn, delta, qkv, y,
-//             gate_up, hidden, fc), logits): one decode step by library GEMMs and single kernels
+//             gate_up, hidden, fc), logits, blocks): one decode step, its layers by spsattn_decoder_blocks or
+//             by library GEMMs and single kernels
 PyObject* engine_step_impl(PyObject* const* a, Py_ssize_t n) {
-  if (n != 6) fail(PyExc_TypeError, "engine_step takes 6 arguments");
+  if (n != 7) fail(PyExc_TypeError, "engine_step takes 7 arguments");
   const EngineModel& m = engine_arg(a[0]);
   const auto* d = reinterpret_cast<const spsattn_decoder*>(PyLong_AsVoidPtr(a[1]));
   const auto* source = reinterpret_cast<const spsattn_token_source*>(PyLong_AsVoidPtr(a[2]));
@@ -208,6 +209,7 @@ PyObject* engine_step_impl(PyObject* const* a, Py_ssize_t n) {
   require(d && source && groups && buf.size() == 8, "engine_step needs its argument blocks and eight buffers");
   Tensor &x = buf[0], &xn = buf[1], &delta = buf[2], &qkv = buf[3], &y = buf[4], &gate_up = buf[5], &hidden = buf[6], &fc = buf[7];
   Tensor logits = tensor_arg(a[5], "logits");
+  const bool blocks = bool_arg(a[6]);
   unlocked([&] {
     const c10::cuda::CUDAGuard guard(x.device());
     void* stream = stream_of(x);
@@ -215,6 +217,11 @@ PyObject* engine_step_impl(PyObject* const* a, Py_ssize_t n) {
     const int ns = d->slots, b = d->batch;
     const int64_t C = m.C, D = m.head_dim;
     check_rc(spsattn_decoder_start(d, source, status, stream), "spsattn_decoder_start");
+    if (blocks) {
+      check_rc(spsattn_decoder_blocks(d, xn.data_ptr(), status, stream), "spsattn_decoder_blocks");
+      at::mm_out(logits, xn.view({b, ns, C}).select(1, d->pred_slot), m.lm_head);
+      return;
+    }
     spsattn_extra extras[2] = {};
     for (int s = 0; s < ns; ++s) {
       extras[s].k = reinterpret_cast<const uint16_t*>(d->k2) + (size_t)s * b * C;

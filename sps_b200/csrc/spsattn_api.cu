@@ -16,6 +16,7 @@
 #include "cache_fill.cuh"
 #include "decode.cuh"
 #include "decode_sm100.cuh"
+#include "decoder_rows.cuh"
 #include "decoder_step.cuh"
 #include "device_once.h"
 #include "kv_update.cuh"
@@ -1258,8 +1259,8 @@ int spsattn_kv_update(void* nw_k, void* nw_v, int64_t* nw_len, int64_t* nw_pos, 
 
 // ------------------------------------------------------------------------ block glue (norm, gate)
 
-int spsattn_add_rmsnorm(void* x, const void* delta, const void* weight, void* y, int dtype,
-                        long long rows, int C, float eps, void* stream) {
+static int add_rmsnorm(void* x, const void* delta, const void* weight, void* y, int dtype, long long rows, int C, float eps,
+                       int let_go, void* stream) {
   if (!x || !weight || (!y && !delta)) return SPSATTN_ERR_ARG;
   if (rows <= 0 || C <= 0 || !(eps >= 0.f)) return SPSATTN_ERR_ARG;
   if (dtype != SPSATTN_DTYPE_BF16 && dtype != SPSATTN_DTYPE_FP32) return SPSATTN_ERR_ARG;
@@ -1275,6 +1276,7 @@ int spsattn_add_rmsnorm(void* x, const void* delta, const void* weight, void* y,
   p.rows = rows;
   p.C = C;
   p.eps = eps;
+  p.let_go = let_go;
   const unsigned blocks = (unsigned)(rows < 148LL * 16 ? rows : 148LL * 16);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   // Rows of at most 256 vectors: one per thread, the next row under way.  Wider ones: so too where two
@@ -1287,6 +1289,11 @@ int spsattn_add_rmsnorm(void* x, const void* delta, const void* weight, void* y,
                  : ahead     ? (bf16 ? add_rmsnorm_kernel<true, 4, true> : add_rmsnorm_kernel<false, 4, true>)
                              : (bf16 ? add_rmsnorm_kernel<true, 4, false> : add_rmsnorm_kernel<false, 4, false>);
   return launch_dependent(kernel, dim3(blocks), dim3(256), 0, st, p);
+}
+
+int spsattn_add_rmsnorm(void* x, const void* delta, const void* weight, void* y, int dtype,
+                        long long rows, int C, float eps, void* stream) {
+  return add_rmsnorm(x, delta, weight, y, dtype, rows, C, eps, 0, stream);
 }
 
 int spsattn_swiglu(const void* gate_up, void* y, int dtype, long long rows, int I, void* stream) {
@@ -1355,6 +1362,59 @@ int launch_skinny(SkinnyParams p, cudaStream_t st) {
   return launch_dependent(kernel, dim3((unsigned)blocks), dim3((unsigned)threads), (size_t)(ring + fixed), st, p);
 }
 
+// [rows, K] operand with contiguous rows, K a multiple of 64, as [64, rows, K / 64]: a box is box_rows rows of
+// `groups` pieces of 64 columns, each piece a tile of its own, 128-byte swizzle; what lies outside reads as zeros
+int encode_rows_map(CUtensorMap* tm, const void* ptr, long long rows, int K, int box_rows, int groups) {
+  EncodeTiledFn enc = get_encode_fn();
+  if (!enc) return SPSATTN_ERR_DRIVER;
+  cuuint64_t dims[3] = {64, (cuuint64_t)rows, (cuuint64_t)(K / 64)};
+  cuuint64_t strides[2] = {(cuuint64_t)K * 2, 128};
+  cuuint32_t box[3] = {64, (cuuint32_t)box_rows, (cuuint32_t)groups};
+  cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : (int)r;
+}
+
+template <int EPI>
+int launch_rows_gemm(RowsGemmParams p, const void* w, const void* x, cudaStream_t st) {
+  const int sms = multiprocessors(), parts = EPI == kRowsSwiglu ? 2 : 1, step = 8 * parts;
+  const int w_rows = parts * p.F, most = EPI == kRowsSwiglu ? kRowsMaxN : kRowsHeldN;
+  // A block reads (bn + bm) rows of K columns.  The cheapest sizes by that and the number of waves; ties go
+  // to the wider input tile, which reads the weights once.
+  long long best = 0;
+  for (int bm = (p.rows + 15) / 16 * 16, tiles_r = 1; bm >= 16; tiles_r *= 2, bm = ((p.rows + tiles_r - 1) / tiles_r + 15) / 16 * 16) {
+    for (int bn = step; bn <= most; bn += step) {
+      const long long blocks = (long long)((w_rows + bn - 1) / bn) * tiles_r, waves = (blocks + sms - 1) / sms;
+      const long long cost = waves * (bn + bm + 16);
+      if (best == 0 || cost < best) best = cost, p.bn = bn, p.bm = bm;
+    }
+    if (tiles_r >= 4 || bm == 16) break;
+  }
+  // stages as wide as still gives three of them
+  int stage = 0, chunks = 0;
+  for (p.groups = 8;; p.groups /= 2) {
+    stage = p.groups * (p.bn + p.bm) * 128;
+    chunks = (p.K / 64 + p.groups - 1) / p.groups;
+    p.stages = 200 * 1024 / stage;
+    if (p.stages > kRowsMaxStages) p.stages = kRowsMaxStages;
+    if (p.stages > chunks) p.stages = chunks;
+    if (p.stages >= 3 || p.stages == chunks || p.groups == 1) break;
+  }
+  CUtensorMap tw, tx;
+  int rc = encode_rows_map(&tw, w, w_rows, p.K, p.bn / parts, parts == 2 ? 1 : p.groups);
+  if (rc == 0) rc = encode_rows_map(&tx, x, p.rows, p.K, p.bm, p.groups);
+  if (rc != 0) return rc;
+  // (the M side of the last stage reads 64 rows from its start: bm may be less, and bn with it)
+  const int bytes = p.stages * stage + 8192 + 1024;
+  static std::atomic<uint64_t> sized{0};
+  if ((rc = allow_shared_memory(sized, rows_gemm_kernel<EPI>, 200 * 1024 + 8192 + 1024)) != 0) return rc;
+  const int bf = p.bn / parts;
+  return launch_dependent(rows_gemm_kernel<EPI>, dim3((unsigned)((p.F + bf - 1) / bf), (unsigned)((p.rows + p.bm - 1) / p.bm)),
+                          dim3(kRowsThreads), (size_t)bytes, st, tw, tx, p);
+}
+
 int launch_token_start(const spsattn_decoder* d, const spsattn_token_source* src, bool choose_only, int* status,
                        cudaStream_t st) {
   if (!d || !src || d->batch <= 0 || d->vocab <= 0) return SPSATTN_ERR_ARG;
@@ -1410,13 +1470,31 @@ int launch_token_start(const spsattn_decoder* d, const spsattn_token_source* src
              : launch_dependent(token_start_kernel<false>, dim3((unsigned)d->batch), dim3(kStartThreads), 0, st, p);
 }
 
-// sizes that the fused step takes
+bool decoder_sizes(const spsattn_decoder* d) {
+  return d && d->param_dtype == SPSATTN_DTYPE_BF16 && d->batch > 0 && d->n_layer > 0 && (d->slots == 1 || d->slots == 2) &&
+         d->n_head > 0 && d->vocab > 0 && d->hidden == d->n_head * d->head_dim && d->intermediate > 0;
+}
+
+// sizes that the projections of decoder_step.cuh take (the norm's sums are those of a row of at most 256 vectors)
+bool skinny_sizes(const spsattn_decoder* d) {
+  return d->batch * d->slots <= kSkinnyMaxRows && d->hidden % 16 == 0 && d->hidden <= kSkinnyMaxCols && d->intermediate % 16 == 0;
+}
+
+// sizes that those of decoder_rows.cuh take
+bool rows_sizes(const spsattn_decoder* d) {
+  return d->batch * d->slots <= kRowsMaxRows && d->hidden % 64 == 0 && d->head_dim % 16 == 0 && d->intermediate % 64 == 0 &&
+         d->freqs_out != nullptr && aligned16(d->freqs_out);
+}
+
+// Which of the two, where both do.  us per token, decoder_step.cuh / decoder_rows.cuh: 768 columns, 12 layers 8 rows
+// 296 / 335, 10 rows 338 / 326, 16 rows 371 / 326; 512, 4 layers 98 / 111, 105 / 106, 110 / 104; 2048, 6 layers 328 / 344, 363 / 341,
+// 418 / 342 (library projections 384).
+bool rows_preferred(const spsattn_decoder* d) { return rows_sizes(d) && (d->batch * d->slots > 8 || !skinny_sizes(d)); }
+
+// sizes that the fused step takes: its head is decoder_step.cuh's
 bool fused_step_sizes(const spsattn_decoder* d) {
-  if (!d || d->param_dtype != SPSATTN_DTYPE_BF16 || d->batch <= 0 || d->n_layer <= 0) return false;
-  if ((d->slots != 1 && d->slots != 2) || d->n_head <= 0 || d->vocab <= 0) return false;
-  if (d->hidden != d->n_head * d->head_dim || d->batch * d->slots > kSkinnyMaxRows) return false;
-  // the norm's sums are those of a row of at most 256 vectors
-  return d->hidden % 16 == 0 && d->hidden <= kSkinnyMaxCols && d->intermediate > 0 && d->intermediate % 16 == 0;
+  return decoder_sizes(d) && d->batch <= kSkinnyMaxRows && d->hidden % 16 == 0 && d->hidden <= kSkinnyMaxCols &&
+         (skinny_sizes(d) || rows_sizes(d));
 }
 
 // what its kernels move by 16 bytes (weights may be views into a buffer of the caller's)
@@ -1436,6 +1514,75 @@ int fused_step_pointers(const spsattn_decoder* d) {
   return rc;
 }
 
+// every slot sees the step's input row, only the <predict> slot its own (decode_attention.py:354-361)
+void step_extras(const spsattn_decoder* d, spsattn_extra (&extras)[2]) {
+  memset(extras, 0, sizeof(extras));
+  for (int s = 0; s < d->slots; ++s) {
+    extras[s].k = reinterpret_cast<const uint16_t*>(d->k2) + (size_t)s * d->batch * d->hidden;
+    extras[s].v = reinterpret_cast<const uint16_t*>(d->v2) + (size_t)s * d->batch * d->hidden;
+    extras[s].query_mask = s == 0 ? (1u << d->slots) - 1 : 2u;
+  }
+}
+
+// All layers of a step by the projections of decoder_rows.cuh: x moves on, ssq is that of the last row.  The normalised
+// rows go through y, which is free whenever a norm has run: the attention's output is read by c_proj alone.
+int launch_rows_layers(const spsattn_decoder* d, int* status, cudaStream_t st) {
+  const int C = d->hidden, I = d->intermediate, rows = d->batch * d->slots;
+  spsattn_extra extras[2];
+  step_extras(d, extras);
+  auto norm = [&](const void* weight) {
+    return add_rmsnorm(d->x, nullptr, weight, d->y, SPSATTN_DTYPE_BF16, rows, C, d->norm_eps, 1, st);
+  };
+  RowsGemmParams base;
+  memset(&base, 0, sizeof(base));
+  base.rows = rows;
+  base.slots = d->slots;
+  base.batch = d->batch;
+  base.head_dim = d->head_dim;
+  base.status = status;
+  int rc = 0;
+  for (int layer = 0; layer < d->n_layer; ++layer) {
+    const spsattn_decoder_layer& w = d->layers[layer];
+    if ((rc = norm(w.attn_norm)) != 0) return rc;
+    RowsGemmParams p = base;
+    p.K = C;
+    p.F = 3 * C;
+    p.q = reinterpret_cast<uint16_t*>(d->q);
+    p.k = reinterpret_cast<uint16_t*>(d->k2);
+    p.v = reinterpret_cast<uint16_t*>(d->v2);
+    p.freqs = reinterpret_cast<const float2*>(d->freqs_out);
+    if ((rc = launch_rows_gemm<kRowsQkv>(p, w.c_attn, d->y, st)) != 0) return rc;
+    bool ring_later = false;
+    rc = decode_impl(d->q, d->slots, d->y, SPSATTN_DTYPE_BF16, w.segments, d->n_segments, extras, d->slots, &w.append, true,
+                     d->batch, d->n_head, d->head_dim, SPSATTN_DTYPE_BF16, 1.0f / sqrtf((float)d->head_dim), d->workspace,
+                     d->workspace_bytes, nullptr, 0, status, st, &ring_later);
+    if (rc != 0) return rc;
+    p = base;
+    if (ring_later) {
+      p.ring_len = w.append.nw_len;
+      p.ring_pos = w.append.nw_pos;
+      p.ring_tokens = w.append.window_tokens;
+      p.active = w.append.active;
+    }
+    p.K = C;
+    p.F = C;
+    p.out = reinterpret_cast<uint16_t*>(d->x);
+    if ((rc = launch_rows_gemm<kRowsResidual>(p, w.c_proj, d->y, st)) != 0 || (rc = norm(w.mlp_norm)) != 0) return rc;
+    p = base;
+    p.K = C;
+    p.F = I;
+    p.out = reinterpret_cast<uint16_t*>(d->mlp_hidden);
+    if ((rc = launch_rows_gemm<kRowsSwiglu>(p, w.gate_up, d->y, st)) != 0) return rc;
+    p = base;
+    p.K = I;
+    p.F = C;
+    p.out = reinterpret_cast<uint16_t*>(d->x);
+    if (layer + 1 == d->n_layer) p.ssq_out = d->ssq;
+    if ((rc = launch_rows_gemm<kRowsResidual>(p, w.down, d->mlp_hidden, st)) != 0) return rc;
+  }
+  return 0;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1453,6 +1600,19 @@ int spsattn_decoder_step_supported(const spsattn_decoder* d) {
   return fused_step_sizes(d) && fused_step_pointers(d) == 0 ? 1 : 0;
 }
 
+int spsattn_decoder_blocks_supported(const spsattn_decoder* d) {
+  return decoder_sizes(d) && rows_sizes(d) && fused_step_pointers(d) == 0 ? 1 : 0;
+}
+
+int spsattn_decoder_blocks(const spsattn_decoder* d, void* xn, int* device_status, void* stream) {
+  if (!spsattn_decoder_blocks_supported(d) || !xn) return SPSATTN_ERR_ARG;
+  if (d->n_segments < 1 || d->n_segments > 2) return SPSATTN_ERR_ARG;
+  if (!aligned16(xn)) return SPSATTN_ERR_ALIGN;
+  const int rc = launch_rows_layers(d, device_status, reinterpret_cast<cudaStream_t>(stream));
+  if (rc != 0) return rc;
+  return add_rmsnorm(d->x, nullptr, d->out_norm, xn, SPSATTN_DTYPE_BF16, d->batch * d->slots, d->hidden, d->norm_eps, 0, stream);
+}
+
 int spsattn_decoder_step(const spsattn_decoder* d, const spsattn_token_source* source, void* logits_out,
                          int* device_status, void* stream) {
   if (!fused_step_sizes(d) || !source || !logits_out) return SPSATTN_ERR_ARG;
@@ -1464,14 +1624,8 @@ int spsattn_decoder_step(const spsattn_decoder* d, const spsattn_token_source* s
   rc = launch_token_start(d, source, false, device_status, st);
   if (rc != 0) return rc;
   const int C = d->hidden, I = d->intermediate, rows = d->batch * d->slots;
-  // every slot sees the step's input row, only the <predict> slot its own (decode_attention.py:354-361)
   spsattn_extra extras[2];
-  memset(extras, 0, sizeof(extras));
-  for (int s = 0; s < d->slots; ++s) {
-    extras[s].k = reinterpret_cast<const uint16_t*>(d->k2) + (size_t)s * d->batch * C;
-    extras[s].v = reinterpret_cast<const uint16_t*>(d->v2) + (size_t)s * d->batch * C;
-    extras[s].query_mask = s == 0 ? (1u << d->slots) - 1 : 2u;
-  }
+  step_extras(d, extras);
   SkinnyParams base;
   memset(&base, 0, sizeof(base));
   base.rows = rows;
@@ -1483,7 +1637,9 @@ int spsattn_decoder_step(const spsattn_decoder* d, const spsattn_token_source* s
   base.x = reinterpret_cast<const uint16_t*>(d->x);
   base.x_stride = C;
   base.K = C;
-  for (int layer = 0; layer < d->n_layer; ++layer) {
+  const bool by_rows = rows_preferred(d);
+  if (by_rows && (rc = launch_rows_layers(d, device_status, st)) != 0) return rc;
+  for (int layer = 0; layer < d->n_layer && !by_rows; ++layer) {
     const spsattn_decoder_layer& w = d->layers[layer];
     SkinnyParams p = base;
     p.w = reinterpret_cast<const uint16_t*>(w.c_attn);

@@ -388,6 +388,7 @@ class SPSGenerator:
         s.ws_bytes = ws_bytes
         s.decoder = self._bind_decoder(s)
         s.fused = bool(self.lib.spsattn_decoder_step_supported(C.byref(s.decoder)))
+        s.blocks = not s.fused and bool(self.lib.spsattn_decoder_blocks_supported(C.byref(s.decoder)))
         self._step = s
 
     def _bind_decoder(self, s) -> _lib.Decoder:
@@ -429,7 +430,7 @@ class SPSGenerator:
             _lib.check(rc, "spsattn_decoder_step")
             return
         ext, model = self._native()
-        ext.engine_step(model, C.addressof(s.decoder), C.addressof(source), C.addressof(s.groups), s.buffers, logits)
+        ext.engine_step(model, C.addressof(s.decoder), C.addressof(source), C.addressof(s.groups), s.buffers, logits, s.blocks)
 
     @torch.no_grad()
     def decode_one_token(self, state: DecodeState, token_B: Tensor, active_B: Tensor) -> Tensor:

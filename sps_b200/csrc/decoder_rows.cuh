@@ -191,97 +191,107 @@ rows_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     __syncwarp();
   } else {
     // ------------------------------------------------------------------ results
-    // M = 64: row r of the accumulator lies in lane 32 * (r / 16) + r % 16
-    const int rl = warp * 16 + lane, r = r0 + rl;
-    const bool live_row = lane < 16 && rl < p.bm && r < p.rows;
-    const int two = p.slots - 1, bi = r >> two, slot = r & two;
-    const int C = EPI == kRowsQkv ? p.F / 3 : 1;
-    constexpr int kHeld = EPI == kRowsSwiglu ? 1 : kRowsHeldN / 8;
+    // The sums go through shared memory (the ring, whose copies and products are over by then), so that all
+    // threads work, each on vectors of 8 outputs of a row, and rows are written in one piece: with a row per
+    // lane (16 of 32 lanes have one) and everything unrolled the results took 2000 clk, most of them for
+    // instructions that no cache had yet.
+    const int vecs = bf / 8, rows_here = min(p.bm, p.rows - r0), items = rows_here * vecs;
+    const int two = p.slots - 1, C = EPI == kRowsQkv ? p.F / 3 : 1;
+    constexpr int kHeld = EPI == kRowsSwiglu ? 1 : kRowsMaxRows * kRowsHeldN / 8 / 128;
     // what stands beside the sums is asked for while they are made: the old row, or the rotary factors
     uint4 old[EPI == kRowsResidual ? kHeld : 1];
     float4 cs[EPI == kRowsQkv ? kHeld : 1][2];
-    if constexpr (EPI == kRowsResidual) {
+    if constexpr (EPI != kRowsSwiglu) {
 #pragma unroll
-      for (int c = 0; c < kHeld; ++c)
-        if (live_row && c * 8 < p.bn && f0 + c * 8 < p.F)
-          old[c] = __ldcg(reinterpret_cast<const uint4*>(p.out + (size_t)r * p.F + f0 + c * 8));
-    }
-    if constexpr (EPI == kRowsQkv) {
-#pragma unroll
-      for (int c = 0; c < kHeld; ++c) {
-        const int f = f0 + c * 8;
-        if (live_row && c * 8 < p.bn && f < 2 * C) {
-          const float4* fr = reinterpret_cast<const float4*>(p.freqs + (size_t)bi * (p.head_dim / 2) + (f >= C ? f - C : f) % p.head_dim / 2);
-          cs[c][0] = __ldg(fr);
-          cs[c][1] = __ldg(fr + 1);
+      for (int k = 0; k < kHeld; ++k) {
+        const int i = tid + 128 * k, rl = i / vecs, f = f0 + (i - rl * vecs) * 8, r = r0 + rl;
+        if (i < items && f < p.F) {
+          if constexpr (EPI == kRowsResidual) old[k] = __ldcg(reinterpret_cast<const uint4*>(p.out + (size_t)r * p.F + f));
+          if constexpr (EPI == kRowsQkv) {
+            if (f < 2 * C) {
+              const float4* fr = reinterpret_cast<const float4*>(p.freqs + (size_t)(r >> two) * (p.head_dim / 2) + (f >= C ? f - C : f) % p.head_dim / 2);
+              cs[k][0] = __ldcg(fr);
+              cs[k][1] = __ldcg(fr + 1);
+            }
+          }
         }
       }
     }
-    const bool ok = mbar_wait(done, 0, abort_flag, p.status);
-    __syncwarp();
+    const bool ok = __all_sync(0xffffffffu, mbar_wait(done, 0, abort_flag, p.status));
+    const int pitch = p.bn * 4 + 16;                 // bytes of a row of sums
     if (ok) {
       tc_fence_after();
-      const uint32_t at = tmem + ((uint32_t)(warp * 32) << 16);
-      if constexpr (EPI == kRowsSwiglu) {
-        for (int c = 0; c < bf; c += 8) {
-          uint32_t g[8], u[8];
-          tmem_ld8(at + c, g);
-          tmem_ld8(at + bf + c, u);
-          tmem_wait_ld();
-          uint32_t o[4];
-#pragma unroll
-          for (int e = 0; e < 8; e += 2) {
-            const float g0 = round_bf16(__uint_as_float(g[e])), g1 = round_bf16(__uint_as_float(g[e + 1]));
-            o[e / 2] = pack2<false>(round_bf16(silu_f(g0)) * round_bf16(__uint_as_float(u[e])),
-                                    round_bf16(silu_f(g1)) * round_bf16(__uint_as_float(u[e + 1])));
-          }
-          if (live_row && f0 + c < p.F)
-            *reinterpret_cast<uint4*>(p.out + (size_t)r * p.F + f0 + c) = make_uint4(o[0], o[1], o[2], o[3]);
-        }
-      } else {
-#pragma unroll
-        for (int c = 0; c < kHeld; ++c) {
-          const int f = f0 + c * 8;
-          if (c * 8 >= p.bn || f >= p.F) break;
-          uint32_t a[8];
-          tmem_ld8(at + c * 8, a);
-          tmem_wait_ld();
-          uint32_t o[4];
-          uint16_t* dst;
-          if constexpr (EPI == kRowsResidual) {
-            const uint32_t w[4] = {old[c].x, old[c].y, old[c].z, old[c].w};
-            float sq = 0.f;
-#pragma unroll
-            for (int e = 0; e < 8; e += 2) {
-              float o0, o1;
-              unpack2<false>(w[e / 2], o0, o1);
-              o0 = round_bf16(o0 + round_bf16(__uint_as_float(a[e])));
-              o1 = round_bf16(o1 + round_bf16(__uint_as_float(a[e + 1])));
-              o[e / 2] = pack2<false>(o0, o1);
-              sq = fmaf(o0, o0, sq);
-              sq = fmaf(o1, o1, sq);
-            }
-            if (p.ssq_out != nullptr && live_row) p.ssq_out[(size_t)r * (p.F / 8) + f / 8] = sq;
-            dst = p.out + (size_t)r * p.F + f;
-          } else {
-            const int which = (f >= C) + (f >= 2 * C), fi = f - which * C;
-            const float q[8] = {cs[c][0].x, cs[c][0].y, cs[c][0].z, cs[c][0].w, cs[c][1].x, cs[c][1].y, cs[c][1].z, cs[c][1].w};
-#pragma unroll
-            for (int e = 0; e < 8; e += 2) {
-              float v0 = round_bf16(__uint_as_float(a[e])), v1 = round_bf16(__uint_as_float(a[e + 1]));
-              if (which < 2) {
-                const float x0 = v0, x1 = v1;
-                v0 = __fsub_rn(__fmul_rn(x0, q[e]), __fmul_rn(x1, q[e + 1]));
-                v1 = __fadd_rn(__fmul_rn(x0, q[e + 1]), __fmul_rn(x1, q[e]));
-              }
-              o[e / 2] = pack2<false>(v0, v1);
-            }
-            dst = which == 0 ? p.q + (size_t)r * C + fi : (which == 1 ? p.k : p.v) + ((size_t)slot * p.batch + bi) * C + fi;
-          }
-          if (live_row) *reinterpret_cast<uint4*>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+      // M = 64: row r of the accumulator lies in lane 32 * (r / 16) + r % 16
+      const uint32_t at = tmem + ((uint32_t)(warp * 32) << 16), to = smem + (warp * 16 + lane) * pitch;
+#pragma unroll 1
+      for (int c = 0; c < p.bn; c += 8) {
+        uint32_t a[8];
+        tmem_ld8(at + c, a);
+        tmem_wait_ld();
+        if (lane < 16) {
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(to + c * 4), "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]) : "memory");
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(to + c * 4 + 16), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]) : "memory");
         }
       }
       tc_fence_before();
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    auto sums = [&](uint32_t from, float (&v)[8]) {
+      const uint4 lo = lds16(from), hi = lds16(from + 16);
+      const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = round_bf16(__uint_as_float(w[e]));
+    };
+    auto result = [&](int k) {
+      const int i = tid + 128 * k, rl = i / vecs, c = (i - rl * vecs) * 8, f = f0 + c, r = r0 + rl;
+      if (!ok || i >= items || f >= p.F) return;
+      float v[8];
+      sums(smem + rl * pitch + c * 4, v);
+      uint16_t* dst;
+      if constexpr (EPI == kRowsSwiglu) {
+        float u[8];
+        sums(smem + rl * pitch + (bf + c) * 4, u);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = round_bf16(silu_f(v[e])) * u[e];
+        dst = p.out + (size_t)r * p.F + f;
+      } else if constexpr (EPI == kRowsResidual) {
+        const uint32_t w[4] = {old[k].x, old[k].y, old[k].z, old[k].w};
+        float sq = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) {
+          float o0, o1;
+          unpack2<false>(w[e / 2], o0, o1);
+          v[e] = round_bf16(o0 + v[e]);
+          v[e + 1] = round_bf16(o1 + v[e + 1]);
+          sq = fmaf(v[e], v[e], sq);
+          sq = fmaf(v[e + 1], v[e + 1], sq);
+        }
+        if (p.ssq_out != nullptr) p.ssq_out[(size_t)r * (p.F / 8) + f / 8] = sq;
+        dst = p.out + (size_t)r * p.F + f;
+      } else {
+        const int which = (f >= C) + (f >= 2 * C), fi = f - which * C;
+        if (which < 2) {
+          const float q[8] = {cs[k][0].x, cs[k][0].y, cs[k][0].z, cs[k][0].w, cs[k][1].x, cs[k][1].y, cs[k][1].z, cs[k][1].w};
+#pragma unroll
+          for (int e = 0; e < 8; e += 2) {
+            const float x0 = v[e], x1 = v[e + 1];
+            v[e] = __fsub_rn(__fmul_rn(x0, q[e]), __fmul_rn(x1, q[e + 1]));
+            v[e + 1] = __fadd_rn(__fmul_rn(x0, q[e + 1]), __fmul_rn(x1, q[e]));
+          }
+        }
+        dst = which == 0 ? p.q + (size_t)r * C + fi
+                         : (which == 1 ? p.k : p.v) + ((size_t)(r & two) * p.batch + (r >> two)) * C + fi;
+      }
+      *reinterpret_cast<uint4*>(dst) = make_uint4(pack2<false>(v[0], v[1]), pack2<false>(v[2], v[3]), pack2<false>(v[4], v[5]),
+                                                  pack2<false>(v[6], v[7]));
+    };
+    if constexpr (EPI == kRowsSwiglu) {
+#pragma unroll 1
+      for (int k = 0; 128 * k < items; ++k) result(k);
+    } else {
+#pragma unroll
+      for (int k = 0; k < kHeld; ++k)
+        if (128 * k < items) result(k);
     }
   }
   __syncthreads();

@@ -1406,8 +1406,10 @@ int launch_rows_gemm(RowsGemmParams p, const void* w, const void* x, cudaStream_
   int rc = encode_rows_map(&tw, w, w_rows, p.K, p.bn / parts, parts == 2 ? 1 : p.groups);
   if (rc == 0) rc = encode_rows_map(&tx, x, p.rows, p.K, p.bm, p.groups);
   if (rc != 0) return rc;
-  // (the M side of the last stage reads 64 rows from its start: bm may be less, and bn with it)
-  const int bytes = p.stages * stage + 8192 + 1024;
+  // (the M side of the last stage reads 64 rows from its start: bm may be less, and bn with it; the sums
+  // of 64 rows take the ring's place)
+  const int ring = p.stages * stage + 8192, sums = kRowsMaxRows * (p.bn * 4 + 16);
+  const int bytes = (ring > sums ? ring : sums) + 1024;
   static std::atomic<uint64_t> sized{0};
   if ((rc = allow_shared_memory(sized, rows_gemm_kernel<EPI>, 200 * 1024 + 8192 + 1024)) != 0) return rc;
   const int bf = p.bn / parts;

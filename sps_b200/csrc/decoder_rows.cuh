@@ -7,15 +7,15 @@
 // copy bandwidth; q/k/v 7.2, 3.9), and the element-wise kernels behind them cost 2.7 us each.  Hence
 //   * one block per `bn` weight rows and `bm` input rows, sized so that a projection is one wave: the
 //     weights are the N side of tcgen05.mma (any multiple of 8), the rows its M = 64;
-//   * TMA brings both operands, up to 256 columns a stage (one copy each), through a ring as deep as shared
+//   * TMA brings both operands, up to 512 columns a stage (one copy each), through a ring as deep as shared
 //     memory allows: with 64 columns a stage the waits and issues around a stage took 430 clk, its products 124
 //     (2048 x 8192: 34 us);
 //   * the launches of a step are programmatic dependents of one another: a block asks for its whole ring
 //     of weights before it waits for the kernel before it, the input rows follow after the wait;
 //   * tensor memory is allocated after that wait: a block that held some while the attention before it
 //     still had blocks without theirs would wait for them, and they for it.
-// us per token, captured, library projections with single kernels / now: 12 layers of 768 columns 18 rows 464 / 357, 32
-// rows 460 / 334; 12 x 1024, 32 rows 544 / 405; 6 x 2048, 24 rows 417 / 401, 64 rows 522 / 481.
+// us per token, captured, library projections with single kernels / now: 12 layers of 768 columns 18 rows 464 / 351, 32
+// rows 460 / 334; 12 x 1024, 32 rows 544 / 397; 6 x 2048, 24 rows 417 / 401, 64 rows 522 / 481.
 // What is left at 2048 columns: 31 clk per 16 columns of a chain (2048 x 8192: 512 of them, 8 us), 300 clk per stage.
 // The contraction of one output is one chain of products in ascending k, never split, rounded to bf16 where
 // the separate kernels (library product, model_glue.cuh, rope.cuh) round theirs: the same bits as theirs at every

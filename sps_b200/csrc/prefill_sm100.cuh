@@ -72,16 +72,10 @@ constexpr int kPrefillThreads = 192;
 constexpr int kScanItems = 6;    // ids per thread where a block works out its document starts itself
 constexpr int kScanRows = kScanItems * kPrefillThreads;
 
-#ifndef SPSATTN_P_SPLIT
-#define SPSATTN_P_SPLIT_DEFAULT 1
-#else
-#define SPSATTN_P_SPLIT_DEFAULT (SPSATTN_P_SPLIT != 0)
-#endif
-
 template <int D>
 struct PrefillCfg {
   static constexpr int kStagesK = 2;
-  static constexpr int kStagesV = (D == 128) ? 1 : 2;
+  static constexpr int kStagesV = 2;       // (head_dim 128 with one: 1000 us at [4, 16, 8192, 128], full window, 993 with two)
   static constexpr int kSBufs = (D <= 64) ? 1 : 2;             // S accumulators in TMEM
   static constexpr uint32_t kTmemCols = (D <= 64) ? 128 : (D == 128) ? 256 : 512;
   // Heads narrower than 64 keep the 128-byte rows of shared memory: the tensor maps end at D and
@@ -92,12 +86,10 @@ struct PrefillCfg {
   static constexpr int kQSubBytes = kTileM * 128;              // 128 rows x 64 elements
   static constexpr int kKVBytes = kTileN * kDP * 2;              // one K or V tile
   static constexpr int kKVSubBytes = kTileN * 128;             // 64 rows x 64 elements
-  static constexpr int kPBytes = (D <= 64 && SPSATTN_P_SPLIT_DEFAULT) ? 0 : kTileM * kTileN * 2;
   static constexpr int kOffQ = 0;
   static constexpr int kOffK = kOffQ + kQBytes;
   static constexpr int kOffV = kOffK + kStagesK * kKVBytes;
-  static constexpr int kOffP = kOffV + kStagesV * kKVBytes;
-  static constexpr int kOffBar = kOffP + kPBytes;
+  static constexpr int kOffBar = kOffV + kStagesV * kKVBytes;
   static constexpr int kSmemBytes = kOffBar + 256 + 1024;      // barriers + alignment slack
   static constexpr int kBlocksPerSM = (D <= 64) ? 3 : (D == 128) ? 2 : 1;
   // head_dim 128 and 256 (two S accumulators): P never touches shared memory.  The softmax thread writes
@@ -111,10 +103,7 @@ struct PrefillCfg {
   // allocation: 128 + 32 columns per block, three blocks per SM = 480 of 512), so the next Q K^T
   // does not have to wait for this tile's P V.  No shared-memory stores, no swizzle arithmetic,
   // no proxy fence; the P tile's 16 KB of shared memory are not needed.
-#ifndef SPSATTN_P_SPLIT
-#define SPSATTN_P_SPLIT 1
-#endif
-  static constexpr bool kPSplit = (D <= 64) && (SPSATTN_P_SPLIT != 0);
+  static constexpr bool kPSplit = (D <= 64);
   static constexpr uint32_t kPCols = kTileN / 2;
   // head_dim 16, 32 and 256: the probabilities keep more than 16 bits.  P goes to tensor memory as
   // two 16-bit terms, p = hi + lo, and the product runs over both: these widths leave the tensor
@@ -294,7 +283,6 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   const uint32_t sQ = smem_base + Cfg::kOffQ;
   const uint32_t sK = smem_base + Cfg::kOffK;
   const uint32_t sV = smem_base + Cfg::kOffV;
-  const uint32_t sP = smem_base + Cfg::kOffP;
   const uint32_t bar0 = smem_base + Cfg::kOffBar;
   // barrier slots (8 bytes each)
   const uint32_t bar_q_full = bar0;
@@ -501,11 +489,9 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         // field, which lives in the low 32 bits
         const uint64_t dq64 = make_smem_desc_sw128(sQ, 16, 1024);
         const uint64_t dk64 = make_smem_desc_sw128(sK, 16, 1024);
-        const uint64_t dp64 = make_smem_desc_sw128(sP, 16, 1024);
         const uint64_t dv64 = make_smem_desc_sw128(sV, Cfg::kKVSubBytes, 1024);
         const uint32_t dq_lo = (uint32_t)dq64, dq_hi = (uint32_t)(dq64 >> 32);
         const uint32_t dk_lo = (uint32_t)dk64, dk_hi = (uint32_t)(dk64 >> 32);
-        const uint32_t dp_lo = (uint32_t)dp64, dp_hi = (uint32_t)(dp64 >> 32);
         const uint32_t dv_lo = (uint32_t)dv64, dv_hi = (uint32_t)(dv64 >> 32);
         auto issue_qk = [&](int j) {
           const int st = j % Cfg::kStagesK;
@@ -548,28 +534,17 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           const uint32_t vb0 = dv_lo + ((st * Cfg::kKVBytes) >> 4);
           const uint32_t od = tmem + Cfg::kColO;
           if (elect_one()) {
-            // P: K-major, one 64-key sub-tile; V: MN-major, 16 key rows = 2048 bytes per step
-            if constexpr (Cfg::kPTmem || Cfg::kPSplit) {
-              // A from tensor memory: 16 keys = 8 packed columns per step
-              const uint32_t pa = Cfg::kPSplit ? tmem_p : tmem + (j % Cfg::kSBufs) * kTileN;
+            // V: MN-major, 16 key rows = 2048 bytes per step
+            // A from tensor memory: 16 keys = 8 packed columns per step
+            const uint32_t pa = Cfg::kPSplit ? tmem_p : tmem + (j % Cfg::kSBufs) * kTileN;
+#pragma unroll
+            for (int kk = 0; kk < kTileN / 16; ++kk)
+              umma_ts(od, pa + 8 * kk, vb0 + ((kk * 2048) >> 4), dv_hi, idesc_pv, j > 0 || kk > 0);
+            if constexpr (Cfg::kPLo) {
+              const uint32_t pl = Cfg::kPSplit ? tmem + Cfg::kColPLo : pa + Cfg::kColPLo;
 #pragma unroll
               for (int kk = 0; kk < kTileN / 16; ++kk)
-                umma_ts(od, pa + 8 * kk, vb0 + ((kk * 2048) >> 4), dv_hi, idesc_pv, j > 0 || kk > 0);
-              if constexpr (Cfg::kPLo) {
-                const uint32_t pl = Cfg::kPSplit ? tmem + Cfg::kColPLo : pa + Cfg::kColPLo;
-#pragma unroll
-                for (int kk = 0; kk < kTileN / 16; ++kk)
-                  umma_ts(od, pl + 8 * kk, vb0 + ((kk * 2048) >> 4), dv_hi, idesc_pv, true);
-              }
-            } else {
-              if (j > 0) {
-                umma_ss<true>(od, dp_lo, dp_hi, vb0, dv_hi, idesc_pv);
-              } else {
-                umma_ss<false>(od, dp_lo, dp_hi, vb0, dv_hi, idesc_pv);
-              }
-#pragma unroll
-              for (int kk = 1; kk < kTileN / 16; ++kk)
-                umma_ss<true>(od, dp_lo + ((kk * 32) >> 4), dp_hi, vb0 + ((kk * 2048) >> 4), dv_hi, idesc_pv);
+                umma_ts(od, pl + 8 * kk, vb0 + ((kk * 2048) >> 4), dv_hi, idesc_pv, true);
             }
             umma_commit(bar_pv_done);
             umma_commit(bar_v_empty + 8 * st);
@@ -784,15 +759,6 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           tmem_st16(at, pl);
           tmem_st16(at + 16, pl + 16);
         }
-        // P -> shared memory, K-major 128B-swizzled: 16-byte chunk ch of row r sits at
-        // r * 128 + ((ch ^ (r & 7)) << 4) of the [128 x 64] tile
-#pragma unroll
-        for (int ch = 0; ch < ((Cfg::kPTmem || Cfg::kPSplit) ? 0 : 8); ++ch) {
-          const uint32_t addr = sP + row * 128 + ((ch ^ (row & 7)) << 4);
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(pk[ch * 4]),
-                       "r"(pk[ch * 4 + 1]), "r"(pk[ch * 4 + 2]), "r"(pk[ch * 4 + 3])
-                       : "memory");
-        }
         if (tid == 0) SPS_TRACE(j, 6);
         if (Cfg::kPTmem && j > 0) {
           if (!mbar_wait(bar_pv_done, (j - 1) & 1, abort_flag, prm.status)) {
@@ -814,8 +780,7 @@ prefill_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           tmem_wait_st();
         }
         if (tid == 0) SPS_TRACE(j, 7);
-        if constexpr (Cfg::kPTmem || Cfg::kPSplit) tmem_wait_st();
-        else fence_proxy_async_smem();
+        tmem_wait_st();
         tc_fence_before();
         softmax_arrive(bar_p_full, lane);
         if (tid == 0) SPS_TRACE(j, 8);

@@ -19,7 +19,8 @@ struct RmsNormParams {
   long long rows;
   int C;
   float eps;
-  int let_go;          // dependents may start at once: they wait themselves before they read y
+  int let_go;          // inside a decode step: dependents may start at once (they wait themselves before they read
+                       // y), and nothing that may still run writes the weight
 };
 
 __device__ __forceinline__ float round_bf16(float f) {
@@ -33,8 +34,9 @@ __device__ __forceinline__ float round_bf16(float f) {
 // kAhead: a block has its next row on the way while it works on this one.  That takes registers (with
 // kRowVecs 1 six blocks per SM still fit, 174 us against 202 with five; with 4 only two), which wide rows
 // need for more blocks: without it 65536 bf16 rows of 4096 357 -> 260 us, 16384 fp32 rows of 8192 310 -> 177.
-template <bool BF16, int kRowVecs, bool kAhead>
-__global__ void __launch_bounds__(256, kRowVecs == 1 ? 6 : kAhead ? 2 : 4) add_rmsnorm_kernel(const RmsNormParams p) {
+// kStep: inside a decode step, rows of at most 256 vectors; the few blocks have registers to keep the weight.
+template <bool BF16, int kRowVecs, bool kAhead, bool kStep = false>
+__global__ void __launch_bounds__(256, kStep ? 2 : kRowVecs == 1 ? 6 : kAhead ? 2 : 4) add_rmsnorm_kernel(const RmsNormParams p) {
   constexpr int V = BF16 ? 8 : 4;   // elements per 16-byte access
   __shared__ float s_part[2][8];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -72,9 +74,12 @@ __global__ void __launch_bounds__(256, kRowVecs == 1 ? 6 : kAhead ? 2 : 4) add_r
       px[at] = pack(f);
     }
   };
+  // kStep: the weight is read before the wait, not behind the barrier (us per token: 12 layers of 1024 columns, 32 rows
+  // 395 -> 379; 12 x 768, 18 rows 345 -> 339; 4 x 2048, 32 rows 337 -> 332).
+  uint4 wgt = make_uint4(0, 0, 0, 0);
   auto store_y = [&](size_t at, int i, const float (&f)[V], float scale) {
     float g[V], r[V];
-    unpack(__ldg(pw + i), g);
+    unpack(kStep ? wgt : __ldg(pw + i), g);
 #pragma unroll
     for (int e = 0; e < V; ++e) r[e] = BF16 ? round_bf16(f[e] * scale) * g[e] : f[e] * scale * g[e];
     py[at] = pack(r);
@@ -82,7 +87,10 @@ __global__ void __launch_bounds__(256, kRowVecs == 1 ? 6 : kAhead ? 2 : 4) add_r
 
   // Bound: HBM.  A block synchronises once per row (every thread adds the eight warp sums itself, in the
   // same order): 65536 rows of 2048 with delta 250 -> 174 us, 6.2 TB/s.
-  if (p.let_go) grid_launch_dependents();
+  if (p.let_go) {
+    grid_launch_dependents();
+    if (kStep && tid < n_vec) wgt = __ldg(pw + tid);
+  }
   grid_dependency_wait();
   uint4 nx[kRowVecs], nd[kRowVecs];
   auto fetch = [&](long long row) {

@@ -1285,7 +1285,8 @@ static int add_rmsnorm(void* x, const void* delta, const void* weight, void* y, 
   // that four blocks fit an SM.
   const int vecs = C / vec;
   const bool bf16 = dtype == SPSATTN_DTYPE_BF16, ahead = rows <= 2 * 148 || (!bf16 && vecs <= 1024);
-  auto* kernel = vecs <= 256 ? (bf16 ? add_rmsnorm_kernel<true, 1, true> : add_rmsnorm_kernel<false, 1, true>)
+  auto* kernel = let_go && bf16 && vecs <= 256 ? add_rmsnorm_kernel<true, 1, true, true>
+                 : vecs <= 256 ? (bf16 ? add_rmsnorm_kernel<true, 1, true> : add_rmsnorm_kernel<false, 1, true>)
                  : ahead     ? (bf16 ? add_rmsnorm_kernel<true, 4, true> : add_rmsnorm_kernel<false, 4, true>)
                              : (bf16 ? add_rmsnorm_kernel<true, 4, false> : add_rmsnorm_kernel<false, 4, false>);
   return launch_dependent(kernel, dim3(blocks), dim3(256), 0, st, p);

@@ -23,6 +23,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "decoder_rows_ring.h"
 #include "model_glue.cuh"
 
 namespace spsattn {
@@ -72,18 +73,28 @@ __device__ __forceinline__ void umma_ss_if(uint32_t d_tmem, uint32_t a_lo, uint3
       : "memory");
 }
 
+// A wait expired, of whichever warp of the block: no copy and no product stays in flight when its memory is given
+// up.  (A function of its own, and the loops over groups are not unrolled: the instructions of a launch come from
+// caches that do not have them yet.  12 layers of 768 columns, 16 rows, us per token: without this 328, with it on
+// every launch's way 342, so 338, with those loops short as well 314.)
+__device__ __noinline__ void rows_give_up(uint32_t full0, int asked, int stages, uint32_t products) {
+  int unused = 0;
+  rows_landed(asked, stages, [&](int st, int phase) { mbar_wait(full0 + 8 * st, phase, &unused, nullptr); });
+  mbar_wait(products, 0, &unused, nullptr);
+}
+
 template <int EPI>
 __global__ void __launch_bounds__(kRowsThreads, 1)
 rows_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                  const __grid_constant__ RowsGemmParams p) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t s_full[kRowsMaxStages], s_empty[kRowsMaxStages], s_done;
+  __shared__ __align__(8) uint64_t s_full[kRowsMaxStages], s_empty[kRowsMaxStages], s_done, s_quit;
   __shared__ uint32_t s_tmem;
-  __shared__ int s_abort;
+  __shared__ int s_abort, s_asked, s_stopped;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   grid_launch_dependents();
   const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t full0 = smem_u32(s_full), empty0 = smem_u32(s_empty), done = smem_u32(&s_done);
+  const uint32_t full0 = smem_u32(s_full), empty0 = smem_u32(s_empty), done = smem_u32(&s_done), quit = smem_u32(&s_quit);
   const int x_sub = p.bm * 128, x_bytes = p.groups * x_sub;       // 64 columns of the input rows; a stage of them
   const int w_sub = p.bn * 128;
   const int stage_bytes = x_bytes + p.groups * w_sub;
@@ -97,6 +108,7 @@ rows_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     mbar_arrive_expect_tx(full0 + 8 * st, (uint32_t)stage_bytes);
     if constexpr (EPI == kRowsSwiglu) {
       // gate rows and up rows of 64 columns lie under one another
+#pragma unroll 1
       for (int g = 0; g < p.groups; ++g) {
         tma_load_3d(dst + g * w_sub, &tm_w, full0 + 8 * st, 0, f0, j * p.groups + g);
         tma_load_3d(dst + g * w_sub + bf * 128, &tm_w, full0 + 8 * st, 0, p.F + f0, j * p.groups + g);
@@ -109,12 +121,14 @@ rows_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 
   if (warp == 4) {
     if (lane == 0) {
-      s_abort = 0;
+      s_abort = s_stopped = 0;
+      s_asked = chunks;
       for (int i = 0; i < p.stages; ++i) {
         mbar_init(full0 + 8 * i, 1);
         mbar_init(empty0 + 8 * i, 1);
       }
       mbar_init(done, 1);
+      mbar_init(quit, 1);
       fence_barrier_init();
       tma_prefetch_desc(&tm_w);
       tma_prefetch_desc(&tm_x);
@@ -148,18 +162,13 @@ rows_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   if (warp == 4) {
     // ------------------------------------------------------------------ loads
     if (elect_one()) {
-      int st = 0, phase = 0, asked = first;
-      for (; asked < chunks; ++asked) {
-        if (!mbar_wait(empty0 + 8 * st, phase, abort_flag, p.status)) break;
-        load_w(st, asked);
-        load_x(st, asked);
-        if (++st == p.stages) st = 0, phase ^= 1;
-      }
-      if (asked < chunks) {
-        // a step that was given up leaves no copy in flight: the last of each stage lands first
-        int unused = 0;
-        for (int j = max(asked - p.stages, 0); j < asked; ++j) mbar_wait(full0 + 8 * (j % p.stages), (j / p.stages) & 1, &unused, nullptr);
-      }
+      const int asked = rows_feed(
+          first, chunks, p.stages, [&](int st, int phase) { return mbar_wait(empty0 + 8 * st, phase, abort_flag, p.status); },
+          [&](int st, int j) {
+            load_w(st, j);
+            load_x(st, j);
+          });
+      if (asked < chunks) s_asked = asked;
     }
     __syncwarp();
   } else if (warp == 5) {
@@ -172,12 +181,13 @@ rows_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     // and with the whole warp around every stage (a vote, an election and a reconvergence each) a stage took
     // 300 clk more.
     if (elect_one()) {
-      int st = 0, phase = 0;
-      for (int j = 0; j < chunks; ++j) {
+      int st = 0, phase = 0, j = 0;
+      for (; j < chunks; ++j) {
         if (!mbar_wait(full0 + 8 * st, phase, abort_flag, p.status)) break;
         tc_fence_after();
         const uint32_t xa = x_lo + ((uint32_t)(st * stage_bytes) >> 4), wa = w_lo + ((uint32_t)(st * stage_bytes) >> 4);
         const int groups = min(p.groups, all_groups - j * p.groups);
+#pragma unroll 1
         for (int g = 0; g < groups; ++g) {
           const uint32_t x = xa + ((uint32_t)(g * x_sub) >> 4), w = wa + ((uint32_t)(g * w_sub) >> 4);
 #pragma unroll
@@ -186,6 +196,10 @@ rows_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         umma_commit(empty0 + 8 * st);
         if (j == chunks - 1) umma_commit(done);
         if (++st == p.stages) st = 0, phase ^= 1;
+      }
+      if (j < chunks) {
+        umma_commit(quit);
+        s_stopped = 1;
       }
     }
     __syncwarp();
@@ -295,6 +309,10 @@ rows_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     }
   }
   __syncthreads();
+  if (*abort_flag != 0) {
+    if (tid == 128) rows_give_up(full0, s_asked, p.stages, s_stopped ? quit : done);
+    __syncthreads();
+  }
   if (warp == 5) {
     tc_fence_after();
     tmem_dealloc<128>(tmem);

@@ -491,7 +491,8 @@ int spsattn_decoder_choose(const spsattn_decoder* d, const spsattn_token_source*
 int spsattn_decoder_step_supported(const spsattn_decoder* d);
 /* The layers of a step between its start and its head, for at most 64 rows of any batch (bf16, hidden and
  * intermediate multiples of 64, head_dim of 16, freqs_out, pointers at 16-byte boundaries): the residual
- * stream in x moves on through all layers, xn [rows, C] receives its final norm.
+ * stream in x moves on through all layers, xn [rows, C] receives its final norm.  Whatever stands before it on
+ * the stream is complete before anything is read that it may write.
  * spsattn_decoder_blocks_supported: 1 = yes. */
 int spsattn_decoder_blocks_supported(const spsattn_decoder* d);
 int spsattn_decoder_blocks(const spsattn_decoder* d, void* xn, int* device_status, void* stream);

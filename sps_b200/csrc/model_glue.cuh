@@ -19,9 +19,13 @@ struct RmsNormParams {
   long long rows;
   int C;
   float eps;
-  int let_go;          // inside a decode step: dependents may start at once (they wait themselves before they read
-                       // y), and nothing that may still run writes the weight
+  int let_go;          // when dependents may start (they wait themselves before they read y): NormLetGo
 };
+
+// At once only inside a decode step: what dependents touch before their own wait (weights, rows of a cache), and
+// this kernel's own weight, is then no longer being written by anything.  After the wait: where a step's launches begin
+// and what stands before them is not known, as in token_start_kernel.
+enum NormLetGo { kLetGoAtEnd = 0, kLetGoAtOnce = 1, kLetGoAfterWait = 2 };
 
 __device__ __forceinline__ float round_bf16(float f) {
   return __bfloat162float(__float2bfloat16_rn(f));
@@ -87,11 +91,10 @@ __global__ void __launch_bounds__(256, kStep ? 2 : kRowVecs == 1 ? 6 : kAhead ? 
 
   // Bound: HBM.  A block synchronises once per row (every thread adds the eight warp sums itself, in the
   // same order): 65536 rows of 2048 with delta 250 -> 174 us, 6.2 TB/s.
-  if (p.let_go) {
-    grid_launch_dependents();
-    if (kStep && tid < n_vec) wgt = __ldg(pw + tid);
-  }
-  grid_dependency_wait();
+  if (p.let_go != kLetGoAtOnce) grid_dependency_wait();
+  if (p.let_go != kLetGoAtEnd) grid_launch_dependents();
+  if (kStep && tid < n_vec) wgt = __ldg(pw + tid);
+  if (p.let_go == kLetGoAtOnce) grid_dependency_wait();
   uint4 nx[kRowVecs], nd[kRowVecs];
   auto fetch = [&](long long row) {
     if (!in_regs || row >= p.rows) return;

@@ -1260,7 +1260,7 @@ int spsattn_kv_update(void* nw_k, void* nw_v, int64_t* nw_len, int64_t* nw_pos, 
 // ------------------------------------------------------------------------ block glue (norm, gate)
 
 static int add_rmsnorm(void* x, const void* delta, const void* weight, void* y, int dtype, long long rows, int C, float eps,
-                       int let_go, void* stream) {
+                       NormLetGo let_go, void* stream) {
   if (!x || !weight || (!y && !delta)) return SPSATTN_ERR_ARG;
   if (rows <= 0 || C <= 0 || !(eps >= 0.f)) return SPSATTN_ERR_ARG;
   if (dtype != SPSATTN_DTYPE_BF16 && dtype != SPSATTN_DTYPE_FP32) return SPSATTN_ERR_ARG;
@@ -1285,7 +1285,7 @@ static int add_rmsnorm(void* x, const void* delta, const void* weight, void* y, 
   // that four blocks fit an SM.
   const int vecs = C / vec;
   const bool bf16 = dtype == SPSATTN_DTYPE_BF16, ahead = rows <= 2 * 148 || (!bf16 && vecs <= 1024);
-  auto* kernel = let_go && bf16 && vecs <= 256 ? add_rmsnorm_kernel<true, 1, true, true>
+  auto* kernel = let_go != kLetGoAtEnd && bf16 && vecs <= 256 ? add_rmsnorm_kernel<true, 1, true, true>
                  : vecs <= 256 ? (bf16 ? add_rmsnorm_kernel<true, 1, true> : add_rmsnorm_kernel<false, 1, true>)
                  : ahead     ? (bf16 ? add_rmsnorm_kernel<true, 4, true> : add_rmsnorm_kernel<false, 4, true>)
                              : (bf16 ? add_rmsnorm_kernel<true, 4, false> : add_rmsnorm_kernel<false, 4, false>);
@@ -1294,7 +1294,7 @@ static int add_rmsnorm(void* x, const void* delta, const void* weight, void* y, 
 
 int spsattn_add_rmsnorm(void* x, const void* delta, const void* weight, void* y, int dtype,
                         long long rows, int C, float eps, void* stream) {
-  return add_rmsnorm(x, delta, weight, y, dtype, rows, C, eps, 0, stream);
+  return add_rmsnorm(x, delta, weight, y, dtype, rows, C, eps, kLetGoAtEnd, stream);
 }
 
 int spsattn_swiglu(const void* gate_up, void* y, int dtype, long long rows, int I, void* stream) {
@@ -1527,14 +1527,15 @@ void step_extras(const spsattn_decoder* d, spsattn_extra (&extras)[2]) {
   }
 }
 
-// All layers of a step by the projections of decoder_rows.cuh: x moves on, ssq is that of the last row.  The normalised
+// All layers of a step by the projections of decoder_rows.cuh: x moves on, ssq is that of the last row.  first:
+// kLetGoAtOnce behind a launch that lets its dependents go after its own wait alone (token_start_kernel).  The normalised
 // rows go through y, which is free whenever a norm has run: the attention's output is read by c_proj alone.
-int launch_rows_layers(const spsattn_decoder* d, int* status, cudaStream_t st) {
+int launch_rows_layers(const spsattn_decoder* d, NormLetGo first, int* status, cudaStream_t st) {
   const int C = d->hidden, I = d->intermediate, rows = d->batch * d->slots;
   spsattn_extra extras[2];
   step_extras(d, extras);
-  auto norm = [&](const void* weight) {
-    return add_rmsnorm(d->x, nullptr, weight, d->y, SPSATTN_DTYPE_BF16, rows, C, d->norm_eps, 1, st);
+  auto norm = [&](const void* weight, NormLetGo let_go) {
+    return add_rmsnorm(d->x, nullptr, weight, d->y, SPSATTN_DTYPE_BF16, rows, C, d->norm_eps, let_go, st);
   };
   RowsGemmParams base;
   memset(&base, 0, sizeof(base));
@@ -1546,7 +1547,7 @@ int launch_rows_layers(const spsattn_decoder* d, int* status, cudaStream_t st) {
   int rc = 0;
   for (int layer = 0; layer < d->n_layer; ++layer) {
     const spsattn_decoder_layer& w = d->layers[layer];
-    if ((rc = norm(w.attn_norm)) != 0) return rc;
+    if ((rc = norm(w.attn_norm, layer == 0 ? first : kLetGoAtOnce)) != 0) return rc;
     RowsGemmParams p = base;
     p.K = C;
     p.F = 3 * C;
@@ -1570,7 +1571,7 @@ int launch_rows_layers(const spsattn_decoder* d, int* status, cudaStream_t st) {
     p.K = C;
     p.F = C;
     p.out = reinterpret_cast<uint16_t*>(d->x);
-    if ((rc = launch_rows_gemm<kRowsResidual>(p, w.c_proj, d->y, st)) != 0 || (rc = norm(w.mlp_norm)) != 0) return rc;
+    if ((rc = launch_rows_gemm<kRowsResidual>(p, w.c_proj, d->y, st)) != 0 || (rc = norm(w.mlp_norm, kLetGoAtOnce)) != 0) return rc;
     p = base;
     p.K = C;
     p.F = I;
@@ -1611,9 +1612,10 @@ int spsattn_decoder_blocks(const spsattn_decoder* d, void* xn, int* device_statu
   if (!spsattn_decoder_blocks_supported(d) || !xn) return SPSATTN_ERR_ARG;
   if (d->n_segments < 1 || d->n_segments > 2) return SPSATTN_ERR_ARG;
   if (!aligned16(xn)) return SPSATTN_ERR_ALIGN;
-  const int rc = launch_rows_layers(d, device_status, reinterpret_cast<cudaStream_t>(stream));
+  // (no launch of this call need stand before it)
+  const int rc = launch_rows_layers(d, kLetGoAfterWait, device_status, reinterpret_cast<cudaStream_t>(stream));
   if (rc != 0) return rc;
-  return add_rmsnorm(d->x, nullptr, d->out_norm, xn, SPSATTN_DTYPE_BF16, d->batch * d->slots, d->hidden, d->norm_eps, 0, stream);
+  return add_rmsnorm(d->x, nullptr, d->out_norm, xn, SPSATTN_DTYPE_BF16, d->batch * d->slots, d->hidden, d->norm_eps, kLetGoAtEnd, stream);
 }
 
 int spsattn_decoder_step(const spsattn_decoder* d, const spsattn_token_source* source, void* logits_out,
@@ -1641,7 +1643,7 @@ int spsattn_decoder_step(const spsattn_decoder* d, const spsattn_token_source* s
   base.x_stride = C;
   base.K = C;
   const bool by_rows = rows_preferred(d);
-  if (by_rows && (rc = launch_rows_layers(d, device_status, st)) != 0) return rc;
+  if (by_rows && (rc = launch_rows_layers(d, kLetGoAtOnce, device_status, st)) != 0) return rc;
   for (int layer = 0; layer < d->n_layer && !by_rows; ++layer) {
     const spsattn_decoder_layer& w = d->layers[layer];
     SkinnyParams p = base;

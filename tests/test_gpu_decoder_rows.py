@@ -54,3 +54,46 @@ def test_step_by_row_tiles_matches_the_separate_kernels(variant, batch, heads, h
         a, b = getattr(states[0], name).float(), getattr(states[1], name).float()
         # row by row: a row in a wrong place is as far off as its own norm
         assert bool(((a - b).norm(dim=-1) <= 2.0 ** -4 * b.norm(dim=-1)).all()), name
+
+
+def test_layers_directly_behind_a_launch_that_writes_their_caches():
+    """spsattn_decoder_blocks has no launch of its own before the first layer: what stands before it on the
+    stream may have let its dependents go and still be writing the cache rows that the layer's attention reads."""
+    import ctypes as C
+    import sps_b200
+    from sps_b200 import _lib
+    from sps_b200.attention import _status
+    from sps_b200.generation import random_state_dict
+    prompt, batch, hidden, heads, window = 120, 6, 512, 8, 16
+    dims = sps_b200.SPSDims(block_size=prompt + 8, vocab_size=500, n_layer=2, n_head=heads, hidden_size=hidden, intermediate_size=1024,
+                            eos_token_id=497, pad_token_id=499, predict_token_id=498, window_size=window)
+    engine = sps_b200.SPSGenerator(random_state_dict(dims, seed=3), dims, variant="reverse_sps")
+    ids = torch.randint(0, 497, (batch, prompt), generator=torch.Generator().manual_seed(2))
+    lib, status = engine.lib, _status(engine.device).data_ptr()
+    stream = torch.cuda.current_stream().cuda_stream
+    outs = []
+    for wait in (True, False, False, False):
+        state, _ = engine.prefill(ids, 8)                # rings full: a new row takes an old one's place, the length stays
+        engine._bind_step(state)
+        s = engine._step
+        token, active = torch.full((batch,), 7, device="cuda"), torch.ones(batch, dtype=torch.bool, device="cuda")
+        source = _lib.TokenSource()
+        source.token_in, source.active_in = token.data_ptr(), active.data_ptr()
+        _lib.check(lib.spsattn_decoder_start(C.byref(s.decoder), C.byref(source), status, stream), "start")
+        g = torch.Generator(device="cuda").manual_seed(4)
+        q = torch.randn(s.q.shape, generator=g, device="cuda").to(s.q.dtype)
+        for buf in (s.k2, s.v2):
+            buf.copy_(torch.randn(buf.shape, generator=g, device="cuda"))
+        torch.cuda.synchronize()
+        segs, n_seg, extras, append = s.layer_args[0]
+        out = torch.empty_like(q)
+        _lib.check(lib.spsattn_decode_step(q.data_ptr(), 2, out.data_ptr(), _lib.DTYPE_BF16, segs, n_seg, extras, 2, C.byref(append), batch,
+                                           heads, hidden // heads, _lib.DTYPE_BF16, 0.125, s.ws.data_ptr(), s.ws_bytes, status, stream), "step")
+        if wait:
+            torch.cuda.synchronize()
+        _lib.check(lib.spsattn_decoder_blocks(C.byref(s.decoder), s.xn.data_ptr(), status, stream), "blocks")
+        sps_b200.check_device_status()
+        outs.append([t.clone() for t in (out, s.xn, state.nw_k, state.nw_v, state.br_k, state.br_v, state.nw_pos, state.br_len)])
+    assert state.nw_len.unique().tolist() == [window] and state.br_len[0].unique().tolist() == [prompt + 2]
+    for other in outs[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(outs[0], other))

@@ -23,7 +23,7 @@ NATIVE_STAMP = os.path.join(PKG_DIR, "_native.stamp")     # what _native.so was 
 ABI_HEADER = os.path.join("..", "..", "include", "spsattn.h")
 SOURCES = ["spsattn_api.cu"]
 HEADERS = ["common.cuh", "mask.cuh", "prefill_sm100.cuh", "prefill_wide_sm100.cuh", "prefill_bwd_sm100.cuh", "prefill_aux.cuh", "decode.cuh", "decode_sm100.cuh",
-           "kv_update.cuh", "model_glue.cuh", "rope.cuh", "cache_fill.cuh", "decoder_step.cuh", "decoder_rows.cuh", "decoder_rows_ring.h", "prompt.cuh", "device_once.h", ABI_HEADER]
+           "kv_update.cuh", "model_glue.cuh", "rope.cuh", "cache_fill.cuh", "decoder_step.cuh", "decoder_rows.cuh", "decoder_rows_ring.h", "decoder_rows_plan.h", "prompt.cuh", "device_once.h", ABI_HEADER]
 NATIVE_SOURCES = ["native.cpp"]
 NATIVE_HEADERS = ["native_engine.h"]
 

@@ -17,6 +17,7 @@
 #include "decode.cuh"
 #include "decode_sm100.cuh"
 #include "decoder_rows.cuh"
+#include "decoder_rows_plan.h"
 #include "decoder_step.cuh"
 #include "device_once.h"
 #include "kv_update.cuh"
@@ -1380,19 +1381,10 @@ int encode_rows_map(CUtensorMap* tm, const void* ptr, long long rows, int K, int
 
 template <int EPI>
 int launch_rows_gemm(RowsGemmParams p, const void* w, const void* x, cudaStream_t st) {
-  const int sms = multiprocessors(), parts = EPI == kRowsSwiglu ? 2 : 1, step = 8 * parts;
-  const int w_rows = parts * p.F, most = EPI == kRowsSwiglu ? kRowsMaxN : kRowsHeldN;
-  // A block reads (bn + bm) rows of K columns.  The cheapest sizes by that and the number of waves; ties go
-  // to the wider input tile, which reads the weights once.
-  long long best = 0;
-  for (int bm = (p.rows + 15) / 16 * 16, tiles_r = 1; bm >= 16; tiles_r *= 2, bm = ((p.rows + tiles_r - 1) / tiles_r + 15) / 16 * 16) {
-    for (int bn = step; bn <= most; bn += step) {
-      const long long blocks = (long long)((w_rows + bn - 1) / bn) * tiles_r, waves = (blocks + sms - 1) / sms;
-      const long long cost = waves * (bn + bm + 16);
-      if (best == 0 || cost < best) best = cost, p.bn = bn, p.bm = bm;
-    }
-    if (tiles_r >= 4 || bm == 16) break;
-  }
+  const int parts = EPI == kRowsSwiglu ? 2 : 1, w_rows = parts * p.F;
+  const RowsTiles tiles = rows_tiles(w_rows, p.rows, multiprocessors(), 8 * parts, EPI == kRowsSwiglu ? kRowsMaxN : kRowsHeldN);
+  p.bn = tiles.bn;
+  p.bm = tiles.bm;
   // stages as wide as still gives three of them
   int stage = 0, chunks = 0;
   for (p.groups = 8;; p.groups /= 2) {

@@ -3,6 +3,8 @@
 import os
 import subprocess
 
+import pytest
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
@@ -48,3 +50,29 @@ int main() {
     kernel = open(os.path.join(ROOT, "sps_b200", "csrc", "decoder_rows.cuh")).read()
     teardown = kernel[kernel.rindex("if (*abort_flag != 0) {"):]
     assert teardown.index("rows_give_up(full0, s_asked, p.stages") < teardown.index("__syncthreads();") < teardown.index("tmem_dealloc")
+
+
+@pytest.mark.parametrize("weight_rows,step,most", [(64, 8, 64), (768, 8, 64), (2304, 8, 64), (4096, 16, 128), (2048, 8, 64), (22016, 16, 128)])
+def test_blocks_are_planned_as_they_are_launched(tmp_path, weight_rows, step, most):
+    """The plan counts the blocks of its own grid (33 to 48 rows in tiles of 16 are three tiles, not four), and no
+    other sizes of a block are cheaper by the rule that it states."""
+    lines = _run(tmp_path, r"""
+#include "decoder_rows_plan.h"
+#include <cstdio>
+int main() {
+  for (int rows = 1; rows <= 64; ++rows) {
+    const spsattn::RowsTiles t = spsattn::rows_tiles(%d, rows, 148, %d, %d);
+    std::printf("%%d %%d %%d %%lld\n", rows, t.bn, t.bm, t.blocks);
+  }
+}
+""" % (weight_rows, step, most))
+    for rows, bn, bm, blocks in lines:
+        def launched(n, m):
+            return -(-weight_rows // n) * -(-rows // m)
+
+        def cost(n, m):
+            return -(-launched(n, m) // 148) * (n + m + 16)
+
+        assert blocks == launched(bn, bm)
+        assert bn % step == 0 and bn <= most and bm % 16 == 0 and bm <= -(-rows // 16) * 16
+        assert cost(bn, bm) == min(cost(n, m) for n in range(step, most + 1, step) for m in (16, 32, 48, 64) if m < rows + 16)

@@ -22,4 +22,13 @@ inline RowsTiles rows_tiles(int weight_rows, int rows, int multiprocessors, int 
   return best;
 }
 
+// Whether a step of 1 to 16 rows that both could do goes by decoder_rows.cuh rather than decoder_step.cuh.  us per token,
+// decoder_step.cuh / decoder_rows.cuh, one row per sequence:
+//   8 rows:  12 layers of 512 columns 224 / 237, 768 268 / 288, 1024 307 / 312, 6 of 2048 308 / 293 (4 rows 287 / 291)
+//   9 rows:  4 layers of 64 to 256 columns (intermediate 192 to 2048) 77..82 / 78..87, 256 x 1024 84.2 / 83.4, 320 x 320 80.2 / 84.5,
+//            384 x 512 86.7 / 83.5, 512 x 1024 88.6 / 86.7, 2048 x 2048 163 / 139; 12 layers of 768 301 / 289
+//   16 rows: 192 x 512 80.2 / 83.3, 256 x 704 84.6 / 84.8, 320 x 320 84.6 / 83.8, 320 x 832 91.6 / 86.3, 512 x 1024 93.0 / 87.2
+// (a second tile of 8 rows is what costs decoder_step.cuh more than the separate norm costs the other)
+inline bool rows_faster(int rows, int hidden) { return rows > 8 && hidden >= 384; }
+
 }  // namespace spsattn

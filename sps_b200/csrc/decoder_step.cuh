@@ -32,8 +32,8 @@
 namespace spsattn {
 
 enum SkinnyEpilogue { kSkinnyQkv = 0, kSkinnyResidual = 1, kSkinnySwiglu = 2, kSkinnyLogits = 3 };
-// Taken up to 8 rows; from 9 on only where the projections of decoder_rows.cuh do not take the sizes
-// (rows_preferred has both sides measured), and for the head.
+// Taken up to 8 rows, of narrow steps up to 16, and where the projections of decoder_rows.cuh do not take the
+// sizes (rows_faster has both sides measured); for the head.
 constexpr int kSkinnyMaxRows = 16;
 constexpr int kSkinnyMaxCols = 2048;   // of a normalised input: one vector of 8 per thread of add_rmsnorm_kernel
 constexpr int kSkinnyMaxStages = 16;

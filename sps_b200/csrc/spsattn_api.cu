@@ -1481,10 +1481,10 @@ bool rows_sizes(const spsattn_decoder* d) {
          d->freqs_out != nullptr && aligned16(d->freqs_out);
 }
 
-// Which of the two, where both do.  us per token, decoder_step.cuh / decoder_rows.cuh: 768 columns, 12 layers 8 rows
-// 296 / 335, 10 rows 338 / 326, 16 rows 371 / 326; 512, 4 layers 98 / 111, 105 / 106, 110 / 104; 2048, 6 layers 328 / 344, 363 / 341,
-// 418 / 342 (library projections 384).
-bool rows_preferred(const spsattn_decoder* d) { return rows_sizes(d) && (d->batch * d->slots > 8 || !skinny_sizes(d)); }
+// which of the two
+bool rows_preferred(const spsattn_decoder* d) {
+  return rows_sizes(d) && (!skinny_sizes(d) || rows_faster(d->batch * d->slots, d->hidden));
+}
 
 // sizes that the fused step takes: its head is decoder_step.cuh's
 bool fused_step_sizes(const spsattn_decoder* d) {

@@ -76,3 +76,20 @@ int main() {
         assert blocks == launched(bn, bm)
         assert bn % step == 0 and bn <= most and bm % 16 == 0 and bm <= -(-rows // 16) * 16
         assert cost(bn, bm) == min(cost(n, m) for n in range(step, most + 1, step) for m in (16, 32, 48, 64) if m < rows + 16)
+
+
+def test_narrow_steps_keep_the_projections_that_are_faster(tmp_path):
+    """Up to 8 rows, and up to 16 below 384 columns, decoder_step.cuh is ahead (figures beside the rule)."""
+    lines = _run(tmp_path, r"""
+#include "decoder_rows_plan.h"
+#include <cstdio>
+#include <initializer_list>
+int main() {
+  for (int rows = 1; rows <= 16; ++rows)
+    for (int hidden : {64, 128, 192, 256, 320, 384, 512, 768, 2048}) std::printf("%d %d %d\n", rows, hidden, spsattn::rows_faster(rows, hidden));
+}
+""")
+    for rows, hidden, faster in lines:
+        assert faster == (rows > 8 and hidden > 320)
+    api = open(os.path.join(ROOT, "sps_b200", "csrc", "spsattn_api.cu")).read()
+    assert "rows_faster(d->batch * d->slots, d->hidden)" in api

@@ -8,8 +8,11 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("variant,batch,heads,hidden,inter,vocab,prompt,fused", [
-    ("standard", 9, 1, 64, 64, 33, 9, True),            # one group of 64 columns, fewer outputs than a block holds
-    ("reverse_sps", 5, 2, 128, 192, 200, 9, True),      # ten rows; three groups
+    ("standard", 9, 1, 64, 64, 33, 9, True),            # narrow, up to 16 rows: decoder_step.cuh, two tiles of rows
+    ("reverse_sps", 5, 2, 128, 192, 200, 9, True),
+    ("sps", 9, 1, 64, 64, 33, 9, True),                 # 18 rows; one group of 64 columns, fewer outputs than a block holds
+    ("reverse_sps", 9, 2, 128, 192, 200, 9, True),      # three groups
+    ("standard", 9, 6, 384, 192, 200, 9, True),         # the narrowest step of 9 rows that goes by row tiles
     ("sps", 16, 5, 320, 576, 1001, 30, True),           # 32 rows; five and nine groups: a last stage that is not full
     ("standard", 17, 3, 192, 320, 200, 9, False),       # 17 rows, library head
     ("delayed_state", 17, 8, 512, 1024, 500, 140, False),   # 34 rows: three tiles of 16; ring counters left to c_proj

@@ -118,6 +118,15 @@ def left_padded_position_ids(idx: Tensor, pad: int) -> Tensor:
     return torch.where(real, pos, torch.zeros_like(pos))
 
 
+def row_tiles_slower(rows: int, hidden: int, intermediate: int) -> bool:
+    """Whether a step's layers go by library projections although ``spsattn_decoder_blocks`` takes them.  us per token,
+    three layers, ``spsattn_decoder_blocks`` / library: 64 rows 3072 x 8192 280 / 282, 2560 x 10240 265 / 264, 3072 x 12288 340 / 337,
+    4096 x 11008 398 / 393 (52 rows 392 / 377), 4096 x 16384 471 / 463, two layers of 8192 x 28672 845 / 845 (49 rows 821 / 807);
+    48 rows 3072 x 12288 282 / 291, 4096 x 11008 369 / 385, 4096 x 16384 439 / 454; 32 rows of 8192 x 28672 725 / 737, 8 rows
+    654 / 660."""
+    return rows > 48 and hidden * intermediate > 3072 * 8192
+
+
 def suppressed_words(ids, vocab_size: int) -> Tensor:
     """int32 [(vocab_size + 31) // 32]: a bit per token id that is never chosen.  Ids below 0 count from the
     end of the vocabulary, as an index does (a model without a pad token has -1 for it)."""
@@ -388,7 +397,8 @@ class SPSGenerator:
         s.ws_bytes = ws_bytes
         s.decoder = self._bind_decoder(s)
         s.fused = bool(self.lib.spsattn_decoder_step_supported(C.byref(s.decoder)))
-        s.blocks = not s.fused and bool(self.lib.spsattn_decoder_blocks_supported(C.byref(s.decoder)))
+        s.blocks = (not s.fused and bool(self.lib.spsattn_decoder_blocks_supported(C.byref(s.decoder)))
+                    and not row_tiles_slower(ns * b, d.hidden_size, d.intermediate_size))
         self._step = s
 
     def _bind_decoder(self, s) -> _lib.Decoder:

@@ -93,3 +93,10 @@ int main() {
         assert faster == (rows > 8 and hidden > 320)
     api = open(os.path.join(ROOT, "sps_b200", "csrc", "spsattn_api.cu")).read()
     assert "rows_faster(d->batch * d->slots, d->hidden)" in api
+
+
+@pytest.mark.parametrize("rows,hidden,inter,slower", [(64, 4096, 11008, True), (49, 2560, 10240, True), (64, 8192, 28672, True),
+                                                      (48, 4096, 11008, False), (64, 3072, 8192, False), (64, 2048, 8192, False), (1, 8192, 28672, False)])
+def test_wide_steps_of_many_rows_keep_the_library_projections(rows, hidden, inter, slower):
+    from sps_b200.generation import row_tiles_slower
+    assert row_tiles_slower(rows, hidden, inter) is slower

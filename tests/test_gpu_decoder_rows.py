@@ -100,3 +100,14 @@ def test_layers_directly_behind_a_launch_that_writes_their_caches():
     assert state.nw_len.unique().tolist() == [window] and state.br_len[0].unique().tolist() == [prompt + 2]
     for other in outs[1:]:
         assert all(torch.equal(a, b) for a, b in zip(outs[0], other))
+
+
+@pytest.mark.parametrize("batch,blocks", [(24, True), (25, False)])
+def test_route_of_wide_steps(batch, blocks):
+    import sps_b200
+    from sps_b200.generation import random_state_dict
+    dims = sps_b200.SPSDims(block_size=16, vocab_size=500, n_layer=1, n_head=20, hidden_size=2560, intermediate_size=10240, eos_token_id=497,
+                            pad_token_id=499, predict_token_id=498, window_size=5)
+    engine = sps_b200.SPSGenerator(random_state_dict(dims, seed=3), dims, variant="sps")
+    engine._bind_step(engine.build_decode_state(batch, 8))
+    assert not engine._step.fused and engine._step.blocks is blocks

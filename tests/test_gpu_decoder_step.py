@@ -23,6 +23,8 @@ def _engine(variant, layers, heads, hidden, inter, vocab, seed=3, block=64, wind
     ("delayed_state", 8, 16, 1024, 2816, 2048),
     ("standard", 16, 16, 2048, 8192, 50304),  # the widest rows, several rounds of the head
     ("sps", 8, 16, 2048, 8192, 9473),
+    ("standard", 12, 125, 2000, 1040, 500),   # two row tiles of nearly the widest rows (no multiple of 64 columns), heads of 16
+    ("reverse_sps", 8, 62, 1984, 2064, 500),  # an intermediate size that is no multiple of 64, heads of 32
 ])
 def test_fused_step_matches_the_separate_kernels(variant, batch, heads, hidden, inter, vocab):
     import sps_b200

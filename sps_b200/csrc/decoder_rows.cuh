@@ -1,4 +1,4 @@
-// The projections of a decode step of 9 to 64 rows: Y[r, f] = sum_k X[r, k] W[f, k], bf16, fp32
+// The projections of a decode step of 9 to 64 rows (wide models: of 1 to 64): Y[r, f] = sum_k X[r, k] W[f, k], bf16, fp32
 // accumulation, each with what stands behind it in the block (rotary embedding and the split into
 // q, k, v; residual add; SwiGLU).
 //
@@ -14,8 +14,8 @@
 //     of weights before it waits for the kernel before it, the input rows follow after the wait;
 //   * tensor memory is allocated after that wait: a block that held some while the attention before it
 //     still had blocks without theirs would wait for them, and they for it.
-// us per token, captured, library projections with single kernels / now: 12 layers of 768 columns 18 rows 464 / 351, 32
-// rows 460 / 334; 12 x 1024, 32 rows 544 / 397; 6 x 2048, 24 rows 417 / 401, 64 rows 522 / 481.
+// us per token, captured, two rows per sequence, library projections with single kernels / now: 12 layers of 768 columns
+// 18 rows 449 / 320, 32 rows 463 / 322; 12 x 1024, 32 rows 505 / 357; 6 x 2048, 24 rows 385 / 322, 64 rows 469 / 422.
 // What is left at 2048 columns: 31 clk per 16 columns of a chain (2048 x 8192: 512 of them, 8 us), 300 clk per stage.
 // The contraction of one output is one chain of products in ascending k, never split, rounded to bf16 where
 // the separate kernels (library product, model_glue.cuh, rope.cuh) round theirs: the same bits as theirs at every

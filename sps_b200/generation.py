@@ -17,11 +17,12 @@ synchronisation, allocation or Python between tokens.  Reference behaviour being
   * Standard   src/modeling/models/full_attention_model.py:506-740 (one row per token, the cache holds
                the current document, one query per step)
 
-What runs where: a decode step of up to 16 rows in bf16 is a chain of kernels of libspsattn.so alone
-(``spsattn_decoder_step``: choice of the token, counters, embedding; projections fused with their norms, rotary
-embedding, gate and residual; segmented decode attention with the cache update; head).  In the prompt
-prefill and in larger steps, or fp32 ones, the projections and the head are library GEMMs, issued with the
-other kernels from native code (csrc/native_engine.h).  Parameters are bf16 (as the reference
+What runs where: a bf16 decode step of batches up to 16 and widths up to 2048 is a chain of kernels of libspsattn.so
+alone (``spsattn_decoder_step``: choice of the token, counters, embedding; projections fused with their norms, rotary
+embedding, gate and residual; segmented decode attention with the cache update; head).  For larger batches of up to 64
+rows and for wider models the layers are (``spsattn_decoder_blocks``), and the head is a library GEMM.  In the prompt
+prefill, in fp32 steps and in those that neither takes (or ``row_tiles_slower`` leaves), the projections and the head
+are library GEMMs, issued with the other kernels from native code (csrc/native_engine.h).  Parameters are bf16 (as the reference
 generates on CUDA) or fp32; the attention operands and caches are bf16 either way.
 """
 

@@ -1482,8 +1482,13 @@ bool rows_sizes(const spsattn_decoder* d) {
 }
 
 // which of the two
-bool rows_preferred(const spsattn_decoder* d) {
-  return rows_sizes(d) && (!skinny_sizes(d) || rows_faster(d->batch * d->slots, d->hidden));
+bool rows_preferred(const spsattn_decoder* d, cudaStream_t st) {
+  if (!rows_sizes(d) || !skinny_sizes(d)) return rows_sizes(d);
+  const auto faster = [d](bool captured) { return rows_faster(d->batch * d->slots, d->hidden, d->intermediate, captured); };
+  if (faster(true) == faster(false)) return faster(true);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  const bool known = launch_code(cudaStreamIsCapturing(st, &capture)) == 0;
+  return faster(known && capture == cudaStreamCaptureStatusActive);
 }
 
 // sizes that the fused step takes: its head is decoder_step.cuh's
@@ -1634,7 +1639,7 @@ int spsattn_decoder_step(const spsattn_decoder* d, const spsattn_token_source* s
   base.x = reinterpret_cast<const uint16_t*>(d->x);
   base.x_stride = C;
   base.K = C;
-  const bool by_rows = rows_preferred(d);
+  const bool by_rows = rows_preferred(d, st);
   if (by_rows && (rc = launch_rows_layers(d, kLetGoAtOnce, device_status, st)) != 0) return rc;
   for (int layer = 0; layer < d->n_layer && !by_rows; ++layer) {
     const spsattn_decoder_layer& w = d->layers[layer];

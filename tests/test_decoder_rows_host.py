@@ -78,21 +78,23 @@ int main() {
         assert cost(bn, bm) == min(cost(n, m) for n in range(step, most + 1, step) for m in (16, 32, 48, 64) if m < rows + 16)
 
 
-def test_narrow_steps_keep_the_projections_that_are_faster(tmp_path):
-    """Up to 8 rows, and up to 16 below 384 columns, decoder_step.cuh is ahead (figures beside the rule)."""
+def test_steps_of_few_rows_keep_the_projections_that_are_faster(tmp_path):
+    """Up to 8 rows, up to 16 below 384 columns, and where launches are not captured up to more rows the less a layer
+    weighs, decoder_step.cuh is ahead (figures beside the rule)."""
     lines = _run(tmp_path, r"""
 #include "decoder_rows_plan.h"
 #include <cstdio>
 #include <initializer_list>
 int main() {
-  for (int rows = 1; rows <= 16; ++rows)
-    for (int hidden : {64, 128, 192, 256, 320, 384, 512, 768, 2048}) std::printf("%d %d %d\n", rows, hidden, spsattn::rows_faster(rows, hidden));
+  for (int captured : {0, 1})
+    for (int rows = 1; rows <= 16; ++rows)
+      for (int hidden : {64, 256, 320, 384, 512, 768, 1024, 2048})
+        std::printf("%d %d %d %d\n", captured, rows, hidden, spsattn::rows_faster(rows, hidden, hidden * 8 / 3 / 64 * 64, captured));
 }
 """)
-    for rows, hidden, faster in lines:
-        assert faster == (rows > 8 and hidden > 320)
-    api = open(os.path.join(ROOT, "sps_b200", "csrc", "spsattn_api.cu")).read()
-    assert "rows_faster(d->batch * d->slots, d->hidden)" in api
+    first = {384: 17, 512: 17, 768: 13, 1024: 9, 2048: 9}
+    for captured, rows, hidden, faster in lines:
+        assert faster == (hidden >= 384 and rows >= (9 if captured else first[hidden]))
 
 
 @pytest.mark.parametrize("rows,hidden,inter,slower", [(64, 4096, 11008, True), (49, 2560, 10240, True), (64, 8192, 28672, True),

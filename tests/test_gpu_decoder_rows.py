@@ -68,7 +68,8 @@ def _step64(engine, state, token, active):
     ("reverse_sps", 5, 2, 128, 192, 200, 9, True),
     ("sps", 9, 1, 64, 64, 33, 9, True),                 # 18 rows; one group of 64 columns, fewer outputs than a block holds
     ("reverse_sps", 9, 2, 128, 192, 200, 9, True),      # three groups
-    ("standard", 9, 6, 384, 192, 200, 9, True),         # the narrowest step of 9 rows that goes by row tiles
+    ("standard", 9, 16, 1024, 2816, 200, 9, True),      # nine rows by row tiles
+    ("reverse_sps", 7, 12, 768, 2048, 200, 9, True),    # fourteen, of 768 columns
     ("sps", 16, 5, 320, 576, 1001, 30, True),           # 32 rows; five and nine groups: a last stage that is not full
     ("standard", 17, 3, 192, 320, 200, 9, False),       # 17 rows, library head
     ("delayed_state", 17, 8, 512, 1024, 500, 140, False),   # 34 rows: three tiles of 16; ring counters left to c_proj
@@ -116,7 +117,7 @@ def test_step_by_row_tiles_matches_the_separate_kernels(variant, batch, heads, h
 
 @pytest.mark.parametrize("variant,batch,heads,hidden,inter,prompt", [
     ("sps", 9, 8, 128, 320, 30),                # heads of 16, row tiles of 18 rows
-    ("reverse_sps", 5, 8, 512, 1024, 140),      # ten rows
+    ("reverse_sps", 5, 16, 1024, 2816, 140),    # ten rows
     ("standard", 17, 24, 768, 2048, 20),        # heads of 32, library head
     ("delayed_state", 20, 3, 192, 576, 12),     # 40 rows
     ("standard", 1, 10, 2560, 1024, 9),         # one row, heads of 256
@@ -147,6 +148,21 @@ def test_step_by_row_tiles_against_64_bits(variant, batch, heads, hidden, inter,
             for cache, rows in ((state.br_k, k), (state.br_v, v)):
                 for i in active.nonzero().flatten().tolist():
                     assert close(cache[layer, i, :, int(state.br_len[layer, i, 0]) - 1].cpu().double(), rows[i, engine.retained_slot])
+
+
+@pytest.mark.parametrize("variant,batch,heads,hidden,inter", [("standard", 9, 6, 384, 192), ("reverse_sps", 7, 8, 512, 1024)])
+def test_captured_steps_that_go_by_another_route(variant, batch, heads, hidden, inter):
+    """Few rows of a light layer: row tiles in a graph, decoder_step.cuh launch by launch; the same bits."""
+    engine = _engine(variant, 2, heads, hidden, inter, 500, 40)
+    ids = torch.randint(0, 497, (batch, 20), generator=torch.Generator().manual_seed(2))
+    outs = []
+    for graph in (True, False):
+        engine._session = None
+        tokens = engine.generate(ids, 12, stop_on_eos=False, use_graph=graph)
+        assert engine._step.fused
+        st = engine._session.state
+        outs.append([t.clone() for t in (tokens, engine._session.next_logits, st.br_k, st.br_v, st.br_len, st.nw_k, st.nw_v, st.nw_pos)])
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
 
 
 def test_layers_directly_behind_a_launch_that_writes_their_caches():
